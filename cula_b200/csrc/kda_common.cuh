@@ -89,7 +89,8 @@ __device__ __forceinline__ float2 unpack_f16(uint32_t x) {
     return __half22float2(*reinterpret_cast<__half2*>(&x));
 }
 __device__ __forceinline__ float2 unpack_bf16(uint32_t x) {
-    return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&x));
+    // a bf16 is the upper half of an fp32: one shift and one mask (the library conversion takes a permute more per element)
+    return make_float2(__uint_as_float(x << 16), __uint_as_float(x & 0xffff0000u));
 }
 
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {

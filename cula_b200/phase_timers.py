@@ -18,10 +18,10 @@ import torch
 from . import _native
 from .build import TIMERS_LIB, build
 
-FWD_PHASES = ["gate activation", "barrier (group totals)", "in-warp scan, tables", "operand generation, half 0",
-              "MMA wait, half 0 (+ L2 hints)", "operand generation, half 1", "MMA wait, half 1",
-              "Y staging + barrier", "triangular inverse", "Akk pack + W/U MMA issue", "W/U MMA wait", "W/U epilogue",
-              "loads issued under the MMA wait", "Gram epilogue", "L2 norms, beta", "top of the tile (q/k loads issued)"]
+FWD_PHASES = ["gate activation", "barrier (block edges, norms)", "in-warp cumulative sum", "per-channel tables", "-",
+              "operand generation", "wait for the Gram MMAs", "-", "triangular inverse, Y staging, Akk pack", "W/U MMA issue",
+              "W/U MMA wait", "W/U epilogue", "loads issued, diagonal blocks", "Gram epilogue", "L2 norms",
+              "top of the tile (q/k loads issued)"]
 DENSE_PHASES = ["half 0: operands widened into smem", "-",
                 "half 0: store read-out + wait for the states (TMA)", "half 0: MMA issue", "half 0: next operands requested",
                 "half 0: wait for the MMAs",

@@ -345,3 +345,24 @@ def test_forward_is_capturable_in_a_cuda_graph():
         torch.cuda.synchronize()
         assert torch.equal(o_static, o_ref) and torch.equal(ht_static, ht_ref)
     check_status()
+
+
+@pytest.mark.parametrize("gate,safe,l2,g_dtype", [(True, True, True, torch.bfloat16), (True, False, True, torch.float32),
+                                                  (False, False, False, torch.float32), (False, False, True, torch.bfloat16)])
+def test_chunk_parallel_stage_at_block_edges(gate, safe, l2, g_dtype):
+    """Last chunks that end on, before and after every 16-row block edge, for each gate element type and activation, with
+    and without the in-kernel normalisation (the operand shift of the fp16 Gram product is taken only with it)."""
+    lens = [1, 2, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65]
+    H, T = 3, sum(lens)
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32)
+    inp = make_inputs(1, T, H, seed=21, gate_offset=-5.0)
+    inp["A_log"] = inp["A_log"] + 0.3
+    if not gate:
+        inp["g"] = (F.logsigmoid(torch.randn(1, T, H, 128, generator=torch.Generator().manual_seed(3))) / 3.0).clamp(-5, 0)
+    inp["g"] = inp["g"].to(g_dtype)
+    if not l2:
+        inp["q"], inp["k"] = (F.normalize(inp[n].float(), dim=-1).to(torch.bfloat16) for n in ("q", "k"))
+    inp["initial_state"] = torch.randn(len(lens), H, 128, 128, generator=torch.Generator().manual_seed(1))
+    o, ht = run_chunk_kda(inp, cu_seqlens=cu, l2=l2, gate=gate, safe=safe)
+    o_ref, ht_ref = oracle_fwd(inp, cu_seqlens=cu, l2=l2, gate=gate, safe=safe)
+    assert_fwd_close(o, ht, o_ref, ht_ref, ht_tol=2e-3)
