@@ -1,14 +1,18 @@
-"""ctypes binding of libcula_kda.so (C ABI declared in include/cula_kda.h).
+"""Loading of the native parts: the ctypes binding of libcula_kda.so (C ABI declared in include/cula_kda.h) and the Python
+extension _host.so (argument checks, allocation, autograd and launches of the operators; csrc/host/).
 
 There is no fallback: if the library is missing or a call fails, an exception is raised.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "lib", "libcula_kda.so")
+HOST_PATH = os.path.join(_PKG, "lib", "_host.so")
 
 _vp, _ip, _fp, _i, _f = ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_float
 
@@ -63,6 +67,25 @@ def lib():
             fn.restype, fn.argtypes = res, args
         _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """Load the host extension once and bind it to the kernel library; raise if either has not been built."""
+    global _host
+    if _host is None:
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m cula_b200.build` (needs g++).")
+        import torch  # noqa: F401  (its shared libraries must be in the process)
+        loader = importlib.machinery.ExtensionFileLoader("_host", HOST_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_host", HOST_PATH, loader=loader))
+        loader.exec_module(module)
+        module.bind(LIB_PATH)
+        _host = module
+    return _host
 
 
 def check(code: int, what: str):

@@ -1,4 +1,5 @@
-"""Compile the CUDA sources into cula_b200/lib/libcula_kda.so for sm_100a with nvcc.
+"""Compile the CUDA sources into cula_b200/lib/libcula_kda.so for sm_100a with nvcc, and the native host path (argument
+checks, allocation, autograd, launches; C++ on libtorch) into the Python extension cula_b200/lib/_host.so with g++.
 
     python -m cula_b200.build [--force] [--verbose]
 
@@ -12,6 +13,7 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
@@ -32,6 +34,35 @@ def sources():
 def _deps_mtime():
     files = glob.glob(os.path.join(CSRC, "*")) + glob.glob(os.path.join(PKG, "..", "include", "*.h"))
     return max(os.path.getmtime(f) for f in files)
+
+
+HOST_SRC = os.path.join(CSRC, "host")
+HOST_LIB = os.path.join(LIB_DIR, "_host.so")
+
+
+def build_host(force=False):
+    """Build cula_b200/lib/_host.so. It reaches the kernels through the C ABI of libcula_kda.so, which it loads at run time."""
+    deps = glob.glob(os.path.join(HOST_SRC, "*")) + [os.path.join(PKG, "..", "include", "cula_kda.h")]
+    if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) >= max(os.path.getmtime(f) for f in deps):
+        return HOST_LIB
+    import torch
+    from torch.utils import cpp_extension
+    os.makedirs(OBJ_DIR, exist_ok=True)
+    os.makedirs(LIB_DIR, exist_ok=True)
+    cuda_home = os.path.dirname(os.path.dirname(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")))
+    includes = [*cpp_extension.include_paths(), os.path.join(cuda_home, "include"), sysconfig.get_paths()["include"]]
+    flags = ["-O2", "-std=c++17", "-fPIC", "-DTORCH_EXTENSION_NAME=_host", "-DTORCH_API_INCLUDE_EXTENSION_H",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{i}" for i in includes)]
+    procs = []
+    for src in sorted(glob.glob(os.path.join(HOST_SRC, "*.cpp"))):
+        obj = os.path.join(OBJ_DIR, os.path.basename(src)[:-4] + ".host.o")
+        procs.append((obj, subprocess.Popen([os.environ.get("CXX", "g++"), *flags, "-c", src, "-o", obj])))
+    if any(p.wait() != 0 for _, p in procs):
+        raise RuntimeError("g++ failed")
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    subprocess.run([os.environ.get("CXX", "g++"), "-shared", "-o", HOST_LIB, *(o for o, _ in procs), f"-L{torch_lib}", f"-L{cuda_home}/lib64",
+                    "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python", "-lcudart", "-ldl"], check=True)
+    return HOST_LIB
 
 
 TIMERS_LIB = os.path.join(LIB_DIR, "libcula_kda_timers.so")
@@ -69,3 +100,4 @@ def build(force=False, verbose=False, timers=False):
 
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv, timers="--timers" in sys.argv))
+    print(build_host(force="--force" in sys.argv))

@@ -1,0 +1,77 @@
+// Native host path: argument checks, output allocation, autograd and launches of the framework's operators, as a Python
+// extension on libtorch. The same calls in Python cost 30 us (decode) to 400 us (a training step of six to nine launches)
+// of interpreter time per call, several times what their kernels take at small sizes.
+#pragma once
+#include <dlfcn.h>
+#include <torch/extension.h>
+
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <optional>
+#include <string>
+
+#include "../../../include/cula_kda.h"
+
+namespace cula_host {
+
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+constexpr int64_t CHUNK = 64, DIM = 128;
+enum { GATE_NONE = 0, GATE_SOFTPLUS = 1, GATE_LOWER_BOUND = 2 };
+
+// entry points of libcula_kda.so, resolved once by bind()
+#define CULA_KDA_ENTRIES(X)                                                                                          \
+    X(cula_kda_tile_pack_bytes) X(cula_kda_fwd_intra) X(cula_kda_fwd_scan) X(cula_kda_cp_transition) X(cula_kda_cp_fold) \
+    X(cula_kda_decode) X(cula_kda_bwd_scratch_floats) X(cula_kda_bwd_grad_scale) X(cula_kda_bwd_scan)                  \
+    X(cula_kda_bwd_dense) X(cula_kda_bwd_gated) X(cula_kda_gate_fwd) X(cula_kda_gate_bwd)                              \
+    X(cula_kda_beta_sigmoid_fwd) X(cula_kda_beta_sigmoid_bwd) X(cula_kda_short_conv_fwd) X(cula_kda_short_conv_bwd)    \
+    X(cula_kda_rms_norm_gated_fwd) X(cula_kda_rms_norm_gated_bwd) X(cula_kda_strerror)
+struct Lib {
+#define CULA_KDA_MEMBER(name) decltype(&::name) name = nullptr;
+    CULA_KDA_ENTRIES(CULA_KDA_MEMBER)
+#undef CULA_KDA_MEMBER
+};
+extern Lib lib;
+
+inline void check(int code, const char* what) {
+    if (code != 0)
+        throw std::runtime_error(std::string(what) + " failed with code " + std::to_string(code) + ": " + lib.cula_kda_strerror(code));
+}
+// the exceptions the Python functions have always raised
+inline void require(bool ok, const char* message) {
+    if (!ok) {
+        PyErr_SetString(PyExc_AssertionError, message);
+        throw pybind11::error_already_set();
+    }
+}
+inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+inline void* ptr(const OptTensor& t) { return t.has_value() && t->defined() ? t->data_ptr() : nullptr; }
+inline float* fptr(const Tensor& t) { return static_cast<float*>(ptr(t)); }
+inline float* fptr(const OptTensor& t) { return static_cast<float*>(ptr(t)); }
+inline int* iptr(const OptTensor& t) { return static_cast<int*>(ptr(t)); }
+inline bool is_f32(const Tensor& t) { return t.scalar_type() == at::kFloat; }
+inline bool is_bf16(const Tensor& t) { return t.scalar_type() == at::kBFloat16; }
+inline Tensor contiguous_f32(const Tensor& t) { return (is_f32(t) ? t : t.to(at::kFloat)).contiguous(); }
+inline OptTensor contiguous_f32(const OptTensor& t) { return t.has_value() && t->defined() ? OptTensor(contiguous_f32(*t)) : OptTensor(); }
+inline cudaStream_t stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+// B200 guard (cached per device), and the status word of a device: one int in pinned host memory that the kernels write
+// directly in the (rare) case that they have something to report, so that reading it costs neither a copy nor a wait
+void assert_blackwell(const Tensor& t);
+int* status_word(int device_index);
+// status reported by kernels that have already finished: raises like check_status()
+void poll_status(int device_index);
+
+// the index tables of a packed batch (utils.VarlenTables)
+struct Tables {
+    Tensor cu_seqlens, chunk_indices, chunk_offsets, seq_order;
+    int64_t n_seqs = 0, num_chunks = 0, total_tokens = 0;
+};
+
+void bind_attention(pybind11::module_& m);
+void bind_layer_ops(pybind11::module_& m);
+
+}  // namespace cula_host

@@ -164,7 +164,7 @@ kda_bwd_dense_kernel(const BwdDenseParams p, const int num_tiles, const __grid_c
     auto cta_wait = [&](int which, uint32_t parity) -> bool {
         if (tid == 0) {
             if (!*sAbort && !mbar_wait(&bars[which], parity)) {
-                atomicExch(p.status, STATUS_WAIT_TIMEOUT);
+                report_status(p.status, STATUS_WAIT_TIMEOUT);
                 *sAbort = 1;
             }
             umma::fence_before_sync();
@@ -255,7 +255,7 @@ kda_bwd_dense_kernel(const BwdDenseParams p, const int num_tiles, const __grid_c
                     issued1 = true;
                 }
                 if (!mbar_wait(&bars[vh], par)) {
-                    atomicExch(p.status, STATUS_WAIT_TIMEOUT);
+                    report_status(p.status, STATUS_WAIT_TIMEOUT);
                     *sAbort = 1;
                 } else {
                     BD_MARK(2 + 6 * vh);      // wait for the states of this half
@@ -284,7 +284,7 @@ kda_bwd_dense_kernel(const BwdDenseParams p, const int num_tiles, const __grid_c
             } else if (warp != 0) {
                 // ---- dD partial of this half from the fp32 states in shared memory, under the MMAs ----
                 if (!mbar_wait(&bars[vh], par)) {
-                    atomicExch(p.status, STATUS_WAIT_TIMEOUT);
+                    report_status(p.status, STATUS_WAIT_TIMEOUT);
                     *sAbort = 1;
                 }
 #pragma unroll
@@ -518,11 +518,10 @@ bool make_scratch_map(CUtensorMap* map, float* scratch, int first_float, int col
 extern "C" int kda_launch_bwd_dense(const kda::BwdDenseParams* p, int num_chunks, cudaStream_t stream) {
     using namespace kda;
     if (num_chunks <= 0) return 0;
-    cudaError_t e = cudaFuncSetAttribute(kda_bwd_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BD_SMEM);
+    static std::atomic<unsigned long long> done;
+    cudaError_t e = allow_smem(kda_bwd_dense_kernel, BD_SMEM, done);
     if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     const int tiles = num_chunks * p->H;
     static_assert(SCR_DW == SCR_DQG + 64 * 128 && SCR_DKG == SCR_DW + 64 * 128 && SCR_DAU == SCR_DPS + 64 * 64,
                   "the tensor maps below address dQg | dW | dKg and dPs | dAu as stacked matrices");

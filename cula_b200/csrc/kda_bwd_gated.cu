@@ -813,11 +813,10 @@ extern "C" int kda_launch_bwd_gated(const kda::BwdGatedParams* p, int num_chunks
     using namespace kda;
     static_assert(BG_SMEM <= 227 * 1024, "shared memory budget");
     if (num_chunks <= 0) return 0;
-    cudaError_t e = cudaFuncSetAttribute(kda_bwd_gated_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BG_SMEM);
+    static std::atomic<unsigned long long> done;
+    cudaError_t e = allow_smem(kda_bwd_gated_kernel, BG_SMEM, done);
     if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     const int tiles = num_chunks * p->H;
     kda_bwd_gated_kernel<<<tiles < sms ? tiles : sms, BG_THREADS, BG_SMEM, stream>>>(*p, tiles);
     return (int)cudaGetLastError();

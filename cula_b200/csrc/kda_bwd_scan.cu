@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
             if (lane == 0 && use > 0) ok = mbar_wait(&empty[s], (use - 1) & 1);
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (!ok) {
-                if (lane == 0) atomicExch(p.status, STATUS_WAIT_TIMEOUT);
+                if (lane == 0) report_status(p.status, STATUS_WAIT_TIMEOUT);
                 break;
             }
             unsigned char* dst = smem + s * BS_STAGE_BYTES;
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
         const int c = nchunks - 1 - it;
         const int s = it % BS_STAGES;
         if (!mbar_wait(&full[s], (it / BS_STAGES) & 1)) {
-            atomicExch(p.status, STATUS_WAIT_TIMEOUT);
+            report_status(p.status, STATUS_WAIT_TIMEOUT);
             return;
         }
         const uint32_t st = smem_u32(smem + s * BS_STAGE_BYTES);
@@ -320,7 +320,8 @@ extern "C" int kda_launch_bwd_scan(const kda::BwdScanParams* p, cudaStream_t str
     using namespace kda;
     if (p->N <= 0) return 0;
     dim3 grid(2, p->H, p->N);
-    cudaError_t e = cudaFuncSetAttribute(kda_bwd_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BS_SMEM);
+    static std::atomic<unsigned long long> done;
+    cudaError_t e = allow_smem(kda_bwd_scan_kernel, BS_SMEM, done);
     if (e != cudaSuccess) return (int)e;
     kda_bwd_scan_kernel<<<grid, BS_THREADS, BS_SMEM, stream>>>(*p);
     return (int)cudaGetLastError();

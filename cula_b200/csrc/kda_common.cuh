@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace kda {
 
 constexpr int BT = 64;    // chunk length (tokens); fixed at 64 as in cula/kda/chunk.py:54
@@ -49,6 +51,9 @@ constexpr int STATUS_OK = 0;
 constexpr int STATUS_WAIT_TIMEOUT = 1;
 constexpr int STATUS_BAD_INDEX = 2;        // a state-pool index past the end of the pool (decode)
 constexpr int STATUS_RANGE = 3;            // a forward intermediate left the fp16 range (or is not finite)
+
+// A plain store: the word may live in device memory or in pinned host memory (where the host polls it without a copy).
+__device__ __forceinline__ void report_status(int* status, int code) { *reinterpret_cast<volatile int*>(status) = code; }
 
 // ---------------------------------------------------------------------------------------------
 // PTX wrappers
@@ -200,6 +205,42 @@ __device__ __forceinline__ ChunkInfo chunk_info(int c, const int* cu_seqlens, co
         ci.valid = min(BT, T - lc * BT);
     }
     return ci;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Launch-side helpers: attributes that never change are asked for once per device, not on every launch
+// ---------------------------------------------------------------------------------------------
+constexpr int MAX_DEVICES = 64;
+inline int current_device() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return dev;
+}
+inline int sm_count() {
+    static std::atomic<int> counts[MAX_DEVICES];
+    const int dev = current_device();
+    if (dev < 0 || dev >= MAX_DEVICES) {
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        return sms;
+    }
+    int sms = counts[dev].load(std::memory_order_relaxed);
+    if (sms == 0) {
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        counts[dev].store(sms, std::memory_order_relaxed);
+    }
+    return sms;
+}
+// raise the dynamic shared memory limit of one kernel (a function-local static `done` per kernel holds the devices it was
+// raised on)
+template <typename Kernel>
+inline cudaError_t allow_smem(Kernel kernel, int bytes, std::atomic<unsigned long long>& done) {
+    const int dev = current_device();
+    const unsigned long long bit = dev >= 0 && dev < MAX_DEVICES ? 1ull << dev : 0;
+    if (bit && (done.load(std::memory_order_relaxed) & bit)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+    return e;
 }
 
 }  // namespace kda

@@ -101,7 +101,8 @@ __global__ void __launch_bounds__(FOLD_THREADS, 1) kda_cp_fold_kernel(const floa
 extern "C" int kda_launch_cp_fold(const float* c_all, const float* m_all, const float* h0, float* s_out, int n, int H,
                                   long long stride_floats, cudaStream_t stream) {
     using namespace kda;
-    cudaError_t e = cudaFuncSetAttribute(kda_cp_fold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FOLD_SMEM);
+    static std::atomic<unsigned long long> done;
+    cudaError_t e = allow_smem(kda_cp_fold_kernel, FOLD_SMEM, done);
     if (e != cudaSuccess) return (int)e;
     dim3 grid(H, DV / FOLD_COLS);
     kda_cp_fold_kernel<<<grid, FOLD_THREADS, FOLD_SMEM, stream>>>(c_all, m_all, h0, s_out, n, H, (size_t)stride_floats);

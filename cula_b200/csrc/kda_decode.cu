@@ -99,7 +99,7 @@ __device__ __forceinline__ void dec_item(const DecodeParams& p, const int item, 
         return;
     }
     if (slot >= p.pool) {                                   // caller error: report, touch nothing
-        if (tid == 0) atomicExch(p.status, STATUS_BAD_INDEX);
+        if (tid == 0) report_status(p.status, STATUS_BAD_INDEX);
         return;
     }
     float* S = p.state + ((size_t)slot * p.HV + hv) * (size_t)DK * p.V;
@@ -249,9 +249,7 @@ extern "C" int kda_launch_decode(const void* q, const void* k, const void* v, co
     p.state_kv = state_kv; p.scale = scale; p.softplus_beta = softplus_beta; p.softplus_threshold = softplus_threshold;
     p.status = status;
     // enough CTAs to fill the machine several times over, else as few (= as much work per CTA) as possible
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     int slices = 1;
     while (slices < V / 32 && (long long)N * HV * slices < 8LL * sms && (V / 32) % (2 * slices) == 0) slices *= 2;
     p.slices = slices;

@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
     auto wait_mma = [&](int which, uint32_t parity) -> bool {
         if (tid == MMA_THREAD) {
             if (!mbar_wait(&bars[which], parity)) {
-                atomicExch(p.status, STATUS_WAIT_TIMEOUT);
+                report_status(p.status, STATUS_WAIT_TIMEOUT);
                 *sAbort = 1;
             }
             umma::fence_before_sync();
@@ -971,7 +971,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
         // w and u inherit the range of v and of (I + L)^-1: fp16 has no room beyond 65504, so say so instead of
         // handing inf to the scan
         const bool out_of_range = f16x2_not_finite(*reinterpret_cast<const uint32_t*>(&big));
-        if (__any_sync(0xffffffffu, out_of_range) && lane == 0) atomicMax(p.status, STATUS_RANGE);
+        if (__any_sync(0xffffffffu, out_of_range) && lane == 0) report_status(p.status, STATUS_RANGE);
     }
     fence_proxy_async();
     umma::fence_before_sync();
@@ -1009,12 +1009,12 @@ extern "C" int kda_launch_fwd_intra(const kda::IntraParams* p, int num_chunks, c
     using namespace kda;
     if (num_chunks <= 0) return 0;
     const int smem = SM_TOTAL + 1024;
-    auto kernel = p->g_per_head ? kda_fwd_intra_kernel<GK_PER_HEAD> : p->g_fp32 ? kda_fwd_intra_kernel<GK_FP32> : kda_fwd_intra_kernel<GK_BF16>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const int kind = p->g_per_head ? GK_PER_HEAD : p->g_fp32 ? GK_FP32 : GK_BF16;
+    auto kernel = kind == GK_PER_HEAD ? kda_fwd_intra_kernel<GK_PER_HEAD> : kind == GK_FP32 ? kda_fwd_intra_kernel<GK_FP32> : kda_fwd_intra_kernel<GK_BF16>;
+    static std::atomic<unsigned long long> done[3];
+    cudaError_t e = allow_smem(kernel, smem, done[kind]);
     if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     IntraParams q = *p;
     q.num_tiles = num_chunks * p->H;
     const int grid = q.num_tiles < 2 * sms ? q.num_tiles : 2 * sms;     // two resident CTAs per SM

@@ -148,7 +148,7 @@ kda_fwd_scan_kernel(const ScanParams p) {
                 }
                 ok = __shfl_sync(0xffffffffu, ok, 0);
                 if (!ok) {
-                    if (lane == 0) atomicExch(p.status, STATUS_WAIT_TIMEOUT);
+                    if (lane == 0) report_status(p.status, STATUS_WAIT_TIMEOUT);
                     break;
                 }
                 issued = c + 1;
@@ -165,7 +165,7 @@ kda_fwd_scan_kernel(const ScanParams p) {
             // the consumers may have left early: do not exit with bulk copies to this CTA's shared memory in flight
             if (is_m && lane == 0) {
                 for (int cc = max(0, issued - L::STAGES); cc < issued; ++cc)
-                    if (!mbar_wait(&full[cc % L::STAGES], (cc / L::STAGES) & 1)) atomicExch(p.status, STATUS_WAIT_TIMEOUT);
+                    if (!mbar_wait(&full[cc % L::STAGES], (cc / L::STAGES) & 1)) report_status(p.status, STATUS_WAIT_TIMEOUT);
             }
             return;
         }
@@ -173,7 +173,7 @@ kda_fwd_scan_kernel(const ScanParams p) {
             for (int c = 0; c < nchunks; ++c) {
                 const int s = c % L::STAGES, use = c / L::STAGES;
                 if (use > 0 && !mbar_wait(&empty[s], (use - 1) & 1)) {
-                    atomicExch(p.status, STATUS_WAIT_TIMEOUT);
+                    report_status(p.status, STATUS_WAIT_TIMEOUT);
                     break;
                 }
                 const unsigned char* tile = p.tiles + ((size_t)(chunk0 + c) * p.H + h) * TP_BYTES;
@@ -235,7 +235,7 @@ kda_fwd_scan_kernel(const ScanParams p) {
             const int r = mbar_wait_or_quorum(&full[s], (c / L::STAGES) & 1, zero_votes, L::CONSUMERS);
             if (r == 2) break;
             if (r == 1) {
-                atomicExch(p.status, STATUS_WAIT_TIMEOUT);
+                report_status(p.status, STATUS_WAIT_TIMEOUT);
                 return;
             }
             if (voted) {         // nothing to compute: keep the pipeline protocol going for the warps that still work
@@ -243,7 +243,7 @@ kda_fwd_scan_kernel(const ScanParams p) {
                 continue;
             }
         } else if (!mbar_wait(&full[s], (c / L::STAGES) & 1)) {
-            atomicExch(p.status, STATUS_WAIT_TIMEOUT);
+            report_status(p.status, STATUS_WAIT_TIMEOUT);
             return;
         }
         const uint32_t st = smem_u32(smem + s * L::STAGE_BYTES);
@@ -489,29 +489,31 @@ extern "C" int kda_launch_fwd_scan(const kda::ScanParams* p, cudaStream_t stream
     if (p->N <= 0) return 0;
     dim3 grid(2, p->H, p->N);
     cudaError_t e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     const bool both_halves = 2LL * p->H * p->N > sms;      // more half-state CTAs than SMs: eight consumer warps per CTA
     using L2 = ScanLayout<false, 2>;
     if (p->vnew_out) {
         if (both_halves) {
-            e = cudaFuncSetAttribute(kda_fwd_scan_kernel<true, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, L2::SMEM);
+            static std::atomic<unsigned long long> done;
+            e = allow_smem(kda_fwd_scan_kernel<true, false, 2>, L2::SMEM, done);
             if (e != cudaSuccess) return (int)e;
             kda_fwd_scan_kernel<true, false, 2><<<dim3(1, p->H, p->N), (L2::CONSUMERS + 1) * 32, L2::SMEM, stream>>>(*p);
         } else {
-            e = cudaFuncSetAttribute(kda_fwd_scan_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM);
+            static std::atomic<unsigned long long> done2;
+            e = allow_smem(kda_fwd_scan_kernel<true, false>, SCAN_SMEM, done2);
             if (e != cudaSuccess) return (int)e;
             kda_fwd_scan_kernel<true, false><<<grid, SCAN_THREADS, SCAN_SMEM, stream>>>(*p);
         }
     } else {
         if (both_halves) {
-            e = cudaFuncSetAttribute(kda_fwd_scan_kernel<false, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, L2::SMEM);
+            static std::atomic<unsigned long long> done3;
+            e = allow_smem(kda_fwd_scan_kernel<false, false, 2>, L2::SMEM, done3);
             if (e != cudaSuccess) return (int)e;
             e = launch_after_producer(kda_fwd_scan_kernel<false, false, 2>, dim3(1, p->H, p->N), (L2::CONSUMERS + 1) * 32, L2::SMEM, stream, *p);
             if (e != cudaSuccess) return (int)e;
         } else {
-            e = cudaFuncSetAttribute(kda_fwd_scan_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM);
+            static std::atomic<unsigned long long> done4;
+            e = allow_smem(kda_fwd_scan_kernel<false, false>, SCAN_SMEM, done4);
             if (e != cudaSuccess) return (int)e;
             e = launch_after_producer(kda_fwd_scan_kernel<false, false>, grid, SCAN_THREADS, SCAN_SMEM, stream, *p);
             if (e != cudaSuccess) return (int)e;
@@ -524,14 +526,13 @@ extern "C" int kda_launch_fwd_scan(const kda::ScanParams* p, cudaStream_t stream
 extern "C" int kda_launch_fwd_transition(const kda::ScanParams* p, cudaStream_t stream) {
     using namespace kda;
     if (p->N <= 0) return 0;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     ScanParams q = *p;
     q.group_major = 4LL * p->H * p->N > sms;     // see the index mapping at the top of the kernel
     const dim3 grid = q.group_major ? dim3(p->H, p->N, 4) : dim3(4, p->H, p->N);
     constexpr int smem = ScanLayout<true, 1>::SMEM;
-    cudaError_t e = cudaFuncSetAttribute(kda_fwd_scan_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static std::atomic<unsigned long long> done5;
+    cudaError_t e = allow_smem(kda_fwd_scan_kernel<false, true>, smem, done5);
     if (e != cudaSuccess) return (int)e;
     kda_fwd_scan_kernel<false, true><<<grid, SCAN_THREADS, smem, stream>>>(q);
     return (int)cudaGetLastError();

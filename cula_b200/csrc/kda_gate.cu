@@ -143,9 +143,7 @@ __global__ void __launch_bounds__(GATE_THREADS) kda_beta_sigmoid_kernel(const vo
 extern "C" int kda_launch_gate(const kda::GateArgs* a, int backward, cudaStream_t stream) {
     using namespace kda;
     if (a->M <= 0) return 0;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     const int groups = a->H * a->K / 8;
     const int gx = (groups + GATE_THREADS - 1) / GATE_THREADS;
     // about eight CTAs per SM in flight; the backward pass ends in one atomic per thread and channel, so it runs a
@@ -163,9 +161,7 @@ extern "C" int kda_launch_beta_sigmoid(const void* x, int x_fp32, const float* d
                                        cudaStream_t stream) {
     using namespace kda;
     if (n <= 0) return 0;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     long long blocks = (n + GATE_THREADS - 1) / GATE_THREADS;
     if (blocks > 8LL * sms) blocks = 8LL * sms;
     if (backward) kda_beta_sigmoid_kernel<true><<<(unsigned)blocks, GATE_THREADS, 0, stream>>>(x, x_fp32, dy, out, n);

@@ -361,9 +361,7 @@ extern "C" int kda_launch_short_conv(const kda::ConvArgs* a, int num_chunks, int
 extern "C" int kda_launch_rms_norm_gated(const kda::NormArgs* a, int backward, cudaStream_t stream) {
     using namespace kda;
     if (a->R <= 0) return 0;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     long long blocks = (a->R + LO_THREADS / 32 - 1) / (LO_THREADS / 32);
     const long long cap = (backward ? 4LL : 16LL) * sms;     // backward: fewer, longer-lived CTAs keep the dw atomics few
     if (blocks > cap) blocks = cap;

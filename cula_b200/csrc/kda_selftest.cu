@@ -12,7 +12,7 @@ __global__ void kda_selftest_wait_kernel(int* status, int limit) {
         fence_mbar_init();
     }
     __syncthreads();
-    if (threadIdx.x == 0 && !mbar_wait(&bar, 0, limit)) atomicExch(status, STATUS_WAIT_TIMEOUT);
+    if (threadIdx.x == 0 && !mbar_wait(&bar, 0, limit)) report_status(status, STATUS_WAIT_TIMEOUT);
 }
 
 }  // namespace kda

@@ -15,8 +15,9 @@ from __future__ import annotations
 
 import torch
 
-from ..kda.chunk import ChunkKDAFunction, _poll_status
-from ..utils import assert_blackwell
+from .. import _native
+from ..kda.chunk import _segments
+from ..utils import get_varlen_tables
 
 
 @torch.compiler.disable
@@ -48,13 +49,6 @@ def chunk_gated_delta_rule(q, k, v, g, beta, scale=None, initial_state=None, out
             raise ValueError(
                 f"The number of initial states is expected to be equal to the number of input sequences, "
                 f"i.e., {len(cu_seqlens) - 1} rather than {initial_state.shape[0]}.")
-    assert q.dtype == k.dtype == v.dtype == torch.bfloat16, "q, k, v must be in bfloat16."
-    assert q.shape == k.shape and q.shape[-1] == v.shape[-1] == 128, "only head dim 128 is supported for keys and values"
-    assert v.shape[:3] == q.shape[:3], "grouped value heads (HV > H) are not supported"
-    assert g.shape == q.shape[:3] and beta.shape == q.shape[:3], "g and beta must be of shape (batch size, seq len, heads)"
-    assert g.dtype in (torch.float32, torch.bfloat16) and beta.dtype in (torch.float32, torch.bfloat16)
-    if initial_state is not None:
-        assert initial_state.dtype == torch.float32, "initial_state must be in float32."
     A_log = dt_bias_h = dt_bias = None
     H = q.shape[2]
     if use_gate_in_kernel:
@@ -62,13 +56,12 @@ def chunk_gated_delta_rule(q, k, v, g, beta, scale=None, initial_state=None, out
         A_log, dt_bias_h = kwargs["A_log"], kwargs.get("dt_bias")
         if dt_bias_h is not None:      # one bias per head: the kernels take one per (head, channel)
             dt_bias = dt_bias_h.float().reshape(H, 1).expand(H, 128).reshape(H * 128)
-    assert_blackwell(q.device)
-    _poll_status(q.device)
-    if scale is None:
-        scale = k.shape[-1] ** -0.5
-    keep = bool(disable_recompute) and torch.is_grad_enabled() and any(
-        t is not None and t.requires_grad for t in (q, k, v, g, beta, A_log, dt_bias_h, initial_state))
-    # a 3-D g tells the shared autograd function (and the kernels) that the gate is per (token, head)
-    return ChunkKDAFunction.apply(q, k, v, g, beta, A_log, dt_bias, scale, initial_state, output_final_state,
-                                  use_qk_l2norm_in_kernel, use_gate_in_kernel, cu_seqlens, cu_seqlens_cpu, False, None,
-                                  disable_recompute, False, keep)
+    tables = segments = None
+    if cu_seqlens is None:
+        segments = _segments(q)
+    else:
+        tables = get_varlen_tables(cu_seqlens, cu_seqlens_cpu).native
+    # the checks, and the rest, are in the host extension; a 3-D g tells the kernels that the gate is per (token, head)
+    return _native.host().attend(q, k, v, g, beta, scale, initial_state, output_final_state, use_qk_l2norm_in_kernel,
+                                 use_gate_in_kernel, A_log, dt_bias, tables, False, None, disable_recompute, False, False,
+                                 True, segments)

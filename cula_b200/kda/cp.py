@@ -28,10 +28,27 @@ import torch.distributed as dist
 
 from .. import _native
 from ..utils import CHUNK, VarlenTables, assert_blackwell
-from .chunk import _gate_mode, _ptr, _status_word
+from .chunk import _gate_mode, _ptr, _status_ptr
 
 
 _SEGMENT_TABLES: dict = {}      # (segment bounds, device) -> VarlenTables of the segments of a shard
+
+
+def segment_bounds(T, num_chunks, P):
+    """Segment boundaries on chunk boundaries, in tokens: [0, ..., T]."""
+    return [min(T, ((num_chunks * i) // P) * CHUNK) for i in range(P)] + [T]
+
+
+def segment_tables(bounds, dev):
+    """Index tables of the segments of one sequence, built once per set of boundaries."""
+    key = (tuple(bounds), str(dev))
+    tables = _SEGMENT_TABLES.get(key)
+    if tables is None:
+        if len(_SEGMENT_TABLES) > 16:
+            _SEGMENT_TABLES.clear()
+        cpu = torch.tensor(bounds, dtype=torch.int32)
+        tables = _SEGMENT_TABLES[key] = VarlenTables(cpu.to(dev), cpu)
+    return tables
 
 
 class KDACPContext:
@@ -49,7 +66,7 @@ class CudaBackend:
     """Compute steps of one rank on its GPU through the C ABI."""
 
     def __init__(self, q, k, v, g, beta, scale, use_qk_l2norm_in_kernel, use_gate_in_kernel, safe_gate, lower_bound,
-                 A_log, dt_bias, segments=None, marks=None, tiles=None):
+                 A_log, dt_bias, segments=None, marks=None):
         assert q.shape[0] == 1, "context parallelism expects one sequence (batch size 1)"
         self.marks = marks          # optional list: receives (stage name, CUDA event recorded after the stage)
         self.mark("start")
@@ -58,24 +75,12 @@ class CudaBackend:
         self.T, self.H = q.shape[1], q.shape[2]
         self.dev = q.device
         self.stream = torch.cuda.current_stream(self.dev).cuda_stream
-        self.status = _status_word(self.dev).data_ptr()
+        self.status = _status_ptr(self.dev)
         self.num_chunks = (self.T + CHUNK - 1) // CHUNK
         P = 2 if segments is None else max(1, int(segments))   # the same on every rank, whatever the shard length
-        # segment boundaries on chunk boundaries, in tokens: [0, ..., T]
-        self.bounds = [min(self.T, ((self.num_chunks * i) // P) * CHUNK) for i in range(P)] + [self.T]
+        self.bounds = segment_bounds(self.T, self.num_chunks, P)
         self.n_segments = P
-        self.tables = None
-        if P > 1:
-            key = (tuple(self.bounds), str(self.dev))
-            self.tables = _SEGMENT_TABLES.get(key)
-            if self.tables is None:
-                if len(_SEGMENT_TABLES) > 16:
-                    _SEGMENT_TABLES.clear()
-                cpu = torch.tensor(self.bounds, dtype=torch.int32)
-                self.tables = _SEGMENT_TABLES[key] = VarlenTables(cpu.to(self.dev), cpu)
-        if tiles is not None:           # the chunk-parallel stage has already run (single-GPU segmented forward)
-            self.tiles = tiles
-            return
+        self.tables = segment_tables(self.bounds, self.dev) if P > 1 else None
         self.tiles = torch.empty(self.num_chunks * self.H * self.lib.cula_kda_tile_pack_bytes(), dtype=torch.uint8,
                                  device=self.dev)
         A_log = None if A_log is None else A_log.float().contiguous()
@@ -190,13 +195,6 @@ def auto_segments(num_chunks, heads, device):
     return max(1, min(MAX_AUTO_SEGMENTS, fit))
 
 
-def segmented_forward(q, k, v, g, beta, tiles, initial_state, output_final_state, segments):
-    """Scan + output of one sequence on one GPU in ``segments`` side-by-side pieces (see `auto_segments`); ``tiles``
-    are the tile packs the chunk-parallel stage has already written. Returns (o, final_state or None)."""
-    backend = CudaBackend(q, k, v, g, beta, None, None, None, None, None, None, None, segments=segments, tiles=tiles)
-    return cp_forward(backend, None, 0, 1, initial_state, output_final_state)
-
-
 def gather_with_group(group=None):
     """all-gather into this rank's own memory: [*shape] -> [world, *shape]."""
     def gather(x):
@@ -277,7 +275,7 @@ class CPBackwardState:
                                                       work.data_ptr(), stream), "cula_kda_bwd_grad_scale")
             _native.check(lib.cula_kda_bwd_scan(self.saved["tiles"].data_ptr(), self.do.data_ptr(), None, work.data_ptr(),
                                                 None, None, Y[0].data_ptr(), None, None, None, 1, self.q.shape[1], self.H,
-                                                _status_word(dev).data_ptr(), stream), "cula_kda_bwd_scan")
+                                                _status_ptr(dev), stream), "cula_kda_bwd_scan")
         return Y
 
     def finish(self, Y_all):

@@ -1,7 +1,10 @@
 """Host-side helpers for the KDA path: device guard and the varlen index tables."""
 from __future__ import annotations
 
+import numpy as np
 import torch
+
+from . import _native
 
 CHUNK = 64
 
@@ -47,18 +50,41 @@ class VarlenTables:
         cpu = (cu_seqlens_cpu if cu_seqlens_cpu is not None else cu_seqlens.cpu()).to(torch.int64)
         if cpu.ndim != 1 or cpu.numel() < 1 or int(cpu[0]) != 0 or bool((cpu[1:] < cpu[:-1]).any()):
             raise ValueError("cu_seqlens must be a non-decreasing 1-D tensor starting at 0")
-        dev = cu_seqlens.device
-        self.n_seqs = cpu.numel() - 1
-        self.total_tokens = int(cpu[-1])
-        self.cu_seqlens = cu_seqlens.to(torch.int32).contiguous()
-        idx = prepare_chunk_indices(cpu)
-        self.num_chunks = idx.shape[0]
-        self.chunk_indices = idx.contiguous().to(dev)
-        self.chunk_offsets = prepare_chunk_offsets(cpu).to(dev)
-        lens = cpu[1:] - cpu[:-1]
+        # all tables in one host buffer and one copy: a new packed batch pays for this before its first launch
+        bounds = cpu.numpy()
+        lens = bounds[1:] - bounds[:-1]
+        n = len(lens)
+        n_chunks = (lens + CHUNK - 1) // CHUNK
+        offsets = np.concatenate([[0], np.cumsum(n_chunks)])
+        NT = int(offsets[-1])
+        host = np.empty(3 * n + 2 + 2 * NT, dtype=np.int32)
+        indices = host[:2 * NT].reshape(NT, 2)                      # (sequence, chunk inside the sequence)
+        indices[:, 0] = np.repeat(np.arange(n), n_chunks)
+        indices[:, 1] = np.arange(NT) - np.repeat(offsets[:-1], n_chunks)
+        host[2 * NT:2 * NT + n + 1] = offsets
+        host[2 * NT + n + 1:2 * NT + 2 * n + 2] = bounds
         # longest sequences first: their CTAs start first and the short ones fill in behind them
-        self.seq_order = torch.argsort(lens, descending=True, stable=True).to(torch.int32).to(dev)
+        host[2 * NT + 2 * n + 2:] = np.argsort(-lens, kind="stable")
+        device = torch.from_numpy(host).to(cu_seqlens.device)
+        self.n_seqs, self.num_chunks, self.total_tokens = n, NT, int(bounds[-1])
+        self.chunk_indices = device[:2 * NT].view(NT, 2)
+        self.chunk_offsets, self.cu_seqlens, self.seq_order = device[2 * NT:].split([n + 1, n + 1, n])
         self.seqlens_cpu = cpu
+        self._native = self._segments = None
+
+    @property
+    def native(self):
+        """The same tables as the host extension takes them."""
+        if self._native is None:
+            self._native = _native.host().Tables(self.cu_seqlens, self.chunk_indices, self.chunk_offsets, self.seq_order,
+                                                 self.n_seqs, self.num_chunks, self.total_tokens)
+        return self._native
+
+    def segments(self, count):
+        """These tables as the ``count`` side-by-side segments of one sequence."""
+        if self._segments is None:
+            self._segments = _native.host().Segments(count, self.native)
+        return self._segments
 
 
 _TABLE_CACHE: list = []      # (source tensor, its version, cu_seqlens_cpu or None, tables), most recent last
