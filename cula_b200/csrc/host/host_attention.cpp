@@ -135,8 +135,8 @@ Backward backward_core(const Tensor& q, const Tensor& k, const Tensor& v, const 
     if (opt.gate_mode != GATE_NONE) {            // the two atomically accumulated gradients share one cleared buffer
         const bool bias = dt_bias.has_value() && dt_bias->defined();
         Tensor both = at::zeros({bias ? H + H * DIM : H}, f32);
-        r.dA = both.narrow(0, 0, H);
-        if (bias) r.dbias = both.narrow(0, H, H * DIM);
+        if (bias) r.dbias = both.narrow(0, 0, H * DIM);
+        r.dA = both.narrow(0, both.numel() - H, H);
     }
     check(lib.cula_kda_bwd_gated(ptr(q), ptr(k), ptr(g), g_flags(g), ptr(beta), beta_flags(beta, opt.beta_logit), fptr(A_log), fptr(dt_bias),
                                  fptr(f.akk), fptr(f.mkk), fptr(scratch), fptr(work), ptr(r.dq), ptr(r.dk), ptr(r.dg), ptr(r.dbeta), fptr(r.dA),

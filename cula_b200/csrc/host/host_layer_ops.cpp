@@ -49,7 +49,7 @@ struct Gate : torch::autograd::Function<Gate> {
         const c10::IValue lb = ctx->saved_data["lb"];
         Tensor dg = at::empty_like(g);
         Tensor both = at::zeros({b32.has_value() ? H + H * K : H}, a32.options());       // the two accumulated gradients
-        Tensor dA = both.narrow(0, 0, H), dbias = b32.has_value() ? both.narrow(0, H, H * K) : Tensor();
+        Tensor dbias = b32.has_value() ? both.narrow(0, 0, H * K) : Tensor(), dA = both.narrow(0, both.numel() - H, H);
         check(lib.cula_kda_gate_bwd(ptr(g), is_f32(g), fptr(a32), fptr(b32), ptr(dy), is_f32(dy), ptr(dg), fptr(dA), fptr(dbias), g.numel() / (H * K),
                                     (int)H, (int)K, !lb.isNone(), lb.isNone() ? 0.f : (float)lb.toDouble(), stream_of(g)), "cula_kda_gate_bwd");
         return {dg, dA.view_as(a32), dbias.defined() ? dbias.view_as(*b32) : Tensor(), Tensor(), Tensor()};

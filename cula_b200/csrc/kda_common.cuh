@@ -98,6 +98,43 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t x) {
     return make_float2(__uint_as_float(x << 16), __uint_as_float(x & 0xffff0000u));
 }
 
+// ---- packed fp32 pairs (one instruction per two lanes of arithmetic on sm_100) ----
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 r;
+    asm("{.reg .b64 ra, rb, rc; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; mul.rn.f32x2 rc, ra, rb; mov.b64 {%0, %1}, rc;}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 r;
+    asm("{.reg .b64 ra, rb, rc; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; add.rn.f32x2 rc, ra, rb; mov.b64 {%0, %1}, rc;}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm("{.reg .b64 ra, rb, rc, rd; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; mov.b64 rc, {%6, %7}; "
+        "fma.rn.f32x2 rd, ra, rb, rc; mov.b64 {%0, %1}, rd;}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+__device__ __forceinline__ float2 splat2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ float2 ex2_2(float2 a) { return make_float2(fast_exp2(a.x), fast_exp2(a.y)); }
+// softplus(x) = max(x, 0) + log1p(e), e = exp(-|x|) <= 1, with log1p(e) = 2 atanh(s), s = e / (2 + e) <= 1/3, by its series in
+// s^2 <= 1/9 up to s^12 (next term 1.4e-8 relative): as accurate for strongly negative x (weak decays) as anywhere else.
+__device__ __forceinline__ float2 softplus2(float2 x) {
+    const float2 e = ex2_2(make_float2(-RCP_LN2 * fabsf(x.x), -RCP_LN2 * fabsf(x.y)));
+    const float2 d = add2(e, splat2(2.f));
+    const float2 s = mul2(e, make_float2(fast_rcp(d.x), fast_rcp(d.y))), z = mul2(s, s);
+    float2 q = fma2(z, splat2(2.f / 13.f), splat2(2.f / 11.f));
+    q = fma2(z, q, splat2(2.f / 9.f));
+    q = fma2(z, q, splat2(2.f / 7.f));
+    q = fma2(z, q, splat2(2.f / 5.f));
+    q = fma2(z, q, splat2(2.f / 3.f));
+    q = fma2(z, q, splat2(2.f));
+    return fma2(s, q, make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
+}
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));

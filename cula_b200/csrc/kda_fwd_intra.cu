@@ -121,43 +121,6 @@ __device__ __forceinline__ void mma_tile_3xtf32(const float* A, int lda, const f
     for (int e = 0; e < 4; ++e) acc[e] += corr[e];
 }
 
-// ---- packed fp32 pairs (one instruction per two lanes of arithmetic on sm_100) ----
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    float2 r;
-    asm("{.reg .b64 ra, rb, rc; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; mul.rn.f32x2 rc, ra, rb; mov.b64 {%0, %1}, rc;}"
-        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 r;
-    asm("{.reg .b64 ra, rb, rc; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; add.rn.f32x2 rc, ra, rb; mov.b64 {%0, %1}, rc;}"
-        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 r;
-    asm("{.reg .b64 ra, rb, rc, rd; mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; mov.b64 rc, {%6, %7}; "
-        "fma.rn.f32x2 rd, ra, rb, rc; mov.b64 {%0, %1}, rd;}"
-        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return r;
-}
-__device__ __forceinline__ float2 splat2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ float2 ex2_2(float2 a) { return make_float2(fast_exp2(a.x), fast_exp2(a.y)); }
-// softplus(x) = max(x, 0) + log1p(e), e = exp(-|x|) <= 1, with log1p(e) = 2 atanh(s), s = e / (2 + e) <= 1/3, by its series in
-// s^2 <= 1/9 up to s^12 (next term 1.4e-8 relative): as accurate for strongly negative x (weak decays) as anywhere else.
-__device__ __forceinline__ float2 softplus2(float2 x) {
-    const float2 e = ex2_2(make_float2(-RCP_LN2 * fabsf(x.x), -RCP_LN2 * fabsf(x.y)));
-    const float2 d = add2(e, splat2(2.f));
-    const float2 s = mul2(e, make_float2(fast_rcp(d.x), fast_rcp(d.y))), z = mul2(s, s);
-    float2 q = fma2(z, splat2(2.f / 13.f), splat2(2.f / 11.f));
-    q = fma2(z, q, splat2(2.f / 9.f));
-    q = fma2(z, q, splat2(2.f / 7.f));
-    q = fma2(z, q, splat2(2.f / 5.f));
-    q = fma2(z, q, splat2(2.f / 3.f));
-    q = fma2(z, q, splat2(2.f));
-    return fma2(s, q, make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
-}
 // mma.sync reads only the upper 19 bits of a tf32 operand, i.e. it truncates. Instead of rounding every operand of the
 // diagonal blocks (one more instruction per element), the mean relative error of truncation, -2^-11 / ln 2 = -3.52e-4 per
 // operand for log-uniform mantissas, is taken out by one factor in the per-channel constant of the column operand.

@@ -36,89 +36,112 @@ __device__ __forceinline__ void store8(void* p, int fp32, size_t idx, const floa
             make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
     }
 }
-__device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
-
-// grid.x covers the H*K/8 channel groups (a thread keeps its 8 channels for the whole launch, so the bias and the
-// head's exp(A_log) are loaded once), grid.y strides over the tokens.
+// A warp owns 256 channels (8 per lane, kept for the whole launch: the bias and the head's exp(A_log) are loaded once);
+// the CTA's eight warps and grid.y stride over the tokens. HBM-bound; NB rows per warp are requested before the first is
+// used. The parameter gradients of a CTA are added in shared memory, then one atomic per channel (16 bytes at a time where
+// the buffer is aligned) and head goes out. Measured at 4096 tokens x 32 heads x 128: backward 47 -> 31 us (134 MB: 4.4 TB/s);
+// shared-memory atomics instead of a slot per warp 38 us, two or six CTAs per SM instead of four 44 / 38 us.
 template <bool BWD>
 __global__ void __launch_bounds__(GATE_THREADS) kda_gate_kernel(const GateArgs a) {
-    __shared__ float sDA[66];     // A_log gradient of the heads this block touches: at most 256 * 8 / K + 1, K >= 32
-    const int HK = a.H * a.K, groups = HK / 8;
-    const int grp = blockIdx.x * GATE_THREADS + threadIdx.x;
-    const bool active = grp < groups;
-    const int ch = active ? 8 * grp : 0, h = ch / a.K;
-    const int h_lo = (blockIdx.x * GATE_THREADS * 8) / a.K;       // first head of this block
+    constexpr int WARPS = GATE_THREADS / 32;
+    __shared__ __align__(16) float s_bias[BWD ? WARPS : 1][BWD ? 256 : 4];
+    __shared__ float s_dA[BWD ? 10 : 1];     // at most 256 / 32 + 1 heads meet 256 channels (K >= 32)
+    const int HK = a.H * a.K, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ch0 = 256 * blockIdx.x, ch_raw = ch0 + 8 * lane;
+    const bool active = ch_raw < HK;
+    const int ch = active ? ch_raw : 0, h = ch / a.K, h_lo = ch0 / a.K;
     if (BWD) {
-        for (int i = threadIdx.x; i < 66; i += GATE_THREADS) sDA[i] = 0.f;
+        if (threadIdx.x < 10) s_dA[threadIdx.x] = 0.f;
         __syncthreads();
     }
     const float alpha = __expf(a.A_log[h]);
-    float bias[8], dbias[8], dA = 0.f;
+    float2 bias[4], dbias[4];
+    float dA = 0.f;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        bias[e] = (a.dt_bias && active) ? a.dt_bias[ch + e] : 0.f;
-        dbias[e] = 0.f;
+    for (int e = 0; e < 4; ++e) {
+        bias[e] = a.dt_bias ? make_float2(a.dt_bias[ch + 2 * e], a.dt_bias[ch + 2 * e + 1]) : make_float2(0.f, 0.f);
+        dbias[e] = make_float2(0.f, 0.f);
     }
     if (active) {
-        // rows are taken four at a time and all their loads are issued before the first is used: a thread has only a
-        // handful of rows, and one load per dependent step would make each of them pay a full memory latency
-        constexpr int NB = 4;
-        for (long long mb = blockIdx.y; mb < a.M; mb += (long long)NB * gridDim.y) {
+        constexpr int NB = BWD ? 2 : 4;
+        const long long step = (long long)gridDim.y * WARPS;
+        for (long long mb = (long long)blockIdx.y * WARPS + warp; mb < a.M; mb += NB * step) {
             float gv[NB][8], dy[NB][8];
 #pragma unroll
             for (int i = 0; i < NB; ++i) {
-                const long long m = min(mb + (long long)i * gridDim.y, a.M - 1);      // clamped: the surplus rows are not used
+                const long long m = min(mb + i * step, a.M - 1);      // clamped: the surplus rows are not used
                 const size_t idx = (size_t)m * HK + ch;
                 load8(a.g, a.g_fp32, idx, gv[i]);
                 if (BWD) load8(a.dy, a.dy_fp32, idx, dy[i]);
             }
 #pragma unroll
             for (int i = 0; i < NB; ++i) {
-                const long long m = mb + (long long)i * gridDim.y;
+                const long long m = mb + i * step;
                 if (m >= a.M) break;
                 const size_t idx = (size_t)m * HK + ch;
                 float o[8];
-                if (!BWD) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const float x = gv[i][e] + bias[e];
-                        o[e] = a.use_lower_bound ? a.lower_bound * __fdividef(1.f, 1.f + __expf(-alpha * x)) : -alpha * softplus_f(x);
-                    }
-                    store8(a.out, a.out_fp32, idx, o);
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const float x = gv[i][e] + bias[e];
-                        float v;
-                        if (a.use_lower_bound) {
-                            const float sg = __fdividef(1.f, 1.f + __expf(-alpha * x));
-                            v = dy[i][e] * a.lower_bound * sg * (1.f - sg) * alpha;      // d/dx of lb sigmoid(alpha x)
-                            dA = fmaf(v, x, dA);                                         // d/dA_log = d/d(alpha) * alpha
-                        } else {
-                            v = -dy[i][e] * alpha * __fdividef(1.f, 1.f + __expf(-x));
-                            dA = fmaf(dy[i][e], -alpha * softplus_f(x), dA);
+                for (int e = 0; e < 4; ++e) {
+                    const float2 x = add2(make_float2(gv[i][2 * e], gv[i][2 * e + 1]), bias[e]);
+                    float2 v;
+                    if (a.use_lower_bound) {
+                        const float c = -alpha * RCP_LN2;
+                        const float2 sg = make_float2(fast_rcp(1.f + fast_exp2(c * x.x)), fast_rcp(1.f + fast_exp2(c * x.y)));
+                        if (!BWD) {
+                            v = mul2(splat2(a.lower_bound), sg);
+                        } else {                     // d/dx of lb sigmoid(alpha x); times x it is d/dA_log
+                            const float2 q = mul2(sg, make_float2(1.f - sg.x, 1.f - sg.y));
+                            v = mul2(mul2(make_float2(dy[i][2 * e], dy[i][2 * e + 1]), splat2(a.lower_bound * alpha)), q);
+                            dA = fmaf(v.x, x.x, fmaf(v.y, x.y, dA));
                         }
-                        dbias[e] += v;
-                        o[e] = v;
+                    } else {
+                        const float2 sp = softplus2(x);
+                        if (!BWD) {
+                            v = mul2(splat2(-alpha), sp);
+                        } else {
+                            const float2 d = mul2(make_float2(dy[i][2 * e], dy[i][2 * e + 1]), splat2(-alpha));
+                            v = mul2(d, make_float2(fast_rcp(1.f + fast_exp2(-RCP_LN2 * x.x)), fast_rcp(1.f + fast_exp2(-RCP_LN2 * x.y))));
+                            dA = fmaf(d.x, sp.x, fmaf(d.y, sp.y, dA));
+                        }
                     }
-                    store8(a.out, a.g_fp32, idx, o);
+                    if (BWD) dbias[e] = add2(dbias[e], v);
+                    o[2 * e] = v.x;
+                    o[2 * e + 1] = v.y;
                 }
+                store8(a.out, BWD ? a.g_fp32 : a.out_fp32, idx, o);
             }
         }
     }
     if (BWD) {
-        if (active) {
-            if (a.ddt_bias) {
+        *reinterpret_cast<float4*>(&s_bias[warp][8 * lane]) = make_float4(dbias[0].x, dbias[0].y, dbias[1].x, dbias[1].y);
+        *reinterpret_cast<float4*>(&s_bias[warp][8 * lane + 4]) = make_float4(dbias[2].x, dbias[2].y, dbias[3].x, dbias[3].y);
+        if (a.dA_log) {
+            // the 16 lanes of a 128-channel head are added by shuffles first
+            if (a.K == 128) {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) atomicAdd(&a.ddt_bias[ch + e], dbias[e]);
+                for (int o = 8; o; o >>= 1) dA += __shfl_xor_sync(0xffffffffu, dA, o);
+                if (active && (lane & 15) == 0) atomicAdd(&s_dA[h - h_lo], dA);
+            } else if (active) {
+                atomicAdd(&s_dA[h - h_lo], dA);
             }
-            if (a.dA_log) atomicAdd(&sDA[h - h_lo], dA);
         }
         __syncthreads();
-        if (a.dA_log) {
-            for (int i = threadIdx.x; i < 66; i += GATE_THREADS)
-                if (h_lo + i < a.H && sDA[i] != 0.f) atomicAdd(&a.dA_log[h_lo + i], sDA[i]);
+        if (a.ddt_bias && threadIdx.x < 64 && ch0 + 4 * threadIdx.x < HK) {
+            const int c4 = 4 * threadIdx.x;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) {
+                const float4 x = *reinterpret_cast<const float4*>(&s_bias[w][c4]);
+                v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+            }
+            float* dst = a.ddt_bias + ch0 + c4;
+            if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+                atomicAdd(reinterpret_cast<float4*>(dst), v);
+            } else {
+                atomicAdd(dst, v.x); atomicAdd(dst + 1, v.y); atomicAdd(dst + 2, v.z); atomicAdd(dst + 3, v.w);
+            }
         }
+        if (a.dA_log && threadIdx.x < 10 && h_lo + threadIdx.x < a.H && s_dA[threadIdx.x] != 0.f) atomicAdd(&a.dA_log[h_lo + threadIdx.x], s_dA[threadIdx.x]);
     }
 }
 
@@ -144,12 +167,11 @@ extern "C" int kda_launch_gate(const kda::GateArgs* a, int backward, cudaStream_
     using namespace kda;
     if (a->M <= 0) return 0;
     const int sms = sm_count();
-    const int groups = a->H * a->K / 8;
-    const int gx = (groups + GATE_THREADS - 1) / GATE_THREADS;
-    // about eight CTAs per SM in flight; the backward pass ends in one atomic per thread and channel, so it runs a
-    // quarter as many, longer-lived CTAs
-    long long gy = ((backward ? 2LL : 8LL) * sms + gx - 1) / gx;
-    if (gy > a->M) gy = a->M;
+    const int gx = (a->H * a->K + 255) / 256;
+    // about eight CTAs per SM in flight; the backward pass ends in atomics, so it runs half as many, longer-lived CTAs
+    long long gy = ((backward ? 4LL : 8LL) * sms + gx - 1) / gx;
+    const long long most = (a->M + GATE_THREADS / 32 - 1) / (GATE_THREADS / 32);
+    if (gy > most) gy = most;
     if (gy > 65535) gy = 65535;
     dim3 grid(gx, (unsigned)gy);
     if (backward) kda_gate_kernel<true><<<grid, GATE_THREADS, 0, stream>>>(*a);

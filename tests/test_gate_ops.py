@@ -116,3 +116,25 @@ def test_beta_sigmoid_inside_chunk_kda(beta_dtype):
     torch.cuda.synchronize()
     assert err_ratio(o_ref.detach(), o.detach().float().cpu()) <= 5e-3
     assert dev_b.grad.dtype == beta_dtype and err_ratio(ref_b.grad, dev_b.grad.float().cpu()) <= 2e-2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,H,K", [(1, 1, 32), (7, 3, 40), (9, 2, 128), (129, 5, 96), (1000, 3, 128)])
+@pytest.mark.parametrize("lb", [None, -5.0])
+def test_fused_kda_gate_at_channel_and_row_edges(M, H, K, lb):
+    """Channel counts that leave part of a warp or of the last 256-channel group idle, heads that straddle a group, row
+    counts around a CTA's share."""
+    from cula_b200.kda import fused_kda_gate
+    gen = torch.Generator().manual_seed(8)
+    g, dy = 3.0 * torch.randn(M, H, K, generator=gen), torch.randn(M, H, K, generator=gen)
+    A_log, bias = 0.3 * torch.randn(H, generator=gen), torch.randn(H * K, generator=gen)
+    ref = [t.clone().requires_grad_(True) for t in (g, A_log, bias)]
+    y_ref = kda_gate(*ref, lower_bound=lb)
+    (y_ref * dy).sum().backward()
+    dev = [t.cuda().requires_grad_(True) for t in (g, A_log, bias)]
+    y = fused_kda_gate(*dev, lower_bound=lb)
+    y.backward(dy.cuda())
+    torch.cuda.synchronize()
+    assert err_ratio(y_ref.detach(), y.detach().cpu()) < 1e-5
+    for r, d in zip(ref, dev):
+        assert err_ratio(r.grad, d.grad.cpu()) < 1e-4

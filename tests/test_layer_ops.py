@@ -91,3 +91,48 @@ def test_rms_norm_gated_matches_oracle(D, act):
     assert err_ratio(ref_in[0].grad, dev[0].grad.float().cpu()) < 4e-3
     assert err_ratio(ref_in[1].grad, dev[1].grad.float().cpu()) < 4e-3
     assert err_ratio(ref_in[2].grad, dev[2].grad.cpu()) < 1e-2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,W,tail", [(8, 1, 0), (72, 4, 5), (200, 3, 0), (64, 2, 1)])
+def test_short_conv_at_chunk_and_channel_edges(D, W, tail):
+    """Channel counts that leave part of a warp idle, sequences that end on and around a batch of tokens and a chunk, rows
+    past the last packed token (zero, with zero gradient)."""
+    from cula_b200.kda import short_conv
+    lens = [1, 2, 3, 4, 5, 7, 8, 9, 61, 63, 64, 65, 67, 128]
+    cu = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32)
+    T, gen = int(cu[-1]), torch.Generator().manual_seed(4)
+    x, dy = (torch.randn(1, T + tail, D, generator=gen).to(torch.bfloat16) for _ in range(2))
+    w, b, cache = 0.5 * torch.randn(D, W, generator=gen), 0.1 * torch.randn(D, generator=gen), torch.randn(len(lens), D, W, generator=gen)
+    ref = [x[:, :T].float().requires_grad_(True), w.clone().requires_grad_(True), b.clone().requires_grad_(True)]
+    y_ref, f_ref = short_conv_ref(ref[0], ref[1], ref[2], cache, "silu", cu)
+    (y_ref * dy[:, :T].float()).sum().backward()
+    dev = [t.cuda().requires_grad_(True) for t in (x, w, b)]
+    y, final = short_conv(dev[0], dev[1], dev[2], initial_state=cache.cuda(), output_final_state=True, cu_seqlens=cu.cuda())
+    y.backward(dy.cuda())
+    torch.cuda.synchronize()
+    assert err_ratio(y_ref.detach(), y.detach()[:, :T].float().cpu()) < 4e-3 and not y[:, T:].any()
+    assert err_ratio(f_ref.detach(), final.cpu()) < 1e-6
+    assert err_ratio(ref[0].grad, dev[0].grad[:, :T].float().cpu()) < 4e-3 and not dev[0].grad[:, T:].any()
+    for r, d in zip(ref[1:], dev[1:]):
+        assert err_ratio(r.grad, d.grad.cpu()) < 1e-2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [128, 256, 512, 1024])
+@pytest.mark.parametrize("R", [1, 3, 8, 9, 4099])
+def test_rms_norm_gated_row_remainders(R, D):
+    from cula_b200.kda import rms_norm_gated
+    gen = torch.Generator().manual_seed(6)
+    x, g, dy = (torch.randn(R, D, generator=gen).to(torch.bfloat16) for _ in range(3))
+    w = 1.0 + 0.1 * torch.randn(D, generator=gen)
+    ref = [x.float().requires_grad_(True), g.float().requires_grad_(True), w.clone().requires_grad_(True)]
+    y_ref = rms_norm_gated_ref(*ref, activation="swish")
+    (y_ref * dy.float()).sum().backward()
+    dev = [t.cuda().requires_grad_(True) for t in (x, g, w)]
+    y = rms_norm_gated(*dev, activation="swish")
+    y.backward(dy.cuda())
+    torch.cuda.synchronize()
+    assert err_ratio(y_ref.detach(), y.detach().float().cpu()) < 4e-3
+    for r, d, tol in zip(ref, dev, (4e-3, 4e-3, 1e-2)):
+        assert err_ratio(r.grad, d.grad.float().cpu()) < tol
