@@ -438,7 +438,7 @@ def cp_section(rank, world, dev, flush, steps=10, T_total=CP_TOKENS, H=CP_HEADS)
         cp.MAX_AUTO_SEGMENTS = 1            # the yardstick is the plain single-pass scan of the whole sequence
         o_ref, ht_ref = chunk_kda(full["q"], full["k"], full["v"], full["g"], full["beta"], A_log=full["A_log"],
                                   dt_bias=full["dt_bias"], initial_state=full["initial_state"], output_final_state=True, **kw)
-        cp.MAX_AUTO_SEGMENTS = 4
+        cp.MAX_AUTO_SEGMENTS = 8
         rel = lambda a, b: float((a.double() - b.double()).norm() / b.double().norm())
         # what the carried state contributes: the forward of the last 4096 tokens alone, from a zero state
         tail = {n: full[n][:, -4096:].contiguous() for n in ("q", "k", "v", "g", "beta")}

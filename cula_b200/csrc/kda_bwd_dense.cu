@@ -24,10 +24,9 @@
 //
 // Covers the state-dependent half of chunk_kda_bwd_kernel_wy_dqkg_fused (cula/kda/chunk_bwd.py:145-313) and the
 // dAqk half of chunk_kda_bwd_kernel_dAv (cula/kda/chunk_bwd.py:63-125).
-#include <cuda.h>
-
 #include "kda_common.cuh"
 #include "kda_params.h"
+#include "tensor_map.cuh"
 #include "umma.cuh"
 
 // Optional per-phase cycle counters (compile with -DKDA_PHASE_TIMERS): thread 0 of every CTA adds the clock64() spent
@@ -470,21 +469,8 @@ extern "C" int kda_bwd_dense_read_timers(unsigned long long* out, int reset) {
 
 namespace {
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = [] {
-        void* sym = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) != cudaSuccess ||
-            qres != cudaDriverEntryPointSuccess)
-            sym = nullptr;
-        return reinterpret_cast<EncodeTiledFn>(sym);
-    }();
-    return fn;
-}
+using kda::EncodeTiledFn;
+using kda::encode_tiled_fn;
 
 // fp32 [tiles * 128 rows][128 columns], fetched as boxes of 32 columns x 128 rows with the 128-byte swizzle
 bool make_state_map(CUtensorMap* map, const float* base, int tiles) {

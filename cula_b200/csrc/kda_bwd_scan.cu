@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
             const int s = it % BS_STAGES, use = it / BS_STAGES;
             const int valid = min(BT, len - c * BT);
             bool ok = true;
-            if (lane == 0 && use > 0) ok = mbar_wait(&empty[s], (use - 1) & 1);
+            if (lane == 0 && use > 0) ok = mbar_spin(&empty[s], (use - 1) & 1);
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (!ok) {
                 if (lane == 0) report_status(p.status, STATUS_WAIT_TIMEOUT);
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
     for (int it = 0; it < nchunks; ++it) {
         const int c = nchunks - 1 - it;
         const int s = it % BS_STAGES;
-        if (!mbar_wait(&full[s], (it / BS_STAGES) & 1)) {
+        if (!mbar_spin(&full[s], (it / BS_STAGES) & 1)) {
             report_status(p.status, STATUS_WAIT_TIMEOUT);
             return;
         }

@@ -185,16 +185,29 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
+// One bounded poll: the hardware suspends the warp until the phase completes or the hint (in nanoseconds) runs out, so that
+// waiting warps do not take issue slots from the working ones of their scheduler.
+constexpr uint32_t MBAR_SUSPEND_NS = 16384;
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(MBAR_SUSPEND_NS) : "memory");
     return ok != 0;
 }
-// Bounded wait: gives up after ~a second (by default) and reports false (the caller records a status and unwinds).
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int limit = (1 << 22)) {
-    for (int i = 0; i < limit; ++i) {
+// Bounded wait: gives up after about a second (by default; at least `limit` short polls) and reports false (the caller
+// records a status and unwinds).
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int limit = (1 << 16)) {
+    for (int i = 0; i < limit; ++i)
         if (mbar_test(bar, parity)) return true;
+    return false;
+}
+// The same without the suspend hint: wakes up a little sooner, for the one waiting warp of a CTA whose others are parked on a barrier.
+__device__ __forceinline__ bool mbar_spin(uint64_t* bar, uint32_t parity, int limit = (1 << 22)) {
+    for (int i = 0; i < limit; ++i) {
+        uint32_t ok;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+        if (ok) return true;
         if (i > 64) __nanosleep(64);
     }
     return false;

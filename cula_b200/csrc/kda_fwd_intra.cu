@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
     // On a time-out the status word is set and the whole CTA leaves the tile loop together (TMEM is freed below).
     auto wait_mma = [&](int which, uint32_t parity) -> bool {
         if (tid == MMA_THREAD) {
-            if (!mbar_wait(&bars[which], parity)) {
+            if (!mbar_spin(&bars[which], parity)) {
                 report_status(p.status, STATUS_WAIT_TIMEOUT);
                 *sAbort = 1;
             }

@@ -1,95 +1,88 @@
-// Sequential state scan fused with the output stage.
+// Sequential state scan fused with the output stage, on tcgen05.
 //
-// One CTA per (sequence, head, half of the value columns). Four consumer warps each own 16 value
-// columns of the fp32 state, held TRANSPOSED in mma.sync accumulator registers (S^T: 16 x 128 per
-// warp) for the whole sequence: because the accumulator fragment of one m16n8k16 MMA is exactly the
-// A fragment of the next, the chain
-//     v_new^T = u^T - S^T w^T ;  o^T = S^T qg^T + v_new^T Aqk^T ;  S^T <- S^T diag(decay) + v_new^T kg
-// runs without the state ever leaving registers and without any cross-warp synchronisation. A fifth
-// warp is the producer: it streams the per-chunk tile packs through a 3-stage shared-memory ring
-// with bulk (TMA-engine) copies signalled on mbarriers.
+// One CTA per (sequence, head) carries the fp32 state TRANSPOSED in tensor memory (S^T: lane = value column, column = key
+// channel) over the chunks; per chunk
+//     ACC  = S16 [W | QG]^T             S16: the state as fp16 A operand in tensor memory, one power-of-two scale per lane
+//     v_new^T = u^T - ACC_W             -> fp16 A operand in tensor memory (over the columns it was computed from)
+//     S^T  = S^T diag(decay) + v_new^T KG
+//     o^T  = ACC_QG + v_new^T Aqk^T
+// What bounds it is the latency of that chain, not the tensor pipe: two MMA groups and two register passes per chunk, each
+// handed over by an mbarrier. So everything that is not on the chain runs beside it, in warps of its own:
+//   warps 0-3     output rows and, when asked for, v_new: lane-per-column values are turned into token rows in shared memory
+//                 and leave as one bulk (tensor) store;
+//   warps 4-19    state: S out of tensor memory, fp16 copy back in (chain), then the decayed state (beside the MMAs),
+//                 per-chunk states to HBM when asked for, initial / final state; four warps share a lane quadrant, 32 key
+//                 channels each;
+//   warps 20-27   v_new (chain), 32 tokens each;
+//   warp 28       issues the MMAs;
+//   warp 29       streams the tile packs (2 stages): TMA tensor boxes lay W, QG, KG out as 128-byte-swizzled operand atoms
+//                 (the pack keeps 256-byte rows; its XOR swizzle is that of the atoms), untiled bulk copies bring the rest.
+//
+// The same kernel computes shard transitions S_out = M S_in + C for context parallelism (grid.z: 0 carries C from a zero
+// state, 1 carries the K x K matrix M from the identity with u = 0; no output rows).
 //
 // Replaces chunk_gated_delta_rule_fwd_h (cula/ops/chunk_delta_h.py:1991-2168) and chunk_gla_fwd_o
 // (cula/ops/fwd_o.py:1755-1852); the per-chunk states h and v_new only go to HBM when the caller
-// asks for them (backward recomputation, return_intermediate_states).
+// asks for them (backward recomputation, return_intermediate_states). Every wait is bounded: on expiry the status word is
+// set, all roles unwind to the end of the kernel, and the tensor memory is freed.
 #include "kda_common.cuh"
 #include "kda_params.h"
+#include "tensor_map.cuh"
+#include "umma.cuh"
 
 namespace kda {
 
-constexpr int SCAN_STAGES = 3;
-constexpr int SCAN_STAGE_BYTES = TP_HEAD_BYTES + 8192;   // W,QG,KG,AQK,DECAY + one U half = 66048
-constexpr int SCAN_STG_BYTES = 4096;                     // per-warp staging for coalesced stores
-constexpr int SCAN_CONSUMERS = 4;
-constexpr int SCAN_THREADS = (SCAN_CONSUMERS + 1) * 32;
-constexpr int SCAN_SMEM = SCAN_STAGES * SCAN_STAGE_BYTES + SCAN_CONSUMERS * SCAN_STG_BYTES + 64;
-constexpr int ST_U = TP_HEAD_BYTES;                      // offset of the U half inside a stage
+constexpr int SC_STAGES = 2;
+constexpr int SC_OUT_WARPS = 4, SC_STATE_WARPS = 16, SC_VALUE_WARPS = 8;
+constexpr int SC_MMA_WARP = SC_OUT_WARPS + SC_STATE_WARPS + SC_VALUE_WARPS, SC_LOAD_WARP = SC_MMA_WARP + 1;
+constexpr int SC_THREADS = 32 * (SC_LOAD_WARP + 1);
+// shared-memory stage: B operands as [2 k-atoms of 64 channels][W 64 rows | QG 64 rows][128 B], KG as [2 mn-atoms][64 tokens]
+// [128 B], then the rest of the pack as it is
+constexpr int ST_WQ = 0, ST_KG = 32768, ST_AQK = 49152, ST_U = 57344, ST_DECAY = 73728, SC_STAGE_BYTES = 74752;
+static_assert(SC_STAGE_BYTES % 1024 == 0, "operand atoms are 1024-byte aligned");
+constexpr int OST_BYTES = 64 * 256;                          // staged token rows
+constexpr int SC_OST = SC_STAGES * SC_STAGE_BYTES, SC_MISC = SC_OST + 2 * OST_BYTES;
+constexpr int SC_SMEM = SC_MISC + 8448 + 1024;
+// tensor-memory columns: the state, its fp16 copy, two [W | QG] accumulators (by chunk parity, so that the next chunk's product
+// does not wait until this one's outputs have been read), the Aqk product
+constexpr uint32_t TM_S32 = 0, TM_S16 = 128, TM_ACC = 192, TM_QG = 64 /* inside an accumulator */, TM_O2 = 448;
 
-// Shared-memory layout of a pipeline stage. The full scan stages the whole head of a tile pack plus one U half and
-// runs one CTA per SM; the transition scan needs only W, KG, DECAY and the U half, packs them tightly, keeps two
-// stages (the producer warp pulls the chunks after those into L2) and so fits two CTAs per SM.
-// NVH = value halves per CTA. 1: a CTA carries 64 value columns on 4 consumer warps (grid.x = 2), three stages.
-// 2: both halves on 8 consumer warps (two per scheduler, so one warp's dependent chain fills the other's bubbles in
-// the tensor pipe), the whole tile pack per stage, two stages; used when there are more scan CTAs than SMs.
-template <bool TRANSITION, int NVH>
-struct ScanLayout {
-    static constexpr int CONSUMERS = SCAN_CONSUMERS * NVH;
-    static constexpr int STAGES = NVH == 2 ? 2 : SCAN_STAGES, STAGE_BYTES = TP_HEAD_BYTES + 8192 * NVH;
-    static constexpr int W = TP_W, KG = TP_KG, DECAY = TP_DECAY, U = ST_U;
-    static constexpr int STG = CONSUMERS * SCAN_STG_BYTES;
-    static constexpr int SMEM = STAGES * STAGE_BYTES + STG + 64;
-    static constexpr int CTAS_PER_SM = 1;
-};
-template <>
-struct ScanLayout<true, 1> {
-    static constexpr int CONSUMERS = SCAN_CONSUMERS;
-    static constexpr int STAGES = 2;
-    static constexpr int W = 0, KG = 16384, DECAY = 32768, U = 33280, STAGE_BYTES = 41472;
-    static constexpr int STG = 0;
-    static constexpr int SMEM = STAGES * STAGE_BYTES + STG + 64;
-    static constexpr int CTAS_PER_SM = 2;
-};
-
-// Bounded wait that also ends when *votes reaches `quorum` (the CTA has nothing left to compute).
-// Returns 0 = barrier phase completed, 1 = gave up (time-out), 2 = quorum reached.
-__device__ __forceinline__ int mbar_wait_or_quorum(uint64_t* bar, uint32_t parity, volatile int* votes, int quorum) {
-    for (int i = 0; i < (1 << 22); ++i) {
-        if (mbar_test(bar, parity)) return 0;
-        if (*votes >= quorum) return 2;
-        if (i > 64) __nanosleep(64);
-    }
-    return 1;
+__device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const CUtensorMap* map, int x, int y, int z, int w, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                 :: "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tma_store_rows(const CUtensorMap* map, uint32_t smem_src, int h, int row) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+                 :: "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_src), "r"(0), "r"(h), "r"(row) : "memory");
+}
+__device__ __forceinline__ uint64_t sc_sdesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+    return umma::make_sdesc(addr, lbo, sbo) | (2ull << 61);     // 128-byte swizzle
+}
+// arrival of a whole warp (its tensor-memory and shared-memory accesses before this point are ordered first)
+__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
 }
 
-// TRANSITION: the affine action of a whole shard on the state, S_out = M S_in + C, from the same recurrence with
-// four column groups per (sequence, head): groups 0,1 carry C (zero start, normal u; written to p.ht) and groups
-// 2,3 carry the K x K matrix M = prod_c (D_c - kg_c^T w_c) (identity start, u = 0; written to p.m_out). No output
-// rows are produced. Used by context parallelism.
-template <bool STORE_HV, bool TRANSITION, int NVH = 1>
-__global__ void __launch_bounds__((SCAN_CONSUMERS * NVH + 1) * 32, ScanLayout<TRANSITION, NVH>::CTAS_PER_SM)
-kda_fwd_scan_kernel(const ScanParams p) {
-    static_assert(NVH == 1 || !TRANSITION, "both value halves per CTA: not for the transition scan");
-    using L = ScanLayout<TRANSITION, NVH>;
-    extern __shared__ __align__(128) unsigned char smem[];
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::STAGES * L::STAGE_BYTES + L::STG);
-    uint64_t* empty = full + L::STAGES;
-    // Columns of the transition matrix M that have become exactly zero stay zero (their recurrence is linear and has
-    // no source term), so a warp whose 16 columns are all zero votes once and stops computing; when all consumer warps
-    // of an M-carrying CTA have voted, the CTA is finished -- bit-identical results, and with strong gates (the decay
-    // of one chunk underflows fp32) these CTAs free their SMs for the C-carrying ones after a chunk or two.
-    volatile int* zero_votes = reinterpret_cast<volatile int*>(empty + L::STAGES);
+__global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanParams p, const __grid_constant__ CUtensorMap map,
+                                                                     const __grid_constant__ CUtensorMap map_o) {
+    extern __shared__ unsigned char sc_smem_raw[];
+    unsigned char* sm = sc_smem_raw + ((1024u - (smem_u32(sc_smem_raw) & 1023u)) & 1023u);
+    const uint32_t smb = smem_u32(sm);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + SC_MISC);
+    uint64_t *full = bars, *empty = bars + 2, *b_s16 = bars + 4, *b_dec = bars + 6, *b_acc = bars + 7, *b_s32 = bars + 9, *b_o = bars + 10,
+             *b_ost = bars + 12, *b_vsum = bars + 13, *b_max = bars + 14 /* [4] */;
+    // A wait by phase parity must not fall two completions behind. v_new can be ready, and have been read, for a chunk while the
+    // other side still waits for the chunk before it, so these two are pairs: chunk c uses barrier c & 1 in its phase c / 2.
+    uint64_t *b_v16 = bars + 18 /* [2] */, *b_oread = bars + 20 /* [2] */;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + SC_MISC + 192);
+    float* sDown = reinterpret_cast<float*>(sm + SC_MISC + 256);         // [4 chunks][128 value columns] 1 / scale of S16: the output warps may be a chunk behind
+    float* sMax = reinterpret_cast<float*>(sm + SC_MISC + 2304);         // [2 chunk parities][4 key quarters][128] largest |S| of a column
+    float* sVsum = reinterpret_cast<float*>(sm + SC_MISC + 6400);        // [2 chunk parities][2 token halves][128] sum of |v_new|
+
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // Grid: (column group, head, sequence). When the transition scan has more CTAs than SMs it is launched as
-    // (head, sequence, column group) instead: block indices are handed to the SMs in linear order, so all C-carrying
-    // CTAs (groups 0, 1) come first, one per SM, and the M-carrying ones (groups 2, 3) become their co-residents; when
-    // the M CTAs finish early (see zero_votes) every C CTA is left with an SM of its own. (With fewer CTAs than SMs the
-    // original order keeps the four CTAs of a head on neighbouring SMs, which read the same tile packs.)
-    const bool gm = TRANSITION && p.group_major;
-    const int cgrp = gm ? blockIdx.z : blockIdx.x, seq_slot = gm ? blockIdx.y : blockIdx.z;
-    const bool is_m = TRANSITION && cgrp >= 2;           // this CTA carries columns of M
-    const int vh = NVH == 2 ? ((warp >> 2) & 1) : (cgrp & 1), h = gm ? blockIdx.x : blockIdx.y;
-    const int pw = warp & 3;                             // 16-column slice of the value half
-    const int n = p.seq_order ? p.seq_order[seq_slot] : seq_slot;
+    const int h = blockIdx.x, n = p.seq_order ? p.seq_order[blockIdx.y] : blockIdx.y;
+    const bool is_m = blockIdx.z == 1, want_o = p.o != nullptr, want_out = want_o || p.vnew_out;
     int bos, len, chunk0;
     if (p.cu_seqlens) {
         bos = p.cu_seqlens[n];
@@ -103,437 +96,419 @@ kda_fwd_scan_kernel(const ScanParams p) {
     const int nchunks = (len + BT - 1) / BT;
 
     if (tid == 0) {
-        for (int s = 0; s < L::STAGES; ++s) {
+        for (int s = 0; s < SC_STAGES; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], L::CONSUMERS);
+            mbar_init(&empty[s], 1 + SC_STATE_WARPS + (is_m ? 0 : SC_VALUE_WARPS));
         }
-        *zero_votes = 0;
+        mbar_init(b_s16, SC_STATE_WARPS);
+        mbar_init(b_dec, SC_STATE_WARPS);
+        mbar_init(b_acc, 1);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&b_v16[b], SC_VALUE_WARPS);
+            mbar_init(&b_oread[b], SC_OUT_WARPS);
+        }
+        mbar_init(b_vsum, SC_VALUE_WARPS);
+        mbar_init(b_s32, 1);
+        mbar_init(b_o, 1);
+        mbar_init(b_ost, SC_OUT_WARPS);
+        for (int q = 0; q < 4; ++q) mbar_init(&b_max[q], SC_STATE_WARPS / 4);
         fence_mbar_init();
     }
+    if (warp == SC_MMA_WARP) umma::tmem_alloc(tmem_slot, 512);
+    umma::fence_before_sync();
     __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tmem = *tmem_slot;
     // Everything this kernel reads (tile packs, initial states) may come from the kernels before it in the stream; with
     // programmatic stream serialization the CTA can be resident before they have finished, so wait here (a no-op when
-    // the launch does not carry the attribute). Only scheduling, the index arithmetic and the barrier set-up above overlap.
+    // the launch does not carry the attribute). Only scheduling, the index arithmetic and the set-up above overlap.
     pdl_wait();
 
-    if (warp == L::CONSUMERS) {
-        // ------------------------------- producer warp -------------------------------
-        if (TRANSITION) {
-            const int u_off = vh ? TP_U1 : TP_U0;
-            int issued = 0;                       // chunks whose copies have been issued
-            for (int c = 0; c < nchunks; ++c) {
-                const int s = c % L::STAGES, use = c / L::STAGES;
-                bool ok = true;
-                int quorum = 0;
-                if (lane == 0) {
-                    if (is_m && *zero_votes >= L::CONSUMERS) quorum = 1;
-                    if (!quorum && use > 0) {
-                        const int r = mbar_wait_or_quorum(&empty[s], (use - 1) & 1, zero_votes, is_m ? L::CONSUMERS : (1 << 30));
-                        ok = r != 1;
-                        quorum = r == 2;
-                    }
-                }
-                quorum = __shfl_sync(0xffffffffu, quorum, 0);
-                if (quorum) break;
-                if (lane == 0) {
-                    if (ok) {
-                        const unsigned char* tile = p.tiles + ((size_t)(chunk0 + c) * p.H + h) * TP_BYTES;
-                        unsigned char* dst = smem + s * L::STAGE_BYTES;
-                        mbar_arrive_expect_tx(&full[s], is_m ? L::U : L::STAGE_BYTES);
-                        bulk_g2s(dst + L::W, tile + TP_W, 16384, &full[s]);
-                        bulk_g2s(dst + L::KG, tile + TP_KG, 16384, &full[s]);
-                        bulk_g2s(dst + L::DECAY, tile + TP_DECAY, 512, &full[s]);
-                        if (!is_m) bulk_g2s(dst + L::U, tile + u_off, 8192, &full[s]);
-                    }
-                }
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                if (!ok) {
-                    if (lane == 0) report_status(p.status, STATUS_WAIT_TIMEOUT);
-                    break;
-                }
-                issued = c + 1;
-                const int cn = c + L::STAGES;                 // not yet being copied: pull it into L2
-                if (cn < nchunks) {
-                    const unsigned char* tile = p.tiles + ((size_t)(chunk0 + cn) * p.H + h) * TP_BYTES;
-                    for (int i = lane; i < (is_m ? 260 : 324); i += 32) {
-                        const int off = i < 128 ? TP_W + i * 128 : i < 256 ? TP_KG + (i - 128) * 128
-                                      : i < 260 ? TP_DECAY + (i - 256) * 128 : u_off + (i - 260) * 128;
-                        prefetch_l2(tile + off);
-                    }
-                }
-            }
-            // the consumers may have left early: do not exit with bulk copies to this CTA's shared memory in flight
-            if (is_m && lane == 0) {
-                for (int cc = max(0, issued - L::STAGES); cc < issued; ++cc)
-                    if (!mbar_wait(&full[cc % L::STAGES], (cc / L::STAGES) & 1)) report_status(p.status, STATUS_WAIT_TIMEOUT);
-            }
-            return;
-        }
+    auto wait = [&](uint64_t* bar, int phase) -> bool {
+        if (mbar_wait(bar, phase & 1)) return true;
+        report_status(p.status, STATUS_WAIT_TIMEOUT);
+        return false;
+    };
+
+    if (warp == SC_LOAD_WARP) {
+        // ------------------------------- producer -------------------------------
         if (lane == 0) {
+            int issued = 0;
+            bool ok = true;
             for (int c = 0; c < nchunks; ++c) {
-                const int s = c % L::STAGES, use = c / L::STAGES;
-                if (use > 0 && !mbar_wait(&empty[s], (use - 1) & 1)) {
-                    report_status(p.status, STATUS_WAIT_TIMEOUT);
-                    break;
+                const int s = c % SC_STAGES, use = c / SC_STAGES;
+                if (use > 0 && !(ok = wait(&empty[s], use - 1))) break;
+                const int t_id = (chunk0 + c) * p.H + h;
+                const unsigned char* tile = p.tiles + (size_t)t_id * TP_BYTES;
+                unsigned char* dst = sm + s * SC_STAGE_BYTES;
+                const uint32_t d = smb + s * SC_STAGE_BYTES;
+                mbar_arrive_expect_tx(&full[s], 16384 + 16384 + 512 + (is_m ? 0 : 16384) + (want_o ? 16384 + 8192 : 0));
+#pragma unroll
+                for (int a = 0; a < 2; ++a) {
+                    tma_load_4d(d + ST_WQ + a * 16384, &map, 0, a, 0, t_id, &full[s]);
+                    if (want_o) tma_load_4d(d + ST_WQ + a * 16384 + 8192, &map, 0, a, 64, t_id, &full[s]);
                 }
-                const unsigned char* tile = p.tiles + ((size_t)(chunk0 + c) * p.H + h) * TP_BYTES;
-                unsigned char* dst = smem + s * L::STAGE_BYTES;
-                mbar_arrive_expect_tx(&full[s], L::STAGE_BYTES);
-                if (NVH == 2) {
-                    bulk_g2s(dst, tile, TP_BYTES, &full[s]);          // head + both U halves are contiguous
-                } else {
-                    bulk_g2s(dst, tile, TP_HEAD_BYTES, &full[s]);
-                    bulk_g2s(dst + ST_U, tile + ((cgrp & 1) ? TP_U1 : TP_U0), 8192, &full[s]);
-                }
+                bulk_g2s(dst + ST_DECAY, tile + TP_DECAY, 512, &full[s]);
+                if (!is_m) bulk_g2s(dst + ST_U, tile + TP_U0, 16384, &full[s]);
+#pragma unroll
+                for (int a = 0; a < 2; ++a) tma_load_4d(d + ST_KG + a * 8192, &map, 0, a, 128, t_id, &full[s]);
+                if (want_o) bulk_g2s(dst + ST_AQK, tile + TP_AQK, 8192, &full[s]);
+                issued = c + 1;
             }
+            // do not leave with copies to this CTA's shared memory in flight
+            if (!ok)
+                for (int c = max(0, issued - SC_STAGES); c < issued; ++c) mbar_wait(&full[c % SC_STAGES], (c / SC_STAGES) & 1);
         }
-        return;
+    } else if (warp == SC_MMA_WARP) {
+        // ------------------------------- MMA issue (the whole warp in step, one elected lane issues) -------------------------------
+        const uint32_t id_wq = umma::make_idesc(umma::FMT_F16, 128, want_o ? 128 : 64, false, false);
+        const uint32_t id_kg = umma::make_idesc(umma::FMT_F16, 128, 128, false, true);
+        const uint32_t id_o2 = umma::make_idesc(umma::FMT_F16, 128, 64, false, false);
+        for (int c = 0; c < nchunks; ++c) {
+            const int s = c % SC_STAGES;
+            // descriptors differ in their address field (16-byte units) only
+            const uint64_t d_wq = sc_sdesc(smb + s * SC_STAGE_BYTES + ST_WQ, 16, 1024), d_kg = sc_sdesc(smb + s * SC_STAGE_BYTES + ST_KG, 8192, 1024),
+                           d_aqk = sc_sdesc(smb + s * SC_STAGE_BYTES + ST_AQK, 16, 1024);
+            const uint32_t acc = tmem + TM_ACC + 128 * (c & 1);
+            if (!wait(&full[s], c / SC_STAGES)) break;
+            if (!wait(b_s16, c)) break;
+            umma::fence_after_sync();
+            if (umma::elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < 8; ++ks)
+                    umma::mma_f16_ta(acc, tmem + TM_S16 + 8 * ks, d_wq + (((ks >> 2) * 16384 + (ks & 3) * 32) >> 4), id_wq, ks != 0);
+                umma::commit(b_acc);
+            }
+            __syncwarp();
+            if (!wait(b_dec, c) || !wait(&b_v16[c & 1], c >> 1)) break;
+            umma::fence_after_sync();
+            if (umma::elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks)       // v_new^T: tokens 0..31 in columns 0..15, tokens 32..63 in columns 32..47 of the W accumulator
+                    umma::mma_f16_ta(tmem + TM_S32, acc + 32 * (ks >> 1) + 8 * (ks & 1), d_kg + ((ks * 2048) >> 4), id_kg, 1);
+                umma::commit(b_s32);
+            }
+            __syncwarp();
+            // the previous chunk's outputs and v_new have been read: TM_O2 is free, and so is the next product's accumulator
+            if (want_out && c > 0 && !wait(&b_oread[(c - 1) & 1], (c - 1) >> 1)) break;
+            if (umma::elect_one()) {
+                if (want_o) {
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks)
+                        umma::mma_f16_ta(tmem + TM_O2, acc + 32 * (ks >> 1) + 8 * (ks & 1), d_aqk + ((ks * 32) >> 4), id_o2, ks != 0);
+                    umma::commit(b_o);
+                }
+                umma::commit(&empty[s]);
+            }
+            __syncwarp();
+        }
     }
-
-    // ---------------------------------- consumer warps ----------------------------------
-    const int g = lane >> 2, t = lane & 3;
-    const int m = lane >> 3, r = lane & 7;          // ldmatrix/stmatrix: matrix index, row inside it
-    const int vb = vh * 64 + pw * 16;               // first value column of this warp
-    unsigned char* stg = smem + L::STAGES * L::STAGE_BYTES + warp * SCAN_STG_BYTES;   // unused by the transition scan
-    const uint32_t stg_u32 = smem_u32(stg);
-
-    float S[16][4];
-    if (is_m) {
-#pragma unroll
-        for (int jt = 0; jt < 16; ++jt) {
-            const int k0 = 8 * jt + 2 * t;
-            S[jt][0] = (k0 == vb + g) ? 1.f : 0.f;
-            S[jt][1] = (k0 + 1 == vb + g) ? 1.f : 0.f;
-            S[jt][2] = (k0 == vb + g + 8) ? 1.f : 0.f;
-            S[jt][3] = (k0 + 1 == vb + g + 8) ? 1.f : 0.f;
-        }
-    } else if (!TRANSITION && p.h0) {
-        const float* h0 = p.h0 + ((size_t)n * p.H + h) * DK * DV;
-#pragma unroll
-        for (int jt = 0; jt < 16; ++jt) {
-            int k0 = 8 * jt + 2 * t;
-            S[jt][0] = h0[(size_t)k0 * DV + vb + g];
-            S[jt][1] = h0[(size_t)(k0 + 1) * DV + vb + g];
-            S[jt][2] = h0[(size_t)k0 * DV + vb + g + 8];
-            S[jt][3] = h0[(size_t)(k0 + 1) * DV + vb + g + 8];
-        }
-    } else {
-#pragma unroll
-        for (int jt = 0; jt < 16; ++jt) S[jt][0] = S[jt][1] = S[jt][2] = S[jt][3] = 0.f;
-    }
-
-    // per-lane swizzled column-group offsets for the four k-step pairs of a 256-byte-row operand
-    uint32_t x256[4];
-#pragma unroll
-    for (int kp = 0; kp < 4; ++kp) x256[kp] = (uint32_t)(((4 * kp + m) ^ r) << 4);
-
-    bool voted = false;          // this warp's columns of M are exactly zero (transition scan only)
-    for (int c = 0; c < nchunks; ++c) {
-        const int s = c % L::STAGES;
-        if (is_m) {
-            if (*zero_votes >= L::CONSUMERS) break;
-            const int r = mbar_wait_or_quorum(&full[s], (c / L::STAGES) & 1, zero_votes, L::CONSUMERS);
-            if (r == 2) break;
-            if (r == 1) {
-                report_status(p.status, STATUS_WAIT_TIMEOUT);
-                return;
-            }
-            if (voted) {         // nothing to compute: keep the pipeline protocol going for the warps that still work
-                if (lane == 0) mbar_arrive(&empty[s]);
-                continue;
-            }
-        } else if (!mbar_wait(&full[s], (c / L::STAGES) & 1)) {
-            report_status(p.status, STATUS_WAIT_TIMEOUT);
-            return;
-        }
-        const uint32_t st = smem_u32(smem + s * L::STAGE_BYTES);
-        const int valid = min(BT, len - c * BT);
-        const size_t tile_idx = (size_t)(chunk0 + c) * p.H + h;
-
-        // ---- S as fp16 A fragments (8 k-steps over the 128 key channels), scaled by a per-warp power
-        //      of two so that the largest entry sits near 2^13: fp16 then carries 11 significant bits
-        //      whatever the magnitude of the state, and cannot overflow ----
-        float smax = 0.f;
-#pragma unroll
-        for (int jt = 0; jt < 16; ++jt)
-            smax = fmaxf(smax, fmaxf(fmaxf(fabsf(S[jt][0]), fabsf(S[jt][1])), fmaxf(fabsf(S[jt][2]), fabsf(S[jt][3]))));
-#pragma unroll
-        for (int o = 16; o; o >>= 1) smax = fmaxf(smax, __shfl_xor_sync(0xffffffffu, smax, o));
-        if (is_m && smax == 0.f) {      // all 16 columns of this warp are exactly zero, and will stay zero
-            voted = true;
-            if (lane == 0) {
-                atomicAdd(const_cast<int*>(zero_votes), 1);
-                mbar_arrive(&empty[s]);
-            }
-            continue;
-        }
-        int shift = 13 - (((__float_as_int(smax) >> 23) & 0xff) - 127);
-        shift = max(-100, min(100, shift));
-        const float s_up = __int_as_float((shift + 127) << 23), s_down = __int_as_float((127 - shift) << 23);
-        uint32_t sa[8][4];
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-            sa[ks][0] = pack_f16(S[2 * ks][0] * s_up, S[2 * ks][1] * s_up);
-            sa[ks][1] = pack_f16(S[2 * ks][2] * s_up, S[2 * ks][3] * s_up);
-            sa[ks][2] = pack_f16(S[2 * ks + 1][0] * s_up, S[2 * ks + 1][1] * s_up);
-            sa[ks][3] = pack_f16(S[2 * ks + 1][2] * s_up, S[2 * ks + 1][3] * s_up);
-        }
-        if (STORE_HV) {
-            if (p.h_out) {
-                // incoming state of this chunk, bf16 [128 k][128 v]; this warp owns a 32-byte column slice
-#pragma unroll
-                for (int ks = 0; ks < 8; ++ks) {
-                    int krow = 8 * (2 * ks + (m >> 1)) + r;
-                    stsm_x4_t(stg_u32 + krow * 32 + (m & 1) * 16,
-                              pack_bf16(S[2 * ks][0], S[2 * ks][1]), pack_bf16(S[2 * ks][2], S[2 * ks][3]),
-                              pack_bf16(S[2 * ks + 1][0], S[2 * ks + 1][1]), pack_bf16(S[2 * ks + 1][2], S[2 * ks + 1][3]));
-                }
-                __syncwarp();
-                unsigned char* hg = reinterpret_cast<unsigned char*>(p.h_out) + tile_idx * (size_t)(DK * DV * 2);
-#pragma unroll
-                for (int it = 0; it < 8; ++it) {
-                    int row = it * 16 + (lane >> 1), hf = lane & 1;
-                    uint4 val = *reinterpret_cast<const uint4*>(stg + row * 32 + hf * 16);
-                    *reinterpret_cast<uint4*>(hg + (size_t)row * 256 + vb * 2 + hf * 16) = val;
-                }
-                __syncwarp();
-            }
-            if (p.h32_out) {
-                // the same state in fp32 [128 k][128 v] for the backward pass
-                float* hg = p.h32_out + tile_idx * (size_t)(DK * DV);
-#pragma unroll
-                for (int jt = 0; jt < 16; ++jt) {
-                    int k0 = 8 * jt + 2 * t;
-                    hg[(size_t)k0 * DV + vb + g] = S[jt][0];
-                    hg[(size_t)(k0 + 1) * DV + vb + g] = S[jt][1];
-                    hg[(size_t)k0 * DV + vb + g + 8] = S[jt][2];
-                    hg[(size_t)(k0 + 1) * DV + vb + g + 8] = S[jt][3];
-                }
-            }
-        }
-
-        // ---- acc = S^T w^T : [16 v] x [64 tokens], contraction over 128 key channels ----
-        float acc[8][4];
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-#pragma unroll
-        for (int kp = 0; kp < 4; ++kp) {
-#pragma unroll
-            for (int nt = 0; nt < 8; ++nt) {
-                uint32_t b0, b1, b2, b3;
-                ldsm_x4(st + L::W + (8 * nt + r) * 256 + x256[kp], b0, b1, b2, b3);
-                mma_f16(acc[nt], sa[2 * kp], b0, b1);
-                mma_f16(acc[nt], sa[2 * kp + 1], b2, b3);
-            }
-        }
-        // ---- v_new^T = u^T - acc  (u = 0 for the transition matrix) ----
+    else if (warp >= SC_OUT_WARPS && warp < SC_OUT_WARPS + SC_STATE_WARPS) {
+        // ------------------------------- state: lane = value column v, 32 key channels per warp -------------------------------
+        const int q = warp & 3, kq = (warp - SC_OUT_WARPS) >> 2, v = 32 * q + lane, k0 = 32 * kq;
+        const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
+        float s[32];
         if (is_m) {
 #pragma unroll
-            for (int nt = 0; nt < 8; ++nt) {
-                acc[nt][0] *= -s_down; acc[nt][1] *= -s_down; acc[nt][2] *= -s_down; acc[nt][3] *= -s_down;
-            }
+            for (int k = 0; k < 32; ++k) s[k] = k0 + k == v ? 1.f : 0.f;
+        } else if (p.h0) {
+            const float* h0 = p.h0 + ((size_t)n * p.H + h) * DK * DV + (size_t)k0 * DV + v;
+#pragma unroll
+            for (int k = 0; k < 32; ++k) s[k] = h0[(size_t)k * DV];
         } else {
 #pragma unroll
-        for (int np = 0; np < 4; ++np) {
-            uint32_t r0, r1, r2, r3;
-            int row = 8 * (2 * np + (m >> 1)) + r, ch = 2 * pw + (m & 1);
-            ldsm_x4_t(st + L::U + (NVH == 2 ? vh * 8192 : 0) + row * 128 + ((ch ^ r) << 4), r0, r1, r2, r3);
-            float2 f;
-            f = unpack_f16(r0); acc[2 * np][0] = fmaf(-s_down, acc[2 * np][0], f.x); acc[2 * np][1] = fmaf(-s_down, acc[2 * np][1], f.y);
-            f = unpack_f16(r1); acc[2 * np][2] = fmaf(-s_down, acc[2 * np][2], f.x); acc[2 * np][3] = fmaf(-s_down, acc[2 * np][3], f.y);
-            f = unpack_f16(r2); acc[2 * np + 1][0] = fmaf(-s_down, acc[2 * np + 1][0], f.x); acc[2 * np + 1][1] = fmaf(-s_down, acc[2 * np + 1][1], f.y);
-            f = unpack_f16(r3); acc[2 * np + 1][2] = fmaf(-s_down, acc[2 * np + 1][2], f.x); acc[2 * np + 1][3] = fmaf(-s_down, acc[2 * np + 1][3], f.y);
+            for (int k = 0; k < 32; ++k) s[k] = 0.f;
         }
-        }
-        uint32_t va[4][4];   // v_new^T as fp16 A fragments (4 k-steps over the 64 tokens)
+        auto load_state = [&]() {
+            umma::ld_32x32b_x32(tl + TM_S32 + k0, reinterpret_cast<uint32_t(&)[32]>(s));
+            umma::wait_ld();
+        };
+        // Largest |entry| of the value column: this warp's quarter of the keys here, the others from the partner warps.
+        auto publish_max = [&](int c) -> float {
+            float m0 = 0.f, m1 = 0.f;
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-            va[ks][0] = pack_f16(acc[2 * ks][0], acc[2 * ks][1]);
-            va[ks][1] = pack_f16(acc[2 * ks][2], acc[2 * ks][3]);
-            va[ks][2] = pack_f16(acc[2 * ks + 1][0], acc[2 * ks + 1][1]);
-            va[ks][3] = pack_f16(acc[2 * ks + 1][2], acc[2 * ks + 1][3]);
-        }
-        if (STORE_HV) {
-            // v_new, fp16 [64 tokens][128 v]
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-                int trow = 8 * (2 * ks + (m >> 1)) + r;
-                stsm_x4_t(stg_u32 + trow * 32 + (m & 1) * 16, va[ks][0], va[ks][1], va[ks][2], va[ks][3]);
+            for (int k = 0; k < 32; k += 2) {
+                m0 = fmaxf(m0, fabsf(s[k]));
+                m1 = fmaxf(m1, fabsf(s[k + 1]));
             }
-            __syncwarp();
-            unsigned char* vg = reinterpret_cast<unsigned char*>(p.vnew_out) + tile_idx * (size_t)(BT * DV * 2);
-#pragma unroll
-            for (int it = 0; it < 4; ++it) {
-                int row = it * 16 + (lane >> 1), hf = lane & 1;
-                uint4 val = *reinterpret_cast<const uint4*>(stg + row * 32 + hf * 16);
-                *reinterpret_cast<uint4*>(vg + (size_t)row * 256 + vb * 2 + hf * 16) = val;
+            m0 = fmaxf(m0, m1);
+            sMax[(c & 1) * 512 + kq * 128 + v] = m0;
+            warp_arrive(&b_max[q], lane);
+            return m0;
+        };
+        bool ok = true;
+        if (nchunks > 0) publish_max(0);
+        for (int c = 0; c < nchunks; ++c) {
+            // The scale of the fp16 copy has to be known when the state arrives, not a reduction over it later. A bound is
+            // enough, fp16 being a floating-point format: |S_c| <= max |S_{c-1}| + sum |v_new| max |kg|, with decays <= 1 and
+            // |kg| <= 1 for unit keys (a factor of 32 is left for others); both terms are ready before the MMA that makes S_c is.
+            const int pc = max(c - 1, 0);
+            if (!(ok = wait(&b_max[q], pc))) break;
+            const float* mx = sMax + (pc & 1) * 512 + v;
+            float bound = fmaxf(fmaxf(mx[0], mx[128]), fmaxf(mx[256], mx[384]));
+            if (c > 0) {
+                if (!(ok = wait(b_vsum, c - 1))) break;
+                bound += sVsum[(pc & 1) * 256 + v] + sVsum[(pc & 1) * 256 + 128 + v];
             }
-            __syncwarp();
+            int shift = 10 - (((__float_as_int(bound) >> 23) & 0xff) - 127);
+            shift = max(-100, min(100, shift));
+            const float2 up = splat2(__int_as_float((shift + 127) << 23));
+            if (kq == 0) sDown[(c & 3) * 128 + v] = __int_as_float((127 - shift) << 23);
+            if (c > 0) {
+                if (!(ok = wait(b_s32, c - 1))) break;
+                umma::fence_after_sync();
+                load_state();
+            }
+            {
+                uint32_t pk[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    const float2 x = mul2(make_float2(s[2 * e], s[2 * e + 1]), up);
+                    pk[e] = pack_f16(x.x, x.y);
+                }
+                umma::st_32x32b_x16(tl + TM_S16 + 16 * kq, pk);
+            }
+            umma::wait_st();
+            umma::fence_before_sync();
+            warp_arrive(b_s16, lane);
+            // ---- beside the MMAs: the decayed state, then the state entering this chunk to HBM if asked for ----
+            const int st = c % SC_STAGES;
+            if (!(ok = wait(&full[st], c / SC_STAGES))) break;
+            const float* dec = reinterpret_cast<const float*>(sm + st * SC_STAGE_BYTES + ST_DECAY) + k0;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                uint32_t r[8];
+#pragma unroll
+                for (int e = 0; e < 8; e += 4) {
+                    const float4 d = *reinterpret_cast<const float4*>(dec + 8 * b + e);
+                    const float2 x = mul2(make_float2(s[8 * b + e], s[8 * b + e + 1]), make_float2(d.x, d.y));
+                    const float2 y = mul2(make_float2(s[8 * b + e + 2], s[8 * b + e + 3]), make_float2(d.z, d.w));
+                    r[e] = __float_as_uint(x.x); r[e + 1] = __float_as_uint(x.y); r[e + 2] = __float_as_uint(y.x); r[e + 3] = __float_as_uint(y.y);
+                }
+                umma::st_32x32b_x8(tl + TM_S32 + k0 + 8 * b, r);
+            }
+            warp_arrive(&empty[st], lane);
+            umma::wait_st();
+            umma::fence_before_sync();
+            warp_arrive(b_dec, lane);
+            // keys far from unit length can defeat the bound: say so instead of carrying inf on
+            if (c > 0 && publish_max(c) * up.x > 65504.f) report_status(p.status, STATUS_RANGE);
+            const size_t tile_idx = (size_t)(chunk0 + c) * p.H + h;
+            if (p.h32_out) {
+                float* hg = p.h32_out + tile_idx * (size_t)(DK * DV) + (size_t)k0 * DV + v;
+#pragma unroll
+                for (int k = 0; k < 32; ++k) hg[(size_t)k * DV] = s[k];
+            }
+            if (p.h_out) {
+                __nv_bfloat16* hg = reinterpret_cast<__nv_bfloat16*>(p.h_out) + tile_idx * (size_t)(DK * DV) + (size_t)k0 * DV + v;
+#pragma unroll
+                for (int k = 0; k < 32; ++k) hg[(size_t)k * DV] = __float2bfloat16_rn(s[k]);
+            }
         }
-
-        // ---- o^T = S^T qg^T + v_new^T Aqk^T (skipped when no output is wanted: backward recomputation) ----
-        if (!TRANSITION && (!STORE_HV || p.o != nullptr)) {
-            float oacc[8][4];
+        float* final_dst = is_m ? p.m_out : p.ht;
+        if (ok && nchunks > 0 && (ok = wait(b_s32, nchunks - 1))) {
+            umma::fence_after_sync();
+            load_state();
+        }
+        if (ok && final_dst) {
+            float* ht = final_dst + ((size_t)n * p.H + h) * DK * DV + (size_t)k0 * DV + v;
 #pragma unroll
-            for (int nt = 0; nt < 8; ++nt) oacc[nt][0] = oacc[nt][1] = oacc[nt][2] = oacc[nt][3] = 0.f;
+            for (int k = 0; k < 32; ++k) ht[(size_t)k * DV] = s[k];
+        }
+    } else if (warp >= SC_OUT_WARPS + SC_STATE_WARPS) {
+        // ------------------------------- v_new: lane = value column v, 32 tokens per warp -------------------------------
+        const int q = warp & 3, th = (warp - SC_OUT_WARPS - SC_STATE_WARPS) >> 2, v = 32 * q + lane, t0 = 32 * th;
+        const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
+        // u[token][v] of the pack: value halves of 128-byte token rows, 16-byte groups XOR-swizzled by the token
+        const int ub = ST_U + (v >> 6) * 8192 + (v & 7) * 2, uc = (v & 63) >> 3;
+        for (int c = 0; c < nchunks; ++c) {
+            const int st = c % SC_STAGES;
+            uint32_t u2[16];                          // this lane's u of 32 tokens, two per register
+            if (!is_m) {
+                if (!wait(&full[st], c / SC_STAGES)) break;
+                const unsigned char* us = sm + st * SC_STAGE_BYTES + ub;
 #pragma unroll
-            for (int kp = 0; kp < 4; ++kp) {
+                for (int e = 0; e < 16; ++e) {
+                    const uint32_t a = *reinterpret_cast<const uint16_t*>(us + (t0 + 2 * e) * 128 + ((uc ^ ((2 * e) & 7)) << 4));
+                    const uint32_t b = *reinterpret_cast<const uint16_t*>(us + (t0 + 2 * e + 1) * 128 + ((uc ^ ((2 * e + 1) & 7)) << 4));
+                    u2[e] = __byte_perm(a, b, 0x5410);
+                }
+                warp_arrive(&empty[st], lane);
+            } else {
 #pragma unroll
-                for (int nt = 0; nt < 8; ++nt) {
-                    uint32_t b0, b1, b2, b3;
-                    ldsm_x4(st + TP_QG + (8 * nt + r) * 256 + x256[kp], b0, b1, b2, b3);
-                    mma_f16(oacc[nt], sa[2 * kp], b0, b1);
-                    mma_f16(oacc[nt], sa[2 * kp + 1], b2, b3);
+                for (int e = 0; e < 16; ++e) u2[e] = 0;
+            }
+            if (!wait(b_s16, c) || !wait(b_acc, c)) break;
+            umma::fence_after_sync();
+            const uint32_t acc = tl + TM_ACC + 128 * (c & 1) + t0;
+            const float2 down = splat2(-sDown[(c & 3) * 128 + v]);
+            float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                uint32_t r[16], pk[8];
+                umma::ld_32x32b_x16(acc + 16 * b, r);
+                umma::wait_ld();
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float2 x = fma2(make_float2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])), down, unpack_f16(u2[8 * b + e]));
+                    pk[e] = pack_f16(x.x, x.y);
+                    sum.x += fabsf(x.x);
+                    sum.y += fabsf(x.y);
+                }
+                umma::st_32x32b_x8(acc + 8 * b, pk);      // columns this warp has already read
+            }
+            umma::wait_st();
+            umma::fence_before_sync();
+            warp_arrive(&b_v16[c & 1], lane);
+            sVsum[(c & 1) * 256 + th * 128 + v] = sum.x + sum.y;
+            warp_arrive(b_vsum, lane);
+        }
+    } else {
+        // ------------------------------- output rows (and v_new): lane = value column v, all tokens -------------------------------
+        const int q = warp, v = 32 * q + lane;
+        const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
+        const int odd = lane & 1;
+        const uint32_t sel = odd ? 0x3276u : 0x5410u;
+        // a register holds the 16-bit values of tokens 2e and 2e + 1 of this column; neighbouring lanes trade halves, so that the
+        // even lane stores token 2e of both columns and the odd lane token 2e + 1
+        auto stage = [&](unsigned char* buf, int t0, const uint32_t (&w)[8]) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const uint32_t x = __shfl_xor_sync(0xffffffffu, w[e], 1);
+                *reinterpret_cast<uint32_t*>(buf + (t0 + 2 * e + odd) * 256 + (v & ~1) * 2) = __byte_perm(w[e], x, sel);
+            }
+        };
+        int turns = 0;                               // staged matrices so far: the two buffers alternate
+        // All rows staged: thread 0 sends a whole matrix with one bulk copy (v_new, or a full chunk of o); a ragged last chunk
+        // goes out row by row. Passing the barrier of turn t also means that the copy of turn t - 1 has been read out.
+        auto turn_over = [&]() -> bool {
+            fence_proxy_async();
+            if (tid == 0) bulk_wait_read_all();
+            warp_arrive(b_ost, lane);
+            return wait(b_ost, turns++);
+        };
+        for (int c = 0; want_out && c < nchunks; ++c) {
+            const uint32_t acc = tl + TM_ACC + 128 * (c & 1);
+            if (p.vnew_out) {
+                if (!wait(&b_v16[c & 1], c >> 1)) break;
+                umma::fence_after_sync();
+                unsigned char* buf = sm + SC_OST + (turns & 1) * OST_BYTES;
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    uint32_t w[8];
+                    umma::ld_32x32b_x8(acc + 32 * (b >> 1) + 8 * (b & 1), w);
+                    umma::wait_ld();
+                    stage(buf, 16 * b, w);
+                }
+                if (!want_o) {
+                    umma::fence_before_sync();
+                    warp_arrive(&b_oread[c & 1], lane);
+                }
+                if (!turn_over()) break;
+                if (tid == 0) {
+                    bulk_s2g(reinterpret_cast<unsigned char*>(p.vnew_out) + ((size_t)(chunk0 + c) * p.H + h) * (size_t)(BT * DV * 2), buf, OST_BYTES);
+                    bulk_commit();
                 }
             }
+            if (want_o) {
+                if (!wait(b_o, c)) break;
+                umma::fence_after_sync();
+                const float2 down = splat2(sDown[(c & 3) * 128 + v]);
+                unsigned char* buf = sm + SC_OST + (turns & 1) * OST_BYTES;
 #pragma unroll
-            for (int nt = 0; nt < 8; ++nt) {
-                oacc[nt][0] *= s_down; oacc[nt][1] *= s_down; oacc[nt][2] *= s_down; oacc[nt][3] *= s_down;
-            }
-#pragma unroll
-            for (int nt = 0; nt < 8; ++nt) {
-#pragma unroll
-                for (int ksp = 0; ksp < 2; ++ksp) {
-                    if (32 * ksp <= 8 * nt + 7) {      // causal: skip column blocks right of the diagonal
-                        uint32_t b0, b1, b2, b3;
-                        ldsm_x4(st + TP_AQK + (8 * nt + r) * 128 + (((4 * ksp + m) ^ r) << 4), b0, b1, b2, b3);
-                        mma_f16(oacc[nt], va[2 * ksp], b0, b1);
-                        if (32 * ksp + 16 <= 8 * nt + 7) mma_f16(oacc[nt], va[2 * ksp + 1], b2, b3);
+                for (int b = 0; b < 4; ++b) {
+                    uint32_t r[16], r2[16], w[8];
+                    umma::ld_32x32b_x16(acc + TM_QG + 16 * b, r);
+                    umma::ld_32x32b_x16(tl + TM_O2 + 16 * b, r2);
+                    umma::wait_ld();
+                    if (b == 3) {
+                        umma::fence_before_sync();
+                        warp_arrive(&b_oread[c & 1], lane);
                     }
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const float2 o = fma2(make_float2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])), down,
+                                              make_float2(__uint_as_float(r2[2 * e]), __uint_as_float(r2[2 * e + 1])));
+                        w[e] = pack_bf16(o.x, o.y);
+                    }
+                    stage(buf, 16 * b, w);
                 }
-            }
-#pragma unroll
-            for (int np = 0; np < 4; ++np) {
-                int trow = 8 * (2 * np + (m >> 1)) + r;
-                stsm_x4_t(stg_u32 + trow * 32 + (m & 1) * 16,
-                          pack_bf16(oacc[2 * np][0], oacc[2 * np][1]), pack_bf16(oacc[2 * np][2], oacc[2 * np][3]),
-                          pack_bf16(oacc[2 * np + 1][0], oacc[2 * np + 1][1]), pack_bf16(oacc[2 * np + 1][2], oacc[2 * np + 1][3]));
-            }
-            __syncwarp();
-            unsigned char* og = reinterpret_cast<unsigned char*>(p.o) +
-                                ((size_t)(bos + c * BT) * p.H + h) * (size_t)(DV * 2) + vb * 2;
-#pragma unroll
-            for (int it = 0; it < 4; ++it) {
-                int row = it * 16 + (lane >> 1), hf = lane & 1;
-                if (row < valid) {
-                    uint4 val = *reinterpret_cast<const uint4*>(stg + row * 32 + hf * 16);
-                    *reinterpret_cast<uint4*>(og + (size_t)row * p.H * (DV * 2) + hf * 16) = val;
-                }
-            }
-            __syncwarp();
-        }
-
-        // ---- S^T <- S^T diag(decay) + v_new^T kg ----
-        {
-            const float* dec = reinterpret_cast<const float*>(smem + s * L::STAGE_BYTES + L::DECAY);
-#pragma unroll
-            for (int jt = 0; jt < 16; ++jt) {
-                float2 d2 = *reinterpret_cast<const float2*>(dec + 8 * jt + 2 * t);
-                S[jt][0] *= d2.x; S[jt][1] *= d2.y; S[jt][2] *= d2.x; S[jt][3] *= d2.y;
-            }
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-#pragma unroll
-                for (int jp = 0; jp < 8; ++jp) {
-                    uint32_t b0, b1, b2, b3;
-                    int row = 16 * ks + (m & 1) * 8 + r, ch = 2 * jp + (m >> 1);
-                    ldsm_x4_t(st + L::KG + row * 256 + ((ch ^ r) << 4), b0, b1, b2, b3);
-                    mma_f16(S[2 * jp], va[ks], b0, b1);
-                    mma_f16(S[2 * jp + 1], va[ks], b2, b3);
+                if (!turn_over()) break;
+                const int rows = min(BT, len - c * BT);
+                if (rows == BT) {
+                    if (tid == 0) {
+                        tma_store_rows(&map_o, smem_u32(buf), h, bos + c * BT);
+                        bulk_commit();
+                    }
+                } else {
+                    for (int row = tid >> 4; row < rows; row += 8)
+                        *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(p.o) + ((size_t)(bos + c * BT + row) * p.H + h) * (DV * 2) + (tid & 15) * 16) =
+                            *reinterpret_cast<const uint4*>(buf + row * 256 + (tid & 15) * 16);
                 }
             }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[s]);
+        if (tid == 0) bulk_wait_all();
     }
-
-    float* final_dst = is_m ? p.m_out : p.ht;
-    if (final_dst) {
-        float* ht = final_dst + ((size_t)n * p.H + h) * DK * DV;
-#pragma unroll
-        for (int jt = 0; jt < 16; ++jt) {
-            int k0 = 8 * jt + 2 * t;
-            ht[(size_t)k0 * DV + vb + g] = S[jt][0];
-            ht[(size_t)(k0 + 1) * DV + vb + g] = S[jt][1];
-            ht[(size_t)k0 * DV + vb + g + 8] = S[jt][2];
-            ht[(size_t)(k0 + 1) * DV + vb + g + 8] = S[jt][3];
-        }
-    }
+    __syncthreads();
+    if (warp == SC_MMA_WARP) umma::tmem_dealloc(tmem, 512);
 }
 
 }  // namespace kda
 
-extern "C" int kda_fwd_scan_smem_bytes() { return kda::SCAN_SMEM; }
+extern "C" int kda_fwd_scan_smem_bytes() { return kda::SC_SMEM; }
 
 namespace {
-// Launch with programmatic stream serialization: the grid may be scheduled while the previous kernel of the stream (the
-// chunk-parallel stage) is still draining; every thread calls pdl_wait() before it reads anything.
-template <typename Kernel>
-cudaError_t launch_after_producer(Kernel kernel, dim3 grid, int threads, int smem, cudaStream_t stream, const kda::ScanParams& p) {
+// W, QG and KG of the tile packs as a rank-4 tensor of fp16: 64 channels, 2 channel halves, 192 rows (64 of each matrix),
+// tiles; fetched as boxes of 64 channels x 64 rows.
+bool make_pack_map(CUtensorMap* map, const unsigned char* tiles, long long num_tiles) {
+    kda::EncodeTiledFn fn = kda::encode_tiled_fn();
+    if (!fn) return false;
+    static_assert(kda::TP_W == 0 && kda::TP_QG == 16384 && kda::TP_KG == 32768 && kda::TP_BYTES % 16 == 0, "three stacked matrices of 256-byte rows");
+    const cuuint64_t dims[4] = {64, 2, 192, (cuuint64_t)num_tiles};
+    const cuuint64_t strides[3] = {128, 256, kda::TP_BYTES};
+    const cuuint32_t box[4] = {64, 1, 64, 1}, elem[4] = {1, 1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<unsigned char*>(tiles), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// o as [tokens][heads][128], stored as boxes of 64 tokens of one head
+bool make_out_map(CUtensorMap* map, void* o, int H) {
+    kda::EncodeTiledFn fn = kda::encode_tiled_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[3] = {128, (cuuint64_t)H, 1ull << 30};
+    const cuuint64_t strides[2] = {256, (cuuint64_t)H * 256};
+    const cuuint32_t box[3] = {128, 1, 64}, elem[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, o, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+              CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+int launch_scan(const kda::ScanParams* p, int groups, cudaStream_t stream) {
+    using namespace kda;
+    if (p->N <= 0) return 0;
+    static std::atomic<unsigned long long> done;
+    cudaError_t e = allow_smem(kda_fwd_scan_kernel, SC_SMEM, done);
+    if (e != cudaSuccess) return (int)e;
+    CUtensorMap map, map_o = {};
+    // the numbers of tiles and tokens are not known here for a packed batch; the kernel's coordinates stay inside the caller's tensors
+    if (!make_pack_map(&map, p->tiles, 1ll << 24) || (p->o && !make_out_map(&map_o, p->o, p->H))) return (int)cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.gridDim = dim3(p->H, p->N, groups);
+    cfg.blockDim = dim3(SC_THREADS);
+    cfg.dynamicSmemBytes = SC_SMEM;
     cfg.stream = stream;
+    // Programmatic stream serialization: the grid may be scheduled while the previous kernel of the stream (the
+    // chunk-parallel stage) is still draining; every thread calls pdl_wait() before it reads anything.
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, p);
+    e = cudaLaunchKernelEx(&cfg, kda_fwd_scan_kernel, *p, map, map_o);
+    if (e != cudaSuccess) return (int)e;
+    return (int)cudaGetLastError();
 }
 }  // namespace
 
-extern "C" int kda_launch_fwd_scan(const kda::ScanParams* p, cudaStream_t stream) {
-    using namespace kda;
-    if (p->N <= 0) return 0;
-    dim3 grid(2, p->H, p->N);
-    cudaError_t e;
-    const int sms = sm_count();
-    const bool both_halves = 2LL * p->H * p->N > sms;      // more half-state CTAs than SMs: eight consumer warps per CTA
-    using L2 = ScanLayout<false, 2>;
-    if (p->vnew_out) {
-        if (both_halves) {
-            static std::atomic<unsigned long long> done;
-            e = allow_smem(kda_fwd_scan_kernel<true, false, 2>, L2::SMEM, done);
-            if (e != cudaSuccess) return (int)e;
-            kda_fwd_scan_kernel<true, false, 2><<<dim3(1, p->H, p->N), (L2::CONSUMERS + 1) * 32, L2::SMEM, stream>>>(*p);
-        } else {
-            static std::atomic<unsigned long long> done2;
-            e = allow_smem(kda_fwd_scan_kernel<true, false>, SCAN_SMEM, done2);
-            if (e != cudaSuccess) return (int)e;
-            kda_fwd_scan_kernel<true, false><<<grid, SCAN_THREADS, SCAN_SMEM, stream>>>(*p);
-        }
-    } else {
-        if (both_halves) {
-            static std::atomic<unsigned long long> done3;
-            e = allow_smem(kda_fwd_scan_kernel<false, false, 2>, L2::SMEM, done3);
-            if (e != cudaSuccess) return (int)e;
-            e = launch_after_producer(kda_fwd_scan_kernel<false, false, 2>, dim3(1, p->H, p->N), (L2::CONSUMERS + 1) * 32, L2::SMEM, stream, *p);
-            if (e != cudaSuccess) return (int)e;
-        } else {
-            static std::atomic<unsigned long long> done4;
-            e = allow_smem(kda_fwd_scan_kernel<false, false>, SCAN_SMEM, done4);
-            if (e != cudaSuccess) return (int)e;
-            e = launch_after_producer(kda_fwd_scan_kernel<false, false>, grid, SCAN_THREADS, SCAN_SMEM, stream, *p);
-            if (e != cudaSuccess) return (int)e;
-        }
-    }
-    return (int)cudaGetLastError();
-}
+extern "C" int kda_launch_fwd_scan(const kda::ScanParams* p, cudaStream_t stream) { return launch_scan(p, 1, stream); }
 
 // Affine shard transitions of every (sequence, head): p->ht receives C, p->m_out receives M; p->o / p->h0 unused.
-extern "C" int kda_launch_fwd_transition(const kda::ScanParams* p, cudaStream_t stream) {
-    using namespace kda;
-    if (p->N <= 0) return 0;
-    const int sms = sm_count();
-    ScanParams q = *p;
-    q.group_major = 4LL * p->H * p->N > sms;     // see the index mapping at the top of the kernel
-    const dim3 grid = q.group_major ? dim3(p->H, p->N, 4) : dim3(4, p->H, p->N);
-    constexpr int smem = ScanLayout<true, 1>::SMEM;
-    static std::atomic<unsigned long long> done5;
-    cudaError_t e = allow_smem(kda_fwd_scan_kernel<false, true>, smem, done5);
-    if (e != cudaSuccess) return (int)e;
-    kda_fwd_scan_kernel<false, true><<<grid, SCAN_THREADS, smem, stream>>>(q);
-    return (int)cudaGetLastError();
-}
+extern "C" int kda_launch_fwd_transition(const kda::ScanParams* p, cudaStream_t stream) { return launch_scan(p, 2, stream); }

@@ -58,7 +58,7 @@ def _tables(cu_seqlens, cu_seqlens_cpu):
 
 def _segments(q):
     """One long sequence: few scan CTAs, many dependent steps -> the pieces its scan is cut into (see `cp.auto_segments`)."""
-    if q.dim() != 4 or q.shape[0] != 1 or q.shape[1] < 512 * CHUNK or not q.is_cuda:
+    if q.dim() != 4 or q.shape[0] != 1 or q.shape[1] < 4096 or not q.is_cuda:      # cheap first look; `auto_segments` decides
         return None
     from .cp import auto_segments, segment_bounds, segment_tables
     num_chunks = (q.shape[1] + CHUNK - 1) // CHUNK

@@ -175,24 +175,25 @@ class CudaBackend:
 
 
 _SM_COUNT: dict = {}
-MAX_AUTO_SEGMENTS = 4       # upper bound of `auto_segments`; 1 switches the single-GPU segmentation off
+MAX_AUTO_SEGMENTS = 8       # upper bound of `auto_segments`; 1 switches the single-GPU segmentation off
+AUTO_SEGMENT_CHUNKS = 128   # shortest sequence, in chunks, that `auto_segments` cuts
 
 
 def auto_segments(num_chunks, heads, device):
     """How many side-by-side segments the scan of ONE long sequence should be cut into on a single GPU: the scan is
-    a chain of ``num_chunks`` dependent steps that occupies only ``2 * heads`` CTAs, so while SMs are idle a second
-    pass pays for itself -- a transition scan per segment (cheaper: no output products), a fold, and then all
-    segments scanned side by side from their now-known incoming states. Per chunk the two passes cost about
-    (0.9 + 1.7) / P microseconds against 1.7 for the plain scan; below a few hundred chunks the extra launches eat
-    the gain. The role of the intra-card mode of flash-linear-attention's merge kernel
+    a chain of ``num_chunks`` dependent steps that occupies only ``heads`` CTAs, so while SMs are idle a second
+    pass pays for itself -- a transition scan of all segments but the last (two CTAs per segment and head), a fold per
+    boundary, and then all segments scanned side by side from their now-known incoming states. Both passes cost about
+    the same per chunk, so that three segments are the least that gains; all CTAs of a pass have to find an SM of their
+    own; and below some hundred chunks the extra launches eat the gain (a step is about 1.6 us, a fold and its launch
+    8 us). The role of the intra-card mode of flash-linear-attention's merge kernel
     (fla/ops/cp/chunk_delta_h.py:321-357)."""
     key = str(device)
     if key not in _SM_COUNT:
         _SM_COUNT[key] = torch.cuda.get_device_properties(device).multi_processor_count
-    fit = _SM_COUNT[key] // (2 * heads)          # segments whose four-warp scan CTAs all find an SM
-    if num_chunks < 512 or fit < 2:
-        return 1
-    return max(1, min(MAX_AUTO_SEGMENTS, fit))
+    sms = _SM_COUNT[key]
+    P = min(MAX_AUTO_SEGMENTS, sms // (2 * heads) + 1, sms // heads, num_chunks // 64)
+    return P if P >= 3 and num_chunks >= AUTO_SEGMENT_CHUNKS else 1
 
 
 def gather_with_group(group=None):
