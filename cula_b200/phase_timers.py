@@ -28,8 +28,10 @@ DENSE_PHASES = ["half 0: operands widened into smem", "-",
                 "half 1: operands widened into smem", "-", "half 1: wait for the states (TMA)",
                 "half 1: MMA issue", "half 1: next tile's operands requested", "half 1: wait for the MMAs", "dQg, dW staged, stores issued",
                 "dKg, dPs, dAu staged, dv stored", "store read-out + end-of-tile barrier"]
-BWD_PHASES = ["loads, gate, norms", "cumulative sum", "stage dW, X", "dA", "T1, dL", "Zw + accumulator set-up", "L2 hints",
-              "Gram VJP, row side", "Gram VJP, column side", "reverse cumulative sum", "gate VJP, dg", "L2-norm VJP, stores"]
+BWD_PHASES = [f"{g}: {n}" for g, names in (
+    ("rows", ("inputs landed", "norms, coefficients, gates", "X", "dA", "Zw", "wait for the columns", "row side", "wait, end of the tile")),
+    ("columns", ("inputs landed", "norms, coefficients, gates", "X", "dA", "T1, dL", "wait for the rows", "column side", "wait, end of the tile")))
+    for n in names]
 
 
 def main():
