@@ -68,14 +68,18 @@ constexpr int BG_SMEM = BG_MISC + 1024;
 __device__ __forceinline__ float bg_tf32(float x) {
     return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
 }
-__device__ __forceinline__ float bg_tf32_lo(float x) {      // the low part of a split: truncation is enough (error 2^-21 of the value)
-    return __uint_as_float(__float_as_uint(x) & 0xffffe000u);
-}
 __device__ __forceinline__ void bg_mma(float (&d)[4], const float (&a)[4], float b0, float b1) {
     asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                  : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
                    "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+}
+// the same with a zero accumulator input
+__device__ __forceinline__ void bg_mma0(float (&d)[4], const float (&a)[4], float b0, float b1) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+                 : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
+                   "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)), "f"(0.f));
 }
 __device__ __forceinline__ void bg_cp16(uint32_t smem_dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(smem_dst), "l"(src) : "memory");
@@ -175,6 +179,12 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
     auto ldsm_b = [&](int base, int row0, int ks, float (&f)[4]) {      // f[0..1]: rows row0.., f[2..3]: rows row0 + 8..
         const int row = row0 + lr + 8 * (lm >> 1), ch = 2 * ks + (lm & 1);
         ldsm_x4(smu + base + (ch >> 3) * 8192 + row * 128 + (((ch & 7) ^ (row & 7)) << 4), reinterpret_cast<uint32_t&>(f[0]),
+                reinterpret_cast<uint32_t&>(f[1]), reinterpret_cast<uint32_t&>(f[2]), reinterpret_cast<uint32_t&>(f[3]));
+    };
+    // the same B fragments by address: lane part, 16-row block and 8-column group (the XOR with the group touches two bits only)
+    const uint32_t lane_b = (uint32_t)((lr + 8 * (lm >> 1)) * 128 + (((lm & 1) ^ lr) << 4));
+    auto ldsm_blk = [&](int base, int blk, int n, float (&f)[4]) {
+        ldsm_x4(smu + base + blk * 2048 + (n >> 2) * 8192 + (lane_b ^ (uint32_t)((n & 3) << 5)), reinterpret_cast<uint32_t&>(f[0]),
                 reinterpret_cast<uint32_t&>(f[1]), reinterpret_cast<uint32_t&>(f[2]), reinterpret_cast<uint32_t&>(f[3]));
     };
     // 16 tokens (block b) of a bf16 array: r[h][x] = the pair of tokens a, b of 8-token group 2 b + h, channel ch0 + 8 x
@@ -577,187 +587,172 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
     // split an A fragment {(ch0, a), (ch0, b), (ch0 + 8, a), (ch0 + 8, b)} into tf32 high and low parts, in fragment order. Every
     // pair (i, j) adds +x to the gate gradient of row i and -x to that of row j through two different products; the reverse
     // cumulative sum relies on those two cancelling, so they must agree far better than tf32
+    // (the tensor core reads the upper 19 bits: high part = the value, truncated; low part = what that leaves, exact, then rounded)
     auto split = [&](const float (&v)[4], float (&hi)[4], float (&lo)[4]) {
         const float o[4] = {v[0], v[2], v[1], v[3]};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            hi[e] = bg_tf32(o[e]);
-            lo[e] = bg_tf32_lo(o[e] - hi[e]);
+            hi[e] = o[e];
+            lo[e] = __uint_as_float(__float_as_uint(o[e] - __uint_as_float(__float_as_uint(o[e]) & 0xffffe000u)) + 0x1000u);
         }
     };
-    // The two sides of the Gram VJPs are rolled loops over block pairs with their per-token values in slots: unrolled, with
-    // everything in registers, they were 100 KB of code that every warp ran once per tile, and instruction fetch was the limit.
+    // The factor 2^(r_I - r_{J+1}) of a pair of blocks belongs to the channel, which is the row of these products: it scales the
+    // 16x16 result of the pair, so that the operands of a block are made once and used against every other block.
     if (!col_group) {
-        // ---- 5a. row side: rows of block I against columns of the blocks J <= I ----
-        float nxt[8];
-        auto fetch = [&](int I) {
+        // ---- 5a. row side: columns of block J against rows of the blocks I >= J ----
+        float accP[8][4];
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh)
+        for (int n = 0; n < 8; ++n) {
+            const float gr[2] = {fast_exp2(rt[(n >> 1) * DK + ch0]), fast_exp2(rt[(n >> 1) * DK + ch0 + 8])};
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    nxt[4 * hh + e] = scr[SCR_DQG + (16 * I + 8 * hh + 2 * t4 + (e & 1)) * DK + ch0 + 8 * (e >> 1)];
-        };
-        fetch(0);
-        bg_bar(1);         // the partial sums have been read: Zw goes to its slots
+            for (int e = 0; e < 4; ++e) accP[n][e] = gr[e >> 1] * scr[SCR_DQG + (8 * n + 2 * t4 + (e & 1)) * DK + ch0 + 8 * (e >> 1)];
+        }
 #pragma unroll
-        for (int n = 0; n < 8; ++n) *slot(BG_C1, BG_X2, n) = make_float4(zw[n][0], zw[n][1], zw[n][2], zw[n][3]);
-#pragma unroll 1
-        for (int I = 0; I < 4; ++I) {
-            const float rI[2] = {rt[I * DK + ch0], rt[I * DK + ch0 + 8]};
-            float accP[2][4], accR[2][4];
-            {
-                const float gr[2] = {fast_exp2(rI[0]), fast_exp2(rI[1])};
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const float4 z = *slot(BG_C1, BG_X2, 2 * I + hh);
-                    accR[hh][0] = z.x; accR[hh][1] = z.y; accR[hh][2] = z.z; accR[hh][3] = z.w;
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) accP[hh][e] = gr[e >> 1] * nxt[4 * hh + e];
-                }
-            }
-            if (I < 3) fetch(I + 1);
-#pragma unroll 1
-            for (int J = 0; J <= I; ++J) {
-                const bool diag = J == I;
-                uint32_t kr[2][2];
-                load_raw(BG_K, J, kr);
-                // column factor: 2^(r_{J+1} - g_j) 2^(r_I - r_{J+1}), merged to 2^(r_I - g_j) inside the diagonal block
-                float a[2], cji[2];
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    const float rJ = rt[J * DK + ch0 + 8 * x], rN = rt[(J + 1) * DK + ch0 + 8 * x];
-                    a[x] = diag ? 0.f : rN - rJ;
-                    cji[x] = diag ? 1.f : fast_exp2(rI[x] - rN);
-                }
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int n = 2 * J + hh;
-                    float fP[4], fR[4], v[4], hi[4], lo[4];
-                    ldsm_b(BG_PN, 16 * I, n, fP);
-                    ldsm_b(BG_C2, 16 * I, n, fR);
-                    const float4 g4 = *slot(BG_G, BG_G + 16384, n);
-                    const float gn[4] = {g4.x, g4.y, g4.z, g4.w};
-                    const float2 rk = *reinterpret_cast<const float2*>(rstd_k + 8 * n + 2 * t4);
-#pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        const float2 kk = mul2(unpack_bf16(kr[hh][x]), mul2(rk, splat2(cji[x])));
-                        v[2 * x] = kk.x * fast_exp2(fminf(a[x] - gn[2 * x], 120.f));
-                        v[2 * x + 1] = kk.y * fast_exp2(fminf(a[x] - gn[2 * x + 1], 120.f));
-                    }
-                    split(v, hi, lo);
-                    bg_mma(accP[0], lo, fP[0], fP[1]);
-                    bg_mma(accP[1], lo, fP[2], fP[3]);
-                    bg_mma(accR[0], lo, fR[0], fR[1]);
-                    bg_mma(accR[1], lo, fR[2], fR[3]);
-                    bg_mma(accP[0], hi, fP[0], fP[1]);
-                    bg_mma(accP[1], hi, fP[2], fP[3]);
-                    bg_mma(accR[0], hi, fR[0], fR[1]);
-                    bg_mma(accR[1], hi, fR[2], fR[3]);
-                }
-            }
+        for (int J = 0; J < 4; ++J) {
+            uint32_t kr[2][2];
+            load_raw(BG_K, J, kr);
+            const float rN[2] = {rt[(J + 1) * DK + ch0], rt[(J + 1) * DK + ch0 + 8]};
+            const float d[2] = {rN[0] - rt[J * DK + ch0], rN[1] - rt[J * DK + ch0 + 8]};
+            float hi[2][4], lo[2][4];
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
-                const int n = 2 * I + hh;
-                const float4 g4 = *slot(BG_G, BG_G + 16384, n);
-                const float f[4] = {fast_exp2(g4.x), fast_exp2(g4.y), fast_exp2(g4.z), fast_exp2(g4.w)};
-                *slot(BG_DW, BG_DW + 16384, n) = make_float4(p.scale * f[0] * accP[hh][0], p.scale * f[1] * accP[hh][1],
-                                                             p.scale * f[2] * accP[hh][2], p.scale * f[3] * accP[hh][3]);
-                *slot(BG_C1, BG_X2, n) = make_float4(f[0] * accR[hh][0], f[1] * accR[hh][1], f[2] * accR[hh][2], f[3] * accR[hh][3]);
+                const float4 g4 = *slot(BG_G, BG_G + 16384, 2 * J + hh);
+                const float2 rk = *reinterpret_cast<const float2*>(rstd_k + 16 * J + 8 * hh + 2 * t4);
+                const float2 k0 = mul2(unpack_bf16(kr[hh][0]), rk), k1 = mul2(unpack_bf16(kr[hh][1]), rk);
+                const float v[4] = {k0.x * fast_exp2(d[0] - g4.x), k0.y * fast_exp2(d[0] - g4.y), k1.x * fast_exp2(d[1] - g4.z), k1.y * fast_exp2(d[1] - g4.w)};
+                split(v, hi[hh], lo[hh]);
             }
+#pragma unroll
+            for (int I = J; I < 4; ++I) {
+                float bP[2][4], bR[2][4], f[4];
+                ldsm_blk(BG_PN, I, 2 * J, f);
+                bg_mma0(bP[0], lo[0], f[0], f[1]);
+                bg_mma0(bP[1], lo[0], f[2], f[3]);
+                bg_mma(bP[0], hi[0], f[0], f[1]);
+                bg_mma(bP[1], hi[0], f[2], f[3]);
+                ldsm_blk(BG_C2, I, 2 * J, f);
+                bg_mma0(bR[0], lo[0], f[0], f[1]);
+                bg_mma0(bR[1], lo[0], f[2], f[3]);
+                bg_mma(bR[0], hi[0], f[0], f[1]);
+                bg_mma(bR[1], hi[0], f[2], f[3]);
+                ldsm_blk(BG_PN, I, 2 * J + 1, f);
+                bg_mma(bP[0], lo[1], f[0], f[1]);
+                bg_mma(bP[1], lo[1], f[2], f[3]);
+                bg_mma(bP[0], hi[1], f[0], f[1]);
+                bg_mma(bP[1], hi[1], f[2], f[3]);
+                ldsm_blk(BG_C2, I, 2 * J + 1, f);
+                bg_mma(bR[0], lo[1], f[0], f[1]);
+                bg_mma(bR[1], lo[1], f[2], f[3]);
+                bg_mma(bR[0], hi[1], f[0], f[1]);
+                bg_mma(bR[1], hi[1], f[2], f[3]);
+                float cji[2] = {1.f, 1.f};
+                if (I != J + 1) {
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) cji[x] = fast_exp2(fminf(rt[I * DK + ch0 + 8 * x] - rN[x], 126.f));
+                }
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        accP[2 * I + hh][e] = fmaf(cji[e >> 1], bP[hh][e], accP[2 * I + hh][e]);
+                        zw[2 * I + hh][e] = fmaf(cji[e >> 1], bR[hh][e], zw[2 * I + hh][e]);
+                    }
+            }
+        }
+        bg_bar(1);         // the partial sums have been read: their space takes a half of the results
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            const float4 g4 = *slot(BG_G, BG_G + 16384, n);
+            const float f[4] = {fast_exp2(g4.x), fast_exp2(g4.y), fast_exp2(g4.z), fast_exp2(g4.w)};
+            *slot(BG_DW, BG_DW + 16384, n) = make_float4(p.scale * f[0] * accP[n][0], p.scale * f[1] * accP[n][1], p.scale * f[2] * accP[n][2],
+                                                         p.scale * f[3] * accP[n][3]);
+            *slot(BG_C1, BG_X2, n) = make_float4(f[0] * zw[n][0], f[1] * zw[n][1], f[2] * zw[n][2], f[3] * zw[n][3]);
         }
         BG_MARK(6);   // row side
     }
     float cs[2] = {0.f, 0.f};      // column group: sum over the tokens of dKg * Kg, the gradient that reaches g_last through kg
     if (col_group) {
-        // ---- 5b. column side: columns of block J against rows of the blocks I >= J ----
-        float nxt[8];
-        auto fetch = [&](int J) {
+        // ---- 5b. column side: rows of block I against columns of the blocks J <= I ----
+        float acc[8][4];
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh)
+        for (int n = 0; n < 8; ++n)
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    nxt[4 * hh + e] = scr[SCR_DKG + (16 * J + 8 * hh + 2 * t4 + (e & 1)) * DK + ch0 + 8 * (e >> 1)];
-        };
-        fetch(0);
-#pragma unroll 1
+            for (int e = 0; e < 4; ++e) acc[n][e] = scr[SCR_DKG + (8 * n + 2 * t4 + (e & 1)) * DK + ch0 + 8 * (e >> 1)];
+#pragma unroll
         for (int J = 0; J < 4; ++J) {
-            float acc[2][4], rN[2], dJ[2];
-#pragma unroll
-            for (int x = 0; x < 2; ++x) {
-                rN[x] = rt[(J + 1) * DK + ch0 + 8 * x];
-                dJ[x] = rN[x] - rt[J * DK + ch0 + 8 * x];
-            }
-            {
-                const float gl[2] = {fast_exp2(glast[0] - rN[0]), fast_exp2(glast[1] - rN[1])};
-                uint32_t kr[2][2];
-                load_raw(BG_K, J, kr);
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int n = 2 * J + hh;
-                    const float4 g4 = *slot(BG_G, BG_G + 16384, n);
-                    const float gn[4] = {g4.x, g4.y, g4.z, g4.w};
-                    const float2 rk = *reinterpret_cast<const float2*>(rstd_k + 8 * n + 2 * t4);
-#pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        const float2 kh = mul2(unpack_bf16(kr[hh][x]), rk);
-                        acc[hh][2 * x] = gl[x] * nxt[4 * hh + 2 * x];
-                        acc[hh][2 * x + 1] = gl[x] * nxt[4 * hh + 2 * x + 1];
-                        cs[x] = fmaf(kh.x * fast_exp2(dJ[x] - gn[2 * x]), acc[hh][2 * x], cs[x]);
-                        cs[x] = fmaf(kh.y * fast_exp2(dJ[x] - gn[2 * x + 1]), acc[hh][2 * x + 1], cs[x]);
-                    }
-                }
-            }
-            if (J < 3) fetch(J + 1);
-#pragma unroll 1
-            for (int I = J; I < 4; ++I) {
-                const bool diag = J == I;
-                uint32_t qr[2][2], kr[2][2];
-                load_raw(BG_Q, I, qr);
-                load_raw(BG_K, I, kr);
-                // row factor: 2^(g_i - r_I) 2^(r_I - r_{J+1}), merged to 2^(g_i - r_{J+1}) inside the diagonal block
-                float a[2], cji[2];
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    a[x] = diag ? dJ[x] : 0.f;
-                    cji[x] = diag ? 1.f : fast_exp2(rt[I * DK + ch0 + 8 * x] - rN[x]);
-                }
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int n = 2 * I + hh, tok = 8 * n + 2 * t4;
-                    float fP[4], fR[4], vq[4], vk[4], hi[4], lo[4];
-                    ldsm_b(BG_PT, 16 * J, n, fP);
-                    ldsm_b(BG_X, 16 * J, n, fR);
-                    const float4 g4 = *slot(BG_G, BG_G + 16384, n);
-                    const float gn[4] = {g4.x, g4.y, g4.z, g4.w};
-                    const float2 rq = mul2(*reinterpret_cast<const float2*>(rstd_q + tok), splat2(p.scale)),
-                                 rk = *reinterpret_cast<const float2*>(rstd_k + tok);
-#pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        const float2 f = mul2(make_float2(fast_exp2(fminf(gn[2 * x] - a[x], 120.f)), fast_exp2(fminf(gn[2 * x + 1] - a[x], 120.f))),
-                                              splat2(cji[x]));
-                        const float2 tq = mul2(mul2(unpack_bf16(qr[hh][x]), rq), f), tk = mul2(mul2(unpack_bf16(kr[hh][x]), rk), f);
-                        vq[2 * x] = tq.x; vq[2 * x + 1] = tq.y;
-                        vk[2 * x] = tk.x; vk[2 * x + 1] = tk.y;
-                    }
-                    split(vq, hi, lo);
-                    bg_mma(acc[0], lo, fP[0], fP[1]);
-                    bg_mma(acc[1], lo, fP[2], fP[3]);
-                    bg_mma(acc[0], hi, fP[0], fP[1]);
-                    bg_mma(acc[1], hi, fP[2], fP[3]);
-                    split(vk, hi, lo);
-                    bg_mma(acc[0], lo, fR[0], fR[1]);
-                    bg_mma(acc[1], lo, fR[2], fR[3]);
-                    bg_mma(acc[0], hi, fR[0], fR[1]);
-                    bg_mma(acc[1], hi, fR[2], fR[3]);
-                }
-            }
+            uint32_t kr[2][2];
+            load_raw(BG_K, J, kr);
+            const float rN[2] = {rt[(J + 1) * DK + ch0], rt[(J + 1) * DK + ch0 + 8]};
+            const float d[2] = {rN[0] - rt[J * DK + ch0], rN[1] - rt[J * DK + ch0 + 8]};
+            const float gl[2] = {fast_exp2(glast[0] - rN[0]), fast_exp2(glast[1] - rN[1])};
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
                 const int n = 2 * J + hh;
                 const float4 g4 = *slot(BG_G, BG_G + 16384, n);
-                *slot(BG_AN, BG_AT, n) = make_float4(fast_exp2(dJ[0] - g4.x) * acc[hh][0], fast_exp2(dJ[0] - g4.y) * acc[hh][1],
-                                                     fast_exp2(dJ[1] - g4.z) * acc[hh][2], fast_exp2(dJ[1] - g4.w) * acc[hh][3]);
+                const float2 rk = *reinterpret_cast<const float2*>(rstd_k + 8 * n + 2 * t4);
+                const float2 k0 = mul2(unpack_bf16(kr[hh][0]), rk), k1 = mul2(unpack_bf16(kr[hh][1]), rk);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[n][e] *= gl[e >> 1];
+                cs[0] = fmaf(k0.x * fast_exp2(d[0] - g4.x), acc[n][0], fmaf(k0.y * fast_exp2(d[0] - g4.y), acc[n][1], cs[0]));
+                cs[1] = fmaf(k1.x * fast_exp2(d[1] - g4.z), acc[n][2], fmaf(k1.y * fast_exp2(d[1] - g4.w), acc[n][3], cs[1]));
             }
+        }
+#pragma unroll
+        for (int I = 0; I < 4; ++I) {
+            uint32_t qr[2][2], kr[2][2];
+            load_raw(BG_Q, I, qr);
+            load_raw(BG_K, I, kr);
+            float qhi[2][4], qlo[2][4], khi[2][4], klo[2][4];
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const int n = 2 * I + hh, tok = 8 * n + 2 * t4;
+                const float4 g4 = *slot(BG_G, BG_G + 16384, n);
+                const float2 rq = mul2(*reinterpret_cast<const float2*>(rstd_q + tok), splat2(p.scale)), rk = *reinterpret_cast<const float2*>(rstd_k + tok);
+                const float2 e0 = make_float2(fast_exp2(g4.x), fast_exp2(g4.y)), e1 = make_float2(fast_exp2(g4.z), fast_exp2(g4.w));
+                const float2 q0 = mul2(mul2(unpack_bf16(qr[hh][0]), rq), e0), q1 = mul2(mul2(unpack_bf16(qr[hh][1]), rq), e1);
+                const float2 k0 = mul2(mul2(unpack_bf16(kr[hh][0]), rk), e0), k1 = mul2(mul2(unpack_bf16(kr[hh][1]), rk), e1);
+                const float vq[4] = {q0.x, q0.y, q1.x, q1.y}, vk[4] = {k0.x, k0.y, k1.x, k1.y};
+                split(vq, qhi[hh], qlo[hh]);
+                split(vk, khi[hh], klo[hh]);
+            }
+#pragma unroll
+            for (int J = 0; J <= I; ++J) {
+                float bl[2][4], f[4];
+                ldsm_blk(BG_PT, J, 2 * I, f);
+                bg_mma0(bl[0], qlo[0], f[0], f[1]);
+                bg_mma0(bl[1], qlo[0], f[2], f[3]);
+                bg_mma(bl[0], qhi[0], f[0], f[1]);
+                bg_mma(bl[1], qhi[0], f[2], f[3]);
+                ldsm_blk(BG_PT, J, 2 * I + 1, f);
+                bg_mma(bl[0], qlo[1], f[0], f[1]);
+                bg_mma(bl[1], qlo[1], f[2], f[3]);
+                bg_mma(bl[0], qhi[1], f[0], f[1]);
+                bg_mma(bl[1], qhi[1], f[2], f[3]);
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    ldsm_blk(BG_X, J, 2 * I + hh, f);
+                    bg_mma(bl[0], klo[hh], f[0], f[1]);
+                    bg_mma(bl[1], klo[hh], f[2], f[3]);
+                    bg_mma(bl[0], khi[hh], f[0], f[1]);
+                    bg_mma(bl[1], khi[hh], f[2], f[3]);
+                }
+                float cji[2] = {1.f, 1.f};
+                if (I != J + 1) {
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) cji[x] = fast_exp2(fminf(rt[I * DK + ch0 + 8 * x] - rt[(J + 1) * DK + ch0 + 8 * x], 126.f));
+                }
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[2 * J + hh][e] = fmaf(cji[e >> 1], bl[hh][e], acc[2 * J + hh][e]);
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            const float4 g4 = *slot(BG_G, BG_G + 16384, n);
+            const float d[2] = {rt[(n / 2 + 1) * DK + ch0] - rt[(n / 2) * DK + ch0], rt[(n / 2 + 1) * DK + ch0 + 8] - rt[(n / 2) * DK + ch0 + 8]};
+            *slot(BG_AN, BG_AT, n) = make_float4(fast_exp2(d[0] - g4.x) * acc[n][0], fast_exp2(d[0] - g4.y) * acc[n][1],
+                                                 fast_exp2(d[1] - g4.z) * acc[n][2], fast_exp2(d[1] - g4.w) * acc[n][3]);
         }
         BG_MARK(6);   // column side
     }
