@@ -194,17 +194,71 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
         ldsm_x4_t(smu + base + row * 256 + ((((uint32_t)(2 * cw + (lm & 1))) ^ (row & 7)) << 4), r[0][0], r[0][1], r[1][0], r[1][1]);
     };
 
-    int tile = blockIdx.x;
-    if (tile < num_tiles) {
-        const int c = tile / p.H, h = tile - c * p.H;
-        const ChunkInfo ci = chunk_info(c, p.cu_seqlens, p.chunk_indices, p.T);
-        if (col_group) { loads.g(ci, h, gt); loads.dw(tile, gt); }
-        else loads.qk(ci, h, gt);
-    }
+    float* rt = reinterpret_cast<float*>(sm + BG_R);
+    float* pZ = reinterpret_cast<float*>(sm + BG_X2);            // [8 slices][64] partial sums over channels
+    float* pL = reinterpret_cast<float*>(sm + BG_X2 + 2048);     // [2 column halves][64]
+    auto slot = [&](int base_lo, int base_hi, int n) -> float4* {     // one float4 per thread of a group and 8 tokens
+        return reinterpret_cast<float4*>(sm + (n < 4 ? base_lo : base_hi) + ((n & 3) * 256 + gt) * 16);
+    };
+    // split an A fragment {(ch0, a), (ch0, b), (ch0 + 8, a), (ch0 + 8, b)} into tf32 high and low parts, in fragment order. Every
+    // pair (i, j) adds +x to the gate gradient of row i and -x to that of row j through two different products; the reverse
+    // cumulative sum relies on those two cancelling, so they must agree far better than tf32
+    // (the tensor core reads the upper 19 bits: high part = the value, truncated; low part = what that leaves, exact, then rounded)
+    auto split = [&](const float (&v)[4], float (&hi)[4], float (&lo)[4]) {
+        const float o[4] = {v[0], v[2], v[1], v[3]};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            hi[e] = o[e];
+            lo[e] = __uint_as_float(__float_as_uint(o[e] - __uint_as_float(__float_as_uint(o[e]) & 0xffffe000u)) + 0x1000u);
+        }
+    };
+    auto sync_all = [&]() { asm volatile("bar.sync 0, 512;" ::: "memory"); };
+    // dA = dAu + stril(dW X^T) -> C2: a 16x16 tile per warp of the CTA, tiles on and below the diagonal
+    auto dA_tile = [&](const float* scr) {
+        const int mt = warp & 3, nh = warp >> 2;
+        if (nh <= mt) {
+            const int r0 = 16 * mt + g8;
+            float2 u[2][2];
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int rr = 0; rr < 2; ++rr)
+                    u[nt][rr] = *reinterpret_cast<const float2*>(scr + SCR_DAU + (r0 + 8 * rr) * BT + 16 * nh + 8 * nt + 2 * t4);
+            float acc[2][4];
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+#pragma unroll 4
+            for (int ks = 0; ks < 16; ++ks) {
+                float fa[4], fb[4];
+                ldsm_a(BG_DW, 16 * mt, ks, fa);
+                ldsm_b(BG_X, 16 * nh, ks, fb);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) fa[e] = bg_tf32(fa[e]);
+                bg_mma(acc[0], fa, fb[0], fb[1]);
+                bg_mma(acc[1], fa, fb[2], fb[3]);
+            }
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int rr = 0; rr < 2; ++rr) {
+                    const int row = r0 + 8 * rr, col = 16 * nh + 8 * nt + 2 * t4, p0 = bg_pos(col);
+                    *reinterpret_cast<float*>(sm + BG_C2 + bg_off(row, p0)) = col < row ? bg_tf32(acc[nt][2 * rr] + u[nt][rr].x) : 0.f;
+                    *reinterpret_cast<float*>(sm + BG_C2 + bg_off(row, p0 + 4)) = col + 1 < row ? bg_tf32(acc[nt][2 * rr + 1] + u[nt][rr].y) : 0.f;
+                }
+        }
+    };
 #ifdef KDA_PHASE_TIMERS
     long long bg_t0_ = clock64();
 #endif
-    for (; tile < num_tiles; tile += gridDim.x) {
+    // The two groups run separate tile loops, so that neither holds the other's registers (one loop with branches spilled 850
+    // bytes a thread); the six CTA barriers per tile match up.
+    if (!col_group) {
+    if ((int)blockIdx.x < num_tiles) {
+        const int c = blockIdx.x / p.H, h = blockIdx.x - c * p.H;
+        loads.qk(chunk_info(c, p.cu_seqlens, p.chunk_indices, p.T), h, gt);
+    }
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+    const int next = tile + gridDim.x;
     const int c = tile / p.H, h = tile - c * p.H;
     const ChunkInfo ci = chunk_info(c, p.cu_seqlens, p.chunk_indices, p.T);
     const size_t tok_stride = (size_t)p.H * DK;
@@ -217,49 +271,14 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
         bias[0] = p.dt_bias[h * DK + ch0];
         bias[1] = p.dt_bias[h * DK + ch0 + 8];
     }
-    // ---- 0. coefficient matrices (a lane per row, so that both orientations are stored without bank conflicts): A by the
-    //         column group, dPs by the row group ----
-    const float* cm_src = col_group ? p.akk + (size_t)tile * 4096 : scr + SCR_DPS;
-    float4 cm[4];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) cm[n] = *reinterpret_cast<const float4*>(cm_src + (gt & 63) * 64 + 4 * ((gt >> 6) + 4 * n));
     uint32_t beta_bits = 0;
     if (tid < 64) {
         const size_t bi = (size_t)(ci.row0 + min(tid, ci.valid - 1)) * p.H + h;
         beta_bits = p.beta_fp32 ? reinterpret_cast<const uint32_t*>(p.beta)[bi] : (uint32_t)reinterpret_cast<const uint16_t*>(p.beta)[bi] << 16;
     }
     bg_cp_wait();
-    __syncthreads();
+    sync_all();
     BG_MARK(0);       // inputs landed
-    {   // norms: 8 threads per row, 16 channels each
-        const int row = tid >> 3, part = tid & 7;
-        float s[2];
-#pragma unroll
-        for (int which = 0; which < 2; ++which) {
-            float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const uint4 v = *reinterpret_cast<const uint4*>(sm + (which ? BG_K : BG_Q) + row * 256 + (((2 * part + e) ^ (row & 7)) << 4));
-                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float2 f = unpack_bf16(w[i]);
-                    acc = fma2(f, f, acc);
-                }
-            }
-            s[which] = acc.x + acc.y;
-        }
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-            s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
-            s[1] += __shfl_xor_sync(0xffffffffu, s[1], o);
-        }
-        if (part == 0) {
-            const bool live = row < ci.valid;
-            rstd_q[row] = live ? (p.use_l2norm ? rsqrtf(s[0] + 1e-6f) : 1.f) : 0.f;
-            rstd_k[row] = live ? (p.use_l2norm ? rsqrtf(s[1] + 1e-6f) : 1.f) : 0.f;
-        }
-    }
     if (tid < 64) {
         float b = 0.f;
         if (tid < ci.valid) {
@@ -268,30 +287,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
         }
         sBeta[tid] = b;
     }
-    {
-        unsigned char* nat = sm + (col_group ? BG_AN : BG_PN);
-        unsigned char* tr = sm + (col_group ? BG_AT : BG_PT);
-        const int row = gt & 63, prow = bg_pos(row);
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            const int c4 = 4 * ((gt >> 6) + 4 * n);
-            const float v[4] = {bg_tf32(cm[n].x), bg_tf32(cm[n].y), bg_tf32(cm[n].z), bg_tf32(cm[n].w)};
-            const int p0 = bg_pos(c4);                 // tokens c4, c4 + 2 sit at p0, p0 + 1 and c4 + 1, c4 + 3 at p0 + 4, p0 + 5
-            if (row >= 32 || c4 < 32) {
-                *reinterpret_cast<float2*>(nat + bg_off(row, p0)) = make_float2(v[0], v[2]);
-                *reinterpret_cast<float2*>(nat + bg_off(row, p0 + 4)) = make_float2(v[1], v[3]);
-            }
-#pragma unroll
-            for (int e = 0; e < 4; ++e) *reinterpret_cast<float*>(tr + bg_off(c4 + e, prow)) = v[e];
-        }
-    }
     // ---- 1. cumulative gate (log2 domain), kept relative to the first row of each 16-row block ----
-    float* rt = reinterpret_cast<float*>(sm + BG_R);
-    float glast[2];
-    uint32_t graw[8][2];      // column group, bf16 gates: the raw values, for the gate VJP
-    auto slot = [&](int base_lo, int base_hi, int n) -> float4* {     // one float4 per thread of a group and 8 tokens
-        return reinterpret_cast<float4*>(sm + (n < 4 ? base_lo : base_hi) + ((n & 3) * 256 + gt) * 16);
-    };
     float G[8][4], r[2][5];
     auto raw_gates = [&](int n2, float (&v)[2][4]) {      // raw gate values of 8-token groups 2 n2, 2 n2 + 1
         if constexpr (GK == BG_PER_HEAD) {
@@ -315,7 +311,6 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
             for (int hh = 0; hh < 2; ++hh)
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    graw[2 * n2 + hh][x] = w[hh][x];
                     const float2 f = unpack_bf16(w[hh][x]);
                     v[hh][2 * x] = f.x;
                     v[hh][2 * x + 1] = f.y;
@@ -371,81 +366,354 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
             }
         }
     }
-    glast[0] = r[0][4]; glast[1] = r[1][4];
-    if (!col_group && t4 == 0) {
+    if (t4 == 0) {
 #pragma unroll
         for (int x = 0; x < 2; ++x)
 #pragma unroll
             for (int b = 0; b < 5; ++b) rt[b * DK + ch0 + 8 * x] = r[x][b];
     }
-    __syncthreads();          // norms, beta, coefficient matrices, block anchors; the raw gates have been read
+    sync_all();       // norms, beta, coefficient matrices, block anchors; the raw gates have been read
     BG_MARK(1);
+    // ---- 2. X = beta k-hat 2^G, rounded to tf32; the gates into their slots ----
+    {
 #pragma unroll
-    for (int n = 0; n < 8; ++n)      // both groups hold the same gates: each stores one half
-        if ((n >> 2) == (col_group ? 1 : 0)) *slot(BG_G, BG_G + 16384, n) = make_float4(G[n][0], G[n][1], G[n][2], G[n][3]);
-    // ---- 2. X = beta k-hat 2^G, rounded to tf32: each group one half of the tokens of its channels ----
-#pragma unroll
-    for (int b2 = 0; b2 < 4; ++b2) {
-        if ((b2 >> 1) == (col_group ? 1 : 0)) {
+        for (int b2 = 0; b2 < 4; ++b2) {
             uint32_t kr[2][2];
             load_raw(BG_K, b2, kr);
             const float gr[2] = {fast_exp2(r[0][b2]), fast_exp2(r[1][b2])};
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
-                const int tok = 16 * b2 + 8 * hh + 2 * t4;
+                const int n = 2 * b2 + hh, tok = 8 * n + 2 * t4;
+                *slot(BG_G, BG_G + 16384, n) = make_float4(G[n][0], G[n][1], G[n][2], G[n][3]);
                 const float2 rk = *reinterpret_cast<const float2*>(rstd_k + tok), be = *reinterpret_cast<const float2*>(sBeta + tok);
                 const float2 f = mul2(rk, be);
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    const float2 kk = unpack_bf16(kr[hh][x]);
-                    *reinterpret_cast<float*>(sm + BG_X + bg_off(tok, ch0 + 8 * x)) = bg_tf32(f.x * kk.x * gr[x] * fast_exp2(G[2 * b2 + hh][2 * x]));
-                    *reinterpret_cast<float*>(sm + BG_X + bg_off(tok + 1, ch0 + 8 * x)) = bg_tf32(f.y * kk.y * gr[x] * fast_exp2(G[2 * b2 + hh][2 * x + 1]));
+                    const float2 kk = mul2(mul2(unpack_bf16(kr[hh][x]), f), splat2(gr[x]));
+                    *reinterpret_cast<float*>(sm + BG_X + bg_off(tok, ch0 + 8 * x)) = bg_tf32(kk.x * fast_exp2(G[n][2 * x]));
+                    *reinterpret_cast<float*>(sm + BG_X + bg_off(tok + 1, ch0 + 8 * x)) = bg_tf32(kk.y * fast_exp2(G[n][2 * x + 1]));
                 }
             }
         }
     }
-    __syncthreads();
+    sync_all();
     BG_MARK(2);       // X
-    // ---- 3. dA = dAu + stril(dW X^T) -> C2: a 16x16 tile per warp, tiles on and below the diagonal ----
+    dA_tile(scr);
+    sync_all();
+    BG_MARK(3);       // dA
+    // ---- 4c. Zw = A^T dW (gradient w.r.t. X) in transposed fragments; its part of dbeta; then it becomes the initial value
+    //          of the dk+ accumulators, which carry 2^(g_i - r_I) at the end ----
+    float zw[8][4];
     {
-        const int mt = warp & 3, nh = warp >> 2;
-        if (nh <= mt) {
-            const int r0 = 16 * mt + g8;
-            float2 u[2][2];
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt)
+        for (int n = 0; n < 8; ++n) zw[n][0] = zw[n][1] = zw[n][2] = zw[n][3] = 0.f;
 #pragma unroll
-                for (int rr = 0; rr < 2; ++rr)
-                    u[nt][rr] = *reinterpret_cast<const float2*>(scr + SCR_DAU + (r0 + 8 * rr) * BT + 16 * nh + 8 * nt + 2 * t4);
-            float acc[2][4];
+        for (int ks = 0; ks < 8; ++ks) {
+            const int tok = 8 * ks + 2 * t4;
+            const float fa[4] = {bg_tf32(*reinterpret_cast<const float*>(sm + BG_DW + bg_off(tok, ch0))),
+                                 bg_tf32(*reinterpret_cast<const float*>(sm + BG_DW + bg_off(tok, ch0 + 8))),
+                                 bg_tf32(*reinterpret_cast<const float*>(sm + BG_DW + bg_off(tok + 1, ch0))),
+                                 bg_tf32(*reinterpret_cast<const float*>(sm + BG_DW + bg_off(tok + 1, ch0 + 8)))};
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-#pragma unroll 4
-            for (int ks = 0; ks < 16; ++ks) {
-                float fa[4], fb[4];
-                ldsm_a(BG_DW, 16 * mt, ks, fa);
-                ldsm_b(BG_X, 16 * nh, ks, fb);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) fa[e] = bg_tf32(fa[e]);
-                bg_mma(acc[0], fa, fb[0], fb[1]);
-                bg_mma(acc[1], fa, fb[2], fb[3]);
+            for (int I = 0; I <= ks / 2; ++I) {
+                float fb[4];
+                ldsm_b(BG_AT, 16 * I, ks, fb);
+                bg_mma(zw[2 * I], fa, fb[0], fb[1]);
+                bg_mma(zw[2 * I + 1], fa, fb[2], fb[3]);
             }
+        }
+        float s[16];
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt)
+        for (int b = 0; b < 4; ++b) {
+            uint32_t kr[2][2];
+            load_raw(BG_K, b, kr);
+            const float gr[2] = {fast_exp2(r[0][b]), fast_exp2(r[1][b])};
 #pragma unroll
-                for (int rr = 0; rr < 2; ++rr) {
-                    const int row = r0 + 8 * rr, col = 16 * nh + 8 * nt + 2 * t4, p0 = bg_pos(col);
-                    *reinterpret_cast<float*>(sm + BG_C2 + bg_off(row, p0)) = col < row ? bg_tf32(acc[nt][2 * rr] + u[nt][rr].x) : 0.f;
-                    *reinterpret_cast<float*>(sm + BG_C2 + bg_off(row, p0 + 4)) = col + 1 < row ? bg_tf32(acc[nt][2 * rr + 1] + u[nt][rr].y) : 0.f;
+            for (int hh = 0; hh < 2; ++hh) {
+                const int n = 2 * b + hh, tok = 8 * n + 2 * t4;
+                const float2 rk = *reinterpret_cast<const float2*>(rstd_k + tok), be = *reinterpret_cast<const float2*>(sBeta + tok);
+                float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const float2 kk = unpack_bf16(kr[hh][x]);
+                    sum.x = fmaf(zw[n][2 * x], kk.x * gr[x] * fast_exp2(G[n][2 * x]), sum.x);
+                    sum.y = fmaf(zw[n][2 * x + 1], kk.y * gr[x] * fast_exp2(G[n][2 * x + 1]), sum.y);
+                    zw[n][2 * x] *= be.x * gr[x];
+                    zw[n][2 * x + 1] *= be.y * gr[x];
                 }
+                s[2 * n] = sum.x * rk.x;
+                s[2 * n + 1] = sum.y * rk.y;
+            }
+        }
+        bg_reduce8<16>(s, g8);
+        *reinterpret_cast<float2*>(pZ + cw * 64 + 8 * g8 + 2 * t4) = make_float2(s[0], s[1]);
+    }
+    BG_MARK(4);       // Zw
+    sync_all();
+    BG_MARK(5);       // wait for the other group
+    if (tid < 64) {   // dbeta is complete
+        float v = scr[SCR_DBU + tid] + (pL[tid] + pL[64 + tid]);
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v += pZ[w * 64 + tid];
+        if (tid < ci.valid) {
+            const size_t bi = (size_t)(ci.row0 + tid) * p.H + h;
+            v *= gs_inv;
+            if (p.beta_logit) v *= sBeta[tid] * (1.f - sBeta[tid]);       // chain rule through the in-kernel sigmoid
+            if (p.beta_fp32) reinterpret_cast<float*>(p.dbeta)[bi] = v;
+            else reinterpret_cast<__nv_bfloat16*>(p.dbeta)[bi] = __float2bfloat16_rn(v);
         }
     }
-    __syncthreads();
+    // The factor 2^(r_I - r_{J+1}) of a pair of blocks belongs to the channel, which is the row of these products: it scales the
+    // 16x16 result of the pair, so that the operands of a block are made once and used against every other block.
+    {
+        // ---- 5a. row side: columns of block J against rows of the blocks I >= J ----
+        float accP[8][4];
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            const float gr[2] = {fast_exp2(rt[(n >> 1) * DK + ch0]), fast_exp2(rt[(n >> 1) * DK + ch0 + 8])};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) accP[n][e] = gr[e >> 1] * scr[SCR_DQG + (8 * n + 2 * t4 + (e & 1)) * DK + ch0 + 8 * (e >> 1)];
+        }
+#pragma unroll
+        for (int J = 0; J < 4; ++J) {
+            uint32_t kr[2][2];
+            load_raw(BG_K, J, kr);
+            const float rN[2] = {rt[(J + 1) * DK + ch0], rt[(J + 1) * DK + ch0 + 8]};
+            const float d[2] = {rN[0] - rt[J * DK + ch0], rN[1] - rt[J * DK + ch0 + 8]};
+            float hi[2][4], lo[2][4];
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const float4 g4 = *slot(BG_G, BG_G + 16384, 2 * J + hh);
+                const float2 rk = *reinterpret_cast<const float2*>(rstd_k + 16 * J + 8 * hh + 2 * t4);
+                const float2 k0 = mul2(unpack_bf16(kr[hh][0]), rk), k1 = mul2(unpack_bf16(kr[hh][1]), rk);
+                const float v[4] = {k0.x * fast_exp2(d[0] - g4.x), k0.y * fast_exp2(d[0] - g4.y), k1.x * fast_exp2(d[1] - g4.z), k1.y * fast_exp2(d[1] - g4.w)};
+                split(v, hi[hh], lo[hh]);
+            }
+#pragma unroll
+            for (int I = J; I < 4; ++I) {
+                float bP[2][4], bR[2][4], f[4];
+                ldsm_blk(BG_PN, I, 2 * J, f);
+                bg_mma0(bP[0], lo[0], f[0], f[1]);
+                bg_mma0(bP[1], lo[0], f[2], f[3]);
+                bg_mma(bP[0], hi[0], f[0], f[1]);
+                bg_mma(bP[1], hi[0], f[2], f[3]);
+                ldsm_blk(BG_C2, I, 2 * J, f);
+                bg_mma0(bR[0], lo[0], f[0], f[1]);
+                bg_mma0(bR[1], lo[0], f[2], f[3]);
+                bg_mma(bR[0], hi[0], f[0], f[1]);
+                bg_mma(bR[1], hi[0], f[2], f[3]);
+                ldsm_blk(BG_PN, I, 2 * J + 1, f);
+                bg_mma(bP[0], lo[1], f[0], f[1]);
+                bg_mma(bP[1], lo[1], f[2], f[3]);
+                bg_mma(bP[0], hi[1], f[0], f[1]);
+                bg_mma(bP[1], hi[1], f[2], f[3]);
+                ldsm_blk(BG_C2, I, 2 * J + 1, f);
+                bg_mma(bR[0], lo[1], f[0], f[1]);
+                bg_mma(bR[1], lo[1], f[2], f[3]);
+                bg_mma(bR[0], hi[1], f[0], f[1]);
+                bg_mma(bR[1], hi[1], f[2], f[3]);
+                float cji[2] = {1.f, 1.f};
+                if (I != J + 1) {
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) cji[x] = fast_exp2(fminf(rt[I * DK + ch0 + 8 * x] - rN[x], 126.f));
+                }
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        accP[2 * I + hh][e] = fmaf(cji[e >> 1], bP[hh][e], accP[2 * I + hh][e]);
+                        zw[2 * I + hh][e] = fmaf(cji[e >> 1], bR[hh][e], zw[2 * I + hh][e]);
+                    }
+            }
+        }
+        bg_bar(1);         // the partial sums have been read: their space takes a half of the results
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            const float4 g4 = *slot(BG_G, BG_G + 16384, n);
+            const float f[4] = {fast_exp2(g4.x), fast_exp2(g4.y), fast_exp2(g4.z), fast_exp2(g4.w)};
+            *slot(BG_DW, BG_DW + 16384, n) = make_float4(p.scale * f[0] * accP[n][0], p.scale * f[1] * accP[n][1], p.scale * f[2] * accP[n][2],
+                                                         p.scale * f[3] * accP[n][3]);
+            *slot(BG_C1, BG_X2, n) = make_float4(f[0] * zw[n][0], f[1] * zw[n][1], f[2] * zw[n][2], f[3] * zw[n][3]);
+        }
+    }
+    BG_MARK(6);       // row side
+    sync_all();       // dk- is ready for the row group, dq and dk+ for the column group
+    BG_MARK(7);
+    {
+        // ---- 6a. dk, the L2-norm VJP, dq and dk out ----
+        float* part = reinterpret_cast<float*>(sm + BG_C2);      // [2][8 slices][64], then totals [2][64]
+        if (p.use_l2norm) {
+#pragma unroll 1
+            for (int b = 0; b < 4; ++b) {
+                uint32_t qr[2][2], kr[2][2];
+                load_raw(BG_Q, b, qr);
+                load_raw(BG_K, b, kr);
+                float s[8];                  // q . dq of the four tokens, then k . dk
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int n = 2 * b + hh;
+                    const float4 dq = *slot(BG_DW, BG_DW + 16384, n), dp = *slot(BG_C1, BG_X2, n), dm = *slot(BG_AN, BG_AT, n);
+                    const float2 q0 = unpack_bf16(qr[hh][0]), q1 = unpack_bf16(qr[hh][1]), k0 = unpack_bf16(kr[hh][0]), k1 = unpack_bf16(kr[hh][1]);
+                    s[2 * hh] = dq.x * q0.x + dq.z * q1.x;
+                    s[2 * hh + 1] = dq.y * q0.y + dq.w * q1.y;
+                    s[4 + 2 * hh] = (dp.x + dm.x) * k0.x + (dp.z + dm.z) * k1.x;
+                    s[4 + 2 * hh + 1] = (dp.y + dm.y) * k0.y + (dp.w + dm.w) * k1.y;
+                }
+                bg_reduce8<8>(s, g8);        // lane (g, t) holds value g
+                part[512 * (g8 >> 2) + cw * 64 + 16 * b + 8 * ((g8 >> 1) & 1) + 2 * t4 + (g8 & 1)] = s[0];
+            }
+            bg_bar(1);
+            if (gt < 128) {
+                const int which = gt >> 6, row = gt & 63;
+                float v = 0.f;
+#pragma unroll
+                for (int w = 0; w < 8; ++w) v += part[512 * which + 64 * w + row];
+                const float rs = which ? rstd_k[row] : rstd_q[row];
+                part[1024 + gt] = v * rs * rs;                  // q-hat (q-hat . dq) = q rstd^2 (q . dq)
+            }
+            bg_bar(1);
+        }
+#pragma unroll 1
+        for (int b = 0; b < 4; ++b) {
+            uint32_t qr[2][2], kr[2][2];
+            load_raw(BG_Q, b, qr);
+            load_raw(BG_K, b, kr);
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const int n = 2 * b + hh, tok = 8 * n + 2 * t4;
+                const float4 dq = *slot(BG_DW, BG_DW + 16384, n), dp = *slot(BG_C1, BG_X2, n), dm = *slot(BG_AN, BG_AT, n);
+                const float2 fq = mul2(*reinterpret_cast<const float2*>(rstd_q + tok), splat2(gs_inv)),
+                             fk = mul2(*reinterpret_cast<const float2*>(rstd_k + tok), splat2(gs_inv));
+                float2 tq = make_float2(0.f, 0.f), tk = tq;
+                if (p.use_l2norm) {
+                    tq = *reinterpret_cast<const float2*>(part + 1024 + tok);
+                    tk = *reinterpret_cast<const float2*>(part + 1088 + tok);
+                }
+                const float dqv[4] = {dq.x, dq.y, dq.z, dq.w}, dkv[4] = {dp.x + dm.x, dp.y + dm.y, dp.z + dm.z, dp.w + dm.w};
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const float2 q2 = unpack_bf16(qr[hh][x]), k2 = unpack_bf16(kr[hh][x]);
+                    qr[hh][x] = pack_bf16(fq.x * (dqv[2 * x] - q2.x * tq.x), fq.y * (dqv[2 * x + 1] - q2.y * tq.y));
+                    kr[hh][x] = pack_bf16(fk.x * (dkv[2 * x] - k2.x * tk.x), fk.y * (dkv[2 * x + 1] - k2.y * tk.y));
+                }
+            }
+            const uint32_t row = 16 * b + raw_row, off = row * 256 + ((((uint32_t)(2 * cw + (lm & 1))) ^ (row & 7)) << 4);
+            stsm_x4_t(smu + BG_PN + off, qr[0][0], qr[0][1], qr[1][0], qr[1][1]);
+            stsm_x4_t(smu + BG_PT + off, kr[0][0], kr[0][1], kr[1][0], kr[1][1]);
+        }
+        // both groups are done with the raw q and k rows, this one with its slots: the next tile's rows may come
+        asm volatile("bar.sync 3, 512;" ::: "memory");
+        if (next < num_tiles) {
+            const int cn = next / p.H, hn = next - cn * p.H;
+            loads.qk(chunk_info(cn, p.cu_seqlens, p.chunk_indices, p.T), hn, gt);
+            loads.dw(next, gt);
+        }
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const int idx = gt + 256 * n, row = idx >> 4, chn = idx & 15;
+            if (row < ci.valid) {
+                const size_t off = base + (size_t)row * tok_stride + 8 * chn;
+                const uint32_t so = (uint32_t)(row * 256 + ((chn ^ (row & 7)) << 4));
+                *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.dq) + off) = *reinterpret_cast<const uint4*>(sm + BG_PN + so);
+                *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.dk) + off) = *reinterpret_cast<const uint4*>(sm + BG_PT + so);
+            }
+        }
+    }
+    }  // tile loop: the first barrier of the next tile orders the reuse of everything written after the last one
+    } else {
+    if ((int)blockIdx.x < num_tiles) {
+        const int c = blockIdx.x / p.H, h = blockIdx.x - c * p.H;
+        loads.g(chunk_info(c, p.cu_seqlens, p.chunk_indices, p.T), h, gt);
+        loads.dw(blockIdx.x, gt);
+    }
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+    const int next = tile + gridDim.x;
+    const int c = tile / p.H, h = tile - c * p.H;
+    const ChunkInfo ci = chunk_info(c, p.cu_seqlens, p.chunk_indices, p.T);
+    const size_t tok_stride = (size_t)p.H * DK;
+    const size_t base = (size_t)ci.row0 * tok_stride + (size_t)h * DK;
+    const float* scr = p.scratch + (size_t)tile * (size_t)BWD_SCRATCH_FLOATS;
+    const float gs_inv = p.gscale[1];
+    const float alpha = p.gate_mode != GATE_NONE ? __expf(p.A_log[h]) : 0.f;
+    float bias[2] = {0.f, 0.f};
+    if (p.gate_mode != GATE_NONE && p.dt_bias) {
+        bias[0] = p.dt_bias[h * DK + ch0];
+        bias[1] = p.dt_bias[h * DK + ch0 + 8];
+    }
+    // ---- 0. norms and the coefficient matrices A and dPs (a lane per row, so that both orientations are stored without bank
+    //         conflicts), while the row group works out the gates ----
+    uint32_t graw[8][2];      // bf16 gates: the raw values, for the gate VJP
+    {
+        float4 cm[2][4];
+#pragma unroll
+        for (int w = 0; w < 2; ++w)
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+                cm[w][n] = *reinterpret_cast<const float4*>((w ? scr + SCR_DPS : p.akk + (size_t)tile * 4096) + (gt & 63) * 64 + 4 * ((gt >> 6) + 4 * n));
+        bg_cp_wait();
+        sync_all();
+        BG_MARK(0);   // inputs landed
+        {   // norms: 4 threads per row, 32 channels each
+            const int row = gt >> 2, part = gt & 3;
+            float s[2];
+#pragma unroll
+            for (int which = 0; which < 2; ++which) {
+                float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(sm + (which ? BG_K : BG_Q) + row * 256 + (((part + 4 * e) ^ (row & 7)) << 4));
+                    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 f = unpack_bf16(w[i]);
+                        acc = fma2(f, f, acc);
+                    }
+                }
+                s[which] = acc.x + acc.y;
+            }
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+                s[1] += __shfl_xor_sync(0xffffffffu, s[1], o);
+            }
+            if (part == 0) {
+                const bool live = row < ci.valid;
+                rstd_q[row] = live ? (p.use_l2norm ? rsqrtf(s[0] + 1e-6f) : 1.f) : 0.f;
+                rstd_k[row] = live ? (p.use_l2norm ? rsqrtf(s[1] + 1e-6f) : 1.f) : 0.f;
+            }
+        }
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            unsigned char* nat = sm + (w ? BG_PN : BG_AN);
+            unsigned char* tr = sm + (w ? BG_PT : BG_AT);
+            const int row = gt & 63, prow = bg_pos(row);
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                const int c4 = 4 * ((gt >> 6) + 4 * n);
+                const float v[4] = {bg_tf32(cm[w][n].x), bg_tf32(cm[w][n].y), bg_tf32(cm[w][n].z), bg_tf32(cm[w][n].w)};
+                const int p0 = bg_pos(c4);                 // tokens c4, c4 + 2 sit at p0, p0 + 1 and c4 + 1, c4 + 3 at p0 + 4, p0 + 5
+                if (row >= 32 || c4 < 32) {
+                    *reinterpret_cast<float2*>(nat + bg_off(row, p0)) = make_float2(v[0], v[2]);
+                    *reinterpret_cast<float2*>(nat + bg_off(row, p0 + 4)) = make_float2(v[1], v[3]);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) *reinterpret_cast<float*>(tr + bg_off(c4 + e, prow)) = v[e];
+            }
+        }
+        if (GK == BG_BF16) {
+#pragma unroll
+            for (int n2 = 0; n2 < 4; ++n2) load_raw(BG_G, n2, reinterpret_cast<uint32_t(&)[2][2]>(graw[2 * n2]));
+        }
+    }
+    sync_all();
+    BG_MARK(1);
+    const float glast[2] = {rt[4 * DK + ch0], rt[4 * DK + ch0 + 8]};
+    sync_all();
+    BG_MARK(2);       // X
+    dA_tile(scr);
+    sync_all();
     BG_MARK(3);       // dA
-    float zw[8][4];           // row group: Zw, then dk+
-    float* pZ = reinterpret_cast<float*>(sm + BG_X2);            // [8 slices][64] partial sums over channels
-    float* pL = reinterpret_cast<float*>(sm + BG_X2 + 2048);     // [2 column halves][64]
-    if (col_group) {
+    {
         const int rb = cw & 3, half = cw >> 2;
         // ---- 4a. T1^T = A dA^T -> C1 (the tiles on and above the diagonal are all that dL needs) ----
 #pragma unroll
@@ -516,162 +784,28 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
             db[rr] += __shfl_xor_sync(0xffffffffu, db[rr], 2);
             if (t4 == 0) pL[half * 64 + 16 * rb + g8 + 8 * rr] = db[rr];
         }
-        BG_MARK(4);   // column group: T1, dL
-    } else {
-        // ---- 4c. Zw = A^T dW (gradient w.r.t. X) in transposed fragments; its part of dbeta; then it becomes the initial value
-        //          of the dk+ accumulators, which carry 2^(g_i - r_I) at the end ----
-#pragma unroll
-        for (int n = 0; n < 8; ++n) zw[n][0] = zw[n][1] = zw[n][2] = zw[n][3] = 0.f;
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-            const int tok = 8 * ks + 2 * t4;
-            const float fa[4] = {bg_tf32(*reinterpret_cast<const float*>(sm + BG_DW + bg_off(tok, ch0))),
-                                 bg_tf32(*reinterpret_cast<const float*>(sm + BG_DW + bg_off(tok, ch0 + 8))),
-                                 bg_tf32(*reinterpret_cast<const float*>(sm + BG_DW + bg_off(tok + 1, ch0))),
-                                 bg_tf32(*reinterpret_cast<const float*>(sm + BG_DW + bg_off(tok + 1, ch0 + 8)))};
-#pragma unroll
-            for (int I = 0; I <= ks / 2; ++I) {
-                float fb[4];
-                ldsm_b(BG_AT, 16 * I, ks, fb);
-                bg_mma(zw[2 * I], fa, fb[0], fb[1]);
-                bg_mma(zw[2 * I + 1], fa, fb[2], fb[3]);
-            }
-        }
-        float s[16];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            uint32_t kr[2][2];
-            load_raw(BG_K, b, kr);
-            const float gr[2] = {fast_exp2(r[0][b]), fast_exp2(r[1][b])};
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const int n = 2 * b + hh, tok = 8 * n + 2 * t4;
-                const float2 rk = *reinterpret_cast<const float2*>(rstd_k + tok), be = *reinterpret_cast<const float2*>(sBeta + tok);
-                float2 sum = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    const float2 kk = unpack_bf16(kr[hh][x]);
-                    sum.x = fmaf(zw[n][2 * x], kk.x * gr[x] * fast_exp2(G[n][2 * x]), sum.x);
-                    sum.y = fmaf(zw[n][2 * x + 1], kk.y * gr[x] * fast_exp2(G[n][2 * x + 1]), sum.y);
-                    zw[n][2 * x] *= be.x * gr[x];
-                    zw[n][2 * x + 1] *= be.y * gr[x];
-                }
-                s[2 * n] = sum.x * rk.x;
-                s[2 * n + 1] = sum.y * rk.y;
-            }
-        }
-        bg_reduce8<16>(s, g8);
-        *reinterpret_cast<float2*>(pZ + cw * 64 + 8 * g8 + 2 * t4) = make_float2(s[0], s[1]);
-        BG_MARK(4);   // row group: Zw
     }
-    __syncthreads();
+    BG_MARK(4);       // T1, dL
+    sync_all();
     BG_MARK(5);       // wait for the other group
-    if (tid < 64) {   // dbeta is complete
-        float v = scr[SCR_DBU + tid] + (pL[tid] + pL[64 + tid]);
-#pragma unroll
-        for (int w = 0; w < 8; ++w) v += pZ[w * 64 + tid];
-        if (tid < ci.valid) {
-            const size_t bi = (size_t)(ci.row0 + tid) * p.H + h;
-            v *= gs_inv;
-            if (p.beta_logit) v *= sBeta[tid] * (1.f - sBeta[tid]);       // chain rule through the in-kernel sigmoid
-            if (p.beta_fp32) reinterpret_cast<float*>(p.dbeta)[bi] = v;
-            else reinterpret_cast<__nv_bfloat16*>(p.dbeta)[bi] = __float2bfloat16_rn(v);
-        }
-    }
-    const int next = tile + gridDim.x;
-    if (tid == 64 && next < num_tiles) {      // the next tile's contiguous inputs on their way to L2
+    if (gt == 0 && next < num_tiles) {      // the next tile's contiguous inputs on their way to L2
         bulk_prefetch_l2(p.scratch + (size_t)next * (size_t)BWD_SCRATCH_FLOATS, BWD_SCRATCH_FLOATS * 4);
         bulk_prefetch_l2(p.akk + (size_t)next * 4096, 4096 * 4);
         bulk_prefetch_l2(p.mkk + (size_t)next * 4096, 4096 * 4);
     }
-    // split an A fragment {(ch0, a), (ch0, b), (ch0 + 8, a), (ch0 + 8, b)} into tf32 high and low parts, in fragment order. Every
-    // pair (i, j) adds +x to the gate gradient of row i and -x to that of row j through two different products; the reverse
-    // cumulative sum relies on those two cancelling, so they must agree far better than tf32
-    // (the tensor core reads the upper 19 bits: high part = the value, truncated; low part = what that leaves, exact, then rounded)
-    auto split = [&](const float (&v)[4], float (&hi)[4], float (&lo)[4]) {
-        const float o[4] = {v[0], v[2], v[1], v[3]};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            hi[e] = o[e];
-            lo[e] = __uint_as_float(__float_as_uint(o[e] - __uint_as_float(__float_as_uint(o[e]) & 0xffffe000u)) + 0x1000u);
+    if (next < num_tiles) {      // and its token rows, a 128-byte line at a time
+        const int cn = next / p.H, hn = next - cn * p.H;
+        const ChunkInfo cin = chunk_info(cn, p.cu_seqlens, p.chunk_indices, p.T);
+        const int row = gt >> 2, part = gt & 3;
+        if (row < cin.valid) {
+            const size_t o = (size_t)(cin.row0 + row) * tok_stride + (size_t)hn * DK;
+            prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(part < 2 ? p.q : p.k) + o + 64 * (part & 1));
+            if (GK == BG_FP32) prefetch_l2(reinterpret_cast<const float*>(p.g) + o + 32 * part);
+            if (GK == BG_BF16 && part < 2) prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(p.g) + o + 64 * part);
         }
-    };
-    // The factor 2^(r_I - r_{J+1}) of a pair of blocks belongs to the channel, which is the row of these products: it scales the
-    // 16x16 result of the pair, so that the operands of a block are made once and used against every other block.
-    if (!col_group) {
-        // ---- 5a. row side: columns of block J against rows of the blocks I >= J ----
-        float accP[8][4];
-#pragma unroll
-        for (int n = 0; n < 8; ++n) {
-            const float gr[2] = {fast_exp2(rt[(n >> 1) * DK + ch0]), fast_exp2(rt[(n >> 1) * DK + ch0 + 8])};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) accP[n][e] = gr[e >> 1] * scr[SCR_DQG + (8 * n + 2 * t4 + (e & 1)) * DK + ch0 + 8 * (e >> 1)];
-        }
-#pragma unroll
-        for (int J = 0; J < 4; ++J) {
-            uint32_t kr[2][2];
-            load_raw(BG_K, J, kr);
-            const float rN[2] = {rt[(J + 1) * DK + ch0], rt[(J + 1) * DK + ch0 + 8]};
-            const float d[2] = {rN[0] - rt[J * DK + ch0], rN[1] - rt[J * DK + ch0 + 8]};
-            float hi[2][4], lo[2][4];
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const float4 g4 = *slot(BG_G, BG_G + 16384, 2 * J + hh);
-                const float2 rk = *reinterpret_cast<const float2*>(rstd_k + 16 * J + 8 * hh + 2 * t4);
-                const float2 k0 = mul2(unpack_bf16(kr[hh][0]), rk), k1 = mul2(unpack_bf16(kr[hh][1]), rk);
-                const float v[4] = {k0.x * fast_exp2(d[0] - g4.x), k0.y * fast_exp2(d[0] - g4.y), k1.x * fast_exp2(d[1] - g4.z), k1.y * fast_exp2(d[1] - g4.w)};
-                split(v, hi[hh], lo[hh]);
-            }
-#pragma unroll
-            for (int I = J; I < 4; ++I) {
-                float bP[2][4], bR[2][4], f[4];
-                ldsm_blk(BG_PN, I, 2 * J, f);
-                bg_mma0(bP[0], lo[0], f[0], f[1]);
-                bg_mma0(bP[1], lo[0], f[2], f[3]);
-                bg_mma(bP[0], hi[0], f[0], f[1]);
-                bg_mma(bP[1], hi[0], f[2], f[3]);
-                ldsm_blk(BG_C2, I, 2 * J, f);
-                bg_mma0(bR[0], lo[0], f[0], f[1]);
-                bg_mma0(bR[1], lo[0], f[2], f[3]);
-                bg_mma(bR[0], hi[0], f[0], f[1]);
-                bg_mma(bR[1], hi[0], f[2], f[3]);
-                ldsm_blk(BG_PN, I, 2 * J + 1, f);
-                bg_mma(bP[0], lo[1], f[0], f[1]);
-                bg_mma(bP[1], lo[1], f[2], f[3]);
-                bg_mma(bP[0], hi[1], f[0], f[1]);
-                bg_mma(bP[1], hi[1], f[2], f[3]);
-                ldsm_blk(BG_C2, I, 2 * J + 1, f);
-                bg_mma(bR[0], lo[1], f[0], f[1]);
-                bg_mma(bR[1], lo[1], f[2], f[3]);
-                bg_mma(bR[0], hi[1], f[0], f[1]);
-                bg_mma(bR[1], hi[1], f[2], f[3]);
-                float cji[2] = {1.f, 1.f};
-                if (I != J + 1) {
-#pragma unroll
-                    for (int x = 0; x < 2; ++x) cji[x] = fast_exp2(fminf(rt[I * DK + ch0 + 8 * x] - rN[x], 126.f));
-                }
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        accP[2 * I + hh][e] = fmaf(cji[e >> 1], bP[hh][e], accP[2 * I + hh][e]);
-                        zw[2 * I + hh][e] = fmaf(cji[e >> 1], bR[hh][e], zw[2 * I + hh][e]);
-                    }
-            }
-        }
-        bg_bar(1);         // the partial sums have been read: their space takes a half of the results
-#pragma unroll
-        for (int n = 0; n < 8; ++n) {
-            const float4 g4 = *slot(BG_G, BG_G + 16384, n);
-            const float f[4] = {fast_exp2(g4.x), fast_exp2(g4.y), fast_exp2(g4.z), fast_exp2(g4.w)};
-            *slot(BG_DW, BG_DW + 16384, n) = make_float4(p.scale * f[0] * accP[n][0], p.scale * f[1] * accP[n][1], p.scale * f[2] * accP[n][2],
-                                                         p.scale * f[3] * accP[n][3]);
-            *slot(BG_C1, BG_X2, n) = make_float4(f[0] * zw[n][0], f[1] * zw[n][1], f[2] * zw[n][2], f[3] * zw[n][3]);
-        }
-        BG_MARK(6);   // row side
     }
-    float cs[2] = {0.f, 0.f};      // column group: sum over the tokens of dKg * Kg, the gradient that reaches g_last through kg
-    if (col_group) {
+    float cs[2] = {0.f, 0.f};      // sum over the tokens of dKg * Kg, the gradient that reaches g_last through kg
+    {
         // ---- 5b. column side: rows of block I against columns of the blocks J <= I ----
         float acc[8][4];
 #pragma unroll
@@ -754,90 +888,11 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
             *slot(BG_AN, BG_AT, n) = make_float4(fast_exp2(d[0] - g4.x) * acc[n][0], fast_exp2(d[0] - g4.y) * acc[n][1],
                                                  fast_exp2(d[1] - g4.z) * acc[n][2], fast_exp2(d[1] - g4.w) * acc[n][3]);
         }
-        BG_MARK(6);   // column side
     }
-    __syncthreads();          // dk- is ready for the row group, dq and dk+ for the column group
+    BG_MARK(6);       // column side
+    sync_all();
     BG_MARK(7);
-    if (!col_group) {
-        // ---- 6a. dk, the L2-norm VJP, dq and dk out ----
-        float* part = reinterpret_cast<float*>(sm + BG_C2);      // [2][8 slices][64], then totals [2][64]
-        if (p.use_l2norm) {
-#pragma unroll 1
-            for (int b = 0; b < 4; ++b) {
-                uint32_t qr[2][2], kr[2][2];
-                load_raw(BG_Q, b, qr);
-                load_raw(BG_K, b, kr);
-                float s[8];                  // q . dq of the four tokens, then k . dk
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {
-                    const int n = 2 * b + hh;
-                    const float4 dq = *slot(BG_DW, BG_DW + 16384, n), dp = *slot(BG_C1, BG_X2, n), dm = *slot(BG_AN, BG_AT, n);
-                    const float2 q0 = unpack_bf16(qr[hh][0]), q1 = unpack_bf16(qr[hh][1]), k0 = unpack_bf16(kr[hh][0]), k1 = unpack_bf16(kr[hh][1]);
-                    s[2 * hh] = dq.x * q0.x + dq.z * q1.x;
-                    s[2 * hh + 1] = dq.y * q0.y + dq.w * q1.y;
-                    s[4 + 2 * hh] = (dp.x + dm.x) * k0.x + (dp.z + dm.z) * k1.x;
-                    s[4 + 2 * hh + 1] = (dp.y + dm.y) * k0.y + (dp.w + dm.w) * k1.y;
-                }
-                bg_reduce8<8>(s, g8);        // lane (g, t) holds value g
-                part[512 * (g8 >> 2) + cw * 64 + 16 * b + 8 * ((g8 >> 1) & 1) + 2 * t4 + (g8 & 1)] = s[0];
-            }
-            bg_bar(1);
-            if (gt < 128) {
-                const int which = gt >> 6, row = gt & 63;
-                float v = 0.f;
-#pragma unroll
-                for (int w = 0; w < 8; ++w) v += part[512 * which + 64 * w + row];
-                const float rs = which ? rstd_k[row] : rstd_q[row];
-                part[1024 + gt] = v * rs * rs;                  // q-hat (q-hat . dq) = q rstd^2 (q . dq)
-            }
-            bg_bar(1);
-        }
-#pragma unroll 1
-        for (int b = 0; b < 4; ++b) {
-            uint32_t qr[2][2], kr[2][2];
-            load_raw(BG_Q, b, qr);
-            load_raw(BG_K, b, kr);
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const int n = 2 * b + hh, tok = 8 * n + 2 * t4;
-                const float4 dq = *slot(BG_DW, BG_DW + 16384, n), dp = *slot(BG_C1, BG_X2, n), dm = *slot(BG_AN, BG_AT, n);
-                const float2 fq = mul2(*reinterpret_cast<const float2*>(rstd_q + tok), splat2(gs_inv)),
-                             fk = mul2(*reinterpret_cast<const float2*>(rstd_k + tok), splat2(gs_inv));
-                float2 tq = make_float2(0.f, 0.f), tk = tq;
-                if (p.use_l2norm) {
-                    tq = *reinterpret_cast<const float2*>(part + 1024 + tok);
-                    tk = *reinterpret_cast<const float2*>(part + 1088 + tok);
-                }
-                const float dqv[4] = {dq.x, dq.y, dq.z, dq.w}, dkv[4] = {dp.x + dm.x, dp.y + dm.y, dp.z + dm.z, dp.w + dm.w};
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    const float2 q2 = unpack_bf16(qr[hh][x]), k2 = unpack_bf16(kr[hh][x]);
-                    qr[hh][x] = pack_bf16(fq.x * (dqv[2 * x] - q2.x * tq.x), fq.y * (dqv[2 * x + 1] - q2.y * tq.y));
-                    kr[hh][x] = pack_bf16(fk.x * (dkv[2 * x] - k2.x * tk.x), fk.y * (dkv[2 * x + 1] - k2.y * tk.y));
-                }
-            }
-            const uint32_t row = 16 * b + raw_row, off = row * 256 + ((((uint32_t)(2 * cw + (lm & 1))) ^ (row & 7)) << 4);
-            stsm_x4_t(smu + BG_PN + off, qr[0][0], qr[0][1], qr[1][0], qr[1][1]);
-            stsm_x4_t(smu + BG_PT + off, kr[0][0], kr[0][1], kr[1][0], kr[1][1]);
-        }
-        // both groups are done with the raw q and k rows, this one with its slots: the next tile's rows may come
-        asm volatile("bar.sync 3, 512;" ::: "memory");
-        if (next < num_tiles) {
-            const int cn = next / p.H, hn = next - cn * p.H;
-            loads.qk(chunk_info(cn, p.cu_seqlens, p.chunk_indices, p.T), hn, gt);
-            loads.dw(next, gt);
-        }
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            const int idx = gt + 256 * n, row = idx >> 4, chn = idx & 15;
-            if (row < ci.valid) {
-                const size_t off = base + (size_t)row * tok_stride + 8 * chn;
-                const uint32_t so = (uint32_t)(row * 256 + ((chn ^ (row & 7)) << 4));
-                *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.dq) + off) = *reinterpret_cast<const uint4*>(sm + BG_PN + so);
-                *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.dk) + off) = *reinterpret_cast<const uint4*>(sm + BG_PT + so);
-            }
-        }
-    } else {
+    {
         // ---- 6b. dG, its reverse cumulative sum down the tokens, the gate VJP ----
         float run[2];
 #pragma unroll
@@ -973,7 +1028,8 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
             }
         }
     }
-    }  // tile loop: the first barrier of the next tile orders the reuse of everything written after it
+    }
+    }
 }
 
 }  // namespace kda
