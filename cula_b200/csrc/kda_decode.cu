@@ -13,12 +13,13 @@
 //   layout "vk" (pool, HV, V, K), the reference's default: a warp walks its value rows 8 at a time (8 x 128
 //     floats in registers, lane = 4 consecutive k, the next 8 rows already in flight), both contractions are
 //     4 FMAs + a warp reduction per row;
-//   layout "kv" (pool, HV, K, V): a CTA owns a 32-column value slice; a warp holds 32 key rows (8 lanes x
-//     float4 per row), the contractions reduce over lanes with equal column group and across the 4 warps
-//     through shared memory.
+//   layout "kv" (pool, HV, K, V): a warp owns 16 value columns of all 128 keys (4 lanes x float4 per row, 16 rows in
+//     registers, all 8 KB requested before the first is used) and works alone: the contractions are 16 FMAs per lane
+//     and a reduction over the 8 lanes that share the columns; no barriers between the loads and the stores. (With the
+//     keys spread over the four warps and three CTA barriers per 32 columns, 33 sequences x 32 heads took 34.8 us a call for
+//     138 MB, now 29.7.)
 // Work items = N * HV * slices (K = 128; V any multiple of 32; slices divides V / 32 and is chosen on the host: 1
-// when there are enough states to fill the GPU, more for small batches); four persistent CTAs of 128 threads
-// per SM walk them.
+// when there are enough states to fill the GPU, more for small batches); kv items are 16 columns each.
 #include "kda_common.cuh"
 
 namespace kda {
@@ -34,7 +35,7 @@ struct DecodeParams {
     float* state;         // [pool, HV, V, 128] (vk) or [pool, HV, 128, V] (kv) fp32, updated in place
     const int* indices;   // [N] pool slot of every sequence, or nullptr (slot = n)
     void* o;              // [N, HV, V] bf16
-    int N, H, HV, V, pool, slices;   // slices: CTAs per state, each owning V / slices value rows (vk) or columns (kv)
+    int N, H, HV, V, pool, slices;   // slices: CTAs per state, each owning V / slices value rows (vk only)
     int a_fp32, b_fp32, use_l2norm, state_kv;
     float scale, softplus_beta, softplus_threshold;
     int* status;
@@ -84,12 +85,11 @@ __device__ __forceinline__ void dec_key_vectors(const DecodeParams& p, int n, in
     }
 }
 
-// One work item = one slice of one (sequence, value head) state.
-__device__ __forceinline__ void dec_item(const DecodeParams& p, const int item, float (*red)[4][32], float* s_gate, float* s_kh,
-                                         float* s_qs) {
+// One work item of the (V, K) layout = one slice of one (sequence, value head) state.
+__device__ __forceinline__ void dec_item(const DecodeParams& p, const int item) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int slice = item % p.slices, nh = item / p.slices;
-    const int per_cta = p.V / p.slices;                     // value rows (vk) or columns (kv) of this CTA, a multiple of 32
+    const int per_cta = p.V / p.slices;                     // value rows of this CTA, a multiple of 32
     const int n = nh / p.HV, hv = nh - n * p.HV;
     const int hq = hv / (p.HV / p.H);
     const int slot = p.indices ? p.indices[n] : n;
@@ -107,7 +107,7 @@ __device__ __forceinline__ void dec_item(const DecodeParams& p, const int item, 
     const __nv_bfloat16* vp = reinterpret_cast<const __nv_bfloat16*>(p.v) + ((size_t)n * p.HV + hv) * p.V;
     __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(p.o) + ((size_t)n * p.HV + hv) * p.V;
 
-    if (!p.state_kv) {
+    {
         // ---- (V, K) rows: the warp owns per_cta / 4 value rows and walks them 8 at a time, the next 8 already in
         //      flight while the current 8 are updated; the lane owns keys 4*lane .. 4*lane+3 ----
         const int rows_warp = per_cta >> 2, nb = rows_warp >> 3;
@@ -157,82 +157,86 @@ __device__ __forceinline__ void dec_item(const DecodeParams& p, const int item, 
 #pragma unroll
             for (int i = 0; i < 8; ++i) row[i] = nxt[i];
         }
+    }
+}
+
+// One work item of the (K, V) layout = 16 value columns of one (sequence, value head) state, for one warp. `vec` is the warp's own
+// [3][128] floats: gate, k-hat and scale * q-hat, read key by key.
+__device__ __forceinline__ void dec_item_kv(const DecodeParams& p, const int item, float (*vec)[DK]) {
+    const int lane = threadIdx.x & 31, cols = p.V >> 4;
+    const int cs = item % cols, nh = item / cols;
+    const int n = nh / p.HV, hv = nh - n * p.HV, hq = hv / (p.HV / p.H);
+    const int rg = lane >> 2, c = 16 * cs + 4 * (lane & 3);      // rows rg, rg + 8, ..., columns c .. c + 3
+    const int slot = p.indices ? p.indices[n] : n;
+    __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(p.o) + ((size_t)n * p.HV + hv) * p.V + c;
+    if (slot < 0) {                                         // padded sequence: no state access; its output row is zeroed
+        if (rg == 0)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) op[e] = __float2bfloat16_rn(0.f);
         return;
     }
-
-    // ---- (K, V) rows: the CTA walks its value columns 32 at a time; warp w owns key rows 32w .. 32w+31, lane (rg, cg):
-    //      row group rg = lane / 8 (rows rg, rg+4, ..., rg+28 of the warp's 32), column group cg = lane % 8 ----
+    if (slot >= p.pool) {                                   // caller error: report, touch nothing
+        if (lane == 0) report_status(p.status, STATUS_BAD_INDEX);
+        return;
+    }
+    float* S = p.state + ((size_t)slot * p.HV + hv) * (size_t)DK * p.V + (size_t)rg * p.V + c;
+    float4 row[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) row[i] = __ldcs(reinterpret_cast<const float4*>(S + (size_t)(8 * i) * p.V));
     {
         float gate[4], kh[4], qs[4];
-        dec_key_vectors(p, n, hv, hq, 4 * lane, gate, kh, qs);       // every warp computes the same 128 values
-        if (warp == 0) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                s_gate[4 * lane + e] = gate[e];
-                s_kh[4 * lane + e] = kh[e];
-                s_qs[4 * lane + e] = qs[e];
-            }
-        }
+        dec_key_vectors(p, n, hv, hq, 4 * lane, gate, kh, qs);
+        *reinterpret_cast<float4*>(&vec[0][4 * lane]) = make_float4(gate[0], gate[1], gate[2], gate[3]);
+        *reinterpret_cast<float4*>(&vec[1][4 * lane]) = make_float4(kh[0], kh[1], kh[2], kh[3]);
+        *reinterpret_cast<float4*>(&vec[2][4 * lane]) = make_float4(qs[0], qs[1], qs[2], qs[3]);
+        __syncwarp();
     }
-    const int rg = lane >> 3, cg = lane & 7;
-    for (int c0 = slice * per_cta; c0 < (slice + 1) * per_cta; c0 += 32) {
-    float4 row[8];
+    const float beta = 1.f / (1.f + __expf(-dec_load(p.b, p.b_fp32, (size_t)n * p.HV + hv)));
+    const __nv_bfloat16* vp = reinterpret_cast<const __nv_bfloat16*>(p.v) + ((size_t)n * p.HV + hv) * p.V + c;      // v and o may be unaligned
+    const float2 v0 = make_float2(__bfloat162float(vp[0]), __bfloat162float(vp[1])), v1 = make_float2(__bfloat162float(vp[2]), __bfloat162float(vp[3]));
+    auto over_rows = [&](float4 a) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-        row[i] = __ldcs(reinterpret_cast<const float4*>(S + (size_t)(32 * warp + rg + 4 * i) * p.V + c0 + 4 * cg));
-    __syncthreads();
+        for (int o = 4; o < 32; o <<= 1) {
+            a.x += __shfl_xor_sync(0xffffffffu, a.x, o); a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+            a.z += __shfl_xor_sync(0xffffffffu, a.z, o); a.w += __shfl_xor_sync(0xffffffffu, a.w, o);
+        }
+        return a;
+    };
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int kk = 32 * warp + rg + 4 * i;
-        const float w = s_gate[kk] * s_kh[kk];
+    for (int i = 0; i < 16; ++i) {
+        const float w = vec[0][8 * i + rg] * vec[1][8 * i + rg];
         acc.x = fmaf(row[i].x, w, acc.x); acc.y = fmaf(row[i].y, w, acc.y);
         acc.z = fmaf(row[i].z, w, acc.z); acc.w = fmaf(row[i].w, w, acc.w);
     }
-#pragma unroll
-    for (int o = 8; o < 32; o <<= 1) {
-        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o); acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
-        acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o); acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
-    }
-    if (rg == 0) *reinterpret_cast<float4*>(&red[0][warp][4 * cg]) = acc;
-    __syncthreads();
-    float vn[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const int c = 4 * cg + e;
-        const float hk = (red[0][0][c] + red[0][1][c]) + (red[0][2][c] + red[0][3][c]);
-        vn[e] = beta * (__bfloat162float(vp[c0 + c]) - hk);
-    }
+    acc = over_rows(acc);
+    const float4 vn = make_float4(beta * (v0.x - acc.x), beta * (v0.y - acc.y), beta * (v1.x - acc.z), beta * (v1.y - acc.w));
     acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int kk = 32 * warp + rg + 4 * i;
-        const float gt = s_gate[kk], kh = s_kh[kk], qv = s_qs[kk];
-        row[i].x = fmaf(gt, row[i].x, kh * vn[0]); row[i].y = fmaf(gt, row[i].y, kh * vn[1]);
-        row[i].z = fmaf(gt, row[i].z, kh * vn[2]); row[i].w = fmaf(gt, row[i].w, kh * vn[3]);
-        __stcs(reinterpret_cast<float4*>(S + (size_t)kk * p.V + c0 + 4 * cg), row[i]);
+    for (int i = 0; i < 16; ++i) {
+        const float gt = vec[0][8 * i + rg], kh = vec[1][8 * i + rg], qv = vec[2][8 * i + rg];
+        row[i].x = fmaf(gt, row[i].x, kh * vn.x); row[i].y = fmaf(gt, row[i].y, kh * vn.y);
+        row[i].z = fmaf(gt, row[i].z, kh * vn.z); row[i].w = fmaf(gt, row[i].w, kh * vn.w);
+        __stcs(reinterpret_cast<float4*>(S + (size_t)(8 * i) * p.V), row[i]);
         acc.x = fmaf(row[i].x, qv, acc.x); acc.y = fmaf(row[i].y, qv, acc.y);
         acc.z = fmaf(row[i].z, qv, acc.z); acc.w = fmaf(row[i].w, qv, acc.w);
     }
-#pragma unroll
-    for (int o = 8; o < 32; o <<= 1) {
-        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o); acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
-        acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o); acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
+    acc = over_rows(acc);
+    if (rg == 0) {
+        op[0] = __float2bfloat16_rn(acc.x); op[1] = __float2bfloat16_rn(acc.y);
+        op[2] = __float2bfloat16_rn(acc.z); op[3] = __float2bfloat16_rn(acc.w);
     }
-    if (rg == 0) *reinterpret_cast<float4*>(&red[1][warp][4 * cg]) = acc;
-    __syncthreads();
-    if (tid < 32) op[c0 + tid] = __float2bfloat16_rn((red[1][0][tid] + red[1][1][tid]) + (red[1][2][tid] + red[1][3][tid]));
-    }   // column chunks (the barriers above also order the reuse of `red`)
 }
 
-// Persistent: a few CTAs per SM walk the work items, so the short items do not pay a CTA launch each.
-__global__ void __launch_bounds__(DEC_THREADS, 4) kda_decode_kernel(const DecodeParams p, const int items) {
-    __shared__ float red[2][4][32];
-    __shared__ float s_gate[DK], s_kh[DK], s_qs[DK];
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
-        dec_item(p, item, red, s_gate, s_kh, s_qs);
-        if (p.state_kv) __syncthreads();                    // the shared vectors are rewritten by the next item
-    }
+// One item per CTA (vk) or per warp (kv): a CTA that ends makes room for one that starts with all its loads, so that the memory
+// system always has requests. (As four resident CTAs per SM that walked the items, 256 sequences x 32 heads in vk took 185.6 us a call for
+// 1.08 GB; now 182.5, and 181 to 171 with the same pool over and over. Five or six CTAs per SM spill: 186, 208.)
+__global__ void __launch_bounds__(DEC_THREADS, 4) kda_decode_kernel(const DecodeParams p) { dec_item(p, blockIdx.x); }
+__global__ void __launch_bounds__(DEC_THREADS, 4) kda_decode_kv_kernel(const DecodeParams p, const int items) {
+    __shared__ float vec[DEC_THREADS / 32][3][DK];
+    const int warp = threadIdx.x >> 5;
+    const long long item = (long long)(DEC_THREADS / 32) * blockIdx.x + warp;
+    if (item < items) dec_item_kv(p, (int)item, vec[warp]);
 }
 
 }  // namespace kda
@@ -248,6 +252,12 @@ extern "C" int kda_launch_decode(const void* q, const void* k, const void* v, co
     p.o = o; p.N = N; p.H = H; p.HV = HV; p.V = V; p.pool = pool; p.a_fp32 = a_fp32; p.b_fp32 = b_fp32; p.use_l2norm = use_l2norm;
     p.state_kv = state_kv; p.scale = scale; p.softplus_beta = softplus_beta; p.softplus_threshold = softplus_threshold;
     p.status = status;
+    if (state_kv) {
+        const long long items = (long long)N * HV * (V / 16), ctas = (items + DEC_THREADS / 32 - 1) / (DEC_THREADS / 32);
+        if (items > 0x7fffffffLL) return -1;
+        kda_decode_kv_kernel<<<(int)ctas, DEC_THREADS, 0, stream>>>(p, (int)items);
+        return (int)cudaGetLastError();
+    }
     // enough CTAs to fill the machine several times over, else as few (= as much work per CTA) as possible
     const int sms = sm_count();
     int slices = 1;
@@ -255,7 +265,6 @@ extern "C" int kda_launch_decode(const void* q, const void* k, const void* v, co
     p.slices = slices;
     const long long items = (long long)N * HV * slices;
     if (items > 0x7fffffffLL) return -1;
-    const long long resident = 4LL * sms;                   // launch bounds keep four 128-thread CTAs resident per SM
-    kda_decode_kernel<<<(int)(items < resident ? items : resident), DEC_THREADS, 0, stream>>>(p, (int)items);
+    kda_decode_kernel<<<(int)items, DEC_THREADS, 0, stream>>>(p);
     return (int)cudaGetLastError();
 }
