@@ -108,3 +108,21 @@ def test_argument_errors():
         chunk_gated_delta_rule(q, q, q, torch.zeros(2, 8, 1, 128), g)
     with pytest.raises(AssertionError, match="A_log"):
         chunk_gated_delta_rule(q, q, q, g, g, use_gate_in_kernel=True)
+
+
+@pytest.mark.parametrize("T", [1, 15, 16, 17, 33, 48, 64, 65])
+def test_scalar_gate_backward_at_block_edges(T):
+    """The per-head gate's own path through the gated backward stage, with the last chunk around every 16-row block edge."""
+    B, H = 1, 2
+    gen = torch.Generator().manual_seed(31)
+    rn = lambda *s: torch.randn(*s, generator=gen)
+    leaves = dict(q=rn(B, T, H, 128).to(torch.bfloat16), k=rn(B, T, H, 128).to(torch.bfloat16), v=rn(B, T, H, 128).to(torch.bfloat16),
+                  g=F.logsigmoid(rn(B, T, H)) / 4.0, beta=torch.sigmoid(rn(B, T, H)).to(torch.bfloat16), h0=0.5 * rn(B, H, 128, 128))
+    do, dht = rn(B, T, H, 128).to(torch.bfloat16), 0.3 * rn(B, H, 128, 128)
+    flags = dict(use_qk_l2norm_in_kernel=True, use_gate_in_kernel=False)
+    ref_in = {n: t.detach().float().requires_grad_(True) for n, t in leaves.items()}
+    o_ref, ht_ref = chunk_gdn_oracle(ref_in["q"], ref_in["k"], ref_in["v"], ref_in["g"], ref_in["beta"], initial_state=ref_in["h0"],
+                                     output_final_state=True, **flags)
+    ((o_ref * do.float()).sum() + (ht_ref * dht).sum()).backward()
+    o, ht, got = _run(leaves, flags, do, dht)
+    _check(o, ht, got, o_ref.detach(), ht_ref.detach(), {n: t.grad for n, t in ref_in.items()}, f"T{T}")

@@ -385,3 +385,25 @@ def test_forward_backward_is_capturable_in_a_cuda_graph():
             else:
                 assert torch.equal(grads_static[n], fresh[n].grad), n
     check_status()
+
+
+@pytest.mark.parametrize("g_dtype,gate,safe,l2", [(torch.bfloat16, True, True, True), (torch.float32, False, False, False),
+                                                  (torch.float32, True, False, True)])
+def test_gated_stage_at_block_edges(g_dtype, gate, safe, l2):
+    """Last chunks that end on, before and after every 16-row block edge (the block-pair factors and the split of the rows
+    between the warp groups change there), for both gate element types and activations, from strong to weak decay."""
+    lens = [1, 2, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65]
+    H, T = 2, sum(lens)
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32)
+    inp = make_inputs(1, T, H, seed=23, gate_offset=-5.0)
+    if not gate:
+        inp["g"] = (F.logsigmoid(torch.randn(1, T, H, 128, generator=torch.Generator().manual_seed(3))) / 3.0).clamp(-5, 0)
+    inp["g"] = inp["g"].to(g_dtype)
+    if not l2:
+        inp["q"], inp["k"] = (F.normalize(inp[n].float(), dim=-1).to(torch.bfloat16) for n in ("q", "k"))
+    gen = torch.Generator().manual_seed(1)
+    inp["initial_state"] = torch.randn(len(lens), H, 128, 128, generator=gen)
+    do = torch.randn(1, T, H, 128, generator=gen).to(torch.bfloat16)
+    dht = torch.randn(len(lens), H, 128, 128, generator=gen)
+    ref, got = run_both(inp, do, dht, cu_seqlens=cu, l2=l2, gate=gate, safe=safe)
+    assert_grads(ref, got, SUITE_TOL, "block edges")
