@@ -176,7 +176,7 @@ class CudaBackend:
 
 _SM_COUNT: dict = {}
 MAX_AUTO_SEGMENTS = 8       # upper bound of `auto_segments`; 1 switches the single-GPU segmentation off
-AUTO_SEGMENT_CHUNKS = 128   # shortest sequence, in chunks, that `auto_segments` cuts
+AUTO_SEGMENT_CHUNKS = 24    # shortest segment, in chunks, that `auto_segments` makes
 
 
 def auto_segments(num_chunks, heads, device):
@@ -185,15 +185,15 @@ def auto_segments(num_chunks, heads, device):
     pass pays for itself -- a transition scan of all segments but the last (two CTAs per segment and head), a fold per
     boundary, and then all segments scanned side by side from their now-known incoming states. Both passes cost about
     the same per chunk, so that three segments are the least that gains; all CTAs of a pass have to find an SM of their
-    own; and below some hundred chunks the extra launches eat the gain (a step is about 1.6 us, a fold and its launch
-    8 us). The role of the intra-card mode of flash-linear-attention's merge kernel
+    own; and below some tens of chunks per segment the extra launches eat the gain (a step is about 1.6 us, a fold and
+    its launch 8 us). The role of the intra-card mode of flash-linear-attention's merge kernel
     (fla/ops/cp/chunk_delta_h.py:321-357)."""
     key = str(device)
     if key not in _SM_COUNT:
         _SM_COUNT[key] = torch.cuda.get_device_properties(device).multi_processor_count
     sms = _SM_COUNT[key]
-    P = min(MAX_AUTO_SEGMENTS, sms // (2 * heads) + 1, sms // heads, num_chunks // 64)
-    return P if P >= 3 and num_chunks >= AUTO_SEGMENT_CHUNKS else 1
+    P = min(MAX_AUTO_SEGMENTS, sms // (2 * heads) + 1, sms // heads, num_chunks // AUTO_SEGMENT_CHUNKS)
+    return P if P >= 3 else 1
 
 
 def gather_with_group(group=None):

@@ -366,3 +366,15 @@ def test_chunk_parallel_stage_at_block_edges(gate, safe, l2, g_dtype):
     o, ht = run_chunk_kda(inp, cu_seqlens=cu, l2=l2, gate=gate, safe=safe)
     o_ref, ht_ref = oracle_fwd(inp, cu_seqlens=cu, l2=l2, gate=gate, safe=safe)
     assert_fwd_close(o, ht, o_ref, ht_ref, ht_tol=2e-3)
+
+
+@pytest.mark.parametrize("T,H,h0_std", [(72 * 64 - 1, 1, 0.0), (128 * 64, 3, 1.0), (150 * 64 + 17, 16, 1.0)])
+def test_segmented_scan_matches_oracle(T, H, h0_std):
+    """One sequence at and around the shortest length whose scan is cut into side-by-side segments (weak decay, so that the
+    state that crosses the cuts matters)."""
+    from cula_b200.kda import cp
+    inp = make_inputs(1, T, H, seed=25, gate_offset=-8.0, h0_std=h0_std)
+    assert cp.auto_segments((T + 63) // 64, H, torch.device("cuda")) > 1
+    o, ht = run_chunk_kda(inp)
+    o_ref, ht_ref = oracle_fwd(inp)
+    assert_fwd_close(o, ht, o_ref, ht_ref, ht_tol=2e-3)
