@@ -1,12 +1,19 @@
-// Reverse state scan of the backward pass (mirror of kda_fwd_scan.cu).
+// Reverse state scan of the backward pass, on tcgen05 (the mirror of kda_fwd_scan.cu).
 //
-// One CTA per (sequence, head, half of the value columns); four consumer warps each own 16 value columns of
-// the fp32 state gradient dS^T (16 x 128 per warp) in mma.sync accumulator registers and walk the chunks
-// from last to first:
-//     dVn^T  = dS'^T Kg^T + dO^T Aqk                 (gradient w.r.t. v_new; stored for the chunk-parallel stage)
-//     dS^T  <- dS'^T diag(decay) + dO^T Qg - dVn^T W  (gradient w.r.t. the state entering the chunk)
-// A fifth warp streams the forward tile packs (W, QG, KG, AQK, DECAY) and the dO rows of the chunk through a
-// 3-stage shared-memory ring with bulk copies on mbarriers.
+// One CTA per (sequence, head) walks the chunks from last to first and carries the fp32 gradient of the state TRANSPOSED in tensor
+// memory (dS^T: lane = value column, column = key channel); per chunk
+//     ADO    = dO^T Aqk                              dO as fp16 A operand in tensor memory; nothing of this is on the chain
+//     ACC    = S16 KG^T                              S16: dS' as fp16 A operand, one power-of-two scale per lane
+//     dVn^T  = ACC + ADO                             gradient of v_new -> fp16 A operand (negated) and HBM
+//     dS^T   = dS'^T diag(decay) + dO^T QG - dVn^T W (gradient of the state entering the chunk)
+// What bounds a few long sequences is the latency of that chain: two MMA groups and two register passes per chunk. What bounds a
+// full GPU is HBM, 154 KB in and out per chunk. (The register-resident mma.sync version of this scan ran 224 dependent-issue
+// MMAs per warp and chunk: 3.2 us per chunk.) The warps are those of the forward scan:
+//   warps 0-3     dVn: lane-per-column values become token rows in shared memory and leave as one bulk store;
+//   warps 4-19    dS': out of tensor memory, fp16 copy back in (chain), then the decayed state, dS' per chunk to HBM, dht / dh0;
+//   warps 20-27   dVn (chain), 32 tokens each, and between two chunks the next dO as operand;
+//   warp 28       issues the MMAs;
+//   warp 29       streams the tile packs and the dO rows (2 stages) by TMA.
 //
 // Replaces chunk_gated_delta_rule_bwd_dhu (flash-linear-attention, fla/ops/common/chunk_delta_h.py:316-718, called
 // at cula/kda/chunk_bwd.py:541-555) and the dv half of chunk_kda_bwd_kernel_dAv (cula/kda/chunk_bwd.py:63-125).
@@ -15,18 +22,23 @@
 // from max|dO|, max|dht| (kda_grad_scale_kernel), so fp16 MMA operands neither overflow nor go subnormal.
 #include "kda_common.cuh"
 #include "kda_params.h"
+#include "scan_common.cuh"
 
 namespace kda {
 
-constexpr int BS_STAGES = 3;
-constexpr int BS_DO_ROW = 144;                               // padded dO row (64 bf16 + 16 B): conflict-free ldmatrix
-constexpr int BS_DO_BYTES = BT * BS_DO_ROW;                  // 9216
-constexpr int BS_STAGE_BYTES = TP_HEAD_BYTES + BS_DO_BYTES;  // 67072
-constexpr int BS_STG_BYTES = 2048;                           // per-warp staging for the dVn store
-constexpr int BS_CONSUMERS = 4;
-constexpr int BS_THREADS = (BS_CONSUMERS + 1) * 32;
-constexpr int BS_SMEM = BS_STAGES * BS_STAGE_BYTES + BS_CONSUMERS * BS_STG_BYTES + 64;
-constexpr int BS_DO = TP_HEAD_BYTES;
+constexpr int BS_STAGES = 2;
+constexpr int BS_OUT_WARPS = 4, BS_STATE_WARPS = 16, BS_VALUE_WARPS = 8;
+constexpr int BS_MMA_WARP = BS_OUT_WARPS + BS_STATE_WARPS + BS_VALUE_WARPS, BS_LOAD_WARP = BS_MMA_WARP + 1;
+constexpr int BS_THREADS = 32 * (BS_LOAD_WARP + 1);
+// shared-memory stage: W, QG, KG as [2 atoms of 64 channels][64 tokens][128 B], Aqk, the dO rows as they are, the decays
+constexpr int BS_W = 0, BS_QG = 16384, BS_KG = 32768, BS_AQK = 49152, BS_DO = 57344, BS_DECAY = 73728, BS_STAGE_BYTES = 74752;
+static_assert(BS_STAGE_BYTES % 1024 == 0, "operand atoms are 1024-byte aligned");
+constexpr int BS_OST_BYTES = BT * DV * 2;                    // staged dVn rows
+constexpr int BS_OST = BS_STAGES * BS_STAGE_BYTES, BS_MISC = BS_OST + 2 * BS_OST_BYTES;
+constexpr int BS_SMEM = BS_MISC + 8448 + 1024;
+// tensor-memory columns: dS, its fp16 copy, two S16 KG^T accumulators (by turn parity; -dVn replaces what was read), two dO
+// operands (by turn parity), dO^T Aqk
+constexpr uint32_t BM_S32 = 0, BM_S16 = 128, BM_ACC = 192, BM_DO = 320, BM_ADO = 384;
 
 // s = 2^k with max(|dO|, |dht|) * s in [4, 8); written as {s, 1/s}. amax_bits holds the running maximum.
 __global__ void kda_grad_amax_kernel(const __nv_bfloat16* d_o, size_t n_do, const float* dht, size_t n_dht,
@@ -64,13 +76,23 @@ __global__ void kda_grad_scale_kernel(const unsigned int* amax_bits, float* gsca
     gscale[1] = __int_as_float((127 - shift) << 23);
 }
 
-__global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdScanParams p) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + BS_STAGES * BS_STAGE_BYTES + BS_CONSUMERS * BS_STG_BYTES);
-    uint64_t* empty = full + BS_STAGES;
+__global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdScanParams p, const __grid_constant__ CUtensorMap map,
+                                                                     const __grid_constant__ CUtensorMap map_do) {
+    extern __shared__ unsigned char bs_smem_raw[];
+    unsigned char* sm = bs_smem_raw + ((1024u - (smem_u32(bs_smem_raw) & 1023u)) & 1023u);
+    const uint32_t smb = smem_u32(sm);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + BS_MISC);
+    uint64_t *full = bars, *empty = bars + 2, *b_s16 = bars + 4, *b_dec = bars + 5, *b_acc = bars + 6, *b_s32 = bars + 7, *b_do = bars + 8,
+             *b_ado = bars + 9, *b_ost = bars + 10, *b_vsum = bars + 11, *b_max = bars + 12 /* [4] */;
+    // pairs, because a wait by phase parity must not fall two completions behind (see kda_fwd_scan.cu): turn i uses barrier i & 1
+    uint64_t *b_v16 = bars + 16 /* [2] */, *b_oread = bars + 18 /* [2] */;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + BS_MISC + 192);
+    float* sDown = reinterpret_cast<float*>(sm + BS_MISC + 256);         // [4 turns][128 value columns] 1 / scale of S16
+    float* sMax = reinterpret_cast<float*>(sm + BS_MISC + 2304);         // [2 turn parities][4 key quarters][128] largest |dS'| of a column
+    float* sVsum = reinterpret_cast<float*>(sm + BS_MISC + 6400);        // [2 turn parities][2 token halves][128] sum of |dVn| + |dO|
+
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int vh = blockIdx.x, h = blockIdx.y;
-    const int n = p.seq_order ? p.seq_order[blockIdx.z] : blockIdx.z;
+    const int h = blockIdx.x, n = p.seq_order ? p.seq_order[blockIdx.y] : blockIdx.y;
     int bos, len, chunk0;
     if (p.cu_seqlens) {
         bos = p.cu_seqlens[n];
@@ -86,221 +108,321 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
     if (tid == 0) {
         for (int s = 0; s < BS_STAGES; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], BS_CONSUMERS);
+            mbar_init(&empty[s], 1 + BS_STATE_WARPS + BS_VALUE_WARPS);
+        }
+        mbar_init(b_s16, BS_STATE_WARPS);
+        mbar_init(b_dec, BS_STATE_WARPS);
+        mbar_init(b_acc, 1);
+        mbar_init(b_s32, 1);
+        mbar_init(b_do, BS_VALUE_WARPS);
+        mbar_init(b_ado, 1);
+        mbar_init(b_ost, BS_OUT_WARPS);
+        mbar_init(b_vsum, BS_VALUE_WARPS);
+        for (int q = 0; q < 4; ++q) mbar_init(&b_max[q], BS_STATE_WARPS / 4);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&b_v16[b], BS_VALUE_WARPS);
+            mbar_init(&b_oread[b], BS_OUT_WARPS);
         }
         fence_mbar_init();
     }
+    if (warp == BS_MMA_WARP) umma::tmem_alloc(tmem_slot, 512);
+    umma::fence_before_sync();
     __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tmem = *tmem_slot;
 
-    if (warp == BS_CONSUMERS) {
-        // ------------------------------- producer warp (all lanes copy dO rows) -------------------------------
-        const __nv_bfloat16* dop = reinterpret_cast<const __nv_bfloat16*>(p.d_o);
+    auto wait = [&](uint64_t* bar, int phase) -> bool {
+        if (mbar_wait(bar, phase & 1)) return true;
+        report_status(p.status, STATUS_WAIT_TIMEOUT);
+        return false;
+    };
+
+    if (warp == BS_LOAD_WARP) {
+        // ------------------------------- producer -------------------------------
+        if (lane == 0) {
+            int issued = 0;
+            bool ok = true;
+            for (int it = 0; it < nchunks; ++it) {
+                const int c = nchunks - 1 - it, s = it % BS_STAGES, use = it / BS_STAGES;
+                if (use > 0 && !(ok = wait(&empty[s], use - 1))) break;
+                const int t_id = (chunk0 + c) * p.H + h;
+                const unsigned char* tile = p.tiles + (size_t)t_id * TP_BYTES;
+                unsigned char* dst = sm + s * BS_STAGE_BYTES;
+                const uint32_t d = smb + s * BS_STAGE_BYTES;
+                mbar_arrive_expect_tx(&full[s], 4 * 16384 + 8192 + 512);
+                tma_load_3d(d + BS_DO, &map_do, 0, h, bos + c * BT, &full[s]);     // first: the value warps work on it ahead of the chain
+                bulk_g2s(dst + BS_AQK, tile + TP_AQK, 8192, &full[s]);
+#pragma unroll
+                for (int m = 2; m >= 0; --m)       // KG, QG, W
+#pragma unroll
+                    for (int a = 0; a < 2; ++a) tma_load_4d(d + m * 16384 + a * 8192, &map, 0, a, 64 * m, t_id, &full[s]);
+                bulk_g2s(dst + BS_DECAY, tile + TP_DECAY, 512, &full[s]);
+                issued = it + 1;
+            }
+            // do not leave with copies to this CTA's shared memory in flight
+            if (!ok)
+                for (int it = max(0, issued - BS_STAGES); it < issued; ++it) mbar_wait(&full[it % BS_STAGES], (it / BS_STAGES) & 1);
+        }
+    } else if (warp == BS_MMA_WARP) {
+        // ------------------------------- MMA issue (the whole warp in step, one elected lane issues) -------------------------------
+        const uint32_t id_kg = umma::make_idesc(umma::FMT_F16, 128, 64, false, false);
+        const uint32_t id_qw = umma::make_idesc(umma::FMT_F16, 128, 128, false, true);
+        const uint32_t id_a = umma::make_idesc(umma::FMT_F16, 128, 64, false, true);
+        for (int it = 0; it < nchunks; ++it) {
+            const int s = it % BS_STAGES;
+            const uint32_t st = smb + s * BS_STAGE_BYTES;
+            const uint64_t d_kg = sc_sdesc(st + BS_KG, 16, 1024), d_qg = sc_sdesc(st + BS_QG, 8192, 1024), d_w = sc_sdesc(st + BS_W, 8192, 1024),
+                           d_a = sc_sdesc(st + BS_AQK, 8192, 1024);
+            const uint32_t acc = tmem + BM_ACC + 64 * (it & 1), t_do = tmem + BM_DO + 32 * (it & 1);
+            if (!wait(&full[s], it / BS_STAGES) || !wait(b_do, it)) break;
+            umma::fence_after_sync();
+            if (umma::elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks) umma::mma_f16_ta(tmem + BM_ADO, t_do + 8 * ks, d_a + ((ks * 2048) >> 4), id_a, ks != 0);
+                umma::commit(b_ado);
+            }
+            __syncwarp();
+            if (!wait(b_s16, it)) break;
+            umma::fence_after_sync();
+            if (umma::elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < 8; ++ks)
+                    umma::mma_f16_ta(acc, tmem + BM_S16 + 8 * ks, d_kg + (((ks >> 2) * 8192 + (ks & 3) * 32) >> 4), id_kg, ks != 0);
+                umma::commit(b_acc);
+            }
+            __syncwarp();
+            if (!wait(b_dec, it)) break;
+            umma::fence_after_sync();
+            if (umma::elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks) umma::mma_f16_ta(tmem + BM_S32, t_do + 8 * ks, d_qg + ((ks * 2048) >> 4), id_qw, 1);
+            }
+            __syncwarp();
+            if (!wait(&b_v16[it & 1], it >> 1)) break;
+            umma::fence_after_sync();
+            if (umma::elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks)       // -dVn^T: tokens 0..31 in columns 0..15, tokens 32..63 in columns 32..47 of the accumulator
+                    umma::mma_f16_ta(tmem + BM_S32, acc + 32 * (ks >> 1) + 8 * (ks & 1), d_w + ((ks * 2048) >> 4), id_qw, 1);
+                umma::commit(b_s32);
+                umma::commit(&empty[s]);
+            }
+            __syncwarp();
+            // the dVn of the turn before has been read: its accumulator is free for the next turn
+            if (p.dvn_out && it > 0 && !wait(&b_oread[(it - 1) & 1], (it - 1) >> 1)) break;
+        }
+    } else if (warp >= BS_OUT_WARPS && warp < BS_OUT_WARPS + BS_STATE_WARPS) {
+        // ------------------------------- dS: lane = value column v, 32 key channels per warp -------------------------------
+        const int q = warp & 3, kq = (warp - BS_OUT_WARPS) >> 2, v = 32 * q + lane, k0 = 32 * kq;
+        const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
+        float s[32];
+        if (p.dht) {
+            const float gs = p.gscale[0];
+            const float* d0 = p.dht + ((size_t)n * p.H + h) * DK * DV + (size_t)k0 * DV + v;
+#pragma unroll
+            for (int k = 0; k < 32; ++k) s[k] = gs * d0[(size_t)k * DV];
+        } else {
+#pragma unroll
+            for (int k = 0; k < 32; ++k) s[k] = 0.f;
+        }
+        auto load_state = [&]() {
+            umma::ld_32x32b_x32(tl + BM_S32 + k0, reinterpret_cast<uint32_t(&)[32]>(s));
+            umma::wait_ld();
+        };
+        // Largest |entry| of the value column: this warp's quarter of the keys here, the others from the partner warps.
+        auto publish_max = [&](int it) -> float {
+            float m0 = 0.f, m1 = 0.f;
+#pragma unroll
+            for (int k = 0; k < 32; k += 2) {
+                m0 = fmaxf(m0, fabsf(s[k]));
+                m1 = fmaxf(m1, fabsf(s[k + 1]));
+            }
+            m0 = fmaxf(m0, m1);
+            sMax[(it & 1) * 512 + kq * 128 + v] = m0;
+            warp_arrive(&b_max[q], lane);
+            return m0;
+        };
+        bool ok = true;
+        if (nchunks > 0) publish_max(0);
         for (int it = 0; it < nchunks; ++it) {
             const int c = nchunks - 1 - it;
-            const int s = it % BS_STAGES, use = it / BS_STAGES;
-            const int valid = min(BT, len - c * BT);
-            bool ok = true;
-            if (lane == 0 && use > 0) ok = mbar_spin(&empty[s], (use - 1) & 1);
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) {
-                if (lane == 0) report_status(p.status, STATUS_WAIT_TIMEOUT);
-                break;
+            // The scale of the fp16 copy comes from a bound that is known before the state is (see kda_fwd_scan.cu):
+            // |dS| <= max |dS'| + sum |dO| max |qg| + sum |dVn| max |w|, with decays <= 1 and |qg|, |w| <= 1 for unit keys,
+            // beta <= 1 and scale <= 1 (a factor of 32 is left for others).
+            const int pt = max(it - 1, 0);
+            if (!(ok = wait(&b_max[q], pt))) break;
+            const float* mx = sMax + (pt & 1) * 512 + v;
+            float bound = fmaxf(fmaxf(mx[0], mx[128]), fmaxf(mx[256], mx[384]));
+            if (it > 0) {
+                if (!(ok = wait(b_vsum, it - 1))) break;
+                bound += sVsum[(pt & 1) * 256 + v] + sVsum[(pt & 1) * 256 + 128 + v];
             }
-            unsigned char* dst = smem + s * BS_STAGE_BYTES;
-            // rows past the end of the sequence are never copied: clear them so stale bytes cannot inject NaNs
-            for (int i = lane; i < (BT - valid) * 8; i += 32)
-                *reinterpret_cast<uint4*>(dst + BS_DO + (valid + (i >> 3)) * BS_DO_ROW + (i & 7) * 16) = make_uint4(0, 0, 0, 0);
+            int shift = 10 - (((__float_as_int(bound) >> 23) & 0xff) - 127);
+            shift = max(-100, min(100, shift));
+            const float2 up = splat2(__int_as_float((shift + 127) << 23));
+            if (kq == 0) sDown[(it & 3) * 128 + v] = __int_as_float((127 - shift) << 23);
+            if (it > 0) {
+                if (!(ok = wait(b_s32, it - 1))) break;
+                umma::fence_after_sync();
+                load_state();
+            }
+            {
+                uint32_t pk[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    const float2 x = mul2(make_float2(s[2 * e], s[2 * e + 1]), up);
+                    pk[e] = pack_f16(x.x, x.y);
+                }
+                umma::st_32x32b_x16(tl + BM_S16 + 16 * kq, pk);
+            }
+            umma::wait_st();
+            umma::fence_before_sync();
+            warp_arrive(b_s16, lane);
+            // ---- beside the MMAs: the decayed state, then dS' (gradient of the state leaving this chunk) to HBM ----
+            const int st = it % BS_STAGES;
+            if (!(ok = wait(&full[st], it / BS_STAGES))) break;
+            const float* dec = reinterpret_cast<const float*>(sm + st * BS_STAGE_BYTES + BS_DECAY) + k0;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                uint32_t r[8];
+#pragma unroll
+                for (int e = 0; e < 8; e += 4) {
+                    const float4 d = *reinterpret_cast<const float4*>(dec + 8 * b + e);
+                    const float2 x = mul2(make_float2(s[8 * b + e], s[8 * b + e + 1]), make_float2(d.x, d.y));
+                    const float2 y = mul2(make_float2(s[8 * b + e + 2], s[8 * b + e + 3]), make_float2(d.z, d.w));
+                    r[e] = __float_as_uint(x.x); r[e + 1] = __float_as_uint(x.y); r[e + 2] = __float_as_uint(y.x); r[e + 3] = __float_as_uint(y.y);
+                }
+                umma::st_32x32b_x8(tl + BM_S32 + k0 + 8 * b, r);
+            }
+            warp_arrive(&empty[st], lane);
+            umma::wait_st();
+            umma::fence_before_sync();
+            warp_arrive(b_dec, lane);
+            // operands far from the assumption can defeat the bound: say so instead of carrying inf on
+            if (it > 0 && overflows(publish_max(it) * up.x)) report_status(p.status, STATUS_RANGE);
+            if (p.ds_out) {
+                float* dsg = p.ds_out + ((size_t)(chunk0 + c) * p.H + h) * (size_t)(DK * DV) + (size_t)k0 * DV + v;
+#pragma unroll
+                for (int k = 0; k < 32; ++k) dsg[(size_t)k * DV] = s[k];
+            }
+        }
+        if (ok && nchunks > 0 && (ok = wait(b_s32, nchunks - 1))) {
+            umma::fence_after_sync();
+            load_state();
+        }
+        if (ok && p.dh0) {
+            const float gs_inv = p.gscale[1];
+            float* d0 = p.dh0 + ((size_t)n * p.H + h) * DK * DV + (size_t)k0 * DV + v;
+#pragma unroll
+            for (int k = 0; k < 32; ++k) d0[(size_t)k * DV] = gs_inv * s[k];
+        }
+    } else if (warp >= BS_OUT_WARPS + BS_STATE_WARPS) {
+        // ------------------------------- dVn: lane = value column v, 32 tokens per warp -------------------------------
+        const int q = warp & 3, th = (warp - BS_OUT_WARPS - BS_STATE_WARPS) >> 2, v = 32 * q + lane, t0 = 32 * th;
+        const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
+        const float gs = p.gscale[0];
+        float dosum = 0.f;
+        // dO^T of a turn as fp16 A operand, in units of gs; rows past the end of the sequence belong to others and count as zero
+        auto convert = [&](int it) -> bool {
+            const int st = it % BS_STAGES, rows = min(BT, len - (nchunks - 1 - it) * BT) - t0;
+            if (!wait(&full[st], it / BS_STAGES)) return false;
+            const unsigned char* src = sm + st * BS_STAGE_BYTES + BS_DO + t0 * 256 + v * 2;
+            uint32_t pk[16];
+            float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                const uint32_t a = *reinterpret_cast<const uint16_t*>(src + (2 * e) * 256), b = *reinterpret_cast<const uint16_t*>(src + (2 * e + 1) * 256);
+                const float2 f = make_float2(2 * e < rows ? gs * __uint_as_float(a << 16) : 0.f, 2 * e + 1 < rows ? gs * __uint_as_float(b << 16) : 0.f);
+                sum.x += fabsf(f.x);
+                sum.y += fabsf(f.y);
+                pk[e] = pack_f16(f.x, f.y);
+            }
+            dosum = sum.x + sum.y;
+            umma::st_32x32b_x16(tl + BM_DO + 32 * (it & 1) + 16 * th, pk);
+            warp_arrive(&empty[st], lane);
+            umma::wait_st();
+            umma::fence_before_sync();
+            warp_arrive(b_do, lane);
+            return true;
+        };
+        bool ok = nchunks == 0 || convert(0);
+        for (int it = 0; ok && it < nchunks; ++it) {
+            uint32_t ado[32];
+            if (!wait(b_ado, it)) break;
+            umma::fence_after_sync();
+            umma::ld_32x32b_x32(tl + BM_ADO + t0, ado);
+            umma::wait_ld();
+            if (!wait(b_s16, it) || !wait(b_acc, it)) break;
+            umma::fence_after_sync();
+            const uint32_t acc = tl + BM_ACC + 64 * (it & 1) + t0;
+            const float2 down = splat2(sDown[(it & 3) * 128 + v]);
+            float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                uint32_t r[16], pk[8];
+                umma::ld_32x32b_x16(acc + 16 * b, r);
+                umma::wait_ld();
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float2 x = fma2(make_float2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])), down,
+                                          make_float2(__uint_as_float(ado[16 * b + 2 * e]), __uint_as_float(ado[16 * b + 2 * e + 1])));
+                    pk[e] = pack_f16(x.x, x.y) ^ 0x80008000u;
+                    sum.x += fabsf(x.x);
+                    sum.y += fabsf(x.y);
+                }
+                umma::st_32x32b_x8(acc + 8 * b, pk);      // columns this warp has already read
+            }
+            umma::wait_st();
+            umma::fence_before_sync();
+            warp_arrive(&b_v16[it & 1], lane);
+            sVsum[(it & 1) * 256 + th * 128 + v] = sum.x + sum.y + dosum;
+            warp_arrive(b_vsum, lane);
+            // the operand buffer and the product of two turns ago are free: b_acc of this turn came after their last MMA
+            if (it + 1 < nchunks) ok = convert(it + 1);
+        }
+    } else if (p.dvn_out) {
+        // ------------------------------- dVn rows: lane = value column v, all tokens -------------------------------
+        const int q = warp, v = 32 * q + lane;
+        const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
+        const int odd = lane & 1;
+        const uint32_t sel = odd ? 0x3276u : 0x5410u;
+        for (int it = 0; it < nchunks; ++it) {
+            const uint32_t acc = tl + BM_ACC + 64 * (it & 1);
+            if (!wait(&b_v16[it & 1], it >> 1)) break;
+            umma::fence_after_sync();
+            unsigned char* buf = sm + BS_OST + (it & 1) * BS_OST_BYTES;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                uint32_t w[8];
+                umma::ld_32x32b_x8(acc + 32 * (b >> 1) + 8 * (b & 1), w);
+                umma::wait_ld();
+                if (b == 3) {
+                    umma::fence_before_sync();
+                    warp_arrive(&b_oread[it & 1], lane);
+                }
+                // a register holds tokens 2e and 2e + 1 of this column; neighbouring lanes trade halves, so that the even lane
+                // stores token 2e of both columns and the odd lane token 2e + 1
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const uint32_t x = __shfl_xor_sync(0xffffffffu, w[e], 1);
+                    *reinterpret_cast<uint32_t*>(buf + (16 * b + 2 * e + odd) * 256 + (v & ~1) * 2) = __byte_perm(w[e], x, sel) ^ 0x80008000u;
+                }
+            }
+            // passing the barrier of a turn also means that the copy of the turn before has been read out
             fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive_expect_tx(&full[s], TP_HEAD_BYTES + valid * 128);
-                bulk_g2s(dst, p.tiles + ((size_t)(chunk0 + c) * p.H + h) * TP_BYTES, TP_HEAD_BYTES, &full[s]);
+            if (tid == 0) bulk_wait_read_all();
+            warp_arrive(b_ost, lane);
+            if (!wait(b_ost, it)) break;
+            if (tid == 0) {
+                bulk_s2g(reinterpret_cast<unsigned char*>(p.dvn_out) + ((size_t)(chunk0 + nchunks - 1 - it) * p.H + h) * (size_t)(BT * DV * 2), buf,
+                         BS_OST_BYTES);
+                bulk_commit();
             }
-            __syncwarp();
-            for (int row = lane; row < valid; row += 32)
-                bulk_g2s(dst + BS_DO + row * BS_DO_ROW,
-                         dop + ((size_t)(bos + c * BT + row) * p.H + h) * DV + vh * 64, 128, &full[s]);
         }
-        return;
+        if (tid == 0) bulk_wait_all();
     }
-
-    // ---------------------------------- consumer warps ----------------------------------
-    const int g = lane >> 2, t = lane & 3;
-    const int m = lane >> 3, r = lane & 7;
-    const int vb = vh * 64 + warp * 16;
-    unsigned char* stg = smem + BS_STAGES * BS_STAGE_BYTES + warp * BS_STG_BYTES;
-    const uint32_t stg_u32 = smem_u32(stg);
-    const float gs = p.gscale[0], gs_inv = p.gscale[1];
-
-    float S[16][4];     // dS^T tile: rows v (g, g+8), cols k = 8*jt + 2t, +1; units of gs
-    if (p.dht) {
-        const float* d0 = p.dht + ((size_t)n * p.H + h) * DK * DV;
-#pragma unroll
-        for (int jt = 0; jt < 16; ++jt) {
-            int k0 = 8 * jt + 2 * t;
-            S[jt][0] = gs * d0[(size_t)k0 * DV + vb + g];
-            S[jt][1] = gs * d0[(size_t)(k0 + 1) * DV + vb + g];
-            S[jt][2] = gs * d0[(size_t)k0 * DV + vb + g + 8];
-            S[jt][3] = gs * d0[(size_t)(k0 + 1) * DV + vb + g + 8];
-        }
-    } else {
-#pragma unroll
-        for (int jt = 0; jt < 16; ++jt) S[jt][0] = S[jt][1] = S[jt][2] = S[jt][3] = 0.f;
-    }
-    uint32_t x256[4];
-#pragma unroll
-    for (int kp = 0; kp < 4; ++kp) x256[kp] = (uint32_t)(((4 * kp + m) ^ r) << 4);
-
-    for (int it = 0; it < nchunks; ++it) {
-        const int c = nchunks - 1 - it;
-        const int s = it % BS_STAGES;
-        if (!mbar_spin(&full[s], (it / BS_STAGES) & 1)) {
-            report_status(p.status, STATUS_WAIT_TIMEOUT);
-            return;
-        }
-        const uint32_t st = smem_u32(smem + s * BS_STAGE_BYTES);
-        const size_t tile_idx = (size_t)(chunk0 + c) * p.H + h;
-
-        // ---- dS' (gradient w.r.t. the state leaving this chunk) to HBM, fp32 [128 k][128 v] ----
-        if (p.ds_out) {
-            float* dsg = p.ds_out + tile_idx * (size_t)(DK * DV);
-#pragma unroll
-            for (int jt = 0; jt < 16; ++jt) {
-                int k0 = 8 * jt + 2 * t;
-                dsg[(size_t)k0 * DV + vb + g] = S[jt][0];
-                dsg[(size_t)(k0 + 1) * DV + vb + g] = S[jt][1];
-                dsg[(size_t)k0 * DV + vb + g + 8] = S[jt][2];
-                dsg[(size_t)(k0 + 1) * DV + vb + g + 8] = S[jt][3];
-            }
-        }
-        // ---- dS' as fp16 A fragments with a per-warp power-of-two scale ----
-        float smax = 0.f;
-#pragma unroll
-        for (int jt = 0; jt < 16; ++jt)
-            smax = fmaxf(smax, fmaxf(fmaxf(fabsf(S[jt][0]), fabsf(S[jt][1])), fmaxf(fabsf(S[jt][2]), fabsf(S[jt][3]))));
-#pragma unroll
-        for (int o = 16; o; o >>= 1) smax = fmaxf(smax, __shfl_xor_sync(0xffffffffu, smax, o));
-        int shift = 13 - (((__float_as_int(smax) >> 23) & 0xff) - 127);
-        shift = max(-100, min(100, shift));
-        const float s_up = __int_as_float((shift + 127) << 23), s_down = __int_as_float((127 - shift) << 23);
-        uint32_t sa[8][4];
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-            sa[ks][0] = pack_f16(S[2 * ks][0] * s_up, S[2 * ks][1] * s_up);
-            sa[ks][1] = pack_f16(S[2 * ks][2] * s_up, S[2 * ks][3] * s_up);
-            sa[ks][2] = pack_f16(S[2 * ks + 1][0] * s_up, S[2 * ks + 1][1] * s_up);
-            sa[ks][3] = pack_f16(S[2 * ks + 1][2] * s_up, S[2 * ks + 1][3] * s_up);
-        }
-        // ---- dO^T as fp16 A fragments (units of gs): 4 k-steps over the 64 tokens ----
-        uint32_t doa[4][4];
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-            uint32_t r0, r1, r2, r3;
-            ldsm_x4_t(st + BS_DO + (16 * ks + (m >> 1) * 8 + r) * BS_DO_ROW + (2 * warp + (m & 1)) * 16, r0, r1, r2, r3);
-            float2 f;
-            f = unpack_bf16(r0); doa[ks][0] = pack_f16(gs * f.x, gs * f.y);
-            f = unpack_bf16(r1); doa[ks][1] = pack_f16(gs * f.x, gs * f.y);
-            f = unpack_bf16(r2); doa[ks][2] = pack_f16(gs * f.x, gs * f.y);
-            f = unpack_bf16(r3); doa[ks][3] = pack_f16(gs * f.x, gs * f.y);
-        }
-        // ---- dVn^T = dS'^T Kg^T + dO^T Aqk : [16 v] x [64 tokens] ----
-        float acc[8][4];
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-#pragma unroll
-        for (int kp = 0; kp < 4; ++kp) {
-#pragma unroll
-            for (int nt = 0; nt < 8; ++nt) {
-                uint32_t b0, b1, b2, b3;
-                ldsm_x4(st + TP_KG + (8 * nt + r) * 256 + x256[kp], b0, b1, b2, b3);
-                mma_f16(acc[nt], sa[2 * kp], b0, b1);
-                mma_f16(acc[nt], sa[2 * kp + 1], b2, b3);
-            }
-        }
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-            acc[nt][0] *= s_down; acc[nt][1] *= s_down; acc[nt][2] *= s_down; acc[nt][3] *= s_down;
-        }
-        // B[k = token j][n = token i] = Aqk[j][i]: rows j, 16-byte groups along i -> transposed ldmatrix
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-#pragma unroll
-            for (int np = 0; np < 4; ++np) {
-                if (16 * np <= 16 * ks + 15) {          // Aqk[j][i] = 0 for i > j
-                    uint32_t b0, b1, b2, b3;
-                    const int row = 16 * ks + (m & 1) * 8 + r, ch = 2 * np + (m >> 1);
-                    ldsm_x4_t(st + TP_AQK + row * 128 + ((ch ^ r) << 4), b0, b1, b2, b3);
-                    mma_f16(acc[2 * np], doa[ks], b0, b1);
-                    mma_f16(acc[2 * np + 1], doa[ks], b2, b3);
-                }
-            }
-        }
-        uint32_t va[4][4];   // dVn^T as fp16 A fragments
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-            va[ks][0] = pack_f16(acc[2 * ks][0], acc[2 * ks][1]);
-            va[ks][1] = pack_f16(acc[2 * ks][2], acc[2 * ks][3]);
-            va[ks][2] = pack_f16(acc[2 * ks + 1][0], acc[2 * ks + 1][1]);
-            va[ks][3] = pack_f16(acc[2 * ks + 1][2], acc[2 * ks + 1][3]);
-        }
-        if (p.dvn_out) {   // dVn, fp16 [64 tokens][128 v]
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-                int trow = 8 * (2 * ks + (m >> 1)) + r;
-                stsm_x4_t(stg_u32 + trow * 32 + (m & 1) * 16, va[ks][0], va[ks][1], va[ks][2], va[ks][3]);
-            }
-            __syncwarp();
-            unsigned char* vg = reinterpret_cast<unsigned char*>(p.dvn_out) + tile_idx * (size_t)(BT * DV * 2);
-#pragma unroll
-            for (int i4 = 0; i4 < 4; ++i4) {
-                int row = i4 * 16 + (lane >> 1), hf = lane & 1;
-                uint4 val = *reinterpret_cast<const uint4*>(stg + row * 32 + hf * 16);
-                *reinterpret_cast<uint4*>(vg + (size_t)row * 256 + vb * 2 + hf * 16) = val;
-            }
-            __syncwarp();
-        }
-        // ---- dS^T <- dS'^T diag(decay) + dO^T Qg - dVn^T W ----
-        {
-            const float* dec = reinterpret_cast<const float*>(smem + s * BS_STAGE_BYTES + TP_DECAY);
-#pragma unroll
-            for (int jt = 0; jt < 16; ++jt) {
-                float2 d2 = *reinterpret_cast<const float2*>(dec + 8 * jt + 2 * t);
-                S[jt][0] *= d2.x; S[jt][1] *= d2.y; S[jt][2] *= d2.x; S[jt][3] *= d2.y;
-            }
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-                uint32_t vneg[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) vneg[e] = va[ks][e] ^ 0x80008000u;
-#pragma unroll
-                for (int jp = 0; jp < 8; ++jp) {
-                    uint32_t b0, b1, b2, b3;
-                    const int row = 16 * ks + (m & 1) * 8 + r, ch = 2 * jp + (m >> 1);
-                    const uint32_t off = row * 256 + ((ch ^ r) << 4);
-                    ldsm_x4_t(st + TP_QG + off, b0, b1, b2, b3);
-                    mma_f16(S[2 * jp], doa[ks], b0, b1);
-                    mma_f16(S[2 * jp + 1], doa[ks], b2, b3);
-                    ldsm_x4_t(st + TP_W + off, b0, b1, b2, b3);
-                    mma_f16(S[2 * jp], vneg, b0, b1);
-                    mma_f16(S[2 * jp + 1], vneg, b2, b3);
-                }
-            }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[s]);
-    }
-
-    if (p.dh0) {
-        float* d0 = p.dh0 + ((size_t)n * p.H + h) * DK * DV;
-#pragma unroll
-        for (int jt = 0; jt < 16; ++jt) {
-            int k0 = 8 * jt + 2 * t;
-            d0[(size_t)k0 * DV + vb + g] = gs_inv * S[jt][0];
-            d0[(size_t)(k0 + 1) * DV + vb + g] = gs_inv * S[jt][1];
-            d0[(size_t)k0 * DV + vb + g + 8] = gs_inv * S[jt][2];
-            d0[(size_t)(k0 + 1) * DV + vb + g + 8] = gs_inv * S[jt][3];
-        }
-    }
+    __syncthreads();
+    if (warp == BS_MMA_WARP) umma::tmem_dealloc(tmem, 512);
 }
 
 }  // namespace kda
@@ -319,10 +441,13 @@ extern "C" int kda_launch_grad_scale(const void* d_o, size_t n_do, const float* 
 extern "C" int kda_launch_bwd_scan(const kda::BwdScanParams* p, cudaStream_t stream) {
     using namespace kda;
     if (p->N <= 0) return 0;
-    dim3 grid(2, p->H, p->N);
     static std::atomic<unsigned long long> done;
     cudaError_t e = allow_smem(kda_bwd_scan_kernel, BS_SMEM, done);
     if (e != cudaSuccess) return (int)e;
-    kda_bwd_scan_kernel<<<grid, BS_THREADS, BS_SMEM, stream>>>(*p);
+    // packed batches hold T tokens altogether; the number of their tiles is not known here, but the kernel's coordinates stay inside
+    CUtensorMap map, map_do;
+    if (!make_pack_map(&map, p->tiles, 1ll << 24) || !make_rows_map(&map_do, const_cast<void*>(p->d_o), p->H, p->cu_seqlens ? p->T : (long long)p->N * p->T))
+        return (int)cudaErrorInvalidValue;
+    kda_bwd_scan_kernel<<<dim3(p->H, p->N), BS_THREADS, BS_SMEM, stream>>>(*p, map, map_do);
     return (int)cudaGetLastError();
 }

@@ -27,8 +27,7 @@
 // set, all roles unwind to the end of the kernel, and the tensor memory is freed.
 #include "kda_common.cuh"
 #include "kda_params.h"
-#include "tensor_map.cuh"
-#include "umma.cuh"
+#include "scan_common.cuh"
 
 namespace kda {
 
@@ -47,23 +46,10 @@ constexpr int SC_SMEM = SC_MISC + 8448 + 1024;
 // does not wait until this one's outputs have been read), the Aqk product
 constexpr uint32_t TM_S32 = 0, TM_S16 = 128, TM_ACC = 192, TM_QG = 64 /* inside an accumulator */, TM_O2 = 448;
 
-__device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const CUtensorMap* map, int x, int y, int z, int w, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-                 :: "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(bar)) : "memory");
-}
 __device__ __forceinline__ void tma_store_rows(const CUtensorMap* map, uint32_t smem_src, int h, int row) {
     asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
                  :: "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_src), "r"(0), "r"(h), "r"(row) : "memory");
 }
-__device__ __forceinline__ uint64_t sc_sdesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return umma::make_sdesc(addr, lbo, sbo) | (2ull << 61);     // 128-byte swizzle
-}
-// arrival of a whole warp (its tensor-memory and shared-memory accesses before this point are ordered first)
-__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
-    __syncwarp();
-    if (lane == 0) mbar_arrive(bar);
-}
-
 __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanParams p, const __grid_constant__ CUtensorMap map,
                                                                      const __grid_constant__ CUtensorMap map_o) {
     extern __shared__ unsigned char sc_smem_raw[];
@@ -292,7 +278,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
             umma::fence_before_sync();
             warp_arrive(b_dec, lane);
             // keys far from unit length can defeat the bound: say so instead of carrying inf on
-            if (c > 0 && publish_max(c) * up.x > 65504.f) report_status(p.status, STATUS_RANGE);
+            if (c > 0 && overflows(publish_max(c) * up.x)) report_status(p.status, STATUS_RANGE);
             const size_t tile_idx = (size_t)(chunk0 + c) * p.H + h;
             if (p.h32_out) {
                 float* hg = p.h32_out + tile_idx * (size_t)(DK * DV) + (size_t)k0 * DV + v;
@@ -458,29 +444,6 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
 extern "C" int kda_fwd_scan_smem_bytes() { return kda::SC_SMEM; }
 
 namespace {
-// W, QG and KG of the tile packs as a rank-4 tensor of fp16: 64 channels, 2 channel halves, 192 rows (64 of each matrix),
-// tiles; fetched as boxes of 64 channels x 64 rows.
-bool make_pack_map(CUtensorMap* map, const unsigned char* tiles, long long num_tiles) {
-    kda::EncodeTiledFn fn = kda::encode_tiled_fn();
-    if (!fn) return false;
-    static_assert(kda::TP_W == 0 && kda::TP_QG == 16384 && kda::TP_KG == 32768 && kda::TP_BYTES % 16 == 0, "three stacked matrices of 256-byte rows");
-    const cuuint64_t dims[4] = {64, 2, 192, (cuuint64_t)num_tiles};
-    const cuuint64_t strides[3] = {128, 256, kda::TP_BYTES};
-    const cuuint32_t box[4] = {64, 1, 64, 1}, elem[4] = {1, 1, 1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<unsigned char*>(tiles), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-// o as [tokens][heads][128], stored as boxes of 64 tokens of one head
-bool make_out_map(CUtensorMap* map, void* o, int H) {
-    kda::EncodeTiledFn fn = kda::encode_tiled_fn();
-    if (!fn) return false;
-    const cuuint64_t dims[3] = {128, (cuuint64_t)H, 1ull << 30};
-    const cuuint64_t strides[2] = {256, (cuuint64_t)H * 256};
-    const cuuint32_t box[3] = {128, 1, 64}, elem[3] = {1, 1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, o, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-              CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 int launch_scan(const kda::ScanParams* p, int groups, cudaStream_t stream) {
     using namespace kda;
     if (p->N <= 0) return 0;
@@ -489,7 +452,7 @@ int launch_scan(const kda::ScanParams* p, int groups, cudaStream_t stream) {
     if (e != cudaSuccess) return (int)e;
     CUtensorMap map, map_o = {};
     // the numbers of tiles and tokens are not known here for a packed batch; the kernel's coordinates stay inside the caller's tensors
-    if (!make_pack_map(&map, p->tiles, 1ll << 24) || (p->o && !make_out_map(&map_o, p->o, p->H))) return (int)cudaErrorInvalidValue;
+    if (!make_pack_map(&map, p->tiles, 1ll << 24) || (p->o && !make_rows_map(&map_o, p->o, p->H, 1ll << 30))) return (int)cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p->H, p->N, groups);
     cfg.blockDim = dim3(SC_THREADS);

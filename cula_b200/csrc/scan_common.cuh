@@ -1,0 +1,55 @@
+// What the forward and the reverse state scan share: shared-memory operand descriptors, TMA moves of the tile packs and token
+// rows, and the maps for them.
+#pragma once
+#include "kda_common.cuh"
+#include "kda_params.h"
+#include "tensor_map.cuh"
+#include "umma.cuh"
+
+namespace kda {
+
+__device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const CUtensorMap* map, int x, int y, int z, int w, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                 :: "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 :: "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ uint64_t sc_sdesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+    return umma::make_sdesc(addr, lbo, sbo) | (2ull << 61);     // 128-byte swizzle
+}
+// arrival of a whole warp (its tensor-memory and shared-memory accesses before this point are ordered first)
+__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+}
+
+// the largest finite entry of a state, scaled for fp16, does not fit (inf and NaN of the caller pass through unreported)
+__device__ __forceinline__ bool overflows(float scaled_max) { return scaled_max > 65504.f && scaled_max < INFINITY; }
+
+// W, QG and KG of the tile packs as a rank-4 tensor of fp16: 64 channels, 2 channel halves, 192 rows (64 of each matrix),
+// tiles; fetched as boxes of 64 channels x 64 rows.
+inline bool make_pack_map(CUtensorMap* map, const unsigned char* tiles, long long num_tiles) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return false;
+    static_assert(TP_W == 0 && TP_QG == 16384 && TP_KG == 32768 && TP_BYTES % 16 == 0, "three stacked matrices of 256-byte rows");
+    const cuuint64_t dims[4] = {64, 2, 192, (cuuint64_t)num_tiles};
+    const cuuint64_t strides[3] = {128, 256, TP_BYTES};
+    const cuuint32_t box[4] = {64, 1, 64, 1}, elem[4] = {1, 1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<unsigned char*>(tiles), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// Token rows [tokens][heads][128] of bf16, moved as boxes of 64 tokens of one head; rows past `tokens` are read as zeros.
+inline bool make_rows_map(CUtensorMap* map, void* rows, int H, long long tokens) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[3] = {128, (cuuint64_t)H, (cuuint64_t)tokens};
+    const cuuint64_t strides[2] = {256, (cuuint64_t)H * 256};
+    const cuuint32_t box[3] = {128, 1, 64}, elem[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, rows, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+              CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+
+}  // namespace kda
