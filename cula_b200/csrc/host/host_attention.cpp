@@ -31,7 +31,7 @@ int beta_flags(const Tensor& beta, bool logit) { return (is_f32(beta) ? CULA_KDA
 
 // an output in the shape of `like`; rows past the packed tokens are zero
 Tensor output_like(const Tensor& like, const Tables* tab) {
-    Tensor t = at::empty_like(like, like.options(), at::MemoryFormat::Contiguous);
+    Tensor t = device_empty(like.sizes(), like.options());
     if (tab && tab->total_tokens < like.size(1)) t.narrow(1, tab->total_tokens, like.size(1) - tab->total_tokens).zero_();
     return t;
 }
@@ -41,8 +41,8 @@ Tensor output_like(const Tensor& like, const Tables* tab) {
 void segmented_scan(const Tensor& v, const OptTensor& h0, bool want_final, const Segments& segs, Forward& f, cudaStream_t stream, int* status) {
     const int64_t P = segs.count, H = v.size(2), T = v.size(1);
     const auto f32 = v.options().dtype(at::kFloat);
-    Tensor C = at::empty({2, P, H, DIM, DIM}, f32);
-    Tensor states = at::empty({P, H, DIM, DIM}, f32);
+    Tensor C = device_empty({2, P, H, DIM, DIM}, f32);
+    Tensor states = device_empty({P, H, DIM, DIM}, f32);
     const int64_t per = H * DIM * DIM;
     float *c = fptr(C), *m = c + P * per, *s = fptr(states);
     int *cu = iptr(segs.tab.cu_seqlens), *co = iptr(segs.tab.chunk_offsets);
@@ -52,8 +52,8 @@ void segmented_scan(const Tensor& v, const OptTensor& h0, bool want_final, const
     for (int64_t i = 1; i < P; ++i)
         check(lib.cula_kda_cp_fold(c + (i - 1) * per, m + (i - 1) * per, i == 1 && !h0.has_value() ? nullptr : s + (i - 1) * per, s + i * per, 1,
                                    (int)H, 0, stream), "cula_kda_cp_fold");
-    f.o = at::empty_like(v);
-    Tensor ht = want_final ? at::empty({P, H, DIM, DIM}, f32) : Tensor();
+    f.o = device_empty(v.sizes(), v.options());
+    Tensor ht = want_final ? device_empty({P, H, DIM, DIM}, f32) : Tensor();
     check(lib.cula_kda_fwd_scan(ptr(f.tiles), s, ptr(f.o), fptr(ht), nullptr, nullptr, nullptr, cu, co, iptr(segs.tab.seq_order), (int)P, (int)T,
                                 (int)H, status, stream), "cula_kda_fwd_scan");
     if (want_final) f.final_state = ht.narrow(0, P - 1, 1);
@@ -77,9 +77,9 @@ Forward forward_core(const Tensor& q, const Tensor& k, const Tensor& v, const Te
     int *cu = tab ? iptr(tab->cu_seqlens) : nullptr, *ci = tab ? iptr(tab->chunk_indices) : nullptr;
     int *co = tab ? iptr(tab->chunk_offsets) : nullptr, *so = tab ? iptr(tab->seq_order) : nullptr;
     const auto f32 = q.options().dtype(at::kFloat);
-    f.tiles = at::empty({tiles * lib.cula_kda_tile_pack_bytes()}, q.options().dtype(at::kByte));
-    if (store_akk || store_bwd) f.akk = at::empty({tiles, CHUNK, CHUNK}, f32);
-    if (store_bwd) f.mkk = at::empty({tiles, CHUNK, CHUNK}, f32);
+    f.tiles = device_empty({tiles * lib.cula_kda_tile_pack_bytes()}, q.options().dtype(at::kByte));
+    if (store_akk || store_bwd) f.akk = device_empty({tiles, CHUNK, CHUNK}, f32);
+    if (store_bwd) f.mkk = device_empty({tiles, CHUNK, CHUNK}, f32);
     check(lib.cula_kda_fwd_intra(ptr(q), ptr(k), ptr(v), ptr(g), g_flags(g), ptr(beta), beta_flags(beta, opt.beta_logit), fptr(A_log), fptr(dt_bias),
                                  cu, ci, (int)f.num_chunks, (int)T, (int)H, (float)opt.scale, opt.l2norm, opt.gate_mode, (float)opt.lower_bound,
                                  ptr(f.tiles), fptr(f.akk), fptr(f.mkk), status, stream), "cula_kda_fwd_intra");
@@ -88,10 +88,10 @@ Forward forward_core(const Tensor& q, const Tensor& k, const Tensor& v, const Te
         return f;
     }
     if (want_output) f.o = output_like(v, tab);
-    if (want_final) f.final_state = at::empty({n_seqs, H, DIM, DIM}, f32);
-    if (store_states) f.h = at::empty({tiles, DIM, DIM}, q.options().dtype(at::kBFloat16));
-    if (store_bwd) f.h32 = at::empty({tiles, DIM, DIM}, f32);
-    if (store_states || store_bwd) f.vnew = at::empty({tiles, CHUNK, DIM}, q.options().dtype(at::kHalf));
+    if (want_final) f.final_state = device_empty({n_seqs, H, DIM, DIM}, f32);
+    if (store_states) f.h = device_empty({tiles, DIM, DIM}, q.options().dtype(at::kBFloat16));
+    if (store_bwd) f.h32 = device_empty({tiles, DIM, DIM}, f32);
+    if (store_states || store_bwd) f.vnew = device_empty({tiles, CHUNK, DIM}, q.options().dtype(at::kHalf));
     check(lib.cula_kda_fwd_scan(ptr(f.tiles), fptr(h0), ptr(f.o), fptr(f.final_state), ptr(f.h), ptr(f.vnew), fptr(f.h32), cu, co, so, (int)n_seqs,
                                 (int)T, (int)H, status, stream), "cula_kda_fwd_scan");
     return f;
@@ -115,16 +115,16 @@ Backward backward_core(const Tensor& q, const Tensor& k, const Tensor& v, const 
     const auto f32 = q.options().dtype(at::kFloat);
     const Tensor d_o = d_out.contiguous();
     const OptTensor dht = contiguous_f32(d_final);
-    Tensor work = at::empty({4}, f32);           // [0:2] = {s, 1/s}, [2] = running max (as bits)
+    Tensor work = device_empty({4}, f32);           // [0:2] = {s, 1/s}, [2] = running max (as bits)
     check(lib.cula_kda_bwd_grad_scale(ptr(d_o), d_o.numel(), fptr(dht), dht.has_value() ? dht->numel() : 0, reinterpret_cast<unsigned int*>(fptr(work) + 2), fptr(work), stream),
           "cula_kda_bwd_grad_scale");
-    Tensor dvn = at::empty({tiles, CHUNK, DIM}, q.options().dtype(at::kHalf)), ds = at::empty({tiles, DIM, DIM}, f32);
+    Tensor dvn = device_empty({tiles, CHUNK, DIM}, q.options().dtype(at::kHalf)), ds = device_empty({tiles, DIM, DIM}, f32);
     Backward r;
-    if (want_dh0) r.dh0 = at::empty({n_seqs, H, DIM, DIM}, f32);
+    if (want_dh0) r.dh0 = device_empty({n_seqs, H, DIM, DIM}, f32);
     check(lib.cula_kda_bwd_scan(ptr(f.tiles), ptr(d_o), fptr(dht), fptr(work), ptr(dvn), fptr(ds), fptr(r.dh0), cu, co, so, (int)n_seqs, (int)T,
                                 (int)H, status, stream), "cula_kda_bwd_scan");
     r.dv = output_like(v, tab);
-    Tensor scratch = at::empty({tiles, lib.cula_kda_bwd_scratch_floats()}, f32);
+    Tensor scratch = device_empty({tiles, lib.cula_kda_bwd_scratch_floats()}, f32);
     check(lib.cula_kda_bwd_dense(fptr(f.h32), fptr(ds), ptr(f.vnew), ptr(dvn), ptr(d_o), ptr(v), ptr(beta), beta_flags(beta, opt.beta_logit),
                                  fptr(f.akk), fptr(work), ptr(r.dv), fptr(scratch), cu, ci, (int)f.num_chunks, (int)T, (int)H, status, stream),
           "cula_kda_bwd_dense");
@@ -134,7 +134,7 @@ Backward backward_core(const Tensor& q, const Tensor& k, const Tensor& v, const 
     r.dbeta = output_like(beta, tab);
     if (opt.gate_mode != GATE_NONE) {            // the two atomically accumulated gradients share one cleared buffer
         const bool bias = dt_bias.has_value() && dt_bias->defined();
-        Tensor both = at::zeros({bias ? H + H * DIM : H}, f32);
+        Tensor both = device_zeros({bias ? H + H * DIM : H}, f32, stream);
         if (bias) r.dbias = both.narrow(0, 0, H * DIM);
         r.dA = both.narrow(0, both.numel() - H, H);
     }
@@ -395,7 +395,7 @@ Tensor decode(const Tensor& A_log_in, const OptTensor& dt_bias_in, const Tensor&
         }
         if (!out.is_contiguous()) throw pybind11::value_error("out must be contiguous");
     } else {
-        out = at::empty({s0, s1, HV, V}, q.options());
+        out = device_empty({s0, s1, HV, V}, q.options());
     }
     check(lib.cula_kda_decode(ptr(q), ptr(k), ptr(v), ptr(a), is_f32(a), ptr(b), is_f32(b), fptr(A_log), fptr(dt_bias), fptr(state), iptr(idx), ptr(out),
                               (int)N, (int)H, (int)HV, (int)V, (int)pool, (float)scale.value_or(1.0 / std::sqrt((double)K)), l2norm,

@@ -6,6 +6,7 @@
 #include <torch/extension.h>
 
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -56,6 +57,15 @@ inline bool is_f32(const Tensor& t) { return t.scalar_type() == at::kFloat; }
 inline bool is_bf16(const Tensor& t) { return t.scalar_type() == at::kBFloat16; }
 inline Tensor contiguous_f32(const Tensor& t) { return (is_f32(t) ? t : t.to(at::kFloat)).contiguous(); }
 inline OptTensor contiguous_f32(const OptTensor& t) { return t.has_value() && t->defined() ? OptTensor(contiguous_f32(*t)) : OptTensor(); }
+// Output allocations of the native path, straight from the allocator: through the dispatcher at::empty takes 1.7 us, and at::zeros
+// 6 us with a kernel of its own, on a path that allocates up to 16 tensors per call.
+inline Tensor device_empty(at::IntArrayRef sizes, const at::TensorOptions& options) { return Tensor(at::detail::empty_cuda(sizes, options)); }
+inline Tensor device_zeros(at::IntArrayRef sizes, const at::TensorOptions& options, cudaStream_t stream) {
+    Tensor t = device_empty(sizes, options);
+    const cudaError_t e = t.numel() ? cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), stream) : cudaSuccess;
+    if (e != cudaSuccess) throw std::runtime_error(std::string("cudaMemsetAsync failed: ") + cudaGetErrorString(e));
+    return t;
+}
 inline cudaStream_t stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
 // B200 guard (cached per device), and the status word of a device: one int in pinned host memory that the kernels write

@@ -21,7 +21,7 @@ bool is_float(const Tensor& t) { return is_bf16(t) || is_f32(t); }
 Tensor gate_forward(const Tensor& g, const Tensor& a32, const OptTensor& b32, std::optional<double> lower_bound, at::ScalarType out_dtype) {
     c10::cuda::CUDAGuard guard(g.device());
     const int64_t H = g.size(-2), K = g.size(-1);
-    Tensor y = at::empty_like(g, g.options().dtype(out_dtype));
+    Tensor y = device_empty(g.sizes(), g.options().dtype(out_dtype));
     check(lib.cula_kda_gate_fwd(ptr(g), is_f32(g), fptr(a32), fptr(b32), ptr(y), out_dtype == at::kFloat, g.numel() / (H * K), (int)H, (int)K,
                                 lower_bound.has_value(), (float)lower_bound.value_or(0.0), stream_of(g)), "cula_kda_gate_fwd");
     return y;
@@ -47,12 +47,12 @@ struct Gate : torch::autograd::Function<Gate> {
         Tensor dy = grads[0].contiguous();
         if (!is_float(dy)) dy = dy.to(at::kFloat);
         const c10::IValue lb = ctx->saved_data["lb"];
-        Tensor dg = at::empty_like(g);
-        Tensor both = at::zeros({b32.has_value() ? H + H * K : H}, a32.options());       // the two accumulated gradients
-        Tensor dbias = b32.has_value() ? both.narrow(0, 0, H * K) : Tensor(), dA = both.narrow(0, both.numel() - H, H);
+        Tensor dg = device_empty(g.sizes(), g.options());
+        Tensor dA = device_zeros(a32.sizes(), a32.options(), stream_of(g));             // the two accumulated gradients
+        Tensor dbias = b32.has_value() ? device_zeros(b32->sizes(), a32.options(), stream_of(g)) : Tensor();
         check(lib.cula_kda_gate_bwd(ptr(g), is_f32(g), fptr(a32), fptr(b32), ptr(dy), is_f32(dy), ptr(dg), fptr(dA), fptr(dbias), g.numel() / (H * K),
                                     (int)H, (int)K, !lb.isNone(), lb.isNone() ? 0.f : (float)lb.toDouble(), stream_of(g)), "cula_kda_gate_bwd");
-        return {dg, dA.view_as(a32), dbias.defined() ? dbias.view_as(*b32) : Tensor(), Tensor(), Tensor()};
+        return {dg, dA, dbias, Tensor(), Tensor()};
     }
 };
 
@@ -70,7 +70,7 @@ Tensor kda_gate(const Tensor& g, const Tensor& A_log, const OptTensor& dt_bias, 
 // ------------------------------------------------ beta activation ------------------------------------------------
 Tensor beta_forward(const Tensor& x) {
     c10::cuda::CUDAGuard guard(x.device());
-    Tensor y = at::empty_like(x, x.options().dtype(at::kFloat));
+    Tensor y = device_empty(x.sizes(), x.options().dtype(at::kFloat));
     check(lib.cula_kda_beta_sigmoid_fwd(ptr(x), is_f32(x), fptr(y), x.numel(), stream_of(x)), "cula_kda_beta_sigmoid_fwd");
     return y;
 }
@@ -85,7 +85,7 @@ struct Beta : torch::autograd::Function<Beta> {
         if (!grads[0].defined()) return {Tensor()};
         const Tensor x = ctx->get_saved_variables()[0], dy = contiguous_f32(grads[0]);
         c10::cuda::CUDAGuard guard(x.device());
-        Tensor dx = at::empty_like(x);
+        Tensor dx = device_empty(x.sizes(), x.options());
         check(lib.cula_kda_beta_sigmoid_bwd(ptr(x), is_f32(x), fptr(dy), ptr(dx), x.numel(), stream_of(x)), "cula_kda_beta_sigmoid_bwd");
         return {dx};
     }
@@ -104,9 +104,9 @@ std::pair<Tensor, Tensor> conv_forward(const Tensor& x, const Tensor& w32, const
     c10::cuda::CUDAGuard guard(x.device());
     const int64_t B = x.size(0), T = x.size(1), D = x.size(2), W = w32.size(-1);
     const int64_t n_seqs = tab ? tab->n_seqs : B, num_chunks = tab ? tab->num_chunks : B * ((T + CHUNK - 1) / CHUNK);
-    Tensor y = at::empty_like(x);
+    Tensor y = device_empty(x.sizes(), x.options());
     if (tab && tab->total_tokens < T) y.narrow(1, tab->total_tokens, T - tab->total_tokens).zero_();     // rows past the packed tokens
-    Tensor fin = want_final ? at::zeros({n_seqs, D, W}, w32.options()) : Tensor();
+    Tensor fin = want_final ? device_zeros({n_seqs, D, W}, w32.options(), stream_of(x)) : Tensor();
     check(lib.cula_kda_short_conv_fwd(ptr(x), fptr(w32), fptr(b32), fptr(c32), ptr(y), fptr(fin), tab ? iptr(tab->cu_seqlens) : nullptr,
                                       tab ? iptr(tab->chunk_indices) : nullptr, (int)num_chunks, (int)T, (int)D, (int)W, silu, stream_of(x)),
           "cula_kda_short_conv_fwd");
@@ -139,7 +139,7 @@ struct Conv : torch::autograd::Function<Conv> {
         const int64_t B = x.size(0), T = x.size(1), D = x.size(2), W = w32.size(-1);
         Tensor dy = grads[0].contiguous();
         if (!is_bf16(dy)) dy = dy.to(at::kBFloat16);
-        Tensor dx = at::empty_like(x), cu, ci;
+        Tensor dx = device_empty(x.sizes(), x.options()), cu, ci;
         int64_t num_chunks = B * ((T + CHUNK - 1) / CHUNK);
         if (auto it = ctx->saved_data.find("tab"); it != ctx->saved_data.end()) {
             auto t = it->second.toTensorVector();
@@ -147,12 +147,12 @@ struct Conv : torch::autograd::Function<Conv> {
             cu = t[0]; ci = t[1]; num_chunks = n[0];
             if (n[1] < T) dx.narrow(1, n[1], T - n[1]).zero_();
         }
-        Tensor both = at::zeros({b32.has_value() ? D * W + D : D * W}, w32.options());     // the two accumulated gradients
-        Tensor dw = both.narrow(0, 0, D * W), db = b32.has_value() ? both.narrow(0, D * W, D) : Tensor();
+        Tensor dw = device_zeros(w32.sizes(), w32.options(), stream_of(x));                // the two accumulated gradients
+        Tensor db = b32.has_value() ? device_zeros(b32->sizes(), w32.options(), stream_of(x)) : Tensor();
         check(lib.cula_kda_short_conv_bwd(ptr(x), fptr(w32), fptr(b32), fptr(c32), ptr(dy), ptr(dx), fptr(dw), fptr(db), (int*)ptr(cu), (int*)ptr(ci),
                                           (int)num_chunks, (int)T, (int)D, (int)W, ctx->saved_data["silu"].toBool(), stream_of(x)),
               "cula_kda_short_conv_bwd");
-        return {dx, dw.view_as(w32), db, Tensor(), Tensor(), Tensor(), Tensor()};
+        return {dx, dw, db, Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
 std::pair<Tensor, OptTensor> short_conv(const Tensor& x, const Tensor& weight_in, const OptTensor& bias, const OptTensor& cache, bool want_final,
@@ -179,7 +179,7 @@ std::pair<Tensor, OptTensor> short_conv(const Tensor& x, const Tensor& weight_in
 std::pair<Tensor, Tensor> norm_forward(const Tensor& x, const Tensor& g, const Tensor& w32, bool swish, double eps) {
     c10::cuda::CUDAGuard guard(x.device());
     const int64_t D = x.size(-1), R = x.numel() / D;
-    Tensor y = at::empty_like(x), rstd = at::empty({R}, w32.options());
+    Tensor y = device_empty(x.sizes(), x.options()), rstd = device_empty({R}, w32.options());
     check(lib.cula_kda_rms_norm_gated_fwd(ptr(x), ptr(g), fptr(w32), ptr(y), fptr(rstd), R, (int)D, swish, (float)eps, stream_of(x)),
           "cula_kda_rms_norm_gated_fwd");
     return {y, rstd};
@@ -202,10 +202,10 @@ struct Norm : torch::autograd::Function<Norm> {
         const int64_t D = x.size(-1), R = x.numel() / D;
         Tensor dy = grads[0].contiguous();
         if (!is_bf16(dy)) dy = dy.to(at::kBFloat16);
-        Tensor dx = at::empty_like(x), dg = at::empty_like(g), dw = at::zeros({D}, w32.options());
+        Tensor dx = device_empty(x.sizes(), x.options()), dg = device_empty(g.sizes(), g.options()), dw = device_zeros(w32.sizes(), w32.options(), stream_of(x));
         check(lib.cula_kda_rms_norm_gated_bwd(ptr(x), ptr(g), fptr(w32), fptr(ctx->saved_data["rstd"].toTensor()), ptr(dy), ptr(dx), ptr(dg), fptr(dw), R,
                                               (int)D, ctx->saved_data["swish"].toBool(), stream_of(x)), "cula_kda_rms_norm_gated_bwd");
-        return {dx, dg, dw.view_as(w32), Tensor(), Tensor()};
+        return {dx, dg, dw, Tensor(), Tensor()};
     }
 };
 Tensor rms_norm_gated(const Tensor& x, const Tensor& g, const Tensor& weight, bool swish, double eps) {
