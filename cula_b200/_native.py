@@ -24,6 +24,8 @@ SIGNATURES = {
     "cula_kda_fwd_intra": (_i, [_vp, _vp, _vp, _vp, _i, _vp, _i, _fp, _fp, _ip, _ip, _i, _i, _i,
                                 _f, _i, _i, _f, _vp, _fp, _fp, _ip, _vp]),
     "cula_kda_fwd_scan": (_i, [_vp, _fp, _vp, _fp, _vp, _vp, _fp, _ip, _ip, _ip, _i, _i, _i, _ip, _vp]),
+    "cula_kda_fwd_pieces": (_i, [_vp, _vp, _vp, _vp, _i, _vp, _i, _fp, _fp, _i, _i, _i, _f, _i, _i, _f, _vp, _fp, _fp, _fp, _vp, _fp,
+                                 _vp, _fp, _fp, _ip, _i, _ip, _vp]),
     "cula_kda_cp_transition": (_i, [_vp, _fp, _fp, _ip, _ip, _i, _i, _i, _ip, _vp]),
     "cula_kda_cp_fold": (_i, [_fp, _fp, _fp, _fp, _i, _i, ctypes.c_longlong, _vp]),
     "cula_kda_decode": (_i, [_vp, _vp, _vp, _vp, _i, _vp, _i, _fp, _fp, _fp, _ip, _vp, _i, _i, _i, _i, _i, _f, _i, _f, _f, _i, _ip, _vp]),

@@ -75,6 +75,63 @@ extern "C" int cula_kda_fwd_scan(const void* d_tiles, const float* d_h0, void* d
     return kda_launch_fwd_scan(&p, static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int cula_kda_fwd_pieces(const void* d_q, const void* d_k, const void* d_v, const void* d_g, int g_is_fp32, const void* d_beta,
+                                   int beta_is_fp32, const float* d_A_log, const float* d_dt_bias, int B, int T, int H, float scale,
+                                   int use_qk_l2norm, int gate_mode, float lower_bound, void* d_tiles, float* d_akk, float* d_mkk,
+                                   const float* d_h0, void* d_o, float* d_ht, void* d_vnew_out, float* d_h32_out, float* d_states,
+                                   const int* h_piece_chunks, int pieces, int* d_status, void* stream) {
+    if (!d_q || !d_k || !d_v || !d_g || !d_beta || !d_tiles || !d_status || !h_piece_chunks || B <= 0 || T <= 0 || H <= 0 || pieces <= 0)
+        return CULA_KDA_EINVAL;
+    if (gate_mode < 0 || gate_mode > 2 || (gate_mode != 0 && !d_A_log)) return CULA_KDA_EINVAL;
+    if (g_is_fp32 & ~(CULA_KDA_G_FP32 | CULA_KDA_G_PER_HEAD)) return CULA_KDA_EINVAL;
+    if ((!d_o && !d_vnew_out) || (d_h32_out && !d_vnew_out) || (pieces > 1 && !d_states)) return CULA_KDA_EINVAL;
+    if (B > 1 && (d_akk || d_mkk || d_vnew_out || d_h32_out)) return CULA_KDA_EINVAL;      // the tiles of a batch come out piece by piece
+    if (misaligned(d_q) || misaligned(d_k) || misaligned(d_v) || misaligned(d_tiles) || misaligned(d_akk) || misaligned(d_mkk) ||
+        (!(g_is_fp32 & CULA_KDA_G_PER_HEAD) && misaligned(d_g)) || misaligned(d_o) || misaligned(d_vnew_out))
+        return CULA_KDA_EALIGN;
+    long long total = 0;
+    for (int i = 0; i < pieces; ++i) {
+        if (h_piece_chunks[i] <= 0) return CULA_KDA_EINVAL;
+        total += h_piece_chunks[i];
+    }
+    if (total != (T + kda::BT - 1) / kda::BT) return CULA_KDA_EINVAL;
+    const bool per_head = (g_is_fp32 & CULA_KDA_G_PER_HEAD) != 0;
+    const size_t g_row = (size_t)H * (per_head ? 1 : kda::DK) * (g_is_fp32 & CULA_KDA_G_FP32 ? 4 : 2);
+    const size_t beta_row = (size_t)H * (beta_is_fp32 & CULA_KDA_BETA_FP32 ? 4 : 2), row = (size_t)H * kda::DK * 2, state = (size_t)B * H * kda::DK * kda::DV;
+    auto at = [](auto* p, size_t bytes) { return p ? reinterpret_cast<decltype(p)>(reinterpret_cast<uintptr_t>(p) + bytes) : p; };
+    int c0 = 0;
+    for (int i = 0; i < pieces; ++i) {
+        const int n = h_piece_chunks[i], t0 = c0 * kda::BT, len = i == pieces - 1 ? T - t0 : n * kda::BT;
+        const size_t tile0 = (size_t)c0 * B * H;
+        kda::IntraParams ip{};
+        ip.q = at(d_q, t0 * row); ip.k = at(d_k, t0 * row); ip.v = at(d_v, t0 * row); ip.g = at(d_g, t0 * g_row); ip.beta = at(d_beta, t0 * beta_row);
+        ip.A_log = d_A_log; ip.dt_bias = d_dt_bias;
+        ip.tiles = static_cast<unsigned char*>(d_tiles) + tile0 * kda::TP_BYTES;
+        ip.akk_out = at(d_akk, tile0 * kda::BT * kda::BT * 4); ip.mkk_out = at(d_mkk, tile0 * kda::BT * kda::BT * 4);
+        ip.status = d_status; ip.T = len; ip.stride = T; ip.H = H;
+        ip.g_fp32 = g_is_fp32 & CULA_KDA_G_FP32; ip.g_per_head = per_head;
+        ip.beta_fp32 = beta_is_fp32 & CULA_KDA_BETA_FP32; ip.beta_logit = (beta_is_fp32 & CULA_KDA_BETA_LOGIT) != 0;
+        ip.use_l2norm = use_qk_l2norm; ip.gate_mode = gate_mode; ip.lower_bound = lower_bound; ip.scale = scale;
+        if (i > 0) {          // runs beside the scan of the piece before, on the SMs that the scan leaves
+            const int rest = kda::sm_count() - B * H;
+            ip.max_ctas = rest > 0 ? 2 * rest : 1;
+            ip.overlap = 1;
+        }
+        int rc = kda_launch_fwd_intra(&ip, B * n, static_cast<cudaStream_t>(stream));
+        if (rc != 0) return rc;
+        kda::ScanParams sp{};
+        sp.tiles = ip.tiles;
+        sp.h0 = i == 0 ? d_h0 : d_states + ((i - 1) & 1) * state;
+        sp.ht = i == pieces - 1 ? d_ht : d_states + (i & 1) * state;
+        sp.o = at(d_o, t0 * row); sp.vnew_out = at(d_vnew_out, tile0 * kda::BT * kda::DV * 2); sp.h32_out = at(d_h32_out, tile0 * kda::DK * kda::DV * 4);
+        sp.status = d_status; sp.T = len; sp.stride = T; sp.H = H; sp.N = B;
+        rc = kda_launch_fwd_scan(&sp, static_cast<cudaStream_t>(stream));
+        if (rc != 0) return rc;
+        c0 += n;
+    }
+    return 0;
+}
+
 extern "C" int cula_kda_cp_transition(const void* d_tiles, float* d_c_out, float* d_m_out, const int* d_cu_seqlens,
                                       const int* d_chunk_offsets, int N, int T, int H, int* d_status, void* stream) {
     if (N == 0) return 0;

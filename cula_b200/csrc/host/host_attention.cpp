@@ -1,6 +1,9 @@
 // chunk_kda / chunk_gated_delta_rule (forward and backward) and the decode step on the native host path.
 #include "host_common.h"
 
+#include <algorithm>
+#include <cmath>
+
 #include <torch/csrc/autograd/python_cpp_function.h>
 
 namespace cula_host {
@@ -59,6 +62,42 @@ void segmented_scan(const Tensor& v, const OptTensor& h0, bool want_final, const
     if (want_final) f.final_state = ht.narrow(0, P - 1, 1);
 }
 
+// How to lay the two stages of a fixed-length batch over the GPU. The scan is a chain per (sequence, head) and needs one SM for each,
+// the chunk-parallel stage takes whatever it is given; run after one another, the scan leaves the other SMs idle. So the chunks are
+// cut into pieces, and a piece's chunk-parallel stage runs beside the scan of the piece before. Sizes for which the two just keep
+// step form a geometric series; the first piece's chunk-parallel stage and the last one's scan are exposed. The times are measured,
+// in us. Above half the SMs the scan leaves too little for this to gain (3 x 4096 x 32 heads: 456 -> 476 us). Measured, whole call:
+// 1 x 65536 x 32 heads 2763 -> 2599 us, 1 x 16384 x 48 1075 -> 950, 1 x 4096 x 32 229.5 -> 211, 2 x 8192 x 32 658 -> 640.
+struct Plan {
+    std::vector<int> pieces;      // chunks per piece
+    double us = 0;
+};
+Plan plan_pieces(int64_t ctas, int64_t nc, int sms) {
+    const double intra = ctas * 0.0535 * 148 / sms;                        // per chunk of every sequence, on the whole GPU
+    const double scan = 1.6 + ctas / 128.0;                                // and its scan (more when many share the memory system)
+    Plan best;
+    best.pieces = {(int)nc};
+    best.us = nc * (intra + scan);
+    if (2 * ctas > sms) return best;
+    const double ratio = std::min(1.5, scan / (intra * sms / (sms - ctas)));
+    for (int n = 2; n <= 8; ++n) {
+        double sum = 0, f = 1;
+        for (int i = 0; i < n; ++i, f *= ratio) sum += f;
+        Plan p;
+        int64_t done = 0;
+        f = 1;
+        for (int i = 0; i < n; ++i, f *= ratio) {
+            const int64_t c = i == n - 1 ? nc - done : std::llround(nc * f / sum);
+            p.pieces.push_back((int)c);
+            done += c;
+        }
+        if (*std::min_element(p.pieces.begin(), p.pieces.end()) < 4) break;
+        p.us = p.pieces[0] * intra + nc * scan + 16 * (n - 1);      // 16: a tail and a ramp of the chunk-parallel stage, launches
+        if (p.us < best.us) best = p;
+    }
+    return best;
+}
+
 // Forward orchestration (the role of cula/kda/chunk_fwd.py:39-152): the chunk-parallel stage writes one tile pack per
 // (chunk, head); the scan consumes them, carries the fp32 state and writes o. All tensors contiguous; A_log, dt_bias fp32.
 Forward forward_core(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const OptTensor& h0,
@@ -80,6 +119,27 @@ Forward forward_core(const Tensor& q, const Tensor& k, const Tensor& v, const Te
     f.tiles = device_empty({tiles * lib.cula_kda_tile_pack_bytes()}, q.options().dtype(at::kByte));
     if (store_akk || store_bwd) f.akk = device_empty({tiles, CHUNK, CHUNK}, f32);
     if (store_bwd) f.mkk = device_empty({tiles, CHUNK, CHUNK}, f32);
+    // a batch of several sequences comes out piece by piece, which what is kept for later cannot
+    if (!tab && !store_states && !(store_akk && !store_bwd) && (B == 1 || !store_bwd)) {
+        const Plan plan = plan_pieces(B * H, f.num_chunks / B, at::cuda::getDeviceProperties(q.device().index())->multiProcessorCount);
+        // side-by-side segments are the other way to fill the GPU, better with few heads (the two cross between 24 and 32)
+        const double nc = (double)f.num_chunks, seg_us = segs ? nc * (H * 0.0535 + 2 * (1.6 + H / 128.0) / segs->count) + 10 * segs->count : 1e30;
+        if (plan.pieces.size() > 1 && 1.06 * plan.us < seg_us) {
+            if (want_output) f.o = device_empty(v.sizes(), v.options());
+            if (want_final) f.final_state = device_empty({B, H, DIM, DIM}, f32);
+            if (store_bwd) {
+                f.h32 = device_empty({tiles, DIM, DIM}, f32);
+                f.vnew = device_empty({tiles, CHUNK, DIM}, q.options().dtype(at::kHalf));
+            }
+            Tensor states = device_empty({2, B, H, DIM, DIM}, f32);
+            check(lib.cula_kda_fwd_pieces(ptr(q), ptr(k), ptr(v), ptr(g), g_flags(g), ptr(beta), beta_flags(beta, opt.beta_logit), fptr(A_log),
+                                          fptr(dt_bias), (int)B, (int)T, (int)H, (float)opt.scale, opt.l2norm, opt.gate_mode,
+                                          (float)opt.lower_bound, ptr(f.tiles), fptr(f.akk), fptr(f.mkk), fptr(h0), ptr(f.o), fptr(f.final_state),
+                                          ptr(f.vnew), fptr(f.h32), fptr(states), plan.pieces.data(), (int)plan.pieces.size(), status, stream),
+                  "cula_kda_fwd_pieces");
+            return f;
+        }
+    }
     check(lib.cula_kda_fwd_intra(ptr(q), ptr(k), ptr(v), ptr(g), g_flags(g), ptr(beta), beta_flags(beta, opt.beta_logit), fptr(A_log), fptr(dt_bias),
                                  cu, ci, (int)f.num_chunks, (int)T, (int)H, (float)opt.scale, opt.l2norm, opt.gate_mode, (float)opt.lower_bound,
                                  ptr(f.tiles), fptr(f.akk), fptr(f.mkk), status, stream), "cula_kda_fwd_intra");

@@ -239,7 +239,8 @@ struct ChunkInfo {
     int row0;    // first token row in the flattened [B*T] token axis
     int valid;   // number of real tokens in this chunk (1..64)
 };
-__device__ __forceinline__ ChunkInfo chunk_info(int c, const int* cu_seqlens, const int* chunk_indices, int T) {
+// stride: tokens from the start of one sequence of a fixed-length batch to the next (0: T)
+__device__ __forceinline__ ChunkInfo chunk_info(int c, const int* cu_seqlens, const int* chunk_indices, int T, int stride = 0) {
     ChunkInfo ci;
     if (cu_seqlens) {
         ci.seq = chunk_indices[2 * c];
@@ -251,7 +252,7 @@ __device__ __forceinline__ ChunkInfo chunk_info(int c, const int* cu_seqlens, co
         int cps = (T + BT - 1) / BT;
         ci.seq = c / cps;
         int lc = c - ci.seq * cps;
-        ci.row0 = ci.seq * T + lc * BT;
+        ci.row0 = ci.seq * (stride ? stride : T) + lc * BT;
         ci.valid = min(BT, T - lc * BT);
     }
     return ci;

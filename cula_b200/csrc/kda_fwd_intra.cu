@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
             int4 v = make_int4(0, 0, 0, 0);
             if (t_id < p.num_tiles) {
                 const int c2 = t_id / p.H;
-                const ChunkInfo ci2 = chunk_info(c2, p.cu_seqlens, p.chunk_indices, p.T);
+                const ChunkInfo ci2 = chunk_info(c2, p.cu_seqlens, p.chunk_indices, p.T, p.stride);
                 v = make_int4(ci2.row0, ci2.valid, t_id - c2 * p.H, t_id);
             }
             sInfo[buf] = v;
@@ -951,6 +951,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
     if (tid == MMA_THREAD) bulk_wait_all();        // staged outputs must be on their way before the shared memory goes away
     __syncthreads();
     if (warp == 0) umma::tmem_dealloc(tmem, 256);
+    pdl_wait();      // an overlapping launch: what follows in the stream counts on the kernel before this one as well
 }
 
 }  // namespace kda
@@ -980,7 +981,19 @@ extern "C" int kda_launch_fwd_intra(const kda::IntraParams* p, int num_chunks, c
     const int sms = sm_count();
     IntraParams q = *p;
     q.num_tiles = num_chunks * p->H;
-    const int grid = q.num_tiles < 2 * sms ? q.num_tiles : 2 * sms;     // two resident CTAs per SM
-    kernel<<<grid, INTRA_THREADS, smem, stream>>>(q);
+    const int most = q.max_ctas > 0 && q.max_ctas < 2 * sms ? q.max_ctas : 2 * sms;     // two resident CTAs per SM
+    const int grid = q.num_tiles < most ? q.num_tiles : most;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(INTRA_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = q.overlap ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, kernel, q);
+    if (e != cudaSuccess) return (int)e;
     return (int)cudaGetLastError();
 }

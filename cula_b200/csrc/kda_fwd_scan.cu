@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
         len = p.cu_seqlens[n + 1] - bos;
         chunk0 = p.chunk_offsets[n];
     } else {
-        bos = n * p.T;
+        bos = n * (p.stride ? p.stride : p.T);
         len = p.T;
         chunk0 = n * ((p.T + BT - 1) / BT);
     }
@@ -108,6 +108,8 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
     // Everything this kernel reads (tile packs, initial states) may come from the kernels before it in the stream; with
     // programmatic stream serialization the CTA can be resident before they have finished, so wait here (a no-op when
     // the launch does not carry the attribute). Only scheduling, the index arithmetic and the set-up above overlap.
+    // A chunk-parallel stage of later tokens that follows may start once every CTA of this grid has its SM.
+    pdl_launch_dependents();
     pdl_wait();
 
     auto wait = [&](uint64_t* bar, int phase) -> bool {

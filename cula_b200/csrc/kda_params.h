@@ -27,6 +27,9 @@ struct IntraParams {
     float* mkk_out;           // [NT*H][64][64] fp32 strict-lower gated k k^T Gram matrix, or null
     int* status;              // device status word
     int T;                    // tokens per sequence when cu_seqlens is null
+    int stride;               // tokens between the starts of two such sequences (0: T)
+    int max_ctas;             // upper bound of the grid (0: two CTAs per SM)
+    int overlap;              // 1: start under the kernel before it in the stream, which writes nothing this one reads
     int H;
     int num_tiles;            // num_chunks * H (filled in by the launcher)
     int g_fp32;
@@ -53,6 +56,7 @@ struct ScanParams {
     const int* seq_order;         // [N] launch order (longest first) or null
     int* status;                  // device status word
     int T;
+    int stride;                   // tokens between the starts of two sequences of a fixed-length batch (0: T)
     int H;
     int N;                        // number of sequences
 };

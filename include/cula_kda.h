@@ -93,6 +93,22 @@ int cula_kda_fwd_scan(const void* d_tiles, const float* d_h0, void* d_o, float* 
                       int N, int T, int H, int* d_status, void* stream);
 
 /*
+ * The whole forward of a fixed-length batch, both stages, in `pieces` spans of h_piece_chunks[i] chunks of every sequence (host array;
+ * the spans add up to all chunks): the chunk-parallel stage of a span runs beside the scan of the span before it. Arguments as above;
+ * d_states: 2 * B * H * 128 * 128 floats of workspace (may be NULL for one piece). With B > 1 the tile packs come out span by span,
+ * and d_akk, d_mkk, d_vnew_out and d_h32_out must be NULL. Everything is launched into `stream`.
+ */
+int cula_kda_fwd_pieces(const void* d_q, const void* d_k, const void* d_v,
+                        const void* d_g, int g_is_fp32,
+                        const void* d_beta, int beta_is_fp32,
+                        const float* d_A_log, const float* d_dt_bias,
+                        int B, int T, int H,
+                        float scale, int use_qk_l2norm, int gate_mode, float lower_bound,
+                        void* d_tiles, float* d_akk, float* d_mkk,
+                        const float* d_h0, void* d_o, float* d_ht, void* d_vnew_out, float* d_h32_out, float* d_states,
+                        const int* h_piece_chunks, int pieces, int* d_status, void* stream);
+
+/*
  * Index tables of a packed batch, computed on the host from HOST memory (h_*): what prepare_chunk_indices
  * (fla/ops/utils/index.py:138-149) and prepare_chunk_offsets_i32 (cula/ops/chunk_delta_h.py:42-47) produce with torch.
  * cula_kda_num_chunks: sum of ceil(len / 64) over the N sequences (< 0 on a bad cu_seqlens).

@@ -378,3 +378,41 @@ def test_segmented_scan_matches_oracle(T, H, h0_std):
     o, ht = run_chunk_kda(inp)
     o_ref, ht_ref = oracle_fwd(inp)
     assert_fwd_close(o, ht, o_ref, ht_ref, ht_tol=2e-3)
+
+
+@pytest.mark.parametrize("B,T,H,pieces,g_dtype", [(1, 64 * 9 - 13, 3, (1, 3, 5), torch.bfloat16), (1, 64 * 9, 2, (5, 2, 1, 1), torch.float32),
+                                                  (3, 64 * 6 - 1, 2, (2, 4), torch.bfloat16), (2, 40, 1, (1,), torch.float32)])
+def test_forward_in_pieces_equals_the_two_stages(B, T, H, pieces, g_dtype):
+    """The pieces hand on the state and lie where the whole run puts its outputs (the last piece ragged, one piece, growing and
+    shrinking ones): against the two stages run one after the other."""
+    from cula_b200 import _native
+    from cula_b200.kda import check_status
+    from cula_b200.kda.chunk import _status_ptr
+    inp = make_inputs(B, T, H, seed=27, gate_offset=-7.0, h0_std=1.0, g_dtype=g_dtype)
+    d = {n: _cuda(t) for n, t in inp.items()}
+    lib, nc, f32 = _native.lib(), (T + 63) // 64, dict(dtype=torch.float32, device="cuda")
+    tiles, stream, status = B * nc * H, torch.cuda.current_stream().cuda_stream, _status_ptr(d["q"].device)
+    ptr = lambda t: None if t is None else t.data_ptr()
+    got = {}
+    for name in ("whole", "pieces"):
+        out = dict(o=torch.zeros(B, T, H, 128, dtype=torch.bfloat16, device="cuda"), ht=torch.zeros(B, H, 128, 128, **f32))
+        if B == 1:
+            out.update(akk=torch.zeros(tiles, 64, 64, **f32), mkk=torch.zeros(tiles, 64, 64, **f32), h32=torch.zeros(tiles, 128, 128, **f32),
+                       vnew=torch.zeros(tiles, 64, 128, dtype=torch.float16, device="cuda"))
+        pack = torch.empty(tiles * lib.cula_kda_tile_pack_bytes(), dtype=torch.uint8, device="cuda")
+        args = [ptr(d[n]) for n in ("q", "k", "v", "g")] + [int(g_dtype == torch.float32), ptr(d["beta"]), 0, ptr(d["A_log"]), ptr(d["dt_bias"])]
+        if name == "whole":
+            _native.check(lib.cula_kda_fwd_intra(*args, None, None, B * nc, T, H, 128 ** -0.5, 1, 2, -5.0, ptr(pack), ptr(out.get("akk")),
+                                                 ptr(out.get("mkk")), status, stream), "intra")
+            _native.check(lib.cula_kda_fwd_scan(ptr(pack), ptr(d["initial_state"]), ptr(out["o"]), ptr(out["ht"]), None, ptr(out.get("vnew")),
+                                                ptr(out.get("h32")), None, None, None, B, T, H, status, stream), "scan")
+        else:
+            states, sizes = torch.empty(2, B, H, 128, 128, **f32), torch.tensor(pieces, dtype=torch.int32)
+            _native.check(lib.cula_kda_fwd_pieces(*args, B, T, H, 128 ** -0.5, 1, 2, -5.0, ptr(pack), ptr(out.get("akk")), ptr(out.get("mkk")),
+                                                  ptr(d["initial_state"]), ptr(out["o"]), ptr(out["ht"]), ptr(out.get("vnew")), ptr(out.get("h32")),
+                                                  ptr(states), sizes.data_ptr(), len(pieces), status, stream), "pieces")
+        torch.cuda.synchronize()
+        check_status()
+        got[name] = out
+    for n, ref in got["whole"].items():
+        assert err_ratio(ref.float().cpu(), got["pieces"][n].float().cpu()) <= 1e-3, n
