@@ -27,6 +27,18 @@ import torch
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
+
+def count_launches(step):
+    """Launches of this library's kernels in one call of `step` (how many depends on the shape), counted by the profiler outside any
+    timed region."""
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        step()
+        torch.cuda.synchronize()
+    return sum(e.count for e in prof.key_averages() if "kda_" in e.key and "_kernel" in e.key)
+
+
 WORKLOADS = {
     # name: (B, T, H, lens or None)
     "fwd_B2_T2048_H32": (2, 2048, 32),
@@ -485,7 +497,7 @@ def run_extra(args, rank, world, local_rank):
     _native.lib()
     kw = dict(use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, safe_gate=True, lower_bound=-5.0)
     H = w["H"]
-    scaling, launches = "weak", 2
+    scaling = "weak"
     if w["kind"] == "fwdbwd":
         B, T = w["B"], w["T"]
         inp = make_inputs(B, T, H, seed=rank, h0_std=0.1)
@@ -498,7 +510,7 @@ def run_extra(args, rank, world, local_rank):
             o, _ = chunk_kda(d["q"], d["k"], d["v"], d["g"], d["beta"], A_log=d["A_log"], dt_bias=d["dt_bias"],
                              initial_state=d["initial_state"], output_final_state=True, **kw)
             o.backward(do)
-        tokens, metric, launches = B * T * world, "chunk_kda forward+backward tokens/s", 9
+        tokens, metric = B * T * world, "chunk_kda forward+backward tokens/s"
         cfg = {"B_per_gpu": B, "T": T, "sharding": "batch x head shards, one per rank, no collective"}
     elif w["kind"] == "gdn":
         # the scalar-gate variant (one decay per token and head) on the headline shape: raw gate activated in-kernel
@@ -525,7 +537,6 @@ def run_extra(args, rank, world, local_rank):
                 o.backward(do)
         tokens = B * T * world
         metric = "chunk_gated_delta_rule forward+backward tokens/s" if w["backward"] else "chunk_gated_delta_rule forward tokens/s"
-        launches = 9 if w["backward"] else 2
         cfg = {"B_per_gpu": B, "T": T, "gate": "one per (token, head), softplus form in-kernel",
                "sharding": "batch x head shards, one per rank, no collective"}
     elif w["kind"] == "varlen":
@@ -551,7 +562,7 @@ def run_extra(args, rank, world, local_rank):
         slots = torch.randperm(N, generator=gen).to(torch.int32).to(dev)
         step = lambda: kda_decode(A_log=dA, dt_bias=dbias, q=dq, k=dk, v=dv, a=da, b=db, initial_state_source=pool,
                                   initial_state_indices=slots)
-        tokens, metric, launches = N * world, "kda_decode tokens/s", 1
+        tokens, metric = N * world, "kda_decode tokens/s"
         state_bytes = 2 * N * H * 128 * 128 * 4
         cfg = {"sequences_per_gpu": N, "state_layout": "vk", "state_bytes_read_plus_written": state_bytes}
     elif w["kind"] == "layer":
@@ -623,7 +634,7 @@ def run_extra(args, rank, world, local_rank):
             "vs_baseline": None, "dtype": "bf16", "data": "synthetic",
             "config": dict({"workload": args.workload, "H": H, "K": 128, "V": 128,
                             "l2": "256 MB flush buffer written before every timed step"}, **cfg),
-            "gpu_launches": launches * args.steps, "clocks": clocks}), flush=True)
+            "gpu_launches": count_launches(step) * args.steps, "clocks": clocks}), flush=True)
     if dist.is_initialized():
         dist.destroy_process_group()
 
@@ -783,7 +794,7 @@ def main():
         "hbm_frac_compulsory": tokens / world * H * BYTES_PER_TOKEN_HEAD / (ms * 1e-3) / 1e9 / peaks["hbm_gbs"],
         "e2e": {"value": tokens / (ms_e2e * 1e-3), "unit": "tokens/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "ms_per_step": ms_e2e, "host_cores_rank0": len(host_cpus)},
-        "gpu_launches": 2 * args.steps,
+        "gpu_launches": count_launches(lambda: fwd(d)) * args.steps,
         "roofline": roofline,
         "cpu_baseline": base,
         "cp": cp,

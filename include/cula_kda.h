@@ -74,7 +74,7 @@ int cula_kda_fwd_intra(const void* d_q, const void* d_k, const void* d_v,
                        void* d_tiles, float* d_akk, float* d_mkk, int* d_status, void* stream);
 
 /*
- * Sequential state scan fused with the output stage, one CTA per (sequence, head, value half).
+ * Sequential state scan fused with the output stage, one CTA per (sequence, head).
  * Replaces chunk_gated_delta_rule_fwd_h(k=kg, w, u, gk, initial_state, output_final_state, cu_seqlens, ...)
  *   (cula/ops/chunk_delta_h.py:1991-2168, called at cula/kda/chunk_fwd.py:111-120) and
  *   chunk_gla_fwd_o(q, v_new, g, A=Aqk, h, o, scale, ...) (cula/ops/fwd_o.py:1755-1852, chunk_fwd.py:131-143).
