@@ -242,6 +242,31 @@ extern "C" int cula_kda_bwd_scan(const void* d_tiles, const void* d_do, const fl
     return kda_launch_bwd_scan(&p, static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int cula_kda_bwd_both_scans(const void* d_tiles, const float* d_h0, void* d_vnew_out, float* d_h32_out, const void* d_do,
+                                       const float* d_dht, const float* d_gscale, void* d_dvn_out, float* d_ds_out, float* d_dh0,
+                                       const int* d_cu_seqlens, const int* d_chunk_offsets, const int* d_seq_order, int N, int T, int H,
+                                       int* d_status, void* stream) {
+    if (N == 0) return 0;
+    if (!d_tiles || !d_vnew_out || !d_h32_out || !d_do || !d_gscale || !d_dvn_out || !d_ds_out || !d_status || N < 0 || H <= 0)
+        return CULA_KDA_EINVAL;
+    if ((d_cu_seqlens == nullptr) != (d_chunk_offsets == nullptr)) return CULA_KDA_EINVAL;
+    if (!d_cu_seqlens && T <= 0) return CULA_KDA_EINVAL;
+    if (misaligned(d_tiles) || misaligned(d_vnew_out) || misaligned(d_do) || misaligned(d_dvn_out) || misaligned(d_ds_out)) return CULA_KDA_EALIGN;
+    kda::ScanParams f{};
+    f.tiles = static_cast<const unsigned char*>(d_tiles);
+    f.h0 = d_h0; f.vnew_out = d_vnew_out; f.h32_out = d_h32_out;
+    f.cu_seqlens = d_cu_seqlens; f.chunk_offsets = d_chunk_offsets; f.seq_order = d_seq_order;
+    f.status = d_status; f.T = T; f.H = H; f.N = N; f.reverse_follows = 1;
+    const int rc = kda_launch_fwd_scan(&f, static_cast<cudaStream_t>(stream));
+    if (rc != 0) return rc;
+    kda::BwdScanParams p{};
+    p.tiles = f.tiles;
+    p.d_o = d_do; p.dht = d_dht; p.gscale = d_gscale; p.dvn_out = d_dvn_out; p.ds_out = d_ds_out; p.dh0 = d_dh0;
+    p.cu_seqlens = d_cu_seqlens; p.chunk_offsets = d_chunk_offsets; p.seq_order = d_seq_order;
+    p.status = d_status; p.T = T; p.H = H; p.N = N; p.beside_forward = 1;
+    return kda_launch_bwd_scan(&p, static_cast<cudaStream_t>(stream));
+}
+
 extern "C" int cula_kda_bwd_dense(const float* d_h32, const float* d_ds, const void* d_vnew, const void* d_dvn,
                                   const void* d_do, const void* d_v, const void* d_beta, int beta_is_fp32,
                                   const float* d_akk, const float* d_gscale, void* d_dv, float* d_scratch,

@@ -100,9 +100,10 @@ Plan plan_pieces(int64_t ctas, int64_t nc, int sms) {
 
 // Forward orchestration (the role of cula/kda/chunk_fwd.py:39-152): the chunk-parallel stage writes one tile pack per
 // (chunk, head); the scan consumes them, carries the fp32 state and writes o. All tensors contiguous; A_log, dt_bias fp32.
+// leave_scan: the scan's buffers are made but backward_core launches it, beside the reverse scan.
 Forward forward_core(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const OptTensor& h0,
                      const OptTensor& A_log, const OptTensor& dt_bias, const Options& opt, const Tables* tab, const Segments* segs, bool want_final,
-                     bool store_states, bool store_akk, bool store_bwd, bool want_output) {
+                     bool store_states, bool store_akk, bool store_bwd, bool want_output, bool leave_scan = false) {
     ++forward_calls;
     c10::cuda::CUDAGuard guard(q.device());
     const int64_t B = q.size(0), T = q.size(1), H = q.size(2);
@@ -120,7 +121,7 @@ Forward forward_core(const Tensor& q, const Tensor& k, const Tensor& v, const Te
     if (store_akk || store_bwd) f.akk = device_empty({tiles, CHUNK, CHUNK}, f32);
     if (store_bwd) f.mkk = device_empty({tiles, CHUNK, CHUNK}, f32);
     // a batch of several sequences comes out piece by piece, which what is kept for later cannot
-    if (!tab && !store_states && !(store_akk && !store_bwd) && (B == 1 || !store_bwd)) {
+    if (!leave_scan && !tab && !store_states && !(store_akk && !store_bwd) && (B == 1 || !store_bwd)) {
         const Plan plan = plan_pieces(B * H, f.num_chunks / B, at::cuda::getDeviceProperties(q.device().index())->multiProcessorCount);
         // side-by-side segments are the other way to fill the GPU, better with few heads (the two cross between 24 and 32)
         const double nc = (double)f.num_chunks, seg_us = segs ? nc * (H * 0.0535 + 2 * (1.6 + H / 128.0) / segs->count) + 10 * segs->count : 1e30;
@@ -152,6 +153,7 @@ Forward forward_core(const Tensor& q, const Tensor& k, const Tensor& v, const Te
     if (store_states) f.h = device_empty({tiles, DIM, DIM}, q.options().dtype(at::kBFloat16));
     if (store_bwd) f.h32 = device_empty({tiles, DIM, DIM}, f32);
     if (store_states || store_bwd) f.vnew = device_empty({tiles, CHUNK, DIM}, q.options().dtype(at::kHalf));
+    if (leave_scan) return f;
     check(lib.cula_kda_fwd_scan(ptr(f.tiles), fptr(h0), ptr(f.o), fptr(f.final_state), ptr(f.h), ptr(f.vnew), fptr(f.h32), cu, co, so, (int)n_seqs,
                                 (int)T, (int)H, status, stream), "cula_kda_fwd_scan");
     return f;
@@ -161,10 +163,25 @@ struct Backward {
     Tensor dq, dk, dv, dg, dbeta, dA, dbias, dh0;
 };
 
-// Backward orchestration (the role of cula/kda/chunk_bwd.py:432-604) from the forward intermediates in `f`.
+// The upstream gradients and the power-of-two scale they are carried in.
+struct Upstream {
+    Tensor d_o, work;             // work: [0:2] = {s, 1/s}, [2] = running max (as bits)
+    OptTensor dht;
+};
+Upstream scale_gradients(const Tensor& d_out, const OptTensor& d_final) {
+    c10::cuda::CUDAGuard guard(d_out.device());
+    Upstream u{d_out.contiguous(), device_empty({4}, d_out.options().dtype(at::kFloat)), contiguous_f32(d_final)};
+    check(lib.cula_kda_bwd_grad_scale(ptr(u.d_o), u.d_o.numel(), fptr(u.dht), u.dht.has_value() ? u.dht->numel() : 0,
+                                      reinterpret_cast<unsigned int*>(fptr(u.work) + 2), fptr(u.work), stream_of(d_out)),
+          "cula_kda_bwd_grad_scale");
+    return u;
+}
+
+// Backward orchestration (the role of cula/kda/chunk_bwd.py:432-604) from the forward intermediates in `f`. With scan_left the
+// forward scan of `f` (from h0) has not run yet: the reverse scan reads none of its results, so the two chains run side by side.
 Backward backward_core(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const OptTensor& A_log,
-                       const OptTensor& dt_bias, const Options& opt, const Tables* tab, const Forward& f, bool want_dh0, const Tensor& d_out,
-                       const OptTensor& d_final) {
+                       const OptTensor& dt_bias, const Options& opt, const Tables* tab, const Forward& f, bool want_dh0, const Upstream& up,
+                       bool scan_left = false, const OptTensor& h0 = {}) {
     c10::cuda::CUDAGuard guard(q.device());
     const int64_t B = q.size(0), T = q.size(1), H = q.size(2);
     cudaStream_t stream = stream_of(q);
@@ -173,16 +190,17 @@ Backward backward_core(const Tensor& q, const Tensor& k, const Tensor& v, const 
     int *cu = tab ? iptr(tab->cu_seqlens) : nullptr, *ci = tab ? iptr(tab->chunk_indices) : nullptr;
     int *co = tab ? iptr(tab->chunk_offsets) : nullptr, *so = tab ? iptr(tab->seq_order) : nullptr;
     const auto f32 = q.options().dtype(at::kFloat);
-    const Tensor d_o = d_out.contiguous();
-    const OptTensor dht = contiguous_f32(d_final);
-    Tensor work = device_empty({4}, f32);           // [0:2] = {s, 1/s}, [2] = running max (as bits)
-    check(lib.cula_kda_bwd_grad_scale(ptr(d_o), d_o.numel(), fptr(dht), dht.has_value() ? dht->numel() : 0, reinterpret_cast<unsigned int*>(fptr(work) + 2), fptr(work), stream),
-          "cula_kda_bwd_grad_scale");
+    const Tensor &d_o = up.d_o, &work = up.work;
+    const OptTensor& dht = up.dht;
     Tensor dvn = device_empty({tiles, CHUNK, DIM}, q.options().dtype(at::kHalf)), ds = device_empty({tiles, DIM, DIM}, f32);
     Backward r;
     if (want_dh0) r.dh0 = device_empty({n_seqs, H, DIM, DIM}, f32);
-    check(lib.cula_kda_bwd_scan(ptr(f.tiles), ptr(d_o), fptr(dht), fptr(work), ptr(dvn), fptr(ds), fptr(r.dh0), cu, co, so, (int)n_seqs, (int)T,
-                                (int)H, status, stream), "cula_kda_bwd_scan");
+    if (scan_left)
+        check(lib.cula_kda_bwd_both_scans(ptr(f.tiles), fptr(h0), ptr(f.vnew), fptr(f.h32), ptr(d_o), fptr(dht), fptr(work), ptr(dvn), fptr(ds),
+                                          fptr(r.dh0), cu, co, so, (int)n_seqs, (int)T, (int)H, status, stream), "cula_kda_bwd_both_scans");
+    else
+        check(lib.cula_kda_bwd_scan(ptr(f.tiles), ptr(d_o), fptr(dht), fptr(work), ptr(dvn), fptr(ds), fptr(r.dh0), cu, co, so, (int)n_seqs, (int)T,
+                                    (int)H, status, stream), "cula_kda_bwd_scan");
     r.dv = output_like(v, tab);
     Tensor scratch = device_empty({tiles, lib.cula_kda_bwd_scratch_floats()}, f32);
     check(lib.cula_kda_bwd_dense(fptr(f.h32), fptr(ds), ptr(f.vnew), ptr(dvn), ptr(d_o), ptr(v), ptr(beta), beta_flags(beta, opt.beta_logit),
@@ -259,17 +277,20 @@ public:
             auto n = ctx->saved_data["tab_sizes"].toIntVector();
             tab = Tables{t[0], t[1], t[2], t[3], n[0], n[1], n[2]};
         }
+        const Tensor d_o = grads[0].defined() ? grads[0] : at::zeros_like(v);
+        const OptTensor dht = grads.size() > 1 && grads[1].defined() ? OptTensor(grads[1]) : OptTensor();
+        const Upstream up = scale_gradients(d_o, dht);      // in front of the recomputation: the reverse scan starts with its scan
         Forward f;
+        bool scan_left = false;
         if (auto it = ctx->saved_data.find("kept"); it != ctx->saved_data.end()) {
             auto t = it->second.toTensorVector();
             f.tiles = t[0]; f.akk = t[1]; f.mkk = t[2]; f.h32 = t[3]; f.vnew = t[4];
             f.num_chunks = tab ? tab->num_chunks : q.size(0) * ((q.size(1) + CHUNK - 1) / CHUNK);
         } else {        // recomputed, as the reference does by default (cula/kda/chunk_bwd.py:459-500)
-            f = forward_core(q, k, v, g, beta, h0, A_log, dt_bias, o, tab ? &*tab : nullptr, nullptr, false, false, false, true, false);
+            f = forward_core(q, k, v, g, beta, h0, A_log, dt_bias, o, tab ? &*tab : nullptr, nullptr, false, false, false, true, false, true);
+            scan_left = true;
         }
-        const Tensor d_o = grads[0].defined() ? grads[0] : at::zeros_like(v);
-        const OptTensor dht = grads.size() > 1 && grads[1].defined() ? OptTensor(grads[1]) : OptTensor();
-        Backward b = backward_core(q, k, v, g, beta, A_log, dt_bias, o, tab ? &*tab : nullptr, f, h0.has_value(), d_o, dht);
+        Backward b = backward_core(q, k, v, g, beta, A_log, dt_bias, o, tab ? &*tab : nullptr, f, h0.has_value(), up, scan_left, h0);
         if (b.dA.defined()) b.dA = b.dA.view_as(*A_log);
         if (b.dbias.defined()) b.dbias = b.dbias.view_as(*dt_bias);
         return {b.dq, b.dk, b.dv, b.dg, b.dbeta, b.dA, b.dbias, b.dh0, Tensor()};
@@ -394,7 +415,7 @@ pybind11::tuple backward_tuple(const Tensor& q, const Tensor& k, const Tensor& v
     auto get = [&](const char* n) { return saved[n].cast<Tensor>(); };
     f.tiles = get("tiles"); f.akk = get("akk"); f.mkk = get("mkk"); f.h32 = get("h32"); f.vnew = get("vnew");
     f.num_chunks = saved["num_chunks"].cast<int64_t>();
-    Backward b = backward_core(q, k, v, g, beta, A_log, dt_bias, o, tab, f, want_dh0, d_o, dht);
+    Backward b = backward_core(q, k, v, g, beta, A_log, dt_bias, o, tab, f, want_dh0, scale_gradients(d_o, dht));
     auto obj = [](const Tensor& t) -> pybind11::object { return t.defined() ? pybind11::cast(t) : pybind11::object(pybind11::none()); };
     return pybind11::make_tuple(obj(b.dq), obj(b.dk), obj(b.dv), obj(b.dg), obj(b.dbeta), obj(b.dA), obj(b.dbias), obj(b.dh0));
 }

@@ -450,6 +450,11 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
     }
     __syncthreads();
     if (warp == BS_MMA_WARP) umma::tmem_dealloc(tmem, 512);
+    // Beside the forward scan: it reads nothing of that scan, and was launched when the tile packs were complete (the trigger
+    // stands behind the forward scan's own wait). What follows in the stream counts on both, so this grid ends after it.
+    // Forward + backward against the two one after the other: 2 x 1000 x 3 heads 198 -> 157 us, 2 x 2048 x 32 (scalar gate) 909 -> 858,
+    // 4 x 8192 x 32, where the forward scan leaves 20 SMs, 6386 -> 6351.
+    pdl_wait();
 }
 
 }  // namespace kda
@@ -475,6 +480,17 @@ extern "C" int kda_launch_bwd_scan(const kda::BwdScanParams* p, cudaStream_t str
     CUtensorMap map, map_do;
     if (!make_pack_map(&map, p->tiles, 1ll << 24) || !make_rows_map(&map_do, const_cast<void*>(p->d_o), p->H, p->cu_seqlens ? p->T : (long long)p->N * p->T))
         return (int)cudaErrorInvalidValue;
-    kda_bwd_scan_kernel<<<dim3(p->H, p->N), BS_THREADS, BS_SMEM, stream>>>(*p, map, map_do);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p->H, p->N);
+    cfg.blockDim = dim3(BS_THREADS);
+    cfg.dynamicSmemBytes = BS_SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p->beside_forward ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, kda_bwd_scan_kernel, *p, map, map_do);
+    if (e != cudaSuccess) return (int)e;
     return (int)cudaGetLastError();
 }

@@ -109,9 +109,11 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
     // Everything this kernel reads (tile packs, initial states) may come from the kernels before it in the stream; with
     // programmatic stream serialization the CTA can be resident before they have finished, so wait here (a no-op when
     // the launch does not carry the attribute). Only scheduling, the index arithmetic and the set-up above overlap.
-    // A chunk-parallel stage of later tokens that follows may start once every CTA of this grid has its SM.
-    pdl_launch_dependents();
+    // A chunk-parallel stage of later tokens that follows may start once every CTA of this grid has its SM; the reverse scan of
+    // the same tiles only once the tiles are complete, i.e. behind the wait.
+    if (!p.reverse_follows) pdl_launch_dependents();
     pdl_wait();
+    if (p.reverse_follows) pdl_launch_dependents();
 
     auto wait = [&](uint64_t* bar, int phase) -> bool {
         if (mbar_wait(bar, phase & 1)) return true;

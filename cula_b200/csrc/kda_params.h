@@ -59,6 +59,7 @@ struct ScanParams {
     int stride;                   // tokens between the starts of two sequences of a fixed-length batch (0: T)
     int H;
     int N;                        // number of sequences
+    int reverse_follows;          // the reverse scan of the same tiles is next in the stream and runs beside this one
 };
 
 struct BwdScanParams {
@@ -76,6 +77,7 @@ struct BwdScanParams {
     int T;
     int H;
     int N;
+    int beside_forward;           // launched behind a forward scan with reverse_follows set
 };
 
 // fp32 scratch record written per (chunk, head) by the dense backward stage, read by the gated stage

@@ -145,6 +145,14 @@ int cula_kda_bwd_scan(const void* d_tiles, const void* d_do, const float* d_dht,
                       const int* d_cu_seqlens, const int* d_chunk_offsets, const int* d_seq_order,
                       int N, int T, int H, int* d_status, void* stream);
 
+/* The forward scan that keeps v_new and the fp32 states for the backward (d_vnew_out, d_h32_out as in cula_kda_fwd_scan) and the
+ * reverse scan beside it. Both read the tile packs and neither the other's results; d_tiles must come from a
+ * cula_kda_fwd_intra call in `stream` before, d_gscale from a cula_kda_bwd_grad_scale call before that one. */
+int cula_kda_bwd_both_scans(const void* d_tiles, const float* d_h0, void* d_vnew_out, float* d_h32_out, const void* d_do,
+                            const float* d_dht, const float* d_gscale, void* d_dvn_out, float* d_ds_out, float* d_dh0,
+                            const int* d_cu_seqlens, const int* d_chunk_offsets, const int* d_seq_order,
+                            int N, int T, int H, int* d_status, void* stream);
+
 /* Chunk-parallel dense products with the carried states (tcgen05 tensor cores; the fp32 states arrive through TMA
  * tensor maps built per call from d_h32 / d_ds); writes d_dv (bf16, final) and the scratch record. d_status: device
  * status word of the bounded waits. Replaces the state-dependent half of chunk_kda_bwd_wy_dqkg_fused (cula/kda/chunk_bwd.py:557-574) and the dAqk

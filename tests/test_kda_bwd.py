@@ -407,3 +407,29 @@ def test_gated_stage_at_block_edges(g_dtype, gate, safe, l2):
     dht = torch.randn(len(lens), H, 128, 128, generator=gen)
     ref, got = run_both(inp, do, dht, cu_seqlens=cu, l2=l2, gate=gate, safe=safe)
     assert_grads(ref, got, SUITE_TOL, "block edges")
+
+
+@pytest.mark.parametrize("B,T,H,lens", [(1, 1, 1, None), (2, 130, 3, None), (3, 200, 37, None), (5, 65, 64, None), (1, 700, 40, [1, 64, 65, 370, 200])])
+def test_side_by_side_scans_equal_scans_one_after_the_other(B, T, H, lens):
+    """Recomputing runs the forward scan and the reverse scan side by side, kept intermediates need the reverse scan alone:
+    the same gradients to the bit, with fewer chains than SMs, about as many, and several times as many."""
+    from cula_b200.kda import check_status, chunk_kda
+    from cula_b200.synthetic import make_inputs_on_device
+    d = make_inputs_on_device(B, T, H, torch.device("cuda"), seed=T, gate_offset=-4.0, h0_std=0.5)
+    cu = None
+    if lens:
+        cu = torch.tensor([0, *np.cumsum(lens)], dtype=torch.int32, device="cuda")
+        d["initial_state"] = 0.5 * torch.randn(len(lens), H, 128, 128, device="cuda")
+    up = torch.randn(B, T, H, 128, device="cuda").to(torch.bfloat16)
+    names = ("q", "k", "v", "g", "beta", "initial_state")
+    grads = []
+    for keep in (True, False, False):
+        leaves = {n: d[n].detach().clone().requires_grad_(True) for n in names}
+        o, ht = chunk_kda(*(leaves[n] for n in names[:5]), initial_state=leaves["initial_state"], output_final_state=True,
+                          use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, safe_gate=True, lower_bound=-5.0, A_log=d["A_log"],
+                          dt_bias=d["dt_bias"], cu_seqlens=cu, disable_recompute=keep)
+        grads.append(torch.autograd.grad([o, ht], list(leaves.values()), [up, ht.detach()]))
+    torch.cuda.synchronize()
+    check_status()
+    for other in grads[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(grads[0], other))
