@@ -452,9 +452,10 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
         auto put = [&](int which, float2 v) { *reinterpret_cast<float2*>(tab + which * 64 + 2 * lane) = v; };
         put(0, add2(dl, splat2(2.f * SH)));                                             // f = 2^(this - G)
         put(1, mul2(ex2_2(rI), splat2(unshift)));                                       // q 2^g = qa * this
-        // 2^(r_I - r_{I+1}) >= 1, <= 2^116 under the safe gate; the clamp keeps an unbounded gate from making inf * 0
+        // 2^(r_I - r_{I+1}) >= 1, <= 2^116 under the safe gate; the clamp keeps an unbounded gate from making inf * 0, also for
+        // the last row of the chunk, whose f is 2^SH
         const float2 cb = sub2(splat2(TF32_DEBIAS2_LOG2 - 2.f * SH), dl);
-        put(2, ex2_2(make_float2(fminf(cb.x, 126.f), fminf(cb.y, 126.f))));
+        put(2, ex2_2(make_float2(fminf(cb.x, 126.f - SH), fminf(cb.y, 126.f - SH))));
         put(3, mul2(ex2_2(sub2(r[4], rN)), splat2(unshift)));                           // kg = kf * 2^(g_last - r_{I+1})
         if (I == 0) put(4, ex2_2(sub2(r[2], r[1])));                                    // copy anchored at block 2
         if (I < 2) put(5, ex2_2(sub2(r[3], rN)));                                       // copy anchored at block 3

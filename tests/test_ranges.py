@@ -1,0 +1,68 @@
+"""Inputs at the ends of what the operators accept: decays, magnitudes and forms that the other tests do not reach.
+Forward, final state and gradients against the CPU oracle; tolerances as in test_kda_bwd.py unless stated."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from oracle.naive_kda import chunk_kda_oracle, err_ratio
+
+NAMES = ("q", "k", "v", "g", "beta", "h0")
+
+
+def make(T=200, H=2, seed=0, B=1):
+    gen = torch.Generator().manual_seed(seed)
+
+    def rn(*s):
+        return torch.randn(*s, generator=gen)
+
+    return dict(q=rn(B, T, H, 128), k=rn(B, T, H, 128), v=rn(B, T, H, 128), g=-0.02 * torch.rand(B, T, H, 128, generator=gen),
+                beta=torch.rand(B, T, H, generator=gen), h0=0.3 * rn(B, H, 128, 128), do=rn(B, T, H, 128), dht=rn(B, H, 128, 128))
+
+
+def unit(x):
+    return F.normalize(x, dim=-1)
+
+
+def forward_backward(c, scale=None, l2=True, reference=True, dtype=torch.float32):
+    """(results of the kernels, results of the oracle in ``dtype``): o, ht and the gradients of NAMES, by name."""
+    from cula_b200.kda import check_status, chunk_kda
+    c = {n: t.to(torch.bfloat16) if n in ("q", "k", "v", "beta", "do") else t for n, t in c.items()}
+    dev = {n: c[n].cuda().requires_grad_(True) for n in NAMES}
+    o, ht = chunk_kda(*(dev[n] for n in NAMES[:5]), scale=scale, initial_state=dev["h0"], output_final_state=True, use_qk_l2norm_in_kernel=l2)
+    grads = torch.autograd.grad([o, ht], list(dev.values()), [c["do"].cuda(), c["dht"].cuda()])
+    torch.cuda.synchronize()
+    check_status()
+    got = dict(o=o, ht=ht, **{"d" + n: g for n, g in zip(NAMES, grads)})
+    got = {n: t.detach().float().cpu() for n, t in got.items()}
+    if not reference:
+        return got, None
+    ref = {n: c[n].to(dtype).requires_grad_(True) for n in NAMES}
+    ro, rh = chunk_kda_oracle(*(ref[n] for n in NAMES[:5]), scale=scale, initial_state=ref["h0"], output_final_state=True,
+                              use_qk_l2norm_in_kernel=l2, dtype=dtype)
+    rg = torch.autograd.grad([ro, rh], list(ref.values()), [c["do"].to(dtype), c["dht"].to(dtype)])
+    return got, dict(o=ro.detach(), ht=rh.detach(), **{"d" + n: g for n, g in zip(NAMES, rg)})
+
+
+def assert_close(got, ref, **tol):
+    bad = []
+    for n, r in ref.items():
+        e = err_ratio(r, got[n])
+        if not e <= tol.get(n, {"o": 5e-3, "ht": 2e-3, "dg": 2e-2, "dbeta": 2e-2}.get(n, 8e-3)):
+            bad.append(f"{n} {e:.2e}")
+    assert not bad, "; ".join(bad)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("l2", [True, False])
+@pytest.mark.parametrize("decay", [7.0, 9.0, 30.0, 1000.0])
+def test_decays_beyond_the_safe_range_stay_finite(decay, l2):
+    """More than about 5.5 nats per token is past what the 16-row anchors carry: contributions inside a block are then lost (the
+    reference does not accept such gates at all), but no factor may meet its inverse as 0 * inf, with normalised rows or without.
+    The final state only needs the factors towards the end of the chunk, which are <= 1: it stays exact."""
+    c = make(seed=1)
+    c["g"] = torch.full_like(c["g"], -decay)
+    if not l2:
+        c["q"], c["k"] = unit(c["q"]), unit(c["k"])
+    got, ref = forward_backward(c, l2=l2)
+    assert torch.isfinite(got["o"]).all()
+    assert err_ratio(ref["ht"], got["ht"]) <= 2e-3
