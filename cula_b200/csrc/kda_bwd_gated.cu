@@ -67,6 +67,12 @@ constexpr int BG_C2 = 212992;                   // dA, then cR; later partial su
 constexpr int BG_MISC = 229376;                 // rstd_q[64], rstd_k[64], beta[64]
 constexpr int BG_SMEM = BG_MISC + 1024;
 
+// The sums of the two Gram phases, and dq, dk+, dk- until they leave, are held times 2^-16. The factor of a block with itself,
+// 2^(r_I - r_{I+1}), reaches 2^116 under the safe gate (2^126, where it is clamped, beyond it) and meets the row's or column's own
+// factor, which takes it back, only after the sum: unscaled, a sum of more than 2^12 would be inf by then, and inf * 0 = NaN where
+// that other factor has underflowed. A power of two changes no bit of what stays in range.
+constexpr float BG_DOWN = 1.f / 65536.f, BG_UP = 65536.f;
+
 // Round to tf32 (nearest, ties away from zero -- what cvt.rna.tf32.f32 does for finite values) with two integer
 // instructions: add half an ulp of the 10-bit mantissa, clear the 13 low bits.
 __device__ __forceinline__ float bg_tf32(float x) {
@@ -442,8 +448,8 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
                     const float2 kk = unpack_bf16(kr[hh][x]);
                     sum.x = fmaf(zw[n][2 * x], kk.x * gr[x] * fast_exp2(G[n][2 * x]), sum.x);
                     sum.y = fmaf(zw[n][2 * x + 1], kk.y * gr[x] * fast_exp2(G[n][2 * x + 1]), sum.y);
-                    zw[n][2 * x] *= be.x * gr[x];
-                    zw[n][2 * x + 1] *= be.y * gr[x];
+                    zw[n][2 * x] *= be.x * (gr[x] * BG_DOWN);
+                    zw[n][2 * x + 1] *= be.y * (gr[x] * BG_DOWN);
                 }
                 s[2 * n] = sum.x * rk.x;
                 s[2 * n + 1] = sum.y * rk.y;
@@ -474,7 +480,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
         float accP[8][4];
 #pragma unroll
         for (int n = 0; n < 8; ++n) {
-            const float gr[2] = {fast_exp2(rt[(n >> 1) * DK + ch0]), fast_exp2(rt[(n >> 1) * DK + ch0 + 8])};
+            const float gr[2] = {BG_DOWN * fast_exp2(rt[(n >> 1) * DK + ch0]), BG_DOWN * fast_exp2(rt[(n >> 1) * DK + ch0 + 8])};
 #pragma unroll
             for (int e = 0; e < 4; ++e) accP[n][e] = gr[e >> 1] * scr[SCR_DQG + (8 * n + 2 * t4 + (e & 1)) * DK + ch0 + 8 * (e >> 1)];
         }
@@ -516,10 +522,10 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
                 bg_mma(bR[1], lo[1], f[2], f[3]);
                 bg_mma(bR[0], hi[1], f[0], f[1]);
                 bg_mma(bR[1], hi[1], f[2], f[3]);
-                float cji[2] = {1.f, 1.f};
+                float cji[2] = {BG_DOWN, BG_DOWN};
                 if (I != J + 1) {
 #pragma unroll
-                    for (int x = 0; x < 2; ++x) cji[x] = fast_exp2(fminf(rt[I * DK + ch0 + 8 * x] - rN[x], 126.f));
+                    for (int x = 0; x < 2; ++x) cji[x] = BG_DOWN * fast_exp2(fminf(rt[I * DK + ch0 + 8 * x] - rN[x], 126.f));
                 }
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh)
@@ -586,8 +592,8 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
             for (int hh = 0; hh < 2; ++hh) {
                 const int n = 2 * b + hh, tok = 8 * n + 2 * t4;
                 const float4 dq = *slot(BG_DW, BG_DW + 16384, n), dp = *slot(BG_C1, BG_X2, n), dm = *slot(BG_AN, BG_AT, n);
-                const float2 fq = mul2(*reinterpret_cast<const float2*>(rstd_q + tok), splat2(gs_inv)),
-                             fk = mul2(*reinterpret_cast<const float2*>(rstd_k + tok), splat2(gs_inv));
+                const float2 fq = mul2(*reinterpret_cast<const float2*>(rstd_q + tok), splat2(gs_inv * BG_UP)),
+                             fk = mul2(*reinterpret_cast<const float2*>(rstd_k + tok), splat2(gs_inv * BG_UP));
                 float2 tq = make_float2(0.f, 0.f), tk = tq;
                 if (p.use_l2norm) {
                     tq = *reinterpret_cast<const float2*>(part + 1024 + tok);
@@ -637,7 +643,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
     const size_t tok_stride = (size_t)p.H * DK;
     const size_t base = (size_t)ci.row0 * tok_stride + (size_t)h * DK;
     const float* scr = p.scratch + (size_t)tile * (size_t)BWD_SCRATCH_FLOATS;
-    const float gs_inv = p.gscale[1];
+    const float gs_up = p.gscale[1] * BG_UP;
     const float alpha = p.gate_mode != GATE_NONE ? __expf(p.A_log[h]) : 0.f;
     float bias[2] = {0.f, 0.f};
     if (p.gate_mode != GATE_NONE && p.dt_bias) {
@@ -808,7 +814,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
             if (GK == BG_BF16 && part < 2) prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(p.g) + o + 64 * part);
         }
     }
-    float cs[2] = {0.f, 0.f};      // sum over the tokens of dKg * Kg, the gradient that reaches g_last through kg
+    float cs[2] = {0.f, 0.f};      // sum over the tokens of dKg * Kg (times BG_DOWN), the gradient that reaches g_last through kg
     {
         // ---- 5b. column side: rows of block I against columns of the blocks J <= I ----
         float acc[8][4];
@@ -822,7 +828,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
             load_raw(BG_K, J, kr);
             const float rN[2] = {rt[(J + 1) * DK + ch0], rt[(J + 1) * DK + ch0 + 8]};
             const float d[2] = {rN[0] - rt[J * DK + ch0], rN[1] - rt[J * DK + ch0 + 8]};
-            const float gl[2] = {fast_exp2(glast[0] - rN[0]), fast_exp2(glast[1] - rN[1])};
+            const float gl[2] = {BG_DOWN * fast_exp2(glast[0] - rN[0]), BG_DOWN * fast_exp2(glast[1] - rN[1])};
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
                 const int n = 2 * J + hh;
@@ -874,10 +880,11 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
                     bg_mma(bl[0], khi[hh], f[0], f[1]);
                     bg_mma(bl[1], khi[hh], f[2], f[3]);
                 }
-                float cji[2] = {1.f, 1.f};
+                float cji[2] = {BG_DOWN, BG_DOWN};
                 if (I != J + 1) {
 #pragma unroll
-                    for (int x = 0; x < 2; ++x) cji[x] = fast_exp2(fminf(rt[I * DK + ch0 + 8 * x] - rt[(J + 1) * DK + ch0 + 8 * x], 126.f));
+                    for (int x = 0; x < 2; ++x)
+                        cji[x] = BG_DOWN * fast_exp2(fminf(rt[I * DK + ch0 + 8 * x] - rt[(J + 1) * DK + ch0 + 8 * x], 126.f));
                 }
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh)
@@ -903,7 +910,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
         for (int x = 0; x < 2; ++x) {     // g_last sits in token 63 (padding rows repeat the last real value): its gradient starts the sum
             cs[x] += __shfl_xor_sync(0xffffffffu, cs[x], 1);
             cs[x] += __shfl_xor_sync(0xffffffffu, cs[x], 2);
-            run[x] = cs[x] + fast_exp2(glast[x]) * scr[SCR_DD + ch0 + 8 * x];
+            run[x] = cs[x] + BG_DOWN * fast_exp2(glast[x]) * scr[SCR_DD + ch0 + 8 * x];
         }
         float dA_part = 0.f, colsum[2] = {0.f, 0.f};
         float* hpart = reinterpret_cast<float*>(sm + BG_X);      // per-head gates: [8 slices][64] sums over channels
@@ -928,7 +935,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
                 const float4 dq = *slot(BG_DW, BG_DW + 16384, n), dp = *slot(BG_C1, BG_X2, n), dm = *slot(BG_AN, BG_AT, n);
                 const float2 rq = *reinterpret_cast<const float2*>(rstd_q + tok), rk = *reinterpret_cast<const float2*>(rstd_k + tok);
                 const float dqv[4] = {dq.x, dq.y, dq.z, dq.w}, dkv[4] = {dp.x - dm.x, dp.y - dm.y, dp.z - dm.z, dp.w - dm.w};
-                const float sa = tok < ci.valid ? gs_inv : 0.f, sb = tok + 1 < ci.valid ? gs_inv : 0.f;
+                const float sa = tok < ci.valid ? gs_up : 0.f, sb = tok + 1 < ci.valid ? gs_up : 0.f;
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
                     const float2 qh = mul2(unpack_bf16(qr[hh][x]), rq), kh = mul2(unpack_bf16(kr[hh][x]), rk);

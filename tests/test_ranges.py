@@ -66,3 +66,28 @@ def test_decays_beyond_the_safe_range_stay_finite(decay, l2):
     got, ref = forward_backward(c, l2=l2)
     assert torch.isfinite(got["o"]).all()
     assert err_ratio(ref["ht"], got["ht"]) <= 2e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("decay,magnitude,per_head", [(5.0, 1.0, False), (5.0, 300.0, False), (5.0, 300.0, True), (9.0, 300.0, False), (30.0, 1.0, False)])
+def test_gradients_at_the_strongest_decays(decay, magnitude, per_head):
+    """-5 nats on every token and channel, the end of the safe range: the factor of a 16-row block with itself is 2^116, and with
+    values of a few hundred the sums that it scales are above 2^12. Beyond the safe range the gradients are not claimed to be
+    accurate, but finite."""
+    from cula_b200.gdn import chunk_gated_delta_rule
+    c = make(seed=2)
+    c["g"], c["v"], c["h0"] = torch.full_like(c["g"], -decay), magnitude * c["v"], magnitude * c["h0"]
+    if per_head:
+        expanded = c["g"]
+        dev = {n: (c[n][..., 0] if n == "g" else c[n]).to(torch.float32 if n in ("g", "h0") else torch.bfloat16).cuda().requires_grad_(True) for n in NAMES}
+        o, ht = chunk_gated_delta_rule(*(dev[n] for n in NAMES[:5]), initial_state=dev["h0"], output_final_state=True, use_qk_l2norm_in_kernel=True)
+        grads = torch.autograd.grad([o, ht], list(dev.values()), [c["do"].to(torch.bfloat16).cuda(), c["dht"].cuda()])
+        got = {n: t.detach().float().cpu() for n, t in dict(o=o, ht=ht, **{"d" + n: g for n, g in zip(NAMES, grads)}).items()}
+        c["g"] = expanded
+        _, ref = forward_backward(c)
+        ref["dg"] = ref["dg"].sum(-1)
+    else:
+        got, ref = forward_backward(c)
+    assert all(torch.isfinite(t).all() for t in got.values()), [n for n, t in got.items() if not torch.isfinite(t).all()]
+    if decay <= 5:
+        assert_close(got, ref)
