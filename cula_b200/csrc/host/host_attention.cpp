@@ -122,7 +122,7 @@ Forward forward_core(const Tensor& q, const Tensor& k, const Tensor& v, const Te
     if (store_bwd) f.mkk = device_empty({tiles, CHUNK, CHUNK}, f32);
     // a batch of several sequences comes out piece by piece, which what is kept for later cannot
     if (!leave_scan && !tab && !store_states && !(store_akk && !store_bwd) && (B == 1 || !store_bwd)) {
-        const Plan plan = plan_pieces(B * H, f.num_chunks / B, at::cuda::getDeviceProperties(q.device().index())->multiProcessorCount);
+        const Plan plan = plan_pieces(B * H, (T + CHUNK - 1) / CHUNK, at::cuda::getDeviceProperties(q.device().index())->multiProcessorCount);
         // side-by-side segments are the other way to fill the GPU, better with few heads (the two cross between 24 and 32)
         const double nc = (double)f.num_chunks, seg_us = segs ? nc * (H * 0.0535 + 2 * (1.6 + H / 128.0) / segs->count) + 10 * segs->count : 1e30;
         if (plan.pieces.size() > 1 && 1.06 * plan.us < seg_us) {
@@ -384,7 +384,7 @@ pybind11::tuple attend(const Tensor& q, const Tensor& k, const Tensor& v, const 
     require(c10::InferenceMode::is_enabled(), "return_intermediate_states is only allowed in inference mode");
     require(!disable_recompute, "return_intermediate_states must be used with disable_recompute=False");
     const int64_t B = q.size(0), H = q.size(2);
-    Tensor h = f.h.view({tab ? 1 : B, tab ? f.num_chunks : f.num_chunks / B, H, DIM, DIM});
+    Tensor h = f.h.view({tab ? 1 : B, tab ? f.num_chunks : (q.size(1) + CHUNK - 1) / CHUNK, H, DIM, DIM});
     return pybind11::make_tuple(obj(f.o), obj(f.final_state), obj(h));
 }
 

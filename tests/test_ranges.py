@@ -91,3 +91,20 @@ def test_gradients_at_the_strongest_decays(decay, magnitude, per_head):
     assert all(torch.isfinite(t).all() for t in got.values()), [n for n, t in got.items() if not torch.isfinite(t).all()]
     if decay <= 5:
         assert_close(got, ref)
+
+
+@pytest.mark.gpu
+def test_empty_batch():
+    """B = 0: empty results, as for any operator of torch, with gradients wanted, kept states and a long T included."""
+    from cula_b200.gdn import chunk_gated_delta_rule
+    from cula_b200.kda import chunk_kda
+    for T in (100, 8192):
+        q, k, v = (torch.empty(0, T, 3, 128, dtype=torch.bfloat16, device="cuda") for _ in range(3))
+        g, beta = torch.empty(0, T, 3, 128, device="cuda"), torch.empty(0, T, 3, device="cuda")
+        o, ht = chunk_kda(q, k, v, g, beta, output_final_state=True)
+        assert o.shape == (0, T, 3, 128) and ht.shape == (0, 3, 128, 128)
+        with torch.inference_mode():
+            o, ht, h = chunk_kda(q, k, v, g, beta, output_final_state=True, return_intermediate_states=True)
+        assert h.shape == (0, (T + 63) // 64, 3, 128, 128)
+        o, _ = chunk_gated_delta_rule(q.clone().requires_grad_(True), k, v, g[..., 0], beta)
+        assert o.shape == (0, T, 3, 128) and o.requires_grad
