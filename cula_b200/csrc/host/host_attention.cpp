@@ -298,6 +298,8 @@ public:
 };
 
 bool any_requires_grad(std::initializer_list<const Tensor*> ts, std::initializer_list<const OptTensor*> os) {
+    for (const Tensor* t : ts) if (has_tangent(*t)) return true;
+    for (const OptTensor* t : os) if (t->has_value() && has_tangent(**t)) return true;
     if (!at::GradMode::is_enabled()) return false;
     for (const Tensor* t : ts) if (t->requires_grad()) return true;
     for (const OptTensor* t : os) if (t->has_value() && (*t)->requires_grad()) return true;

@@ -66,6 +66,8 @@ inline Tensor device_zeros(at::IntArrayRef sizes, const at::TensorOptions& optio
     if (e != cudaSuccess) throw std::runtime_error(std::string("cudaMemsetAsync failed: ") + cudaGetErrorString(e));
     return t;
 }
+// a dual tensor of forward-mode differentiation: no operator here has a forward derivative, and only the autograd function says so
+inline bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
 inline cudaStream_t stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
 // B200 guard (cached per device), and the status word of a device: one int in pinned host memory that the kernels write

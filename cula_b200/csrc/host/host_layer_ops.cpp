@@ -9,6 +9,8 @@ using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
 bool grad_wanted(std::initializer_list<OptTensor> ts) {
+    for (const OptTensor& t : ts)
+        if (t.has_value() && has_tangent(*t)) return true;
     if (!at::GradMode::is_enabled()) return false;
     for (const OptTensor& t : ts)
         if (t.has_value() && t->defined() && t->requires_grad()) return true;

@@ -108,3 +108,29 @@ def test_empty_batch():
         assert h.shape == (0, (T + 63) // 64, 3, 128, 128)
         o, _ = chunk_gated_delta_rule(q.clone().requires_grad_(True), k, v, g[..., 0], beta)
         assert o.shape == (0, T, 3, 128) and o.requires_grad
+
+
+@pytest.mark.gpu
+def test_forward_mode_differentiation_is_refused():
+    """No operator has a forward derivative: a dual tensor raises instead of losing its tangent."""
+    import torch.autograd.forward_ad as fw
+
+    from cula_b200.gdn import chunk_gated_delta_rule
+    from cula_b200.kda import chunk_kda, fused_beta_sigmoid, fused_kda_gate, rms_norm_gated, short_conv
+    c = {n: t.cuda().to(torch.float32 if n in ("g", "h0") else torch.bfloat16) for n, t in make(T=64).items()}
+    c["q"], c["k"] = unit(c["q"]), unit(c["k"])
+    weight, x = torch.ones(128, device="cuda"), c["v"].reshape(1, 64, 256)
+    with fw.dual_level():
+        def dual(t):
+            return fw.make_dual(t, torch.ones_like(t))
+
+        calls = [lambda n=n: chunk_kda(*(dual(c[m]) if m == n else c[m] for m in NAMES[:5])) for n in NAMES[:5]]
+        calls += [lambda: chunk_kda(*(c[m] for m in NAMES[:5]), initial_state=dual(c["h0"])),
+                  lambda: chunk_gated_delta_rule(dual(c["q"]), c["k"], c["v"], c["g"][..., 0], c["beta"]),
+                  lambda: fused_kda_gate(dual(c["g"]), torch.zeros(2, device="cuda")), lambda: fused_beta_sigmoid(dual(c["beta"])),
+                  lambda: short_conv(x, dual(torch.ones(256, 4, device="cuda"))), lambda: rms_norm_gated(c["q"], dual(c["k"]), weight)]
+        for call in calls:
+            with pytest.raises((RuntimeError, NotImplementedError), match="jvp"):
+                call()
+        with torch.no_grad(), pytest.raises((RuntimeError, NotImplementedError), match="jvp"):
+            calls[0]()
