@@ -166,6 +166,15 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
 
     if (warp == BS_LOAD_WARP) {
         // ------------------------------- producer -------------------------------
+        // The ragged last chunk of a sequence, which comes first, fetches its dO rows one by one: a box of 64 rows would reach past
+        // the end of the tensor, and how many rows that has is not known here (T says nothing about a packed batch).
+        const int ragged = len - (nchunks - 1) * BT;
+        if (nchunks > 0 && ragged < BT) {
+            if (lane == 0) mbar_expect_tx(&full[0], ragged * DV * 2);
+            __syncwarp();
+            const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(p.d_o) + ((size_t)(bos + (nchunks - 1) * BT) * p.H + h) * DV;
+            for (int row = lane; row < ragged; row += 32) bulk_g2s(sm + BS_DO + row * DV * 2, src + (size_t)row * p.H * DV, DV * 2, &full[0]);
+        }
         if (lane == 0) {
             int issued = 0;
             bool ok = true;
@@ -176,8 +185,9 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
                 const unsigned char* tile = p.tiles + (size_t)t_id * TP_BYTES;
                 unsigned char* dst = sm + s * BS_STAGE_BYTES;
                 const uint32_t d = smb + s * BS_STAGE_BYTES;
-                mbar_arrive_expect_tx(&full[s], 4 * 16384 + 8192 + 512);
-                tma_load_3d(d + BS_DO, &map_do, 0, h, bos + c * BT, &full[s]);     // first: the value warps work on it ahead of the chain
+                const bool box = it > 0 || ragged == BT;
+                mbar_arrive_expect_tx(&full[s], 3 * 16384 + 8192 + 512 + (box ? 16384 : 0));
+                if (box) tma_load_3d(d + BS_DO, &map_do, 0, h, bos + c * BT, &full[s]);     // first: the value warps work on it ahead of the chain
                 bulk_g2s(dst + BS_AQK, tile + TP_AQK, 8192, &full[s]);
 #pragma unroll
                 for (int m = 2; m >= 0; --m)       // KG, QG, W
@@ -476,9 +486,9 @@ extern "C" int kda_launch_bwd_scan(const kda::BwdScanParams* p, cudaStream_t str
     static std::atomic<unsigned long long> done;
     cudaError_t e = allow_smem(kda_bwd_scan_kernel, BS_SMEM, done);
     if (e != cudaSuccess) return (int)e;
-    // packed batches hold T tokens altogether; the number of their tiles is not known here, but the kernel's coordinates stay inside
+    // the numbers of tiles and tokens are not known here for a packed batch; the kernel's coordinates stay inside the caller's tensors
     CUtensorMap map, map_do;
-    if (!make_pack_map(&map, p->tiles, 1ll << 24) || !make_rows_map(&map_do, const_cast<void*>(p->d_o), p->H, p->cu_seqlens ? p->T : (long long)p->N * p->T))
+    if (!make_pack_map(&map, p->tiles, 1ll << 24) || !make_rows_map(&map_do, const_cast<void*>(p->d_o), p->H, 1ll << 30))
         return (int)cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p->H, p->N);

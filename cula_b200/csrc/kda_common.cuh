@@ -185,6 +185,10 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
+// more bytes for the phase that is open, without an arrival
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
 // One bounded poll: the hardware suspends the warp until the phase completes or the hint (in nanoseconds) runs out, so that
 // waiting warps do not take issue slots from the working ones of their scheduler.
 constexpr uint32_t MBAR_SUSPEND_NS = 16384;

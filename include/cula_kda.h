@@ -8,6 +8,7 @@
  *     cula/ops/chunk_delta_h.py:2119-2138);
  *   - tensors are contiguous, token-major: q/k/g [B*T, H, 128], v/o [B*T, H, 128], beta [B*T, H];
  *     a packed (varlen) batch is one sequence axis of cu_seqlens[N] tokens, B == 1;
+ *   - T is the length of the sequences of a fixed-length batch; with d_cu_seqlens it is not used and may be anything;
  *   - `stream` is a cudaStream_t passed as void*; all work is enqueued on it, nothing synchronises;
  *   - return value: 0 = ok, < 0 = argument error (CULA_KDA_E*), > 0 = a cudaError_t from the launch.
  *     The reference instead throws c10::Error from TORCH_CHECK (csrc/api/kda_sm100.cu:46-50) and

@@ -134,3 +134,46 @@ def test_forward_mode_differentiation_is_refused():
                 call()
         with torch.no_grad(), pytest.raises((RuntimeError, NotImplementedError), match="jvp"):
             calls[0]()
+
+
+@pytest.mark.gpu
+def test_reverse_scan_of_a_packed_batch_does_not_depend_on_T():
+    """Through the C ABI: T is the length of fixed-length sequences and means nothing beside d_cu_seqlens. Zero, a longest length
+    and the packed total give the same bits, with full and ragged last chunks, and nothing past the packed rows is read."""
+    from cula_b200 import _native
+    from cula_b200.kda import check_status
+    from cula_b200.kda.chunk import _status_ptr
+    from cula_b200.utils import VarlenTables
+    lens, H = [64, 1, 130, 0, 128, 63, 200], 2
+    total = sum(lens)
+    c = make(T=total, H=H, seed=3)
+    d = {n: c[n].cuda().to(torch.float32 if n == "g" else torch.bfloat16) for n in ("q", "k", "v", "g", "beta")}
+    do = torch.full((total + 64, H, 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    do[:total] = c["do"][0]
+    tab = VarlenTables(torch.tensor([0, *torch.tensor(lens).cumsum(0)], dtype=torch.int32).cuda())
+    lib, nt, N, f32 = _native.lib(), tab.num_chunks * H, len(lens), dict(dtype=torch.float32, device="cuda")
+    stream, status = torch.cuda.current_stream().cuda_stream, _status_ptr(do.device)
+    pack = torch.empty(nt * lib.cula_kda_tile_pack_bytes(), dtype=torch.uint8, device="cuda")
+    cu, ci, co = (t.data_ptr() for t in (tab.cu_seqlens, tab.chunk_indices, tab.chunk_offsets))
+    _native.check(lib.cula_kda_fwd_intra(*(d[n].data_ptr() for n in ("q", "k", "v", "g")), 1, d["beta"].data_ptr(), 0, None, None, cu, ci, tab.num_chunks,
+                                         0, H, 128 ** -0.5, 1, 0, 0.0, pack.data_ptr(), None, None, status, stream), "intra")
+    gscale = torch.tensor([2.0, 0.5, 0, 0], **f32)
+    dht, h0 = torch.randn(N, H, 128, 128, **f32), torch.randn(N, H, 128, 128, **f32)
+    results = []
+    for T in (total, 0, 200, -1):
+        for both in (False, True):
+            out = [torch.zeros(nt, 64, 128, dtype=torch.float16, device="cuda"), torch.zeros(nt, 128, 128, **f32), torch.zeros(N, H, 128, 128, **f32)]
+            p = [t.data_ptr() for t in out]
+            if both:
+                vnew, h32 = torch.empty_like(out[0]), torch.empty_like(out[1])
+                code = lib.cula_kda_bwd_both_scans(pack.data_ptr(), h0.data_ptr(), vnew.data_ptr(), h32.data_ptr(), do.data_ptr(), dht.data_ptr(),
+                                                   gscale.data_ptr(), *p, cu, co, None, N, T, H, status, stream)
+            else:
+                code = lib.cula_kda_bwd_scan(pack.data_ptr(), do.data_ptr(), dht.data_ptr(), gscale.data_ptr(), *p, cu, co, None, N, T, H, status, stream)
+            _native.check(code, "reverse scan")
+            results.append(out)
+    torch.cuda.synchronize()
+    check_status()
+    assert all(torch.isfinite(t).all() for t in results[0])
+    for other in results[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(results[0], other))
