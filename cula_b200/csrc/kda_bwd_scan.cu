@@ -36,7 +36,7 @@ constexpr int BS_W = 0, BS_QG = 16384, BS_KG = 32768, BS_AQK = 49152, BS_DO = 57
 static_assert(BS_STAGE_BYTES % 1024 == 0, "operand atoms are 1024-byte aligned");
 constexpr int BS_OST_BYTES = BT * DV * 2;                    // staged dVn rows
 constexpr int BS_OST = BS_STAGES * BS_STAGE_BYTES, BS_MISC = BS_OST + 2 * BS_OST_BYTES;
-constexpr int BS_SMEM = BS_MISC + 8448 + 1024;
+constexpr int BS_SMEM = BS_MISC + 8512 + 1024;
 // tensor-memory columns: dS, its fp16 copy, two S16 KG^T accumulators (by turn parity; -dVn replaces what was read), two dO
 // operands (by turn parity), dO^T Aqk
 constexpr uint32_t BM_S32 = 0, BM_S16 = 128, BM_ACC = 192, BM_DO = 320, BM_ADO = 384;
@@ -113,10 +113,11 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
              *b_ado = bars + 9, *b_ost = bars + 10, *b_vsum = bars + 11, *b_max = bars + 12 /* [4] */;
     // pairs, because a wait by phase parity must not fall two completions behind (see kda_fwd_scan.cu): turn i uses barrier i & 1
     uint64_t *b_v16 = bars + 16 /* [2] */, *b_oread = bars + 18 /* [2] */;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + BS_MISC + 192);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + BS_MISC + 240);
     float* sDown = reinterpret_cast<float*>(sm + BS_MISC + 256);         // [4 turns][128 value columns] 1 / scale of S16
-    float* sMax = reinterpret_cast<float*>(sm + BS_MISC + 2304);         // [2 turn parities][4 key quarters][128] largest |dS'| of a column
+    float* sMax = reinterpret_cast<float*>(sm + BS_MISC + 2304);         // [2 turn parities][4 key quarters][128] largest |decayed dS'| of a column
     float* sVsum = reinterpret_cast<float*>(sm + BS_MISC + 6400);        // [2 turn parities][2 token halves][128] sum of |dVn| + |dO|
+    uint32_t* sQW = reinterpret_cast<uint32_t*>(sm + BS_MISC + 8448);    // [4 turns] what |qg| and |w| can reach (see or_operands)
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int h = blockIdx.x, n = p.seq_order ? p.seq_order[blockIdx.y] : blockIdx.y;
@@ -145,6 +146,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
         mbar_init(b_ado, 1);
         mbar_init(b_ost, BS_OUT_WARPS);
         mbar_init(b_vsum, BS_VALUE_WARPS);
+        for (int b = 0; b < 4; ++b) sQW[b] = 0;
         for (int q = 0; q < 4; ++q) mbar_init(&b_max[q], BS_STATE_WARPS / 4);
         for (int b = 0; b < 2; ++b) {
             mbar_init(&b_v16[b], BS_VALUE_WARPS);
@@ -266,35 +268,32 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
             umma::ld_32x32b_x32(tl + BM_S32 + k0, reinterpret_cast<uint32_t(&)[32]>(s));
             umma::wait_ld();
         };
-        // Largest |entry| of the value column: this warp's quarter of the keys here, the others from the partner warps.
-        auto publish_max = [&](int it) -> float {
+        // Largest |entry| of the value column in what turn `it` starts from, the decayed dS' of the turn before (see kda_fwd_scan.cu).
+        auto publish_max = [&](int it, float decay) {
             float m0 = 0.f, m1 = 0.f;
 #pragma unroll
             for (int k = 0; k < 32; k += 2) {
                 m0 = fmaxf(m0, fabsf(s[k]));
                 m1 = fmaxf(m1, fabsf(s[k + 1]));
             }
-            m0 = fmaxf(m0, m1);
-            sMax[(it & 1) * 512 + kq * 128 + v] = m0;
+            sMax[(it & 1) * 512 + kq * 128 + v] = fmaxf(m0, m1) * decay;
             warp_arrive(&b_max[q], lane);
-            return m0;
         };
         bool ok = true;
-        if (nchunks > 0) publish_max(0);
+        if (nchunks > 0) publish_max(0, 1.f);
         for (int it = 0; it < nchunks; ++it) {
             const int c = nchunks - 1 - it;
             // The scale of the fp16 copy comes from a bound that is known before the state is (see kda_fwd_scan.cu):
-            // |dS| <= max |dS'| + sum |dO| max |qg| + sum |dVn| max |w|, with decays <= 1 and |qg|, |w| <= 1 for unit keys,
-            // beta <= 1 and scale <= 1 (a factor of 32 is left for others).
-            const int pt = max(it - 1, 0);
-            if (!(ok = wait(&b_max[q], pt))) break;
-            const float* mx = sMax + (pt & 1) * 512 + v;
+            // |dS| <= max |decayed dS'| + max(|qg|, |w|) (sum |dO| + sum |dVn|).
+            if (!(ok = wait(&b_max[q], it))) break;
+            const float* mx = sMax + (it & 1) * 512 + v;
             float bound = fmaxf(fmaxf(mx[0], mx[128]), fmaxf(mx[256], mx[384]));
             if (it > 0) {
+                const int pt = (it - 1) & 1;
                 if (!(ok = wait(b_vsum, it - 1))) break;
-                bound += sVsum[(pt & 1) * 256 + v] + sVsum[(pt & 1) * 256 + 128 + v];
+                bound = fmaf(or_bound(sQW[(it - 1) & 3]), sVsum[pt * 256 + v] + sVsum[pt * 256 + 128 + v], bound);
             }
-            int shift = 10 - (((__float_as_int(bound) >> 23) & 0xff) - 127);
+            int shift = 13 - (((__float_as_int(bound) >> 23) & 0xff) - 127);
             shift = max(-100, min(100, shift));
             const float2 up = splat2(__int_as_float((shift + 127) << 23));
             if (kq == 0) sDown[(it & 3) * 128 + v] = __int_as_float((127 - shift) << 23);
@@ -319,6 +318,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
             const int st = it % BS_STAGES;
             if (!(ok = wait(&full[st], it / BS_STAGES))) break;
             const float* dec = reinterpret_cast<const float*>(sm + st * BS_STAGE_BYTES + BS_DECAY) + k0;
+            const float dec_lane = dec[lane];
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
                 uint32_t r[8];
@@ -335,8 +335,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
             umma::wait_st();
             umma::fence_before_sync();
             warp_arrive(b_dec, lane);
-            // operands far from the assumption can defeat the bound: say so instead of carrying inf on
-            if (it > 0 && overflows(publish_max(it) * up.x)) report_status(p.status, STATUS_RANGE);
+            publish_max(it + 1, __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(dec_lane))));
             if (p.ds_out) {
                 float* dsg = p.ds_out + ((size_t)(chunk0 + c) * p.H + h) * (size_t)(DK * DV) + (size_t)k0 * DV + v;
 #pragma unroll
@@ -376,10 +375,12 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
             }
             dosum = sum.x + sum.y;
             umma::st_32x32b_x16(tl + BM_DO + 32 * (it & 1) + 16 * th, pk);
-            warp_arrive(&empty[st], lane);
             umma::wait_st();
             umma::fence_before_sync();
             warp_arrive(b_do, lane);
+            static_assert(BS_W == 0 && BS_QG == 16384, "one range");
+            or_operands<32768 / BS_VALUE_WARPS>(sm + st * BS_STAGE_BYTES + (4 * th + q) * (32768 / BS_VALUE_WARPS), lane, &sQW[it & 3]);
+            warp_arrive(&empty[st], lane);
             return true;
         };
         bool ok = nchunks == 0 || convert(0);
@@ -390,6 +391,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
             umma::ld_32x32b_x32(tl + BM_ADO + t0, ado);
             umma::wait_ld();
             if (!wait(b_s16, it) || !wait(b_acc, it)) break;
+            if (q == 0 && th == 0 && lane == 0) sQW[(it + 2) & 3] = 0;      // see kda_fwd_scan.cu
             umma::fence_after_sync();
             const uint32_t acc = tl + BM_ACC + 64 * (it & 1) + t0;
             const float2 down = splat2(sDown[(it & 3) * 128 + v]);

@@ -42,7 +42,7 @@ constexpr int ST_WQ = 0, ST_KG = 32768, ST_AQK = 49152, ST_U = 57344, ST_DECAY =
 static_assert(SC_STAGE_BYTES % 1024 == 0, "operand atoms are 1024-byte aligned");
 constexpr int OST_BYTES = 64 * 256;                          // staged token rows
 constexpr int SC_OST = SC_STAGES * SC_STAGE_BYTES, SC_MISC = SC_OST + 2 * OST_BYTES;
-constexpr int SC_SMEM = SC_MISC + 8448 + 1024;
+constexpr int SC_SMEM = SC_MISC + 8512 + 1024;
 // tensor-memory columns: the state, its fp16 copy, two [W | QG] accumulators (by chunk parity, so that the next chunk's product
 // does not wait until this one's outputs have been read), the Aqk product
 constexpr uint32_t TM_S32 = 0, TM_S16 = 128, TM_ACC = 192, TM_QG = 64 /* inside an accumulator */, TM_O2 = 448;
@@ -62,10 +62,11 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
     // A wait by phase parity must not fall two completions behind. v_new can be ready, and have been read, for a chunk while the
     // other side still waits for the chunk before it, so these two are pairs: chunk c uses barrier c & 1 in its phase c / 2.
     uint64_t *b_v16 = bars + 18 /* [2] */, *b_oread = bars + 20 /* [2] */;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + SC_MISC + 192);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + SC_MISC + 240);
     float* sDown = reinterpret_cast<float*>(sm + SC_MISC + 256);         // [4 chunks][128 value columns] 1 / scale of S16: the output warps may be a chunk behind
-    float* sMax = reinterpret_cast<float*>(sm + SC_MISC + 2304);         // [2 chunk parities][4 key quarters][128] largest |S| of a column
+    float* sMax = reinterpret_cast<float*>(sm + SC_MISC + 2304);         // [2 chunk parities][4 key quarters][128] largest |decayed S| of a column
     float* sVsum = reinterpret_cast<float*>(sm + SC_MISC + 6400);        // [2 chunk parities][2 token halves][128] sum of |v_new|
+    uint32_t* sKg = reinterpret_cast<uint32_t*>(sm + SC_MISC + 8448);    // [4 chunks] what |kg| can reach (see or_operands)
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int h = blockIdx.x, n = p.seq_order ? p.seq_order[blockIdx.y] : blockIdx.y;
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
     if (tid == 0) {
         for (int s = 0; s < SC_STAGES; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1 + SC_STATE_WARPS + (is_m ? 0 : SC_VALUE_WARPS));
+            mbar_init(&empty[s], 1 + SC_STATE_WARPS + SC_VALUE_WARPS);
         }
         mbar_init(b_s16, SC_STATE_WARPS);
         mbar_init(b_dec, SC_STATE_WARPS);
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
             mbar_init(&b_oread[b], SC_OUT_WARPS);
         }
         mbar_init(b_vsum, SC_VALUE_WARPS);
+        for (int b = 0; b < 4; ++b) sKg[b] = 0;
         mbar_init(b_s32, 1);
         mbar_init(b_o, 1);
         mbar_init(b_ost, SC_OUT_WARPS);
@@ -214,34 +216,34 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
             umma::ld_32x32b_x32(tl + TM_S32 + k0, reinterpret_cast<uint32_t(&)[32]>(s));
             umma::wait_ld();
         };
-        // Largest |entry| of the value column: this warp's quarter of the keys here, the others from the partner warps.
-        auto publish_max = [&](int c) -> float {
+        // Largest |entry| of the value column in what chunk c starts from, the decayed state of chunk c - 1 (before chunk 0 the state
+        // itself): this warp's quarter of the keys here, the others from the partner warps. `decay`: largest of the quarter.
+        auto publish_max = [&](int c, float decay) {
             float m0 = 0.f, m1 = 0.f;
 #pragma unroll
             for (int k = 0; k < 32; k += 2) {
                 m0 = fmaxf(m0, fabsf(s[k]));
                 m1 = fmaxf(m1, fabsf(s[k + 1]));
             }
-            m0 = fmaxf(m0, m1);
-            sMax[(c & 1) * 512 + kq * 128 + v] = m0;
+            sMax[(c & 1) * 512 + kq * 128 + v] = fmaxf(m0, m1) * decay;
             warp_arrive(&b_max[q], lane);
-            return m0;
         };
         bool ok = true;
-        if (nchunks > 0) publish_max(0);
+        if (nchunks > 0) publish_max(0, 1.f);
         for (int c = 0; c < nchunks; ++c) {
             // The scale of the fp16 copy has to be known when the state arrives, not a reduction over it later. A bound is
-            // enough, fp16 being a floating-point format: |S_c| <= max |S_{c-1}| + sum |v_new| max |kg|, with decays <= 1 and
-            // |kg| <= 1 for unit keys (a factor of 32 is left for others); both terms are ready before the MMA that makes S_c is.
-            const int pc = max(c - 1, 0);
-            if (!(ok = wait(&b_max[q], pc))) break;
-            const float* mx = sMax + (pc & 1) * 512 + v;
+            // enough, fp16 being a floating-point format: |S_c| <= max |decayed S_{c-1}| + max |kg| sum |v_new|, whose terms are
+            // ready before the MMA that makes S_c is. It holds for any keys and decays, so the copy stays below 2^14; where the
+            // terms of the sum cancel it is some binades smaller, of which fp16 has 28 before it loses bits of the largest entries.
+            if (!(ok = wait(&b_max[q], c))) break;
+            const float* mx = sMax + (c & 1) * 512 + v;
             float bound = fmaxf(fmaxf(mx[0], mx[128]), fmaxf(mx[256], mx[384]));
             if (c > 0) {
+                const int pc = (c - 1) & 1;
                 if (!(ok = wait(b_vsum, c - 1))) break;
-                bound += sVsum[(pc & 1) * 256 + v] + sVsum[(pc & 1) * 256 + 128 + v];
+                bound = fmaf(or_bound(sKg[(c - 1) & 3]), sVsum[pc * 256 + v] + sVsum[pc * 256 + 128 + v], bound);
             }
-            int shift = 10 - (((__float_as_int(bound) >> 23) & 0xff) - 127);
+            int shift = 13 - (((__float_as_int(bound) >> 23) & 0xff) - 127);
             shift = max(-100, min(100, shift));
             const float2 up = splat2(__int_as_float((shift + 127) << 23));
             if (kq == 0) sDown[(c & 3) * 128 + v] = __int_as_float((127 - shift) << 23);
@@ -266,6 +268,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
             const int st = c % SC_STAGES;
             if (!(ok = wait(&full[st], c / SC_STAGES))) break;
             const float* dec = reinterpret_cast<const float*>(sm + st * SC_STAGE_BYTES + ST_DECAY) + k0;
+            const float dec_lane = dec[lane];
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
                 uint32_t r[8];
@@ -282,8 +285,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
             umma::wait_st();
             umma::fence_before_sync();
             warp_arrive(b_dec, lane);
-            // keys far from unit length can defeat the bound: say so instead of carrying inf on
-            if (c > 0 && overflows(publish_max(c) * up.x)) report_status(p.status, STATUS_RANGE);
+            publish_max(c + 1, __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(dec_lane))));      // decays are not negative
             const size_t tile_idx = (size_t)(chunk0 + c) * p.H + h;
             if (p.h32_out) {
                 float* hg = p.h32_out + tile_idx * (size_t)(DK * DV) + (size_t)k0 * DV + v;
@@ -315,8 +317,9 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
         for (int c = 0; c < nchunks; ++c) {
             const int st = c % SC_STAGES;
             uint32_t u2[16];                          // this lane's u of 32 tokens, two per register
+            if (!wait(&full[st], c / SC_STAGES)) break;
+            or_operands<16384 / SC_VALUE_WARPS>(sm + st * SC_STAGE_BYTES + ST_KG + (4 * th + q) * (16384 / SC_VALUE_WARPS), lane, &sKg[c & 3]);
             if (!is_m) {
-                if (!wait(&full[st], c / SC_STAGES)) break;
                 const unsigned char* us = sm + st * SC_STAGE_BYTES + ub;
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
@@ -324,12 +327,13 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
                     const uint32_t b = *reinterpret_cast<const uint16_t*>(us + (t0 + 2 * e + 1) * 128 + ((uc ^ ((2 * e + 1) & 7)) << 4));
                     u2[e] = __byte_perm(a, b, 0x5410);
                 }
-                warp_arrive(&empty[st], lane);
             } else {
 #pragma unroll
                 for (int e = 0; e < 16; ++e) u2[e] = 0;
             }
+            warp_arrive(&empty[st], lane);
             if (!wait(b_s16, c) || !wait(b_acc, c)) break;
+            if (q == 0 && th == 0 && lane == 0) sKg[(c + 2) & 3] = 0;      // chunk c - 2 is behind the state warps, c + 2 ahead of every value warp
             umma::fence_after_sync();
             const uint32_t acc = tl + TM_ACC + 128 * (c & 1) + t0;
             const float2 down = splat2(-sDown[(c & 3) * 128 + v]);

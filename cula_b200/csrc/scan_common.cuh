@@ -25,8 +25,22 @@ __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
     if (lane == 0) mbar_arrive(bar);
 }
 
-// the largest finite entry of a state, scaled for fp16, does not fit (inf and NaN of the caller pass through unreported)
-__device__ __forceinline__ bool overflows(float scaled_max) { return scaled_max > 65504.f && scaled_max < INFINITY; }
+// How large fp16 operands in shared memory can be: the bitwise OR of their words. This warp's BYTES of them are added to `acc`.
+// (A maximum takes eight times the instructions, and the warps that have a stage's operands in hand wait for it on the chain.)
+template <int BYTES>
+__device__ __forceinline__ void or_operands(const unsigned char* part, int lane, uint32_t* acc) {
+    uint32_t x = 0;
+#pragma unroll
+    for (int i = 0; i < BYTES / 512; ++i) {
+        const uint4 v = *reinterpret_cast<const uint4*>(part + i * 512 + lane * 16);
+        x |= v.x | v.y | v.z | v.w;
+    }
+    x = __reduce_or_sync(0xffffffffu, x);
+    if (lane == 0) atomicOr(acc, x);
+}
+// A power of two above every entry: twice that of the ORed exponents, which are at least the largest one. Entries on both sides of 1
+// can make it overshoot by up to 2^16; in the bound behind an fp16 scale that costs none of the 11 bits of the largest entries.
+__device__ __forceinline__ float or_bound(uint32_t x) { return __uint_as_float((((x | x >> 16) & 0x7c00u) << 13) + (113u << 23)); }
 
 // W, QG and KG of the tile packs as a rank-4 tensor of fp16: 64 channels, 2 channel halves, 192 rows (64 of each matrix),
 // tiles; fetched as boxes of 64 channels x 64 rows.

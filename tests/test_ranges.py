@@ -177,3 +177,28 @@ def test_reverse_scan_of_a_packed_batch_does_not_depend_on_T():
     assert all(torch.isfinite(t).all() for t in results[0])
     for other in results[1:]:
         assert all(torch.equal(a, b) for a, b in zip(results[0], other))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,value", [("scale", 900.0), ("aligned_keys", 100.0), ("spread_keys", 100.0), ("small_keys", 1e-3)])
+def test_the_scans_take_any_scale_and_key_length(kind, value):
+    """The fp16 copies of the carried states are scaled by a bound that includes the largest |kg|, |qg|, |w| and decay: a large
+    softmax scale with queries the keys do not see, keys far from unit length that all write to one channel or each to its own."""
+    c, scale, l2 = make(seed=4), None, False
+    if kind == "scale":            # queries orthogonal to the keys and gradients of one sign: the state gradient adds up scale * dO
+        scale, l2 = value, True
+        c["k"][..., 0], c["q"], c["do"], c["dht"] = 0, 0.01 * c["q"], c["do"].abs(), 0 * c["dht"]
+        c["q"][..., 0] = 3
+    else:
+        c["k"] = unit(c["k"])
+        if kind == "aligned_keys":
+            c["k"] = torch.zeros_like(c["k"])
+            c["k"][..., 0] = 1
+            c["v"], c["h0"], c["beta"] = c["v"][:, :1].expand_as(c["v"]), 0 * c["h0"], torch.full_like(c["beta"], 0.6)
+        elif kind == "spread_keys":
+            c["k"] = F.one_hot(torch.arange(200) % 128, 128).float().view(1, 200, 1, 128).expand(1, 200, 2, 128)
+        c["q"], c["k"], c["beta"] = unit(c["q"]), value * c["k"], 1.5 * c["beta"] / max(1, value ** 2)
+    got, ref = forward_backward(c, scale=scale, l2=l2, dtype=torch.float64)
+    # one key and one value over and over: what a token adds to the state falls to the few percent by which the state decays per
+    # token, a difference of fp16 terms (2^-11 each) some 50 times as large, and dk and dg are proportional to it
+    assert_close(got, ref, **({"dk": 5e-2, "dg": 1e-1} if kind == "aligned_keys" else {}))
