@@ -286,9 +286,10 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
     }
     __syncthreads();
 
-    // fp16 operands of the Gram product: 2^SH on either side keeps small gate factors of unit rows out of the subnormals;
-    // rows of unknown length (no normalisation in the kernel) are taken as they are
-    const float SH = p.use_l2norm ? 6.f : 0.f;
+    // fp16 operands of the Gram product: 2^SH on either side keeps small gate factors of unit rows out of the subnormals. Where an
+    // operand may be large, they are taken as they are: rows of unknown length (no normalisation in the kernel), decays that can
+    // be positive (not activated in the kernel), a softmax scale, which rides on q, that 2^6 could carry past 65504
+    const float SH = p.use_l2norm && p.gate_mode != GATE_NONE && fabsf(p.scale) <= 512.f ? 6.f : 0.f;
     const float unshift = fast_exp2(-SH), unshift2 = fast_exp2(-2.f * SH);
     // byte offset of this lane's segment of row A / B inside an atom (c and h toggle bits 6 and 3)
     const uint32_t segA = (uint32_t)(rowA * 128 + ((t ^ (rowA & 7)) << 4) + 8 * sx);

@@ -202,3 +202,44 @@ def test_the_scans_take_any_scale_and_key_length(kind, value):
     # one key and one value over and over: what a token adds to the state falls to the few percent by which the state decays per
     # token, a difference of fp16 terms (2^-11 each) some 50 times as large, and dk and dg are proportional to it
     assert_close(got, ref, **({"dk": 5e-2, "dg": 1e-1} if kind == "aligned_keys" else {}))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale,gate", [(511.0, True), (513.0, True), (2e4, True), (2e4, False), (1e-3, False)])
+def test_softmax_scale_up_to_the_fp16_range(scale, gate):
+    """scale q k and scale q are stored as fp16, whose range is the limit; the operands of the Gram product must not end earlier."""
+    from cula_b200.kda import check_status, chunk_kda
+    c = make(seed=5)
+    raw = (c["g"] * 100 - 2).to(torch.bfloat16)
+    kw = dict(use_gate_in_kernel=True, safe_gate=True, lower_bound=-5.0, A_log=torch.zeros(2)) if gate else {}
+    x = {n: c[n].to(torch.bfloat16) for n in ("q", "k", "v", "beta")}
+    x["q"][..., 0], x["k"][..., 0] = 30, -30           # a channel that holds most of both rows
+    args = [x["q"], x["k"], x["v"], raw if gate else c["g"], x["beta"]]
+    ref, ref_h = chunk_kda_oracle(*args, scale=scale, initial_state=c["h0"], output_final_state=True, use_qk_l2norm_in_kernel=True,
+                                  dtype=torch.float64, **kw)
+    kw = {n: t.cuda() if isinstance(t, torch.Tensor) else t for n, t in kw.items()}
+    o, ht = chunk_kda(*(t.cuda() for t in args), scale=scale, initial_state=c["h0"].cuda(), output_final_state=True, use_qk_l2norm_in_kernel=True, **kw)
+    torch.cuda.synchronize()
+    check_status()
+    assert err_ratio(ref, o.cpu()) <= 5e-3 and err_ratio(ref_h, ht.cpu()) <= 2e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("growth", [0.05, 0.07])
+def test_growing_states(growth):
+    """Positive log decays (a factor of 88 over a chunk at 0.07) with normalised rows, every token with a key of its own: the column
+    factors of the Gram product exceed 1 and must not be shifted towards the end of the fp16 range on top of that."""
+    from cula_b200.gdn import chunk_gated_delta_rule
+    from cula_b200.kda import check_status, chunk_kda
+    c = make(seed=6)
+    c["g"], c["h0"] = torch.full_like(c["g"], growth), 1e-2 * c["h0"]
+    c["k"] = F.one_hot(torch.arange(200) % 128, 128).float().view(1, 200, 1, 128).expand(1, 200, 2, 128)
+    c = {n: t.to(torch.bfloat16) if n in ("q", "k", "v", "beta") else t for n, t in c.items()}
+    ref, ref_h = chunk_kda_oracle(*(c[n] for n in NAMES[:5]), initial_state=c["h0"], output_final_state=True, use_qk_l2norm_in_kernel=True,
+                                  dtype=torch.float64)
+    for fn, g in ((chunk_kda, c["g"]), (chunk_gated_delta_rule, c["g"][..., 0])):
+        o, ht = fn(*(t.cuda() for t in (c["q"], c["k"], c["v"], g, c["beta"])), initial_state=c["h0"].cuda(), output_final_state=True,
+                   use_qk_l2norm_in_kernel=True)
+        torch.cuda.synchronize()
+        check_status()
+        assert err_ratio(ref, o.cpu()) <= 5e-3 and err_ratio(ref_h, ht.cpu()) <= 2e-3
