@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
     volatile int* sAbort = reinterpret_cast<volatile int*>(sm + SM_MISC + 552);
     float* sAlpha = reinterpret_cast<float*>(sm + SM_MISC + 560);        // [2] exp(A_log[h])
     int4* sInfo = reinterpret_cast<int4*>(sm + SM_MISC + 576);           // [2] {first token row, valid rows, head, tile slot}
+    float* sBetaMax = reinterpret_cast<float*>(sm + SM_MISC + 608);      // [2][2 warps] largest |beta| of the tile
     float* sBiasBuf = reinterpret_cast<float*>(sm + SM_BIAS);            // [2][128]
     float* sEdgeA = reinterpret_cast<float*>(sm + SM_EDGE);              // [4][128]
     float* sEdgeT = sEdgeA + 4 * DK;                                     // [4][128]
@@ -272,6 +273,8 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
             float b = p.beta_fp32 ? __uint_as_float(sc_next) : __uint_as_float(sc_next << 16);
             if (p.beta_logit) b = (tid < valid_rows) ? __fdividef(1.f, 1.f + __expf(-b)) : 0.f;    // padding rows stay 0
             sBetaBuf[buf * BT + tid] = b;
+            const uint32_t most = __reduce_max_sync(0xffffffffu, __float_as_uint(b) & 0x7fffffffu);
+            if (lane == 0) sBetaMax[2 * buf + warp] = __uint_as_float(most);
         }
         else if (tid < BT + DK) sBiasBuf[buf * DK + tid - BT] = __uint_as_float(sc_next);
         else if (tid == BT + DK) sAlpha[buf] = p.gate_mode != GATE_NONE ? __expf(__uint_as_float(sc_next)) : 0.f;
@@ -821,6 +824,13 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
         }
     }
     __syncthreads();
+    // A tile whose betas are all small takes them times a power of two (largest in [1/2, 1)) into the fp16 operand, and that out of w
+    // and u again; 1, and no work, from 2^-6 up
+    float beta_up = 1.f;
+    {
+        const float most = fmaxf(sBetaMax[2 * par], sBetaMax[2 * par + 1]);
+        if (most < 0.015625f && most > 0.f) beta_up = __int_as_float(min(253 - (__float_as_int(most) >> 23), 127 + 60) << 23);
+    }
     {
         // second level: block rows 32..63 x columns 0..31. One 16x8 tile per warp (2 m-tiles x 4 n-tiles)
         const int mt = warp >> 2, nt = warp & 3;
@@ -838,7 +848,11 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
         {
             const int half = tid >> 7, row = 32 * half + ((tid >> 2) & 31), ch = 4 * half + (tid & 3);
             const float4 lo = *reinterpret_cast<const float4*>(sAi + row * LROW + 8 * ch), hi = *reinterpret_cast<const float4*>(sAi + row * LROW + 8 * ch + 4);
-            const float4 b0 = *reinterpret_cast<const float4*>(sBeta + 8 * ch), b1 = *reinterpret_cast<const float4*>(sBeta + 8 * ch + 4);
+            float4 b0 = *reinterpret_cast<const float4*>(sBeta + 8 * ch), b1 = *reinterpret_cast<const float4*>(sBeta + 8 * ch + 4);
+            if (beta_up != 1.f) {
+                b0.x *= beta_up; b0.y *= beta_up; b0.z *= beta_up; b0.w *= beta_up;
+                b1.x *= beta_up; b1.y *= beta_up; b1.z *= beta_up; b1.w *= beta_up;
+            }
             const uint4 pk = make_uint4(pack_f16(b0.x * lo.x, b0.y * lo.y), pack_f16(b0.z * lo.z, b0.w * lo.w), pack_f16(b1.x * hi.x, b1.y * hi.y),
                                         pack_f16(b1.z * hi.z, b1.w * hi.w));
             unsigned char* dst = sm + SM_AKK16 + row * 128 + ((ch ^ (row & 7)) << 4);
@@ -861,7 +875,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
         }
         {
             float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            const float2 bc = *reinterpret_cast<const float2*>(sBeta + 8 * nt + 2 * t);
+            const float2 bc = mul2(*reinterpret_cast<const float2*>(sBeta + 8 * nt + 2 * t), splat2(beta_up));
             if (mt == 0) mma_tile_3xtf32<2>(sAi + 32 * LROW + 32, LROW, sT + 8 * nt, TROW, acc, g, t);     // D2inv is lower triangular
             else mma_tile_3xtf32<4>(sAi + 48 * LROW + 32, LROW, sT + 8 * nt, TROW, acc, g, t);
 #pragma unroll
@@ -884,7 +898,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
     __syncthreads();
     PHASE_MARK(8);      // triangular inverse, Y staging, Akk pack
 
-    // ---- 9. [w | u] = Akk diag(beta) [X | Y]: two M=128 x N=128 x K=64 products into TMEM columns 0..127 (w) and 128..255 (u).
+    // ---- 9. [w | u] = Akk diag(beta * beta_up) [X | Y]: two M=128 x N=128 x K=64 products into TMEM columns 0..127 (w) and 128..255 (u).
     //         A = Akk diag(beta) stacked twice (K-major), so TMEM lanes 0..63 and 64..127 both hold the 64 token rows;
     //         B = X, then Y, each as two MN-major 64-channel atoms ----
     if (tid == MMA_THREAD) {
@@ -919,6 +933,14 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
             umma::ld_32x32b_x16(taddr + 32 * cp, r[0]);
             umma::ld_32x32b_x16(taddr + 32 * cp + 16, r[1]);
             umma::wait_ld();
+            if (beta_up != 1.f) {
+                const float down = __int_as_float(0x7f000000 - __float_as_int(beta_up));      // 1 / beta_up
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    r[0][e] = __float_as_uint(down * __uint_as_float(r[0][e]));
+                    r[1][e] = __float_as_uint(down * __uint_as_float(r[1][e]));
+                }
+            }
 #pragma unroll
             for (int hc = 0; hc < 4; ++hc) {
                 const uint32_t* rr = r[hc >> 1] + 8 * (hc & 1);

@@ -243,3 +243,17 @@ def test_growing_states(growth):
         torch.cuda.synchronize()
         check_status()
         assert err_ratio(ref, o.cpu()) <= 5e-3 and err_ratio(ref_h, ht.cpu()) <= 2e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("length,beta", [(1.0, 1e-3), (1.0, 1e-4), (300.0, 1.0), (3000.0, 1.0)])
+def test_small_betas(length, beta):
+    """Step sizes of 1e-5 and less, as keys of length 300 need them: beta rides on the fp16 operand (I + L)^-1, times a power of two
+    where the whole tile is small. (u = beta v itself is stored in fp16: with unit keys 1e-4 is the end.)"""
+    c = make(seed=7)
+    c["q"], c["k"], c["beta"] = unit(c["q"]), length * unit(c["k"]), beta * c["beta"] / length ** 2
+    if length == 1:
+        c["h0"] = 0 * c["h0"]
+    got, ref = forward_backward(c, l2=False, dtype=torch.float64)
+    tol = {"ht": 4e-3, "dk": 1e-2} if length > 1000 else {}      # kg and u near opposite ends of fp16
+    assert_close(got, ref, **tol)
