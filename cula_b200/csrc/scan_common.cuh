@@ -54,8 +54,8 @@ inline bool make_pack_map(CUtensorMap* map, const unsigned char* tiles, long lon
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<unsigned char*>(tiles), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// Token rows [tokens][heads][128] of bf16, moved as boxes of 64 tokens of one head. `tokens` may be an upper bound: the kernels
-// move whole chunks only through this map, which lie inside the tensor.
+// Token rows [tokens][heads][128] of bf16, moved as boxes of 64 tokens of one head; rows past `tokens` are read as zeros. It may be
+// an upper bound where only whole chunks, which lie inside the tensor, are moved.
 inline bool make_rows_map(CUtensorMap* map, void* rows, int H, long long tokens) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
