@@ -63,7 +63,7 @@ def _segments(q):
     from .cp import auto_segments, segment_bounds, segment_tables
     num_chunks = (q.shape[1] + CHUNK - 1) // CHUNK
     P = auto_segments(num_chunks, q.shape[2], q.device)
-    return segment_tables(segment_bounds(q.shape[1], num_chunks, P), q.device).segments(P) if P > 1 else None
+    return segment_tables(segment_bounds(q.shape[1], num_chunks, P), q.device).segments if P > 1 else None
 
 
 def chunk_kda_fwd(q, k, v, g, beta, scale, initial_state, output_final_state, cu_seqlens, cu_seqlens_cpu,

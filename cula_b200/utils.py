@@ -80,10 +80,11 @@ class VarlenTables:
                                                  self.n_seqs, self.num_chunks, self.total_tokens)
         return self._native
 
-    def segments(self, count):
-        """These tables as the ``count`` side-by-side segments of one sequence."""
+    @property
+    def segments(self):
+        """The sequences of these tables as the side-by-side segments of one long sequence."""
         if self._segments is None:
-            self._segments = _native.host().Segments(count, self.native)
+            self._segments = _native.host().Segments(self.n_seqs, self.native)
         return self._segments
 
 

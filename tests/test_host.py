@@ -169,6 +169,25 @@ def test_varlen_tables_are_cached_by_identity_not_by_address():
     assert get_varlen_tables(c) is not tab_c
 
 
+def test_segments_are_as_many_as_the_tables_hold(monkeypatch):
+    """The segments of one long sequence are the sequences of their tables; there is no second count to disagree with them."""
+    from cula_b200 import _native
+    from cula_b200.kda.cp import segment_bounds, segment_tables
+
+    class FakeHost:
+        Tables = staticmethod(lambda *a: a)
+        Segments = staticmethod(lambda count, tables: (count, tables))
+
+    monkeypatch.setattr(_native, "host", lambda: FakeHost)
+    for P in (3, 5, 8, 3):
+        tab = segment_tables(segment_bounds(8192, 128, P), torch.device("cpu"))
+        count, native = tab.segments
+        assert count == tab.n_seqs == P and native[4] == P
+        assert tab.segments is tab.segments
+    monkeypatch.undo()
+    segment_tables.__globals__["_SEGMENT_TABLES"].clear()         # they hold the fake
+
+
 def test_cp_context_kwarg_dispatches_to_the_context_parallel_path(monkeypatch):
     """``chunk_kda(..., cp_context=ctx)`` keeps the reference's one-line call (cula/kda/chunk.py:348-355) and hands
     the shard to ``chunk_kda_cp`` with the group the context carries."""
