@@ -13,29 +13,26 @@ constexpr int BT = 64;    // chunk length (tokens); fixed at 64 as in cula/kda/c
 constexpr int DK = 128;   // key head dim
 constexpr int DV = 128;   // value head dim
 constexpr float RCP_LN2 = 1.4426950408889634f;
-constexpr float LN2 = 0.6931471805599453f;
 
 // ---------------------------------------------------------------------------------------------
-// Forward tile pack: everything the state scan needs for one (chunk, head), contiguous in HBM so
-// that one stage of the scan pipeline is two bulk copies. Each array is stored in the exact image
-// the scan wants in shared memory: row-major with the 16-byte column groups XOR-swizzled by
-// (row & 7), which makes every ldmatrix read bank-conflict free.
+// Forward tile pack: everything the state scans need for one (chunk, head), contiguous in HBM. The
+// matrices are row-major with the 16-byte column groups XOR-swizzled by (row & 7), which is the 128-byte
+// swizzle of tensor-core operand atoms: the scans fetch W, QG and KG as boxes of 64 channels that land as
+// such atoms, and the rest (an atom column already, or no operand) with untiled bulk copies.
 //   W    [64][128] fp16   w  = Akk (beta k 2^g)
 //   QG   [64][128] fp16   qg = scale * q 2^g
 //   KG   [64][128] fp16   kg = k 2^(g_last - g)
 //   AQK  [64][64]  fp16   scale * tril(q k^T gated)
 //   DECAY[128]     fp32   2^(g_last)
-//   U0,U1 [64][64] fp16   u = Akk (beta v), value columns 0..63 and 64..127
+//   U   [2][64][64] fp16  u = Akk (beta v), value columns 0..63, then 64..127
 // ---------------------------------------------------------------------------------------------
 constexpr int TP_W = 0;
 constexpr int TP_QG = 16384;
 constexpr int TP_KG = 32768;
 constexpr int TP_AQK = 49152;
 constexpr int TP_DECAY = 57344;
-constexpr int TP_U0 = 57856;
-constexpr int TP_U1 = 66048;
+constexpr int TP_U = 57856;
 constexpr int TP_BYTES = 74240;
-constexpr int TP_HEAD_BYTES = TP_U0;   // W..DECAY: shared by both value halves
 
 // byte offset of element (row, col) of a 2-byte matrix with 128 columns (256-byte rows)
 __host__ __device__ __forceinline__ int swz256(int row, int col) {
@@ -146,21 +143,6 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t& r0, uint32_t&
 __device__ __forceinline__ void stsm_x4_t(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
     asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};"
                  :: "r"(addr), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
-}
-__device__ __forceinline__ void stsm_x4(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
-    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};"
-                 :: "r"(addr), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
-}
-// D(16x8,f32) += A(16x16) * B(16x8); A row-major fragments, B column fragments.
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 // ---- programmatic dependent launch: a kernel launched with the programmatic-stream-serialization attribute may start

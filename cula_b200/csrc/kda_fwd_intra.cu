@@ -966,7 +966,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
     umma::fence_after_sync();
     if (tid == MMA_THREAD) {       // w, u and Aqk leave as three bulk copies; their buffers are next written by the operand generation
         bulk_s2g(tile + TP_W, sm + SM_STG_W, 16384);
-        bulk_s2g(tile + TP_U0, sm + SM_STG_U, 16384);
+        bulk_s2g(tile + TP_U, sm + SM_STG_U, 16384);
         bulk_s2g(tile + TP_AQK, sm + SM_STG_AQK, 8192);
         bulk_commit();
     }

@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
                     if (want_o) tma_load_4d(d + ST_WQ + a * 16384 + 8192, &map, 0, a, 64, t_id, &full[s]);
                 }
                 bulk_g2s(dst + ST_DECAY, tile + TP_DECAY, 512, &full[s]);
-                if (!is_m) bulk_g2s(dst + ST_U, tile + TP_U0, 16384, &full[s]);
+                if (!is_m) bulk_g2s(dst + ST_U, tile + TP_U, 16384, &full[s]);
 #pragma unroll
                 for (int a = 0; a < 2; ++a) tma_load_4d(d + ST_KG + a * 8192, &map, 0, a, 128, t_id, &full[s]);
                 if (want_o) bulk_g2s(dst + ST_AQK, tile + TP_AQK, 8192, &full[s]);

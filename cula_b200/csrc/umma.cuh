@@ -16,7 +16,7 @@
 namespace kda {
 namespace umma {
 
-constexpr uint32_t FMT_F16 = 0, FMT_BF16 = 1, FMT_TF32 = 2;
+constexpr uint32_t FMT_F16 = 0, FMT_TF32 = 2;
 
 // 32-bit instruction descriptor: fp32 accumulate, dense, no negate.
 __host__ __device__ constexpr uint32_t make_idesc(uint32_t fmt_ab, int M, int N, bool a_mn_major, bool b_mn_major) {
