@@ -272,13 +272,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
         };
         // Largest |entry| of the value column in what turn `it` starts from, the decayed dS' of the turn before (see kda_fwd_scan.cu).
         auto publish_max = [&](int it, float decay) {
-            float m0 = 0.f, m1 = 0.f;
-#pragma unroll
-            for (int k = 0; k < 32; k += 2) {
-                m0 = fmaxf(m0, fabsf(s[k]));
-                m1 = fmaxf(m1, fabsf(s[k + 1]));
-            }
-            sMax[(it & 1) * 512 + kq * 128 + v] = fmaxf(m0, m1) * decay;
+            sMax[(it & 1) * 512 + kq * 128 + v] = abs_max(s) * decay;
             warp_arrive(&b_max[q], lane);
         };
         bool ok = true;
@@ -295,24 +289,15 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
                 if (!(ok = wait(b_vsum, it - 1))) break;
                 bound = fmaf(or_bound(sQW[(it - 1) & 3]), sVsum[pt * 256 + v] + sVsum[pt * 256 + 128 + v], bound);
             }
-            int shift = 13 - (((__float_as_int(bound) >> 23) & 0xff) - 127);
-            shift = max(-100, min(100, shift));
-            const float2 up = splat2(__int_as_float((shift + 127) << 23));
-            if (kq == 0) sDown[(it & 3) * 128 + v] = __int_as_float((127 - shift) << 23);
+            float up, down;
+            fp16_scale(bound, up, down);
+            if (kq == 0) sDown[(it & 3) * 128 + v] = down;
             if (it > 0) {
                 if (!(ok = wait(b_s32, it - 1))) break;
                 umma::fence_after_sync();
                 load_state();
             }
-            {
-                uint32_t pk[16];
-#pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    const float2 x = mul2(make_float2(s[2 * e], s[2 * e + 1]), up);
-                    pk[e] = pack_f16(x.x, x.y);
-                }
-                umma::st_32x32b_x16(tl + BM_S16 + 16 * kq, pk);
-            }
+            store_f16(tl + BM_S16 + 16 * kq, s, up);
             umma::wait_st();
             umma::fence_before_sync();
             warp_arrive(b_s16, lane);
@@ -321,23 +306,12 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
             if (!(ok = wait(&full[st], it / BS_STAGES))) break;
             const float* dec = reinterpret_cast<const float*>(sm + st * BS_STAGE_BYTES + BS_DECAY) + k0;
             const float dec_lane = dec[lane];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                uint32_t r[8];
-#pragma unroll
-                for (int e = 0; e < 8; e += 4) {
-                    const float4 d = *reinterpret_cast<const float4*>(dec + 8 * b + e);
-                    const float2 x = mul2(make_float2(s[8 * b + e], s[8 * b + e + 1]), make_float2(d.x, d.y));
-                    const float2 y = mul2(make_float2(s[8 * b + e + 2], s[8 * b + e + 3]), make_float2(d.z, d.w));
-                    r[e] = __float_as_uint(x.x); r[e + 1] = __float_as_uint(x.y); r[e + 2] = __float_as_uint(y.x); r[e + 3] = __float_as_uint(y.y);
-                }
-                umma::st_32x32b_x8(tl + BM_S32 + k0 + 8 * b, r);
-            }
+            store_decayed(tl + BM_S32 + k0, s, dec);
             warp_arrive(&empty[st], lane);
             umma::wait_st();
             umma::fence_before_sync();
             warp_arrive(b_dec, lane);
-            publish_max(it + 1, __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(dec_lane))));
+            publish_max(it + 1, warp_max_decay(dec_lane));
             if (p.ds_out) {
                 float* dsg = p.ds_out + ((size_t)(chunk0 + c) * p.H + h) * (size_t)(DK * DV) + (size_t)k0 * DV + v;
 #pragma unroll
@@ -425,8 +399,6 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
         // ------------------------------- dVn rows: lane = value column v, all tokens -------------------------------
         const int q = warp, v = 32 * q + lane;
         const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
-        const int odd = lane & 1;
-        const uint32_t sel = odd ? 0x3276u : 0x5410u;
         for (int it = 0; it < nchunks; ++it) {
             const uint32_t acc = tl + BM_ACC + 64 * (it & 1);
             if (!wait(&b_v16[it & 1], it >> 1)) break;
@@ -441,18 +413,9 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
                     umma::fence_before_sync();
                     warp_arrive(&b_oread[it & 1], lane);
                 }
-                // a register holds tokens 2e and 2e + 1 of this column; neighbouring lanes trade halves, so that the even lane
-                // stores token 2e of both columns and the odd lane token 2e + 1
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const uint32_t x = __shfl_xor_sync(0xffffffffu, w[e], 1);
-                    *reinterpret_cast<uint32_t*>(buf + (16 * b + 2 * e + odd) * 256 + (v & ~1) * 2) = __byte_perm(w[e], x, sel) ^ 0x80008000u;
-                }
+                stage_rows(buf, 16 * b, v, w, 0x80008000u);
             }
-            // passing the barrier of a turn also means that the copy of the turn before has been read out
-            fence_proxy_async();
-            if (tid == 0) bulk_wait_read_all();
-            warp_arrive(b_ost, lane);
+            arrive_staged(b_ost, tid);
             if (!wait(b_ost, it)) break;
             if (tid == 0) {
                 bulk_s2g(reinterpret_cast<unsigned char*>(p.dvn_out) + ((size_t)(chunk0 + nchunks - 1 - it) * p.H + h) * (size_t)(BT * DV * 2), buf,

@@ -219,13 +219,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
         // Largest |entry| of the value column in what chunk c starts from, the decayed state of chunk c - 1 (before chunk 0 the state
         // itself): this warp's quarter of the keys here, the others from the partner warps. `decay`: largest of the quarter.
         auto publish_max = [&](int c, float decay) {
-            float m0 = 0.f, m1 = 0.f;
-#pragma unroll
-            for (int k = 0; k < 32; k += 2) {
-                m0 = fmaxf(m0, fabsf(s[k]));
-                m1 = fmaxf(m1, fabsf(s[k + 1]));
-            }
-            sMax[(c & 1) * 512 + kq * 128 + v] = fmaxf(m0, m1) * decay;
+            sMax[(c & 1) * 512 + kq * 128 + v] = abs_max(s) * decay;
             warp_arrive(&b_max[q], lane);
         };
         bool ok = true;
@@ -243,24 +237,15 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
                 if (!(ok = wait(b_vsum, c - 1))) break;
                 bound = fmaf(or_bound(sKg[(c - 1) & 3]), sVsum[pc * 256 + v] + sVsum[pc * 256 + 128 + v], bound);
             }
-            int shift = 13 - (((__float_as_int(bound) >> 23) & 0xff) - 127);
-            shift = max(-100, min(100, shift));
-            const float2 up = splat2(__int_as_float((shift + 127) << 23));
-            if (kq == 0) sDown[(c & 3) * 128 + v] = __int_as_float((127 - shift) << 23);
+            float up, down;
+            fp16_scale(bound, up, down);
+            if (kq == 0) sDown[(c & 3) * 128 + v] = down;
             if (c > 0) {
                 if (!(ok = wait(b_s32, c - 1))) break;
                 umma::fence_after_sync();
                 load_state();
             }
-            {
-                uint32_t pk[16];
-#pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    const float2 x = mul2(make_float2(s[2 * e], s[2 * e + 1]), up);
-                    pk[e] = pack_f16(x.x, x.y);
-                }
-                umma::st_32x32b_x16(tl + TM_S16 + 16 * kq, pk);
-            }
+            store_f16(tl + TM_S16 + 16 * kq, s, up);
             umma::wait_st();
             umma::fence_before_sync();
             warp_arrive(b_s16, lane);
@@ -269,23 +254,12 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
             if (!(ok = wait(&full[st], c / SC_STAGES))) break;
             const float* dec = reinterpret_cast<const float*>(sm + st * SC_STAGE_BYTES + ST_DECAY) + k0;
             const float dec_lane = dec[lane];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                uint32_t r[8];
-#pragma unroll
-                for (int e = 0; e < 8; e += 4) {
-                    const float4 d = *reinterpret_cast<const float4*>(dec + 8 * b + e);
-                    const float2 x = mul2(make_float2(s[8 * b + e], s[8 * b + e + 1]), make_float2(d.x, d.y));
-                    const float2 y = mul2(make_float2(s[8 * b + e + 2], s[8 * b + e + 3]), make_float2(d.z, d.w));
-                    r[e] = __float_as_uint(x.x); r[e + 1] = __float_as_uint(x.y); r[e + 2] = __float_as_uint(y.x); r[e + 3] = __float_as_uint(y.y);
-                }
-                umma::st_32x32b_x8(tl + TM_S32 + k0 + 8 * b, r);
-            }
+            store_decayed(tl + TM_S32 + k0, s, dec);
             warp_arrive(&empty[st], lane);
             umma::wait_st();
             umma::fence_before_sync();
             warp_arrive(b_dec, lane);
-            publish_max(c + 1, __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(dec_lane))));      // decays are not negative
+            publish_max(c + 1, warp_max_decay(dec_lane));
             const size_t tile_idx = (size_t)(chunk0 + c) * p.H + h;
             if (p.h32_out) {
                 float* hg = p.h32_out + tile_idx * (size_t)(DK * DV) + (size_t)k0 * DV + v;
@@ -362,24 +336,11 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
         // ------------------------------- output rows (and v_new): lane = value column v, all tokens -------------------------------
         const int q = warp, v = 32 * q + lane;
         const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
-        const int odd = lane & 1;
-        const uint32_t sel = odd ? 0x3276u : 0x5410u;
-        // a register holds the 16-bit values of tokens 2e and 2e + 1 of this column; neighbouring lanes trade halves, so that the
-        // even lane stores token 2e of both columns and the odd lane token 2e + 1
-        auto stage = [&](unsigned char* buf, int t0, const uint32_t (&w)[8]) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const uint32_t x = __shfl_xor_sync(0xffffffffu, w[e], 1);
-                *reinterpret_cast<uint32_t*>(buf + (t0 + 2 * e + odd) * 256 + (v & ~1) * 2) = __byte_perm(w[e], x, sel);
-            }
-        };
         int turns = 0;                               // staged matrices so far: the two buffers alternate
         // All rows staged: thread 0 sends a whole matrix with one bulk copy (v_new, or a full chunk of o); a ragged last chunk
         // goes out row by row. Passing the barrier of turn t also means that the copy of turn t - 1 has been read out.
         auto turn_over = [&]() -> bool {
-            fence_proxy_async();
-            if (tid == 0) bulk_wait_read_all();
-            warp_arrive(b_ost, lane);
+            arrive_staged(b_ost, tid);
             return wait(b_ost, turns++);
         };
         for (int c = 0; want_out && c < nchunks; ++c) {
@@ -393,7 +354,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
                     uint32_t w[8];
                     umma::ld_32x32b_x8(acc + 32 * (b >> 1) + 8 * (b & 1), w);
                     umma::wait_ld();
-                    stage(buf, 16 * b, w);
+                    stage_rows(buf, 16 * b, v, w);
                 }
                 if (!want_o) {
                     umma::fence_before_sync();
@@ -426,7 +387,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) kda_fwd_scan_kernel(const ScanP
                                               make_float2(__uint_as_float(r2[2 * e]), __uint_as_float(r2[2 * e + 1])));
                         w[e] = pack_bf16(o.x, o.y);
                     }
-                    stage(buf, 16 * b, w);
+                    stage_rows(buf, 16 * b, v, w);
                 }
                 if (!turn_over()) break;
                 const int rows = min(BT, len - c * BT);

@@ -25,6 +25,71 @@ __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
     if (lane == 0) mbar_arrive(bar);
 }
 
+// ---- the carried state, 32 key channels of one value column per lane ----
+__device__ __forceinline__ float abs_max(const float (&s)[32]) {
+    float m0 = 0.f, m1 = 0.f;
+#pragma unroll
+    for (int k = 0; k < 32; k += 2) {
+        m0 = fmaxf(m0, fabsf(s[k]));
+        m1 = fmaxf(m1, fabsf(s[k + 1]));
+    }
+    return fmaxf(m0, m1);
+}
+// Power of two that takes values of at most `bound` below 2^14, and its inverse
+__device__ __forceinline__ void fp16_scale(float bound, float& up, float& down) {
+    int shift = 13 - (((__float_as_int(bound) >> 23) & 0xff) - 127);
+    shift = max(-100, min(100, shift));
+    up = __int_as_float((shift + 127) << 23);
+    down = __int_as_float((127 - shift) << 23);
+}
+// fp16 copy of the state in tensor memory, as A operand
+__device__ __forceinline__ void store_f16(uint32_t taddr, const float (&s)[32], float up) {
+    uint32_t pk[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        const float2 x = mul2(make_float2(s[2 * e], s[2 * e + 1]), splat2(up));
+        pk[e] = pack_f16(x.x, x.y);
+    }
+    umma::st_32x32b_x16(taddr, pk);
+}
+// The state times the decays of its 32 channels, as the accumulator that the chunk's products are added to
+__device__ __forceinline__ void store_decayed(uint32_t taddr, const float (&s)[32], const float* dec) {
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        uint32_t r[8];
+#pragma unroll
+        for (int e = 0; e < 8; e += 4) {
+            const float4 d = *reinterpret_cast<const float4*>(dec + 8 * b + e);
+            const float2 x = mul2(make_float2(s[8 * b + e], s[8 * b + e + 1]), make_float2(d.x, d.y));
+            const float2 y = mul2(make_float2(s[8 * b + e + 2], s[8 * b + e + 3]), make_float2(d.z, d.w));
+            r[e] = __float_as_uint(x.x); r[e + 1] = __float_as_uint(x.y); r[e + 2] = __float_as_uint(y.x); r[e + 3] = __float_as_uint(y.y);
+        }
+        umma::st_32x32b_x8(taddr + 8 * b, r);
+    }
+}
+// Largest of 32 decays, one per lane (they are not negative: as integers they order the same)
+__device__ __forceinline__ float warp_max_decay(float d) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(d))); }
+
+// ---- token rows in shared memory from lane-per-column registers ----
+// A register holds the 16-bit values of tokens t0 + 2e and t0 + 2e + 1 of value column v; neighbouring lanes trade halves, so that
+// the even lane stores the first token of both columns and the odd lane the second. `flip`: bits to toggle (signs).
+__device__ __forceinline__ void stage_rows(unsigned char* buf, int t0, int v, const uint32_t (&w)[8], uint32_t flip = 0) {
+    const int odd = v & 1;
+    const uint32_t sel = odd ? 0x3276u : 0x5410u;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const uint32_t x = __shfl_xor_sync(0xffffffffu, w[e], 1);
+        *reinterpret_cast<uint32_t*>(buf + (t0 + 2 * e + odd) * 256 + (v & ~1) * 2) = __byte_perm(w[e], x, sel) ^ flip;
+    }
+}
+// Everything this thread staged may leave by a bulk copy once all warps have arrived on `bar`; thread 0 also waits until the copy of
+// the turn before has been read out, so that passing the barrier frees that buffer.
+__device__ __forceinline__ void arrive_staged(uint64_t* bar, int tid) {
+    fence_proxy_async();
+    if (tid == 0) bulk_wait_read_all();
+    warp_arrive(bar, tid & 31);
+}
+
 // How large fp16 operands in shared memory can be: the bitwise OR of their words. This warp's BYTES of them are added to `acc`.
 // (A maximum takes eight times the instructions, and the warps that have a stage's operands in hand wait for it on the chain.)
 template <int BYTES>
