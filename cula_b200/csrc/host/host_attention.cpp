@@ -66,8 +66,15 @@ void segmented_scan(const Tensor& v, const OptTensor& h0, bool want_final, const
 // the chunk-parallel stage takes whatever it is given; run after one another, the scan leaves the other SMs idle. So the chunks are
 // cut into pieces, and a piece's chunk-parallel stage runs beside the scan of the piece before. Sizes for which the two just keep
 // step form a geometric series; the first piece's chunk-parallel stage and the last one's scan are exposed. The times are measured,
-// in us. Above half the SMs the scan leaves too little for this to gain (3 x 4096 x 32 heads: 456 -> 476 us). Measured, whole call:
-// 1 x 65536 x 32 heads 2763 -> 2599 us, 1 x 16384 x 48 1075 -> 950, 1 x 4096 x 32 229.5 -> 211, 2 x 8192 x 32 658 -> 640.
+// in us. Above half the SMs the scan leaves too little for this to gain (3 x 4096 x 32 heads: 456 -> 476 us).
+// Both stages one after the other -> in these pieces, us, cold L2, with a bf16 gate / an fp32 gate / a gate per head:
+//   1 x 4096 x 32 heads   238 -> 211     255 -> 227     214 -> 187        2 x 2048 x 32   187 -> 182     204 -> 202     163 -> 156
+//   2 x 8192 x 32         675 -> 639     726 -> 697     585 -> 537        4 x 4096 x 16   349 -> 338     378 -> 370     302 -> 275
+//   1 x 65536 x 32       3418 -> 2465   3610 -> 2719   3051 -> 2338       1 x 16384 x 48 1082 -> 932    1156 -> 1011    949 -> 810
+// The three kernels take 0.053, 0.059 and 0.042 us per tile (8192 tiles). One rate serves all: planned with its own, an fp32 gate
+// came out 1 % slower to 3 % faster and a gate per head 6 % slower to 4 % faster, for other reasons than the plan can know.
+// What keeps its intermediates (training that recomputes, B > 1 that does not) and packed batches have no pieces, and only B = 1
+// without gradients or kept intermediates has segments: few long chains are left as they are there.
 struct Plan {
     std::vector<int> pieces;      // chunks per piece
     double us = 0;

@@ -25,7 +25,7 @@
 //
 // What bounds it: the legacy TF32 pipe is busy for about 10 k of a tile's 44 k cycles, all of them in the two Gram phases (14 to
 // 16 k); the rest is a chain of short dependent phases with 16 warps per SM (41 % of the issue slots) and the 245 KB of the next
-// tile. Measured at 4 x 8192 x 32 heads: 3.48 -> 2.33 ms against one group with token rows in shared memory.
+// tile. Measured at 4 x 8192 x 32 heads: 3.48 -> 2.30 ms against one group with token rows in shared memory.
 #include "kda_common.cuh"
 #include "kda_params.h"
 

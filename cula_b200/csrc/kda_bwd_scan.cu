@@ -8,8 +8,8 @@
 //     dS^T   = dS'^T diag(decay) + dO^T QG - dVn^T W (gradient of the state entering the chunk)
 // What bounds a few long sequences is the latency of that chain: two MMA groups and two register passes per chunk. What bounds a
 // full GPU is HBM, 154 KB in and out per chunk. (The register-resident mma.sync version of this scan ran 224 dependent-issue
-// MMAs per warp and chunk: 3.2 us per chunk, now 2.4. 4 sequences of 128 chunks x 32 heads 661 -> 395..416 us, of which the bytes
-// are 385; 2 x 16 chunks x 3 heads 51.5 -> 41.7 us.) The warps are those of the forward scan:
+// MMAs per warp and chunk: 3.2 us per chunk, now 2.27 with 2 heads. 4 sequences of 128 chunks x 32 heads 661 -> 429 us, cold, of
+// which the bytes are 385.) The warps are those of the forward scan:
 //   warps 0-3     dVn: lane-per-column values become token rows in shared memory and leave as one bulk store;
 //   warps 4-19    dS': out of tensor memory, fp16 copy back in (chain), then the decayed state, dS' per chunk to HBM, dht / dh0;
 //   warps 20-27   dVn (chain), 32 tokens each, and between two chunks the next dO as operand;

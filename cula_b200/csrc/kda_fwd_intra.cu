@@ -26,8 +26,8 @@
 // the tensor pipes and HBM are far from busy). Warp w owns 16-row block w & 3 and channel half w >> 2 of all first phases; its
 // 16-byte row segments make every global access and every operand store a full vector. Two CTAs are resident per SM, so one
 // CTA's operand generation overlaps the other's MMAs, inverse and epilogues.
-// Measured at B=2, T=2048, H=32 (2048 tiles): 140 -> 113 us, 31.7 k -> 24 k warp instructions per tile against the version
-// that formed all of the Gram product as tf32 operands in shared memory, two channel halves one after the other.
+// Measured at B=2, T=2048, H=32 (2048 tiles, cold L2): 143.6 -> 119 us, 31.7 k -> 24 k warp instructions per tile against the
+// version that formed all of the Gram product as tf32 operands in shared memory, two channel halves one after the other.
 #include "kda_common.cuh"
 #include "kda_params.h"
 #include "umma.cuh"

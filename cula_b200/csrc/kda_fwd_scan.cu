@@ -7,8 +7,8 @@
 //     S^T  = S^T diag(decay) + v_new^T KG
 //     o^T  = ACC_QG + v_new^T Aqk^T
 // What bounds it is the latency of that chain, not the tensor pipe: two MMA groups and two register passes per chunk, each
-// handed over by an mbarrier. So everything that is not on the chain runs beside it, in warps of its own. (Measured: 1.6 us per
-// chunk + 6 us; 2.0 with the state in mma.sync registers.)
+// handed over by an mbarrier. So everything that is not on the chain runs beside it, in warps of its own. (Measured, 2 heads: 1.62
+// us per chunk + 10 us, cold; 2.0 per chunk with the state in mma.sync registers. 0.1 of it is the bound on |kg|.)
 //   warps 0-3     output rows and, when asked for, v_new: lane-per-column values are turned into token rows in shared memory
 //                 and leave as one bulk (tensor) store;
 //   warps 4-19    state: S out of tensor memory, fp16 copy back in (chain), then the decayed state (beside the MMAs),

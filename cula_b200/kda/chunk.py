@@ -57,7 +57,9 @@ def _tables(cu_seqlens, cu_seqlens_cpu):
 
 
 def _segments(q):
-    """One long sequence: few scan CTAs, many dependent steps -> the pieces its scan is cut into (see `cp.auto_segments`)."""
+    """One long sequence: few scan CTAs, many dependent steps -> the pieces its scan is cut into (see `cp.auto_segments`). Packed
+    batches and batches of a few long sequences are not cut, nor are the scans of a backward pass: they run one chain per
+    sequence and head, however few there are."""
     if q.dim() != 4 or q.shape[0] != 1 or q.shape[1] < 4096 or not q.is_cuda:      # cheap first look; `auto_segments` decides
         return None
     from .cp import auto_segments, segment_bounds, segment_tables
@@ -124,8 +126,9 @@ def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_sta
             flash-linear-attention's ``FLACPContext`` here, cula/kda/chunk.py:348-355).
 
     Numeric range: the chunk-local intermediates w, u, kg, qg, Aqk travel as fp16 (the reference uses bf16), so
-    ``|v|`` and ``|beta v|`` must stay below 65504; q and k are unrestricted when ``use_qk_l2norm_in_kernel`` is
-    set and are expected to be unit rows otherwise. A value that leaves the range is reported through the device
+    ``|v|``, ``|beta v|``, ``|scale q|`` and ``|scale q k|`` must stay below 65504; q and k are unrestricted when
+    ``use_qk_l2norm_in_kernel`` is set, and otherwise rows of any length that this allows. Decays of more than about 5.4
+    (natural log, per token) on 16 tokens in a row lose the contributions inside such a block. A value that leaves the range is reported through the device
     status word (``check_status``; also raised by the next ``chunk_kda`` call on the device).
 
     Returns ``(o, final_state)`` (``final_state`` is None unless requested).
