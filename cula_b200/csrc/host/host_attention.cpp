@@ -223,10 +223,10 @@ Backward backward_core(const Tensor& q, const Tensor& k, const Tensor& v, const 
         if (bias) r.dbias = both.narrow(0, 0, H * DIM);
         r.dA = both.narrow(0, both.numel() - H, H);
     }
-    check(lib.cula_kda_bwd_gated(ptr(q), ptr(k), ptr(g), g_flags(g), ptr(beta), beta_flags(beta, opt.beta_logit), fptr(A_log), fptr(dt_bias),
-                                 fptr(f.akk), fptr(f.mkk), fptr(scratch), fptr(work), ptr(r.dq), ptr(r.dk), ptr(r.dg), ptr(r.dbeta), fptr(r.dA),
-                                 fptr(r.dbias), cu, ci, (int)f.num_chunks, (int)T, (int)H, (float)opt.scale, opt.l2norm, opt.gate_mode,
-                                 (float)opt.lower_bound, stream), "cula_kda_bwd_gated");
+    check(lib.cula_kda_bwd_gated_checked(ptr(q), ptr(k), ptr(g), g_flags(g), ptr(beta), beta_flags(beta, opt.beta_logit), fptr(A_log), fptr(dt_bias),
+                                         fptr(f.akk), fptr(f.mkk), fptr(scratch), fptr(work), ptr(r.dq), ptr(r.dk), ptr(r.dg), ptr(r.dbeta),
+                                         fptr(r.dA), fptr(r.dbias), cu, ci, (int)f.num_chunks, (int)T, (int)H, (float)opt.scale, opt.l2norm,
+                                         opt.gate_mode, (float)opt.lower_bound, status, stream), "cula_kda_bwd_gated");
     return r;
 }
 

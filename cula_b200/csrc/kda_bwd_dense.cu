@@ -26,6 +26,7 @@
 // dAqk half of chunk_kda_bwd_kernel_dAv (cula/kda/chunk_bwd.py:63-125).
 #include "kda_common.cuh"
 #include "kda_params.h"
+#include "scan_common.cuh"
 #include "tensor_map.cuh"
 #include "umma.cuh"
 
@@ -71,10 +72,6 @@ __device__ __forceinline__ uint64_t bd_sdesc(uint32_t addr, uint32_t lbo, uint32
 __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  :: "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t smem_src, int x, int y, int z) {
-    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
-                 :: "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_src), "r"(x), "r"(y), "r"(z) : "memory");
 }
 // byte offset of the 16-byte group `chunk` (0..7) of row `row` inside an atom
 __device__ __forceinline__ uint32_t atom_off(int row, int chunk) {

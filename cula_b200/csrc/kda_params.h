@@ -140,6 +140,7 @@ struct BwdGatedParams {
     int gate_mode;
     float lower_bound;
     float scale;
+    int* status;                  // device status word (bounded waits) or null
 };
 
 // short causal depthwise convolution (forward and backward)

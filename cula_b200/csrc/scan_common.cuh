@@ -16,6 +16,10 @@ __device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const CUtensorMap
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  :: "r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t smem_src, int x, int y, int z) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+                 :: "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_src), "r"(x), "r"(y), "r"(z) : "memory");
+}
 __device__ __forceinline__ uint64_t sc_sdesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return umma::make_sdesc(addr, lbo, sbo) | (2ull << 61);     // 128-byte swizzle
 }
@@ -119,15 +123,15 @@ inline bool make_pack_map(CUtensorMap* map, const unsigned char* tiles, long lon
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<unsigned char*>(tiles), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// Token rows [tokens][heads][128] of bf16, moved as boxes of 64 tokens of one head; rows past `tokens` are read as zeros. It may be
+// Token rows [tokens][heads][128] of bf16 (or fp32), moved as boxes of 64 tokens of one head; rows past `tokens` are read as zeros. It may be
 // an upper bound where only whole chunks, which lie inside the tensor, are moved.
-inline bool make_rows_map(CUtensorMap* map, void* rows, int H, long long tokens) {
+inline bool make_rows_map(CUtensorMap* map, void* rows, int H, long long tokens, bool fp32 = false) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
     const cuuint64_t dims[3] = {128, (cuuint64_t)H, (cuuint64_t)tokens};
-    const cuuint64_t strides[2] = {256, (cuuint64_t)H * 256};
+    const cuuint64_t row = fp32 ? 512 : 256, strides[2] = {row, (cuuint64_t)H * row};
     const cuuint32_t box[3] = {128, 1, 64}, elem[3] = {1, 1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, rows, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+    return fn(map, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, rows, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
               CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 

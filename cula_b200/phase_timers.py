@@ -28,10 +28,8 @@ DENSE_PHASES = ["half 0: operands widened into smem", "-",
                 "half 1: operands widened into smem", "-", "half 1: wait for the states (TMA)",
                 "half 1: MMA issue", "half 1: next tile's operands requested", "half 1: wait for the MMAs", "dQg, dW staged, stores issued",
                 "dKg, dPs, dAu staged, dv stored", "store read-out + end-of-tile barrier"]
-BWD_PHASES = [f"{g}: {n}" for g, names in (
-    ("rows", ("inputs landed", "norms, coefficients, gates", "X", "dA", "Zw", "wait for the columns", "row side", "wait, end of the tile")),
-    ("columns", ("inputs landed", "norms, coefficients, gates", "X", "dA", "T1, dL", "wait for the rows", "column side", "wait, end of the tile")))
-    for n in names]
+BWD_PHASES = ["inputs landed", "norms, gates, coefficients", "anchors, X, dW^T, q e", "dA", "Zw, q side read, k f, k e", "T1", "P part read",
+              "dL, cR", "R part read", "k side read", "dk, dG, sums", "S13","S11","S12","B7","top issue"]
 
 
 def main():

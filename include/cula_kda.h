@@ -176,6 +176,14 @@ int cula_kda_bwd_gated(const void* d_q, const void* d_k, const void* d_g, int g_
                        const int* d_cu_seqlens, const int* d_chunk_indices, int num_chunks, int T, int H,
                        float scale, int use_qk_l2norm, int gate_mode, float lower_bound, void* stream);
 
+/* The same with the device status word of its bounded waits (cula_kda_bwd_gated reports nowhere). */
+int cula_kda_bwd_gated_checked(const void* d_q, const void* d_k, const void* d_g, int g_is_fp32,
+                               const void* d_beta, int beta_is_fp32, const float* d_A_log, const float* d_dt_bias,
+                               const float* d_akk, const float* d_mkk, const float* d_scratch, const float* d_gscale,
+                               void* d_dq, void* d_dk, void* d_dg, void* d_dbeta, float* d_dA_log, float* d_ddt_bias,
+                               const int* d_cu_seqlens, const int* d_chunk_indices, int num_chunks, int T, int H,
+                               float scale, int use_qk_l2norm, int gate_mode, float lower_bound, int* d_status, void* stream);
+
 /* ------------------------------------------------------------------------------------------------------------
  * Context parallelism (one long sequence split into contiguous shards, one per GPU). The reference reaches this
  * through flash-linear-attention's cp_context (cula/kda/chunk_fwd.py:99-109,122-127; fla/ops/cp/chunk_delta_h.py).

@@ -433,3 +433,28 @@ def test_side_by_side_scans_equal_scans_one_after_the_other(B, T, H, lens):
     check_status()
     for other in grads[1:]:
         assert all(torch.equal(a, b) for a, b in zip(grads[0], other))
+
+
+@pytest.mark.parametrize("g_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T", [1, 15, 16, 17, 63, 64, 65, 200])
+def test_gradients_do_not_depend_on_what_memory_held_before(T, g_dtype):
+    """Work buffers come from the allocator as they are: with every free block full of NaN the gradients are the same to the bit."""
+    from cula_b200.kda import chunk_kda
+    from cula_b200.synthetic import make_inputs_on_device
+    d = make_inputs_on_device(2, T, 3, torch.device("cuda"), seed=T, gate_offset=-4.0, h0_std=0.5)
+    d["g"] = d["g"].to(g_dtype)
+    names = ("q", "k", "v", "g", "beta", "initial_state")
+    grads = []
+    for fill in (0.0, float("nan")):
+        leaves = {n: d[n].detach().clone().requires_grad_(True) for n in names}
+        # one block of every size that the call can ask for, freed again, so that it gets these
+        junk = [torch.full((1 << e,), fill, device="cuda") for e in range(7, 24)]
+        junk += [torch.full((3 << e,), fill, device="cuda") for e in range(7, 22)]
+        torch.cuda.synchronize()
+        del junk
+        o, ht = chunk_kda(*(leaves[n] for n in names[:5]), initial_state=leaves["initial_state"], output_final_state=True,
+                          use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, safe_gate=True, lower_bound=-5.0, A_log=d["A_log"],
+                          dt_bias=d["dt_bias"])
+        grads.append(torch.autograd.grad([o, ht], list(leaves.values()), [torch.ones_like(o), torch.ones_like(ht)]))
+    for n, a, b in zip(names, *grads):
+        assert torch.equal(a, b), n
