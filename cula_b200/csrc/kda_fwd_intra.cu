@@ -22,14 +22,17 @@
 // generation leaves the values (thread (g, t) of a warp owns two rows and 16 channels, and both the A and the B fragment
 // of m16n8k8 want rows by g and contraction columns by t), so they cost no shared-memory traffic at all.
 //
-// What bounds it: instruction latency of the CUDA-core phases (42 % of the issue slots taken with four warps per scheduler;
+// What bounds it: instruction latency of the CUDA-core phases (44 % of the issue slots taken with four warps per scheduler;
 // the tensor pipes and HBM are far from busy). Warp w owns 16-row block w & 3 and channel half w >> 2 of all first phases; its
 // 16-byte row segments make every global access and every operand store a full vector. Two CTAs are resident per SM, so one
 // CTA's operand generation overlaps the other's MMAs, inverse and epilogues.
 // Measured at B=2, T=2048, H=32 (2048 tiles, cold L2): 143.6 -> 119 us, 31.7 k -> 24 k warp instructions per tile against the
-// version that formed all of the Gram product as tf32 operands in shared memory, two channel halves one after the other.
+// version that formed all of the Gram product as tf32 operands in shared memory, two channel halves one after the other; with the
+// q and k rows of whole chunks by TMA where their operands will stand, instead of in registers from tile to tile: 119 -> 112 us, 844 ->
+// 774 us at 4 x 8192 x 32. (Requested right at the start of a tile, where the thread that asks waits for the copies out: 789 us.)
 #include "kda_common.cuh"
 #include "kda_params.h"
+#include "scan_common.cuh"
 #include "umma.cuh"
 
 // Optional per-phase cycle counters (compile with -DKDA_PHASE_TIMERS): thread 0 of every CTA adds the clock64() spent
@@ -126,8 +129,13 @@ __device__ __forceinline__ void mma_tile_3xtf32(const float* A, int lda, const f
 // operand for log-uniform mantissas, is taken out by one factor in the per-channel constant of the column operand.
 constexpr float TF32_DEBIAS2_LOG2 = 2.f * 5.0775e-4f;     // log2 of (1 + 3.52e-4)^2: both operands
 
+// q, k, v rows [tokens][heads][128], 64 channels x 64 tokens of a head at a time, 128-byte swizzle
+struct IntraMaps {
+    CUtensorMap q, k, v;
+};
+
 template <int GK>
-__global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const IntraParams p) {
+__global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const IntraParams p, const __grid_constant__ IntraMaps maps) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const uint32_t sm_u32 = smem_u32(sm);
@@ -157,6 +165,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
     if (tid == 0) {
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
+        mbar_init(&bars[2], 1);          // q and k rows
         *sAbort = 0;
         fence_mbar_init();
     }
@@ -200,8 +209,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
             sInfo[buf] = v;
         }
     };
-    // Register prefetch: the raw gate rows and the q and k rows are fetched one tile ahead, each at the point of the tile from
-    // which their registers are free (the loads come from L2, see the hints below).
+    // Register prefetch: the raw gate rows are fetched one tile ahead, at the point of the tile from which their registers are free.
     // Loads are unconditional (nothing may depend on a loaded value before it is used): a padding row reads the last
     // real row of the chunk instead, and is zeroed where it is used (through its gate, norm and beta factors).
     constexpr int NGR = GK == GK_FP32 ? 8 : (GK == GK_BF16 ? 4 : 1);
@@ -234,19 +242,17 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
             }
         }
     };
-    uint4 qraw[4], kraw[4];         // [row j][c]: 8 bf16 each
-    auto fetch_qk = [&](const int4 nf) {
-        const size_t base2 = (size_t)nf.x * tok_stride + (size_t)nf.z * DK + 64 * hf + 8 * t;
-        const __nv_bfloat16* qp = reinterpret_cast<const __nv_bfloat16*>(p.q) + base2;
-        const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(p.k) + base2;
+    // The q and k rows of a whole chunk come by TMA into the buffer of the A operand, in its layout: each thread finds its values where it
+    // will put the operand. Rows of a ragged chunk (a box would reach past them) are loaded one by one; padding rows read the last real
+    // row and are zeroed through their norms.
+    uint32_t qk_parity = 0;
+    auto request_qk = [&](const int4 nf) {        // one thread
+        if (nf.y < BT) return;
+        mbar_arrive_expect_tx(&bars[2], 32768);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const size_t roff = (size_t)min(rowA + j, nf.y - 1) * tok_stride;
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                qraw[2 * j + c] = *reinterpret_cast<const uint4*>(qp + roff + 32 * c);
-                kraw[2 * j + c] = *reinterpret_cast<const uint4*>(kp + roff + 32 * c);
-            }
+        for (int half = 0; half < 2; ++half) {
+            tma_load_3d(sm_u32 + SM_OPA + half * KATOM_A, &maps.q, 64 * half, nf.z, nf.x, &bars[2]);
+            tma_load_3d(sm_u32 + SM_OPA + half * KATOM_A + 8192, &maps.k, 64 * half, nf.z, nf.x, &bars[2]);
         }
     };
     // Per-tile scalars (beta of the 64 rows, dt_bias and exp(A_log) of the head) are fetched one tile ahead by the
@@ -283,7 +289,6 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
     __syncthreads();
     if ((int)blockIdx.x < p.num_tiles) {
         fetch_g(sInfo[0]);
-        fetch_qk(sInfo[0]);
         load_scalars(sInfo[0]);
         park_scalars(0, sInfo[0].y);
     }
@@ -371,6 +376,10 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
             }
         }
     }
+    if (tid == MMA_THREAD) {       // the previous tile's staged outputs have left the operand buffers
+        bulk_wait_read_all();
+        request_qk(info);
+    }
     PHASE_MARK(0); // gate activation
     {
         if (pr == 0) {       // the block's first row
@@ -410,6 +419,34 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
         }
     }
     PHASE_MARK(2);      // in-warp cumulative sum
+    uint4 qraw[4], kraw[4];         // [row j][c]: 8 bf16 each
+    if (valid == BT) {
+        if (!mbar_wait(&bars[2], qk_parity)) {
+            report_status(p.status, STATUS_WAIT_TIMEOUT);
+            *sAbort = 1;
+        }
+        qk_parity ^= 1;
+        const unsigned char* raw = sm + SM_OPA + hf * KATOM_A;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const uint32_t so = ((j ? segB : segA) & ~15u) ^ (uint32_t)(64 * c);
+                qraw[2 * j + c] = *reinterpret_cast<const uint4*>(raw + so);
+                kraw[2 * j + c] = *reinterpret_cast<const uint4*>(raw + 8192 + so);
+            }
+    } else {
+        const size_t at = base + 64 * hf + 8 * t;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const size_t roff = at + (size_t)min(rowA + j, valid - 1) * tok_stride;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                qraw[2 * j + c] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.q) + roff + 32 * c);
+                kraw[2 * j + c] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.k) + roff + 32 * c);
+            }
+        }
+    }
     // ---- 2. sums of squares of the thread's two q and k rows over this warp's 64 channels ----
     if (p.use_l2norm) {
 #pragma unroll
@@ -433,7 +470,6 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
         }
     }
     PHASE_MARK(14);     // norms
-    if (tid == MMA_THREAD) bulk_wait_read_all();   // the previous tile's staged outputs have left the operand buffers
     __syncthreads();          // block edges and sums of squares are visible
     PHASE_MARK(1);      // barrier
     // ---- 3. per-channel constants of this warp's block and channel half, two channels per lane ----
@@ -481,6 +517,17 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
             rk[j] = live ? b : 0.f;
         }
     }
+    if (valid < BT) {             // the rows of a ragged chunk go where the box puts those of a whole one
+        unsigned char* raw = sm + SM_OPA + hf * KATOM_A;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const uint32_t so = ((j ? segB : segA) & ~15u) ^ (uint32_t)(64 * c);
+                *reinterpret_cast<uint4*>(raw + so) = qraw[2 * j + c];
+                *reinterpret_cast<uint4*>(raw + 8192 + so) = kraw[2 * j + c];
+            }
+    }
     __syncwarp();
     PHASE_MARK(3);      // tables
     // ---- 4. operand generation. Per element only two exponentials: eA = 2^(g_i - r_I) and f = 2^(r_{I+1} - g_i).
@@ -512,8 +559,14 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
             for (int h = 0; h < 2; ++h) {
                 asm volatile("" ::: "memory");          // one step at a time: the registers of four in flight would not fit
                 const float* tp = tab + 32 * c + 8 * t + 4 * (h ^ sx);
-                const bool up = h != sx;
                 float2 kf[2][2];                                             // [row][pair]
+                uint2 qr[2], kr[2];                                          // this thread's values, where their operands will go
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const uint32_t so = (j ? segB : segA) ^ (uint32_t)(64 * c + 8 * h);
+                    qr[j] = *reinterpret_cast<const uint2*>(opa + so);
+                    kr[j] = *reinterpret_cast<const uint2*>(opa + 8192 + so);
+                }
                 uint32_t pa[2][2], pk[2][2], px[2][2], pg[2][2], pq[2][2];
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
@@ -523,8 +576,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
                     float2 ko[2];
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
-                        const uint4 qr = qraw[2 * j], kr = kraw[2 * j];
-                        const uint32_t qw = x ? (up ? qr.w : qr.y) : (up ? qr.z : qr.x), kw = x ? (up ? kr.w : kr.y) : (up ? kr.z : kr.x);
+                        const uint32_t qw = x ? qr[j].y : qr[j].x, kw = x ? kr[j].y : kr[j].x;
                         float2 eA, f;
                         if constexpr (GK == GK_PER_HEAD) {
                             eA = splat2(eP[j]); f = splat2(fP[j]);
@@ -590,9 +642,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
                 if (I < 2) later(48, 5);
                 if (I < 1) later(16, 4);
             }
-            qraw[0] = qraw[1]; qraw[2] = qraw[3];       // the second segment moves into place
-            kraw[0] = kraw[1]; kraw[2] = kraw[3];
-            if constexpr (NX == 8) {
+            if constexpr (NX == 8) {                    // the second segment moves into place
 #pragma unroll
                 for (int x = 0; x < 4; ++x) {
                     GA[x] = GA[x + 4];
@@ -639,12 +689,13 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
         if (nf.y > 0) {
             fetch_g(nf);
             load_scalars(nf);
-            // (the bulk form of the prefetch is issued lane by lane, which costs more instructions than it saves)
-            const int row = tid >> 2, part = tid & 3;
-            if (row < nf.y) {
-                const size_t off = (size_t)(nf.x + row) * tok_stride + (size_t)nf.z * DK + 64 * (part & 1);
-                prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(part < 2 ? p.q : p.k) + off);
-                if (part < 2) prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(p.v) + off);
+            if (tid == INFO_THREAD && nf.y == BT) {       // the next tile's token rows towards L2
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    tma_prefetch_3d(&maps.q, 64 * half, nf.z, nf.x);
+                    tma_prefetch_3d(&maps.k, 64 * half, nf.z, nf.x);
+                    tma_prefetch_3d(&maps.v, 64 * half, nf.z, nf.x);
+                }
             }
         }
     }
@@ -891,8 +942,6 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
             }
         }
     }
-    // the next tile's q and k rows: nothing else of this tile needs many registers
-    if (tile_id + (int)gridDim.x < p.num_tiles) fetch_qk(sInfo[par ^ 1]);
     fence_proxy_async();
     umma::fence_before_sync();
     __syncthreads();
@@ -1017,7 +1066,11 @@ extern "C" int kda_launch_fwd_intra(const kda::IntraParams* p, int num_chunks, c
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = q.overlap ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, kernel, q);
+    // (whole chunks lie inside the tensors, whose length a packed batch does not tell)
+    IntraMaps maps;
+    if (!make_half_rows_map(&maps.q, p->q, p->H) || !make_half_rows_map(&maps.k, p->k, p->H) || !make_half_rows_map(&maps.v, p->v, p->H))
+        return (int)cudaErrorInvalidValue;
+    e = cudaLaunchKernelEx(&cfg, kernel, q, maps);
     if (e != cudaSuccess) return (int)e;
     return (int)cudaGetLastError();
 }

@@ -20,6 +20,10 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t sm
     asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
                  :: "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_src), "r"(x), "r"(y), "r"(z) : "memory");
 }
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int x, int y, int z) {      // towards L2
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
+                 :: "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z) : "memory");
+}
 __device__ __forceinline__ uint64_t sc_sdesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return umma::make_sdesc(addr, lbo, sbo) | (2ull << 61);     // 128-byte swizzle
 }
@@ -134,6 +138,14 @@ inline bool make_rows_map(CUtensorMap* map, void* rows, int H, long long tokens,
     return fn(map, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, rows, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
               CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-
+// The same in boxes of 64 channels, as 128-byte-swizzled atoms; only whole chunks, which lie inside the tensor, are moved.
+inline bool make_half_rows_map(CUtensorMap* map, const void* rows, int H) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[3] = {128, (cuuint64_t)H, 1ull << 30}, strides[2] = {256, (cuuint64_t)H * 256};
+    const cuuint32_t box[3] = {64, 1, 64}, elem[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(rows), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 }  // namespace kda

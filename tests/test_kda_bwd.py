@@ -458,3 +458,38 @@ def test_gradients_do_not_depend_on_what_memory_held_before(T, g_dtype):
         grads.append(torch.autograd.grad([o, ht], list(leaves.values()), [torch.ones_like(o), torch.ones_like(ht)]))
     for n, a, b in zip(names, *grads):
         assert torch.equal(a, b), n
+
+
+@pytest.mark.parametrize("first", [1, 63, 64, 65, 100, 128])
+@pytest.mark.parametrize("g_dtype", [torch.bfloat16, torch.float32])
+def test_a_sequence_does_not_read_its_neighbour(first, g_dtype):
+    """Rows of whole chunks move as boxes, those of ragged ones one by one: NaN in the sequence behind must not reach this one."""
+    from cula_b200.kda import check_status, chunk_kda
+    from cula_b200.synthetic import make_inputs_on_device
+    H, rest = 2, 70
+    d = make_inputs_on_device(1, first + rest, H, torch.device("cuda"), seed=first, gate_offset=-4.0)
+    d["g"] = d["g"].to(g_dtype)
+    names = ("q", "k", "v", "g", "beta")
+    kw = dict(use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, safe_gate=True, lower_bound=-5.0, A_log=d["A_log"], dt_bias=d["dt_bias"])
+    results = []
+    for poison in (False, True):
+        leaves = []
+        for n in names:
+            x = d[n].detach().clone()
+            if poison:
+                x[:, first:] = float("nan")
+            leaves.append((x if poison else x[:, :first].contiguous()).requires_grad_(True))
+        cu = torch.tensor([0, first, first + rest], dtype=torch.int32, device="cuda") if poison else None
+        o, _ = chunk_kda(*leaves, cu_seqlens=cu, **kw)
+        up = torch.ones_like(o)
+        if poison:
+            up[:, first:] = 0
+        results.append([o, *torch.autograd.grad(o, leaves, up)])
+    torch.cuda.synchronize()
+    try:
+        check_status()           # NaN values of the neighbour may be reported
+    except RuntimeError:
+        pass
+    for n, a, b in zip(("o", *names), *results):
+        assert torch.isfinite(b[:, :first].float()).all(), n
+        assert err_ratio(a.detach().float().cpu(), b[:, :first].detach().float().cpu()) <= 1e-6, n
