@@ -29,11 +29,10 @@ extern "C" int cula_kda_tile_pack_bytes(void) { return kda::TP_BYTES; }
 extern "C" int cula_kda_fwd_intra_smem_bytes(void) { return kda_fwd_intra_smem_bytes(); }
 extern "C" int cula_kda_fwd_scan_smem_bytes(void) { return kda_fwd_scan_smem_bytes(); }
 
-extern "C" int cula_kda_fwd_intra(const void* d_q, const void* d_k, const void* d_v, const void* d_g, int g_is_fp32,
-                                  const void* d_beta, int beta_is_fp32, const float* d_A_log, const float* d_dt_bias,
-                                  const int* d_cu_seqlens, const int* d_chunk_indices, int num_chunks, int T, int H,
-                                  float scale, int use_qk_l2norm, int gate_mode, float lower_bound, void* d_tiles,
-                                  float* d_akk, float* d_mkk, int* d_status, void* stream) {
+static int fwd_intra(const void* d_q, const void* d_k, const void* d_v, const void* d_g, int g_is_fp32, const void* d_beta, int beta_is_fp32,
+                     const float* d_A_log, const float* d_dt_bias, const int* d_cu_seqlens, const int* d_chunk_indices, int num_chunks, int T, int H,
+                     float scale, int use_qk_l2norm, int gate_mode, float lower_bound, void* d_tiles, float* d_akk, float* d_mkk, int* d_status,
+                     void* stream, bool overlap) {
     if (num_chunks == 0) return 0;
     if (!d_q || !d_k || !d_v || !d_g || !d_beta || !d_tiles || !d_status || num_chunks < 0 || H <= 0) return CULA_KDA_EINVAL;
     if (gate_mode < 0 || gate_mode > 2 || (gate_mode != 0 && !d_A_log)) return CULA_KDA_EINVAL;
@@ -54,7 +53,17 @@ extern "C" int cula_kda_fwd_intra(const void* d_q, const void* d_k, const void* 
     p.T = T; p.H = H; p.g_fp32 = g_is_fp32 & CULA_KDA_G_FP32; p.g_per_head = (g_is_fp32 & CULA_KDA_G_PER_HEAD) != 0;
     p.beta_fp32 = beta_is_fp32 & CULA_KDA_BETA_FP32; p.beta_logit = (beta_is_fp32 & CULA_KDA_BETA_LOGIT) != 0;
     p.use_l2norm = use_qk_l2norm; p.gate_mode = gate_mode; p.lower_bound = lower_bound; p.scale = scale;
+    p.overlap = overlap;
     return kda_launch_fwd_intra(&p, num_chunks, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int cula_kda_fwd_intra(const void* d_q, const void* d_k, const void* d_v, const void* d_g, int g_is_fp32,
+                                  const void* d_beta, int beta_is_fp32, const float* d_A_log, const float* d_dt_bias,
+                                  const int* d_cu_seqlens, const int* d_chunk_indices, int num_chunks, int T, int H,
+                                  float scale, int use_qk_l2norm, int gate_mode, float lower_bound, void* d_tiles,
+                                  float* d_akk, float* d_mkk, int* d_status, void* stream) {
+    return fwd_intra(d_q, d_k, d_v, d_g, g_is_fp32, d_beta, beta_is_fp32, d_A_log, d_dt_bias, d_cu_seqlens, d_chunk_indices, num_chunks, T, H, scale,
+                     use_qk_l2norm, gate_mode, lower_bound, d_tiles, d_akk, d_mkk, d_status, stream, false);
 }
 
 extern "C" int cula_kda_fwd_scan(const void* d_tiles, const float* d_h0, void* d_o, float* d_ht, void* d_h_out,
@@ -221,6 +230,18 @@ extern "C" int cula_kda_bwd_grad_scale(const void* d_do, long long n_do, const f
     if (!d_do || !d_amax || !d_gscale || n_do < 0 || n_dht < 0) return CULA_KDA_EINVAL;
     if (misaligned(d_do) || misaligned(d_dht)) return CULA_KDA_EALIGN;
     return kda_launch_grad_scale(d_do, (size_t)n_do, d_dht, (size_t)n_dht, d_amax, d_gscale, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int cula_kda_bwd_scale_and_intra(const void* d_do, long long n_do, const float* d_dht, long long n_dht, unsigned int* d_amax,
+                                            float* d_gscale, const void* d_q, const void* d_k, const void* d_v, const void* d_g, int g_is_fp32,
+                                            const void* d_beta, int beta_is_fp32, const float* d_A_log, const float* d_dt_bias,
+                                            const int* d_cu_seqlens, const int* d_chunk_indices, int num_chunks, int T, int H, float scale,
+                                            int use_qk_l2norm, int gate_mode, float lower_bound, void* d_tiles, float* d_akk, float* d_mkk,
+                                            int* d_status, void* stream) {
+    const int rc = cula_kda_bwd_grad_scale(d_do, n_do, d_dht, n_dht, d_amax, d_gscale, stream);
+    if (rc != 0) return rc;
+    return fwd_intra(d_q, d_k, d_v, d_g, g_is_fp32, d_beta, beta_is_fp32, d_A_log, d_dt_bias, d_cu_seqlens, d_chunk_indices, num_chunks, T, H, scale,
+                     use_qk_l2norm, gate_mode, lower_bound, d_tiles, d_akk, d_mkk, d_status, stream, true);
 }
 
 extern "C" int cula_kda_bwd_scan(const void* d_tiles, const void* d_do, const float* d_dht, const float* d_gscale,

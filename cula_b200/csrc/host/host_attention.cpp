@@ -105,13 +105,31 @@ Plan plan_pieces(int64_t ctas, int64_t nc, int sms) {
     return best;
 }
 
+// The upstream gradients and the power-of-two scale they are carried in.
+struct Upstream {
+    Tensor d_o, work;             // work: [0:2] = {s, 1/s}, [2] = running max (as bits)
+    OptTensor dht;
+    int64_t n_dht() const { return dht.has_value() ? dht->numel() : 0; }
+    unsigned int* amax() const { return reinterpret_cast<unsigned int*>(fptr(work) + 2); }
+};
+Upstream upstream(const Tensor& d_out, const OptTensor& d_final) {
+    return {d_out.contiguous(), device_empty({4}, d_out.options().dtype(at::kFloat)), contiguous_f32(d_final)};
+}
+void scale_gradients(const Upstream& u) {
+    c10::cuda::CUDAGuard guard(u.d_o.device());
+    check(lib.cula_kda_bwd_grad_scale(ptr(u.d_o), u.d_o.numel(), fptr(u.dht), u.n_dht(), u.amax(), fptr(u.work), stream_of(u.d_o)),
+          "cula_kda_bwd_grad_scale");
+}
+
 // Forward orchestration (the role of cula/kda/chunk_fwd.py:39-152): the chunk-parallel stage writes one tile pack per
 // (chunk, head); the scan consumes them, carries the fp32 state and writes o. All tensors contiguous; A_log, dt_bias fp32.
-// leave_scan: the scan's buffers are made but backward_core launches it, beside the reverse scan.
+// recompute_for: in front of a backward pass. The scale of its upstream gradients is worked out beside the chunk-parallel stage, and of the
+// scan only the buffers are made: backward_core launches it, beside the reverse scan.
 Forward forward_core(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const OptTensor& h0,
                      const OptTensor& A_log, const OptTensor& dt_bias, const Options& opt, const Tables* tab, const Segments* segs, bool want_final,
-                     bool store_states, bool store_akk, bool store_bwd, bool want_output, bool leave_scan = false) {
+                     bool store_states, bool store_akk, bool store_bwd, bool want_output, const Upstream* recompute_for = nullptr) {
     ++forward_calls;
+    const bool leave_scan = recompute_for != nullptr;
     c10::cuda::CUDAGuard guard(q.device());
     const int64_t B = q.size(0), T = q.size(1), H = q.size(2);
     cudaStream_t stream = stream_of(q);
@@ -148,9 +166,17 @@ Forward forward_core(const Tensor& q, const Tensor& k, const Tensor& v, const Te
             return f;
         }
     }
-    check(lib.cula_kda_fwd_intra(ptr(q), ptr(k), ptr(v), ptr(g), g_flags(g), ptr(beta), beta_flags(beta, opt.beta_logit), fptr(A_log), fptr(dt_bias),
-                                 cu, ci, (int)f.num_chunks, (int)T, (int)H, (float)opt.scale, opt.l2norm, opt.gate_mode, (float)opt.lower_bound,
-                                 ptr(f.tiles), fptr(f.akk), fptr(f.mkk), status, stream), "cula_kda_fwd_intra");
+    if (recompute_for) {
+        const Upstream& u = *recompute_for;
+        check(lib.cula_kda_bwd_scale_and_intra(ptr(u.d_o), u.d_o.numel(), fptr(u.dht), u.n_dht(), u.amax(), fptr(u.work), ptr(q), ptr(k), ptr(v), ptr(g),
+                                               g_flags(g), ptr(beta), beta_flags(beta, opt.beta_logit), fptr(A_log), fptr(dt_bias), cu, ci,
+                                               (int)f.num_chunks, (int)T, (int)H, (float)opt.scale, opt.l2norm, opt.gate_mode, (float)opt.lower_bound,
+                                               ptr(f.tiles), fptr(f.akk), fptr(f.mkk), status, stream), "cula_kda_bwd_scale_and_intra");
+    } else {
+        check(lib.cula_kda_fwd_intra(ptr(q), ptr(k), ptr(v), ptr(g), g_flags(g), ptr(beta), beta_flags(beta, opt.beta_logit), fptr(A_log),
+                                     fptr(dt_bias), cu, ci, (int)f.num_chunks, (int)T, (int)H, (float)opt.scale, opt.l2norm, opt.gate_mode,
+                                     (float)opt.lower_bound, ptr(f.tiles), fptr(f.akk), fptr(f.mkk), status, stream), "cula_kda_fwd_intra");
+    }
     if (segs && segs->count > 1) {
         segmented_scan(v, h0, want_final, *segs, f, stream, status);
         return f;
@@ -169,20 +195,6 @@ Forward forward_core(const Tensor& q, const Tensor& k, const Tensor& v, const Te
 struct Backward {
     Tensor dq, dk, dv, dg, dbeta, dA, dbias, dh0;
 };
-
-// The upstream gradients and the power-of-two scale they are carried in.
-struct Upstream {
-    Tensor d_o, work;             // work: [0:2] = {s, 1/s}, [2] = running max (as bits)
-    OptTensor dht;
-};
-Upstream scale_gradients(const Tensor& d_out, const OptTensor& d_final) {
-    c10::cuda::CUDAGuard guard(d_out.device());
-    Upstream u{d_out.contiguous(), device_empty({4}, d_out.options().dtype(at::kFloat)), contiguous_f32(d_final)};
-    check(lib.cula_kda_bwd_grad_scale(ptr(u.d_o), u.d_o.numel(), fptr(u.dht), u.dht.has_value() ? u.dht->numel() : 0,
-                                      reinterpret_cast<unsigned int*>(fptr(u.work) + 2), fptr(u.work), stream_of(d_out)),
-          "cula_kda_bwd_grad_scale");
-    return u;
-}
 
 // Backward orchestration (the role of cula/kda/chunk_bwd.py:432-604) from the forward intermediates in `f`. With scan_left the
 // forward scan of `f` (from h0) has not run yet: the reverse scan reads none of its results, so the two chains run side by side.
@@ -286,15 +298,16 @@ public:
         }
         const Tensor d_o = grads[0].defined() ? grads[0] : at::zeros_like(v);
         const OptTensor dht = grads.size() > 1 && grads[1].defined() ? OptTensor(grads[1]) : OptTensor();
-        const Upstream up = scale_gradients(d_o, dht);      // in front of the recomputation: the reverse scan starts with its scan
+        const Upstream up = upstream(d_o, dht);
         Forward f;
         bool scan_left = false;
         if (auto it = ctx->saved_data.find("kept"); it != ctx->saved_data.end()) {
             auto t = it->second.toTensorVector();
             f.tiles = t[0]; f.akk = t[1]; f.mkk = t[2]; f.h32 = t[3]; f.vnew = t[4];
             f.num_chunks = tab ? tab->num_chunks : q.size(0) * ((q.size(1) + CHUNK - 1) / CHUNK);
+            scale_gradients(up);
         } else {        // recomputed, as the reference does by default (cula/kda/chunk_bwd.py:459-500)
-            f = forward_core(q, k, v, g, beta, h0, A_log, dt_bias, o, tab ? &*tab : nullptr, nullptr, false, false, false, true, false, true);
+            f = forward_core(q, k, v, g, beta, h0, A_log, dt_bias, o, tab ? &*tab : nullptr, nullptr, false, false, false, true, false, &up);
             scan_left = true;
         }
         Backward b = backward_core(q, k, v, g, beta, A_log, dt_bias, o, tab ? &*tab : nullptr, f, h0.has_value(), up, scan_left, h0);
@@ -424,7 +437,9 @@ pybind11::tuple backward_tuple(const Tensor& q, const Tensor& k, const Tensor& v
     auto get = [&](const char* n) { return saved[n].cast<Tensor>(); };
     f.tiles = get("tiles"); f.akk = get("akk"); f.mkk = get("mkk"); f.h32 = get("h32"); f.vnew = get("vnew");
     f.num_chunks = saved["num_chunks"].cast<int64_t>();
-    Backward b = backward_core(q, k, v, g, beta, A_log, dt_bias, o, tab, f, want_dh0, scale_gradients(d_o, dht));
+    const Upstream up = upstream(d_o, dht);
+    scale_gradients(up);
+    Backward b = backward_core(q, k, v, g, beta, A_log, dt_bias, o, tab, f, want_dh0, up);
     auto obj = [](const Tensor& t) -> pybind11::object { return t.defined() ? pybind11::cast(t) : pybind11::object(pybind11::none()); };
     return pybind11::make_tuple(obj(b.dq), obj(b.dk), obj(b.dv), obj(b.dg), obj(b.dbeta), obj(b.dA), obj(b.dbias), obj(b.dh0));
 }

@@ -26,7 +26,7 @@ enum { GATE_NONE = 0, GATE_SOFTPLUS = 1, GATE_LOWER_BOUND = 2 };
 // entry points of libcula_kda.so, resolved once by bind()
 #define CULA_KDA_ENTRIES(X)                                                                                          \
     X(cula_kda_tile_pack_bytes) X(cula_kda_fwd_intra) X(cula_kda_fwd_scan) X(cula_kda_cp_transition) X(cula_kda_cp_fold) X(cula_kda_fwd_pieces) \
-    X(cula_kda_decode) X(cula_kda_bwd_scratch_floats) X(cula_kda_bwd_grad_scale) X(cula_kda_bwd_scan) X(cula_kda_bwd_both_scans) \
+    X(cula_kda_decode) X(cula_kda_bwd_scratch_floats) X(cula_kda_bwd_grad_scale) X(cula_kda_bwd_scale_and_intra) X(cula_kda_bwd_scan) X(cula_kda_bwd_both_scans) \
     X(cula_kda_bwd_dense) X(cula_kda_bwd_gated_checked) X(cula_kda_gate_fwd) X(cula_kda_gate_bwd)                              \
     X(cula_kda_beta_sigmoid_fwd) X(cula_kda_beta_sigmoid_bwd) X(cula_kda_short_conv_fwd) X(cula_kda_short_conv_bwd)    \
     X(cula_kda_rms_norm_gated_fwd) X(cula_kda_rms_norm_gated_bwd) X(cula_kda_strerror)

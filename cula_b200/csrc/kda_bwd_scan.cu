@@ -42,9 +42,12 @@ constexpr int BS_SMEM = BS_MISC + 8512 + 1024;
 constexpr uint32_t BM_S32 = 0, BM_S16 = 128, BM_ACC = 192, BM_DO = 320, BM_ADO = 384;
 
 constexpr int AMAX_THREADS = 512;
-// s = 2^k with max(|dO|, |dht|) * s in [4, 8); written as {s, 1/s}. amax_bits holds the running maximum.
+// s = 2^k with max(|dO|, |dht|) * s in [4, 8); written as {s, 1/s}. amax_bits holds the running maximum, gscale[0] counts the blocks that
+// are done until the last one writes the scale there (both start as zero). The recomputation of the chunk-parallel stage, which reads none
+// of this, may start under this kernel.
 __global__ void kda_grad_amax_kernel(const __nv_bfloat16* d_o, size_t n_do, const float* dht, size_t n_dht,
-                                     unsigned int* amax_bits) {
+                                     unsigned int* amax_bits, float* gscale) {
+    pdl_launch_dependents();
     float m = 0.f;
     const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nthr = (size_t)gridDim.x * blockDim.x;
     // 16-byte loads over the bulk (the tensors come 16-byte aligned from the C ABI), scalar loads over the tail
@@ -92,15 +95,17 @@ __global__ void kda_grad_amax_kernel(const __nv_bfloat16* d_o, size_t n_do, cons
 #pragma unroll
         for (int w = 0; w < AMAX_THREADS / 32; ++w) m = fmaxf(m, wmax[w]);
         if (m > 0.f) atomicMax(amax_bits, __float_as_uint(m));
+        __threadfence();
+        if (atomicAdd(reinterpret_cast<unsigned int*>(gscale), 1u) == gridDim.x - 1) {
+            __threadfence();
+            m = __uint_as_float(atomicMax(amax_bits, 0u));
+            const int e = ((__float_as_int(m) >> 23) & 0xff) - 127;      // floor(log2 m); m == 0 gives -127
+            int shift = m > 0.f ? 2 - e : 0;
+            shift = max(-120, min(120, shift));
+            gscale[0] = __int_as_float((shift + 127) << 23);
+            gscale[1] = __int_as_float((127 - shift) << 23);
+        }
     }
-}
-__global__ void kda_grad_scale_kernel(const unsigned int* amax_bits, float* gscale) {
-    const float m = __uint_as_float(*amax_bits);
-    int e = ((__float_as_int(m) >> 23) & 0xff) - 127;      // floor(log2 m); m == 0 gives -127
-    int shift = (m > 0.f) ? 2 - e : 0;
-    shift = max(-120, min(120, shift));
-    gscale[0] = __int_as_float((shift + 127) << 23);
-    gscale[1] = __int_as_float((127 - shift) << 23);
 }
 
 __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdScanParams p, const __grid_constant__ CUtensorMap map,
@@ -439,11 +444,15 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
 extern "C" int kda_launch_grad_scale(const void* d_o, size_t n_do, const float* dht, size_t n_dht, unsigned int* amax_bits,
                                      float* gscale, cudaStream_t stream) {
     using namespace kda;
-    cudaError_t e = cudaMemsetAsync(amax_bits, 0, sizeof(unsigned int), stream);
+    const bool one_piece = reinterpret_cast<float*>(amax_bits) == gscale + 2;
+    cudaError_t e = cudaMemsetAsync(gscale, 0, (one_piece ? 3 : 1) * sizeof(float), stream);
+    if (e == cudaSuccess && !one_piece) e = cudaMemsetAsync(amax_bits, 0, sizeof(unsigned int), stream);
     if (e != cudaSuccess) return (int)e;
-    kda_grad_amax_kernel<<<592, AMAX_THREADS, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(d_o), n_do, dht, dht ? n_dht : 0,
-                                                  amax_bits);
-    kda_grad_scale_kernel<<<1, 1, 0, stream>>>(amax_bits, gscale);
+    // a block per 512 16-byte pieces, up to four of 512 threads per SM
+    if (!dht) n_dht = 0;
+    const size_t pieces = (n_do / 8 > n_dht / 4 ? n_do / 8 : n_dht / 4) / AMAX_THREADS + 1, most = (size_t)4 * sm_count();
+    kda_grad_amax_kernel<<<(unsigned)(pieces < most ? pieces : most), AMAX_THREADS, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(d_o), n_do, dht,
+                                                                                                n_dht, amax_bits, gscale);
     return (int)cudaGetLastError();
 }
 

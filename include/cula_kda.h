@@ -136,6 +136,15 @@ int cula_kda_bwd_scratch_floats(void);
 int cula_kda_bwd_grad_scale(const void* d_do, long long n_do, const float* d_dht, long long n_dht,
                             unsigned int* d_amax, float* d_gscale, void* stream);
 
+/* cula_kda_bwd_grad_scale and, side by side with it, cula_kda_fwd_intra (the recomputation in front of a backward pass, which reads nothing
+ * of the upstream gradients). What follows in the stream finds both done. */
+int cula_kda_bwd_scale_and_intra(const void* d_do, long long n_do, const float* d_dht, long long n_dht, unsigned int* d_amax, float* d_gscale,
+                                 const void* d_q, const void* d_k, const void* d_v, const void* d_g, int g_is_fp32, const void* d_beta,
+                                 int beta_is_fp32, const float* d_A_log, const float* d_dt_bias, const int* d_cu_seqlens,
+                                 const int* d_chunk_indices, int num_chunks, int T, int H, float scale, int use_qk_l2norm, int gate_mode,
+                                 float lower_bound, void* d_tiles, float* d_akk, float* d_mkk, int* d_status, void* stream);
+
+
 /* Reverse state scan: d_dvn_out (fp16 [num_chunks*H][64][128], gradient w.r.t. v_new), d_ds_out (fp32
  * [num_chunks*H][128][128], gradient w.r.t. the state leaving each chunk), d_dh0 ([N,H,128,128] fp32 or NULL).
  * d_dvn_out and d_ds_out may both be NULL when only d_dh0 is wanted (first pass of the context-parallel backward).

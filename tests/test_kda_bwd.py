@@ -493,3 +493,26 @@ def test_a_sequence_does_not_read_its_neighbour(first, g_dtype):
     for n, a, b in zip(("o", *names), *results):
         assert torch.isfinite(b[:, :first].float()).all(), n
         assert err_ratio(a.detach().float().cpu(), b[:, :first].detach().float().cpu()) <= 1e-6, n
+
+
+@pytest.mark.parametrize("n_do,n_dht,apart", [(128, 0, False), (129, 5, True), (8 * 512 * 3 + 7, 16384, False), (1 << 22, 4, True), (12_582_912 + 8, 0, False)])
+@pytest.mark.parametrize("magnitude", [0.0, 3e-6, 1.0, 700.0])
+def test_gradient_scale(n_do, n_dht, apart, magnitude):
+    """The power of two that takes the largest upstream gradient into [4, 8), from one block to the most, wherever that value stands."""
+    from cula_b200 import _native
+    lib = _native.lib()
+    gen = torch.Generator(device="cuda").manual_seed(n_do)
+    do = (magnitude * torch.rand(n_do, device="cuda", generator=gen)).to(torch.bfloat16)
+    dht = magnitude * torch.rand(n_dht, device="cuda", generator=gen) if n_dht else None
+    do[n_do - 1] = 3 * magnitude
+    work = torch.full((8,), float("nan"), device="cuda")
+    amax = work.data_ptr() + (16 if apart else 8)
+    for _ in range(2):
+        assert lib.cula_kda_bwd_grad_scale(do.data_ptr(), n_do, dht.data_ptr() if n_dht else None, n_dht, amax, work.data_ptr(),
+                                           torch.cuda.current_stream().cuda_stream) == 0
+    s, inv = work[:2].tolist()
+    most = float(do.float().abs().max())
+    if magnitude == 0.0:
+        assert s == 1.0 and inv == 1.0
+    else:
+        assert 4.0 <= most * s < 8.0 and s * inv == 1.0
