@@ -268,6 +268,21 @@ inline int sm_count() {
     }
     return sms;
 }
+// A launch that may be scheduled while the kernel before it in the stream drains; the kernel calls pdl_launch_dependents() and, before it
+// touches memory, pdl_wait().
+template <typename... P, typename... A>
+inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 // raise the dynamic shared memory limit of one kernel (a function-local static `done` per kernel holds the devices it was
 // raised on)
 template <typename Kernel>

@@ -46,6 +46,7 @@ __global__ void __launch_bounds__(GATE_THREADS) kda_gate_kernel(const GateArgs a
     constexpr int WARPS = GATE_THREADS / 32;
     __shared__ __align__(16) float s_bias[BWD ? WARPS : 1][BWD ? 256 : 4];
     __shared__ float s_dA[BWD ? 10 : 1];     // at most 256 / 32 + 1 heads meet 256 channels (K >= 32)
+    pdl_launch_dependents();
     const int HK = a.H * a.K, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ch0 = 256 * blockIdx.x, ch_raw = ch0 + 8 * lane;
     const bool active = ch_raw < HK;
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(GATE_THREADS) kda_gate_kernel(const GateArgs a
         if (threadIdx.x < 10) s_dA[threadIdx.x] = 0.f;
         __syncthreads();
     }
+    pdl_wait();
     const float alpha = __expf(a.A_log[h]);
     float2 bias[4], dbias[4];
     float dA = 0.f;
@@ -148,6 +150,8 @@ __global__ void __launch_bounds__(GATE_THREADS) kda_gate_kernel(const GateArgs a
 template <bool BWD>
 __global__ void __launch_bounds__(GATE_THREADS) kda_beta_sigmoid_kernel(const void* x, int x_fp32, const float* dy, void* out,
                                                                        long long n) {
+    pdl_launch_dependents();
+    pdl_wait();
     for (long long i = (long long)blockIdx.x * GATE_THREADS + threadIdx.x; i < n; i += (long long)gridDim.x * GATE_THREADS) {
         const float xv = x_fp32 ? reinterpret_cast<const float*>(x)[i] : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(x)[i]);
         const float y = __fdividef(1.f, 1.f + __expf(-xv));
@@ -174,9 +178,7 @@ extern "C" int kda_launch_gate(const kda::GateArgs* a, int backward, cudaStream_
     if (gy > most) gy = most;
     if (gy > 65535) gy = 65535;
     dim3 grid(gx, (unsigned)gy);
-    if (backward) kda_gate_kernel<true><<<grid, GATE_THREADS, 0, stream>>>(*a);
-    else kda_gate_kernel<false><<<grid, GATE_THREADS, 0, stream>>>(*a);
-    return (int)cudaGetLastError();
+    return (int)launch_early(backward ? kda_gate_kernel<true> : kda_gate_kernel<false>, grid, GATE_THREADS, stream, *a);
 }
 
 extern "C" int kda_launch_beta_sigmoid(const void* x, int x_fp32, const float* dy, void* out, long long n, int backward,
@@ -186,7 +188,6 @@ extern "C" int kda_launch_beta_sigmoid(const void* x, int x_fp32, const float* d
     const int sms = sm_count();
     long long blocks = (n + GATE_THREADS - 1) / GATE_THREADS;
     if (blocks > 8LL * sms) blocks = 8LL * sms;
-    if (backward) kda_beta_sigmoid_kernel<true><<<(unsigned)blocks, GATE_THREADS, 0, stream>>>(x, x_fp32, dy, out, n);
-    else kda_beta_sigmoid_kernel<false><<<(unsigned)blocks, GATE_THREADS, 0, stream>>>(x, x_fp32, dy, out, n);
-    return (int)cudaGetLastError();
+    return (int)launch_early(backward ? kda_beta_sigmoid_kernel<true> : kda_beta_sigmoid_kernel<false>, dim3((unsigned)blocks), GATE_THREADS, stream, x,
+                             x_fp32, dy, out, n);
 }

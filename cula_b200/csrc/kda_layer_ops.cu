@@ -74,6 +74,8 @@ __global__ void __launch_bounds__(LO_THREADS) kda_short_conv_kernel(const ConvAr
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ch = GROUP * blockIdx.x + CH * lane, unit = CONV_WARPS * blockIdx.y + warp, c = unit / (BT / UNIT);
     bool live = ch < a.D && c < num_chunks;
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float s_dw[BWD ? CONV_WARPS : 1][GROUP][W + 1];       // weight and bias gradients per warp
     ChunkInfo ci{};
     int t0 = 0, t1 = 0;
@@ -271,6 +273,8 @@ __global__ void __launch_bounds__(LO_THREADS) kda_rms_norm_gated_kernel(const No
     const int lane = threadIdx.x & (LPR - 1), grp = threadIdx.x / LPR;
     const long long row0 = (long long)blockIdx.x * GROUPS + grp, stride = (long long)gridDim.x * GROUPS;
     float2 wv[VPL][4], dw_acc[VPL][4];
+    pdl_launch_dependents();
+    pdl_wait();
 #pragma unroll
     for (int v = 0; v < VPL; ++v)
 #pragma unroll
@@ -393,22 +397,19 @@ extern "C" int kda_launch_short_conv(const kda::ConvArgs* a, int num_chunks, int
     const bool halves = wide || (!backward && (long long)num_chunks * groups < 16LL * sm_count());
     const int units = num_chunks * (halves ? 2 : 1);
     const dim3 grid(groups, (units + CONV_WARPS - 1) / CONV_WARPS);
-#define KDA_CONV_LAUNCH(W)                                                                                            \
-    do {                                                                                                              \
-        if (wide) kda_short_conv_kernel<W, true, 2, 32><<<grid, LO_THREADS, 0, stream>>>(*a, num_chunks);               \
-        else if (backward) kda_short_conv_kernel<W, true, 1, 64><<<grid, LO_THREADS, 0, stream>>>(*a, num_chunks);      \
-        else if (halves) kda_short_conv_kernel<W, false, 1, 32><<<grid, LO_THREADS, 0, stream>>>(*a, num_chunks);       \
-        else kda_short_conv_kernel<W, false, 1, 64><<<grid, LO_THREADS, 0, stream>>>(*a, num_chunks);                   \
-    } while (0)
+    void (*kernel)(const ConvArgs, const int) = nullptr;
+#define KDA_CONV_KERNEL(W)                                                                                          \
+    kernel = wide ? kda_short_conv_kernel<W, true, 2, 32> : backward ? kda_short_conv_kernel<W, true, 1, 64> :       \
+             halves ? kda_short_conv_kernel<W, false, 1, 32> : kda_short_conv_kernel<W, false, 1, 64>
     switch (a->W) {
-        case 1: KDA_CONV_LAUNCH(1); break;
-        case 2: KDA_CONV_LAUNCH(2); break;
-        case 3: KDA_CONV_LAUNCH(3); break;
-        case 4: KDA_CONV_LAUNCH(4); break;
+        case 1: KDA_CONV_KERNEL(1); break;
+        case 2: KDA_CONV_KERNEL(2); break;
+        case 3: KDA_CONV_KERNEL(3); break;
+        case 4: KDA_CONV_KERNEL(4); break;
         default: return -1;
     }
-#undef KDA_CONV_LAUNCH
-    return (int)cudaGetLastError();
+#undef KDA_CONV_KERNEL
+    return (int)launch_early(kernel, grid, LO_THREADS, stream, *a, num_chunks);
 }
 
 extern "C" int kda_launch_rms_norm_gated(const kda::NormArgs* a, int backward, cudaStream_t stream) {
@@ -418,16 +419,13 @@ extern "C" int kda_launch_rms_norm_gated(const kda::NormArgs* a, int backward, c
     long long blocks = (a->R + groups - 1) / groups;
     const long long cap = (backward ? 4LL : 16LL) * sm_count();     // backward: fewer, longer-lived CTAs keep the dw atomics few
     if (blocks > cap) blocks = cap;
-#define KDA_NORM_LAUNCH(L, V)                                                                                        \
-    do {                                                                                                             \
-        if (backward) kda_rms_norm_gated_kernel<L, V, true><<<(unsigned)blocks, LO_THREADS, 0, stream>>>(*a);          \
-        else kda_rms_norm_gated_kernel<L, V, false><<<(unsigned)blocks, LO_THREADS, 0, stream>>>(*a);                  \
-    } while (0)
-    if (a->D == 128) KDA_NORM_LAUNCH(16, 1);
-    else if (a->D == 256) KDA_NORM_LAUNCH(32, 1);
-    else if (a->D == 512) KDA_NORM_LAUNCH(32, 2);
-    else if (a->D == 1024) KDA_NORM_LAUNCH(32, 4);
+    void (*kernel)(const NormArgs) = nullptr;
+#define KDA_NORM_KERNEL(L, V) kernel = backward ? kda_rms_norm_gated_kernel<L, V, true> : kda_rms_norm_gated_kernel<L, V, false>
+    if (a->D == 128) KDA_NORM_KERNEL(16, 1);
+    else if (a->D == 256) KDA_NORM_KERNEL(32, 1);
+    else if (a->D == 512) KDA_NORM_KERNEL(32, 2);
+    else if (a->D == 1024) KDA_NORM_KERNEL(32, 4);
     else return -1;
-#undef KDA_NORM_LAUNCH
-    return (int)cudaGetLastError();
+#undef KDA_NORM_KERNEL
+    return (int)launch_early(kernel, dim3((unsigned)blocks), LO_THREADS, stream, *a);
 }
