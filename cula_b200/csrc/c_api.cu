@@ -385,6 +385,15 @@ extern "C" int cula_kda_beta_sigmoid_bwd(const void* d_x, int x_is_fp32, const f
     return kda_launch_beta_sigmoid(d_x, x_is_fp32, d_dy, d_dx, n, 1, static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int kda_launch_clear(unsigned int* dst, long long words, cudaStream_t stream);
+
+extern "C" int cula_kda_clear(void* d_dst, long long bytes, void* stream) {
+    if (bytes == 0) return 0;
+    if (!d_dst || bytes < 0 || bytes % 4 != 0) return CULA_KDA_EINVAL;
+    if (misaligned(d_dst)) return CULA_KDA_EALIGN;
+    return kda_launch_clear(static_cast<unsigned int*>(d_dst), bytes / 4, static_cast<cudaStream_t>(stream));
+}
+
 extern "C" int kda_launch_short_conv(const kda::ConvArgs* a, int num_chunks, int backward, cudaStream_t stream);
 extern "C" int kda_launch_rms_norm_gated(const kda::NormArgs* a, int backward, cudaStream_t stream);
 

@@ -27,7 +27,7 @@ enum { GATE_NONE = 0, GATE_SOFTPLUS = 1, GATE_LOWER_BOUND = 2 };
 #define CULA_KDA_ENTRIES(X)                                                                                          \
     X(cula_kda_tile_pack_bytes) X(cula_kda_fwd_intra) X(cula_kda_fwd_scan) X(cula_kda_cp_transition) X(cula_kda_cp_fold) X(cula_kda_fwd_pieces) \
     X(cula_kda_decode) X(cula_kda_bwd_scratch_floats) X(cula_kda_bwd_grad_scale) X(cula_kda_bwd_scale_and_intra) X(cula_kda_bwd_scan) X(cula_kda_bwd_both_scans) \
-    X(cula_kda_bwd_dense) X(cula_kda_bwd_gated_checked) X(cula_kda_gate_fwd) X(cula_kda_gate_bwd)                              \
+    X(cula_kda_bwd_dense) X(cula_kda_bwd_gated_checked) X(cula_kda_clear) X(cula_kda_gate_fwd) X(cula_kda_gate_bwd)                              \
     X(cula_kda_beta_sigmoid_fwd) X(cula_kda_beta_sigmoid_bwd) X(cula_kda_short_conv_fwd) X(cula_kda_short_conv_bwd)    \
     X(cula_kda_rms_norm_gated_fwd) X(cula_kda_rms_norm_gated_bwd) X(cula_kda_strerror)
 struct Lib {
@@ -62,8 +62,7 @@ inline OptTensor contiguous_f32(const OptTensor& t) { return t.has_value() && t-
 inline Tensor device_empty(at::IntArrayRef sizes, const at::TensorOptions& options) { return Tensor(at::detail::empty_cuda(sizes, options)); }
 inline Tensor device_zeros(at::IntArrayRef sizes, const at::TensorOptions& options, cudaStream_t stream) {
     Tensor t = device_empty(sizes, options);
-    const cudaError_t e = t.numel() ? cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), stream) : cudaSuccess;
-    if (e != cudaSuccess) throw std::runtime_error(std::string("cudaMemsetAsync failed: ") + cudaGetErrorString(e));
+    check(lib.cula_kda_clear(t.data_ptr(), (long long)t.nbytes(), stream), "cula_kda_clear");
     return t;
 }
 // a dual tensor of forward-mode differentiation: no operator here has a forward derivative, and only the autograd function says so

@@ -165,7 +165,24 @@ __global__ void __launch_bounds__(GATE_THREADS) kda_beta_sigmoid_kernel(const vo
     }
 }
 
+// Zeros for buffers that atomics add to: unlike a memset, which ends and starts a chain of early launches, this is part of it.
+__global__ void __launch_bounds__(GATE_THREADS) kda_clear_kernel(unsigned int* dst, long long words) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const long long i = (long long)blockIdx.x * GATE_THREADS + threadIdx.x, n = (long long)gridDim.x * GATE_THREADS, quads = words / 4;
+    for (long long j = i; j < quads; j += n) reinterpret_cast<uint4*>(dst)[j] = make_uint4(0, 0, 0, 0);
+    for (long long j = 4 * quads + i; j < words; j += n) dst[j] = 0;
+}
+
 }  // namespace kda
+
+extern "C" int kda_launch_clear(unsigned int* dst, long long words, cudaStream_t stream) {
+    using namespace kda;
+    long long blocks = (words / 4 + GATE_THREADS - 1) / GATE_THREADS;
+    const long long most = 4LL * sm_count();
+    blocks = blocks < 1 ? 1 : blocks > most ? most : blocks;
+    return (int)launch_early(kda_clear_kernel, dim3((unsigned)blocks), GATE_THREADS, stream, dst, words);
+}
 
 extern "C" int kda_launch_gate(const kda::GateArgs* a, int backward, cudaStream_t stream) {
     using namespace kda;

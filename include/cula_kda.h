@@ -272,6 +272,9 @@ int cula_kda_gate_bwd(const void* d_g, int g_is_fp32, const float* d_A_log, cons
 int cula_kda_beta_sigmoid_fwd(const void* d_x, int x_is_fp32, float* d_y, long long n, void* stream);
 int cula_kda_beta_sigmoid_bwd(const void* d_x, int x_is_fp32, const float* d_dy, void* d_dx, long long n, void* stream);
 
+/* Zeros for a buffer that kernels add to (16-byte aligned, whole 32-bit words). */
+int cula_kda_clear(void* d_dst, long long bytes, void* stream);
+
 /* ------------------------------------------------------------------------------------------------------------
  * The two layer operators on either side of chunk_kda in a Kimi-Linear block (fla/layers/kda.py:147-165, 191, 306).
  *
