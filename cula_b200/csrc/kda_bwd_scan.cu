@@ -44,9 +44,10 @@ constexpr uint32_t BM_S32 = 0, BM_S16 = 128, BM_ACC = 192, BM_DO = 320, BM_ADO =
 constexpr int AMAX_THREADS = 512;
 // s = 2^k with max(|dO|, |dht|) * s in [4, 8); written as {s, 1/s}. amax_bits holds the running maximum, gscale[0] counts the blocks that
 // are done until the last one writes the scale there (both start as zero). The recomputation of the chunk-parallel stage, which reads none
-// of this, may start under this kernel.
+// of this, may start under this kernel, but under nothing before it: the trigger stands behind the wait.
 __global__ void kda_grad_amax_kernel(const __nv_bfloat16* d_o, size_t n_do, const float* dht, size_t n_dht,
                                      unsigned int* amax_bits, float* gscale) {
+    pdl_wait();
     pdl_launch_dependents();
     float m = 0.f;
     const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nthr = (size_t)gridDim.x * blockDim.x;
@@ -441,19 +442,20 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
 
 }  // namespace kda
 
+extern "C" int kda_launch_clear(unsigned int* dst, long long words, cudaStream_t stream);
+
 extern "C" int kda_launch_grad_scale(const void* d_o, size_t n_do, const float* dht, size_t n_dht, unsigned int* amax_bits,
                                      float* gscale, cudaStream_t stream) {
     using namespace kda;
     const bool one_piece = reinterpret_cast<float*>(amax_bits) == gscale + 2;
-    cudaError_t e = cudaMemsetAsync(gscale, 0, (one_piece ? 3 : 1) * sizeof(float), stream);
-    if (e == cudaSuccess && !one_piece) e = cudaMemsetAsync(amax_bits, 0, sizeof(unsigned int), stream);
-    if (e != cudaSuccess) return (int)e;
+    int rc = kda_launch_clear(reinterpret_cast<unsigned int*>(gscale), one_piece ? 3 : 1, stream);
+    if (rc == 0 && !one_piece) rc = kda_launch_clear(amax_bits, 1, stream);
+    if (rc != 0) return rc;
     // a block per 512 16-byte pieces, up to four of 512 threads per SM
     if (!dht) n_dht = 0;
     const size_t pieces = (n_do / 8 > n_dht / 4 ? n_do / 8 : n_dht / 4) / AMAX_THREADS + 1, most = (size_t)4 * sm_count();
-    kda_grad_amax_kernel<<<(unsigned)(pieces < most ? pieces : most), AMAX_THREADS, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(d_o), n_do, dht,
-                                                                                                n_dht, amax_bits, gscale);
-    return (int)cudaGetLastError();
+    return (int)launch_early(kda_grad_amax_kernel, dim3((unsigned)(pieces < most ? pieces : most)), AMAX_THREADS, stream,
+                             reinterpret_cast<const __nv_bfloat16*>(d_o), n_do, dht, n_dht, amax_bits, gscale);
 }
 
 extern "C" int kda_launch_bwd_scan(const kda::BwdScanParams* p, cudaStream_t stream) {
