@@ -232,8 +232,8 @@ Backward backward_core(const Tensor& q, const Tensor& k, const Tensor& v, const 
     if (opt.gate_mode != GATE_NONE) {            // the two atomically accumulated gradients share one cleared buffer
         const bool bias = dt_bias.has_value() && dt_bias->defined();
         Tensor both = device_zeros({bias ? H + H * DIM : H}, f32, stream);
-        if (bias) r.dbias = both.narrow(0, 0, H * DIM);
-        r.dA = both.narrow(0, both.numel() - H, H);
+        if (bias) r.dbias = part_of(both, 0, dt_bias->sizes());
+        r.dA = part_of(both, both.numel() - H, A_log->sizes());
     }
     check(lib.cula_kda_bwd_gated_checked(ptr(q), ptr(k), ptr(g), g_flags(g), ptr(beta), beta_flags(beta, opt.beta_logit), fptr(A_log), fptr(dt_bias),
                                          fptr(f.akk), fptr(f.mkk), fptr(scratch), fptr(work), ptr(r.dq), ptr(r.dk), ptr(r.dg), ptr(r.dbeta),
@@ -311,8 +311,6 @@ public:
             scan_left = true;
         }
         Backward b = backward_core(q, k, v, g, beta, A_log, dt_bias, o, tab ? &*tab : nullptr, f, h0.has_value(), up, scan_left, h0);
-        if (b.dA.defined()) b.dA = b.dA.view_as(*A_log);
-        if (b.dbias.defined()) b.dbias = b.dbias.view_as(*dt_bias);
         return {b.dq, b.dk, b.dv, b.dg, b.dbeta, b.dA, b.dbias, b.dh0, Tensor()};
     }
 };

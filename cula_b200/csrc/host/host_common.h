@@ -65,6 +65,13 @@ inline Tensor device_zeros(at::IntArrayRef sizes, const at::TensorOptions& optio
     check(lib.cula_kda_clear(t.data_ptr(), (long long)t.nbytes(), stream), "cula_kda_clear");
     return t;
 }
+// contiguous part of an own buffer as a tensor (narrow and view through the dispatcher take 3 us)
+inline Tensor part_of(const Tensor& buffer, int64_t offset, at::IntArrayRef sizes) {
+    Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(buffer.storage()), buffer.key_set(), buffer.dtype());
+    t.unsafeGetTensorImpl()->set_storage_offset(offset);
+    t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+    return t;
+}
 // a dual tensor of forward-mode differentiation: no operator here has a forward derivative, and only the autograd function says so
 inline bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
 inline cudaStream_t stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }

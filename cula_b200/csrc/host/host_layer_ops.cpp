@@ -53,8 +53,8 @@ struct Gate : torch::autograd::Function<Gate> {
         // the two accumulated gradients share one cleared buffer
         const int64_t n_bias = b32.has_value() ? b32->numel() : 0;
         Tensor both = device_zeros({n_bias + a32.numel()}, a32.options(), stream_of(g));
-        Tensor dA = both.narrow(0, n_bias, a32.numel()).view(a32.sizes());
-        Tensor dbias = b32.has_value() ? both.narrow(0, 0, n_bias).view(b32->sizes()) : Tensor();
+        Tensor dA = part_of(both, n_bias, a32.sizes());
+        Tensor dbias = b32.has_value() ? part_of(both, 0, b32->sizes()) : Tensor();
         check(lib.cula_kda_gate_bwd(ptr(g), is_f32(g), fptr(a32), fptr(b32), ptr(dy), is_f32(dy), ptr(dg), fptr(dA), fptr(dbias), g.numel() / (H * K),
                                     (int)H, (int)K, !lb.isNone(), lb.isNone() ? 0.f : (float)lb.toDouble(), stream_of(g)), "cula_kda_gate_bwd");
         return {dg, dA, dbias, Tensor(), Tensor()};
