@@ -319,6 +319,11 @@ kda_bwd_dense_kernel(const BwdDenseParams p, const int num_tiles, const __grid_c
             const bool upper = q < 2;                                // TMEM lanes 0-63
             const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
             uint32_t r[16];
+            // this thread's piece of V, for dbeta_u: asked for now, used last
+            const int v0 = (upper ? 0 : 64) + 16 * cg;
+            const size_t goff = (size_t)(cur.row0 + min(i, cur.valid - 1)) * tok_stride + (size_t)cur_h * DV + v0;
+            const uint4 v_lo = *reinterpret_cast<const uint4*>(Vg + goff);
+            const uint4 v_hi = *reinterpret_cast<const uint4*>(Vg + goff + 8);
             // D1: dQg (lanes 0-63) / -dW (lanes 64-127), 32 of the 128 key channels per warp -> boxes in the [dO; dVn] / [Vn; V] buffers
             {
                 unsigned char* box = sm + BD_A1 + ((upper ? 0 : 4) + cg) * 8192;
@@ -377,14 +382,10 @@ kda_bwd_dense_kernel(const BwdDenseParams p, const int num_tiles, const __grid_c
             }
             // D4: Zu (both lane halves hold it): lanes 0-63 take value columns 0-63, lanes 64-127 columns 64-127
             {
-                const int v0 = (upper ? 0 : 64) + 16 * cg;
                 umma::ld_32x32b_x16(tl + TC_D4 + v0, r);
                 umma::wait_ld();
                 float dbu = 0.f;
                 if (i < cur.valid) {
-                    const size_t goff = (size_t)(cur.row0 + i) * tok_stride + (size_t)cur_h * DV + v0;
-                    const uint4 v_lo = *reinterpret_cast<const uint4*>(Vg + goff);
-                    const uint4 v_hi = *reinterpret_cast<const uint4*>(Vg + goff + 8);
                     const uint32_t vw[8] = {v_lo.x, v_lo.y, v_lo.z, v_lo.w, v_hi.x, v_hi.y, v_hi.z, v_hi.w};
                     const float bsc = gs_inv * sBeta[i];
                     uint32_t out[8];
