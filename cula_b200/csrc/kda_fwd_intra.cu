@@ -784,25 +784,14 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
                 }
             }
         };
-        uint32_t r0[16], r1[16];
-        if (qd & 1) {        // rows 32..63: block 2 against blocks 0, 1; block 3 against 0, 1, 2
-            umma::ld_32x32b_x16(taddr + 16, r0);
-            umma::ld_32x32b_x16(taddr + 32, r1);
+        // rows 32..63: block 2 against blocks 0, 1, block 3 against 0, 1, 2; rows 0..31: block 1 against block 0. Not unrolled: the kernel
+        // runs its code once a tile, the instruction cache does not hold it, and these are 8 KB of 95 (774 -> 762 us at 4 x 8192 x 32).
+#pragma unroll 1
+        for (int pair = qd & 1; pair <= 5 * (qd & 1); ++pair) {
+            uint32_t r[16];
+            umma::ld_32x32b_x16(taddr + 16 * pair, r);
             umma::wait_ld();
-            emit(r0, 2, 0);
-            emit(r1, 2, 1);
-            umma::ld_32x32b_x16(taddr + 48, r0);
-            umma::ld_32x32b_x16(taddr + 64, r1);
-            umma::wait_ld();
-            emit(r0, 3, 0);
-            emit(r1, 3, 1);
-            umma::ld_32x32b_x16(taddr + 80, r0);
-            umma::wait_ld();
-            emit(r0, 3, 2);
-        } else {             // rows 0..31: block 1 against block 0
-            umma::ld_32x32b_x16(taddr, r0);
-            umma::wait_ld();
-            emit(r0, 1, 0);
+            emit(r, pair == 0 ? 1 : pair < 3 ? 2 : 3, pair == 0 ? 0 : pair < 3 ? pair - 1 : pair - 3);
         }
     } else {
         const int cc0 = 2 * ((t & 1) | ((2 * t) & 4));
