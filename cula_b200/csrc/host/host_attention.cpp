@@ -108,12 +108,19 @@ Plan plan_pieces(int64_t ctas, int64_t nc, int sms) {
 // The upstream gradients and the power-of-two scale they are carried in.
 struct Upstream {
     Tensor d_o, work;             // work: [0:2] = {s, 1/s}, [2] = running max (as bits)
+    Tensor sums;                  // the atomically accumulated gradients of dt_bias (if any) and A_log, cleared
     OptTensor dht;
     int64_t n_dht() const { return dht.has_value() ? dht->numel() : 0; }
     unsigned int* amax() const { return reinterpret_cast<unsigned int*>(fptr(work) + 2); }
 };
-Upstream upstream(const Tensor& d_out, const OptTensor& d_final) {
-    return {d_out.contiguous(), device_empty({4}, d_out.options().dtype(at::kFloat)), contiguous_f32(d_final)};
+// (cleared in front of everything: between two kernels of the chain a launch would keep the second from being set up behind the first)
+Upstream upstream(const Tensor& d_out, const OptTensor& d_final, const Tensor& q, const OptTensor& dt_bias, const Options& opt) {
+    c10::cuda::CUDAGuard guard(q.device());
+    const auto f32 = q.options().dtype(at::kFloat);
+    const int64_t H = q.size(2);
+    const bool bias = dt_bias.has_value() && dt_bias->defined();
+    return {d_out.contiguous(), device_empty({4}, d_out.options().dtype(at::kFloat)),
+            opt.gate_mode != GATE_NONE ? device_zeros({bias ? H + H * DIM : H}, f32, stream_of(q)) : Tensor(), contiguous_f32(d_final)};
 }
 void scale_gradients(const Upstream& u) {
     c10::cuda::CUDAGuard guard(u.d_o.device());
@@ -229,11 +236,9 @@ Backward backward_core(const Tensor& q, const Tensor& k, const Tensor& v, const 
     r.dk = output_like(k, tab);
     r.dg = output_like(g, tab);
     r.dbeta = output_like(beta, tab);
-    if (opt.gate_mode != GATE_NONE) {            // the two atomically accumulated gradients share one cleared buffer
-        const bool bias = dt_bias.has_value() && dt_bias->defined();
-        Tensor both = device_zeros({bias ? H + H * DIM : H}, f32, stream);
-        if (bias) r.dbias = part_of(both, 0, dt_bias->sizes());
-        r.dA = part_of(both, both.numel() - H, A_log->sizes());
+    if (opt.gate_mode != GATE_NONE) {
+        if (dt_bias.has_value() && dt_bias->defined()) r.dbias = part_of(up.sums, 0, dt_bias->sizes());
+        r.dA = part_of(up.sums, up.sums.numel() - H, A_log->sizes());
     }
     check(lib.cula_kda_bwd_gated_checked(ptr(q), ptr(k), ptr(g), g_flags(g), ptr(beta), beta_flags(beta, opt.beta_logit), fptr(A_log), fptr(dt_bias),
                                          fptr(f.akk), fptr(f.mkk), fptr(scratch), fptr(work), ptr(r.dq), ptr(r.dk), ptr(r.dg), ptr(r.dbeta),
@@ -298,7 +303,7 @@ public:
         }
         const Tensor d_o = grads[0].defined() ? grads[0] : at::zeros_like(v);
         const OptTensor dht = grads.size() > 1 && grads[1].defined() ? OptTensor(grads[1]) : OptTensor();
-        const Upstream up = upstream(d_o, dht);
+        const Upstream up = upstream(d_o, dht, q, dt_bias, o);
         Forward f;
         bool scan_left = false;
         if (auto it = ctx->saved_data.find("kept"); it != ctx->saved_data.end()) {
@@ -435,7 +440,7 @@ pybind11::tuple backward_tuple(const Tensor& q, const Tensor& k, const Tensor& v
     auto get = [&](const char* n) { return saved[n].cast<Tensor>(); };
     f.tiles = get("tiles"); f.akk = get("akk"); f.mkk = get("mkk"); f.h32 = get("h32"); f.vnew = get("vnew");
     f.num_chunks = saved["num_chunks"].cast<int64_t>();
-    const Upstream up = upstream(d_o, dht);
+    const Upstream up = upstream(d_o, dht, q, dt_bias, o);
     scale_gradients(up);
     Backward b = backward_core(q, k, v, g, beta, A_log, dt_bias, o, tab, f, want_dh0, up);
     auto obj = [](const Tensor& t) -> pybind11::object { return t.defined() ? pybind11::cast(t) : pybind11::object(pybind11::none()); };

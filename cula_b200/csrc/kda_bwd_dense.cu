@@ -97,7 +97,6 @@ kda_bwd_dense_kernel(const BwdDenseParams p, const int num_tiles, const __grid_c
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const size_t tok_stride = (size_t)p.H * DV;
-    const float gs = p.gscale[0], gs_inv = p.gscale[1];
     const __nv_bfloat16* dOg = reinterpret_cast<const __nv_bfloat16*>(p.d_o);
     const __nv_bfloat16* Vg = reinterpret_cast<const __nv_bfloat16*>(p.v);
     // staging role: token row and 8 value columns (of the 64 of a half)
@@ -113,6 +112,8 @@ kda_bwd_dense_kernel(const BwdDenseParams p, const int num_tiles, const __grid_c
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();         // launched while the reverse scan drains; that one ends behind the forward scan, so all it counts on is there
+    const float gs = p.gscale[0], gs_inv = p.gscale[1];
 
     // ---- helpers ----
     auto issue_state_loads = [&](int t_id, int vh) {        // one thread: one value half of S and dS' of a tile
@@ -211,6 +212,7 @@ kda_bwd_dense_kernel(const BwdDenseParams p, const int num_tiles, const __grid_c
     long long bd_t0_ = clock64();
 #endif
     for (; tile < num_tiles; tile += gridDim.x, par ^= 1u) {
+        if (tile + (int)gridDim.x >= num_tiles) pdl_launch_dependents();      // the last tile: the gated stage may be set up behind it
         const int next = tile + gridDim.x;
         const ChunkInfo cur = ci;
         const int cur_h = h;
@@ -515,7 +517,6 @@ extern "C" int kda_launch_bwd_dense(const kda::BwdDenseParams* p, int num_chunks
         !make_scratch_map(&map_out128, p->scratch, SCR_DQG, 128, 192, tiles) ||
         !make_scratch_map(&map_out64, p->scratch, SCR_DPS, 64, 128, tiles))
         return (int)cudaErrorInvalidValue;
-    kda_bwd_dense_kernel<<<tiles < sms ? tiles : sms, BD_THREADS, BD_SMEM, stream>>>(*p, tiles, map_s, map_ds, map_out128,
-                                                                                      map_out64);
-    return (int)cudaGetLastError();
+    return (int)launch_early(kda_bwd_dense_kernel, dim3(tiles < sms ? tiles : sms), BD_THREADS, BD_SMEM, stream, *p, tiles, map_s, map_ds,
+                             map_out128, map_out64);
 }

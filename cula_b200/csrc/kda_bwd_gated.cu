@@ -183,6 +183,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
         fence_mbar_init();
     }
     if (warp == 0) umma::tmem_alloc(tmem_slot, 512);
+    pdl_wait();         // launched while the dense stage drains
     auto geometry = [&](int t) {
         const int c = t / p.H;
         const ChunkInfo ci = chunk_info(c, p.cu_seqlens, p.chunk_indices, p.T);
@@ -523,6 +524,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
         for (int x = 0; x < N2; ++x) v[x] = make_float2(scr[from + (t0 + 2 * x) * DK + ch], scr[from + (t0 + 2 * x + 1) * DK + ch]);
     };
     const int next = tile + gridDim.x;
+    if (next >= num_tiles) pdl_launch_dependents();
     if (warp == 2) {          // (not part of the chain)
         if (next < num_tiles) {
             if (lane == 0) {
@@ -1014,6 +1016,5 @@ extern "C" int kda_launch_bwd_gated(const kda::BwdGatedParams* p, int num_chunks
     if (!make_matrix_map(&maps.a, p->akk, 64, 64, 16384, tiles) || !make_matrix_map(&maps.m, p->mkk, 64, 64, 16384, tiles) ||
         !make_matrix_map(&maps.dw, p->scratch + SCR_DW, 128, 64, rec, tiles) || !make_matrix_map(&maps.ps, p->scratch + SCR_DPS, 64, 128, rec, tiles))
         return (int)cudaErrorInvalidValue;
-    kernel<<<tiles < sms ? tiles : sms, BG_THREADS, BG_SMEM, stream>>>(*p, tiles, maps);
-    return (int)cudaGetLastError();
+    return (int)launch_early(kernel, dim3(tiles < sms ? tiles : sms), BG_THREADS, BG_SMEM, stream, *p, tiles, maps);
 }

@@ -406,6 +406,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) kda_bwd_scan_kernel(const BwdSc
         const int q = warp, v = 32 * q + lane;
         const uint32_t tl = tmem + ((uint32_t)(32 * q) << 16);
         for (int it = 0; it < nchunks; ++it) {
+            if (it + 1 == nchunks) pdl_launch_dependents();      // the last chunk: the dense stage may be set up
             const uint32_t acc = tl + BM_ACC + 64 * (it & 1);
             if (!wait(&b_v16[it & 1], it >> 1)) break;
             umma::fence_after_sync();
@@ -454,7 +455,7 @@ extern "C" int kda_launch_grad_scale(const void* d_o, size_t n_do, const float* 
     // a block per 512 16-byte pieces, up to four of 512 threads per SM
     if (!dht) n_dht = 0;
     const size_t pieces = (n_do / 8 > n_dht / 4 ? n_do / 8 : n_dht / 4) / AMAX_THREADS + 1, most = (size_t)4 * sm_count();
-    return (int)launch_early(kda_grad_amax_kernel, dim3((unsigned)(pieces < most ? pieces : most)), AMAX_THREADS, stream,
+    return (int)launch_early(kda_grad_amax_kernel, dim3((unsigned)(pieces < most ? pieces : most)), AMAX_THREADS, 0, stream,
                              reinterpret_cast<const __nv_bfloat16*>(d_o), n_do, dht, n_dht, amax_bits, gscale);
 }
 

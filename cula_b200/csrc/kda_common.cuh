@@ -271,10 +271,11 @@ inline int sm_count() {
 // A launch that may be scheduled while the kernel before it in the stream drains; the kernel calls pdl_launch_dependents() and, before it
 // touches memory, pdl_wait().
 template <typename... P, typename... A>
-inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t stream, A... args) {
+inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t stream, const A&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -181,7 +181,7 @@ extern "C" int kda_launch_clear(unsigned int* dst, long long words, cudaStream_t
     long long blocks = (words / 4 + GATE_THREADS - 1) / GATE_THREADS;
     const long long most = 4LL * sm_count();
     blocks = blocks < 1 ? 1 : blocks > most ? most : blocks;
-    return (int)launch_early(kda_clear_kernel, dim3((unsigned)blocks), GATE_THREADS, stream, dst, words);
+    return (int)launch_early(kda_clear_kernel, dim3((unsigned)blocks), GATE_THREADS, 0, stream, dst, words);
 }
 
 extern "C" int kda_launch_gate(const kda::GateArgs* a, int backward, cudaStream_t stream) {
@@ -195,7 +195,7 @@ extern "C" int kda_launch_gate(const kda::GateArgs* a, int backward, cudaStream_
     if (gy > most) gy = most;
     if (gy > 65535) gy = 65535;
     dim3 grid(gx, (unsigned)gy);
-    return (int)launch_early(backward ? kda_gate_kernel<true> : kda_gate_kernel<false>, grid, GATE_THREADS, stream, *a);
+    return (int)launch_early(backward ? kda_gate_kernel<true> : kda_gate_kernel<false>, grid, GATE_THREADS, 0, stream, *a);
 }
 
 extern "C" int kda_launch_beta_sigmoid(const void* x, int x_fp32, const float* dy, void* out, long long n, int backward,
@@ -205,6 +205,6 @@ extern "C" int kda_launch_beta_sigmoid(const void* x, int x_fp32, const float* d
     const int sms = sm_count();
     long long blocks = (n + GATE_THREADS - 1) / GATE_THREADS;
     if (blocks > 8LL * sms) blocks = 8LL * sms;
-    return (int)launch_early(backward ? kda_beta_sigmoid_kernel<true> : kda_beta_sigmoid_kernel<false>, dim3((unsigned)blocks), GATE_THREADS, stream, x,
+    return (int)launch_early(backward ? kda_beta_sigmoid_kernel<true> : kda_beta_sigmoid_kernel<false>, dim3((unsigned)blocks), GATE_THREADS, 0, stream, x,
                              x_fp32, dy, out, n);
 }

@@ -409,7 +409,7 @@ extern "C" int kda_launch_short_conv(const kda::ConvArgs* a, int num_chunks, int
         default: return -1;
     }
 #undef KDA_CONV_KERNEL
-    return (int)launch_early(kernel, grid, LO_THREADS, stream, *a, num_chunks);
+    return (int)launch_early(kernel, grid, LO_THREADS, 0, stream, *a, num_chunks);
 }
 
 extern "C" int kda_launch_rms_norm_gated(const kda::NormArgs* a, int backward, cudaStream_t stream) {
@@ -427,5 +427,5 @@ extern "C" int kda_launch_rms_norm_gated(const kda::NormArgs* a, int backward, c
     else if (a->D == 1024) KDA_NORM_KERNEL(32, 4);
     else return -1;
 #undef KDA_NORM_KERNEL
-    return (int)launch_early(kernel, dim3((unsigned)blocks), LO_THREADS, stream, *a);
+    return (int)launch_early(kernel, dim3((unsigned)blocks), LO_THREADS, 0, stream, *a);
 }

@@ -516,3 +516,32 @@ def test_gradient_scale(n_do, n_dht, apart, magnitude):
         assert s == 1.0 and inv == 1.0
     else:
         assert 4.0 <= most * s < 8.0 and s * inv == 1.0
+
+
+@pytest.mark.parametrize("B,T,H,lens", [(1, 1, 1, None), (2, 130, 3, None), (1, 64 * 40, 5, None), (1, 700, 40, [1, 64, 65, 370, 200])])
+def test_stages_launched_behind_one_another_equal_stages_waited_for(B, T, H, lens):
+    """Each stage of the backward pass is launched while the one before it drains: calls queued without a pause, in memory that the
+    calls before them have just given back, have the bits of calls that start on an idle device."""
+    from cula_b200.kda import check_status, chunk_kda
+    from cula_b200.synthetic import make_inputs_on_device
+    names = ("q", "k", "v", "g", "beta")
+    cu = None if lens is None else torch.tensor([0, *np.cumsum(lens)], dtype=torch.int32, device="cuda")
+    data = [make_inputs_on_device(B, T, H, torch.device("cuda"), seed=s, gate_offset=-4.0) for s in range(4)]
+
+    def call(d):
+        leaves = [d[n].detach().requires_grad_(True) for n in names]
+        o, _ = chunk_kda(*leaves, use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, safe_gate=True, lower_bound=-5.0, A_log=d["A_log"],
+                         dt_bias=d["dt_bias"], cu_seqlens=cu)
+        return torch.autograd.grad(o, leaves, d["v"])
+
+    alone = []
+    for d in data:
+        torch.cuda.synchronize()
+        alone.append(call(d))
+    torch.cuda.synchronize()
+    queued = [call(d) for _ in range(3) for d in data]
+    torch.cuda.synchronize()
+    check_status()
+    for i, grads in enumerate(queued):
+        for n, a, b in zip(names, alone[i % 4], grads):
+            assert torch.equal(a, b), (i, n)
