@@ -388,19 +388,17 @@ __global__ void __launch_bounds__(LO_THREADS) kda_rms_norm_gated_kernel(const No
 extern "C" int kda_launch_short_conv(const kda::ConvArgs* a, int num_chunks, int backward, cudaStream_t stream) {
     using namespace kda;
     if (num_chunks <= 0) return 0;
-    auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; };
     // Backward: two pairs of channels per lane halve the instructions that do not depend on the number of channels and double the work
-    // between dependent ones; rows of 8-byte pieces are all it asks for. Forward: one pair (two: 17.5 -> 19.5 us at 4096 x 4096), and
-    // half chunks where whole ones would leave fewer than 16 warps per SM (8192 x 512: 11.5 -> 8.5 us).
-    const bool wide = backward && a->D % 4 == 0 && aligned(a->x) && aligned(a->dy) && aligned(a->dx);
+    // between dependent ones (rows are 16-byte pieces). Forward: one pair (two: 17.5 -> 19.5 us at 4096 x 4096), and half chunks where
+    // whole ones would leave fewer than 16 warps per SM (8192 x 512: 11.5 -> 8.5 us).
+    const bool wide = backward;
     const int groups = (a->D + (wide ? 127 : 63)) / (wide ? 128 : 64);
-    const bool halves = wide || (!backward && (long long)num_chunks * groups < 16LL * sm_count());
+    const bool halves = wide || (long long)num_chunks * groups < 16LL * sm_count();
     const int units = num_chunks * (halves ? 2 : 1);
     const dim3 grid(groups, (units + CONV_WARPS - 1) / CONV_WARPS);
     void (*kernel)(const ConvArgs, const int) = nullptr;
 #define KDA_CONV_KERNEL(W)                                                                                          \
-    kernel = wide ? kda_short_conv_kernel<W, true, 2, 32> : backward ? kda_short_conv_kernel<W, true, 1, 64> :       \
-             halves ? kda_short_conv_kernel<W, false, 1, 32> : kda_short_conv_kernel<W, false, 1, 64>
+    kernel = wide ? kda_short_conv_kernel<W, true, 2, 32> : halves ? kda_short_conv_kernel<W, false, 1, 32> : kda_short_conv_kernel<W, false, 1, 64>
     switch (a->W) {
         case 1: KDA_CONV_KERNEL(1); break;
         case 2: KDA_CONV_KERNEL(2); break;

@@ -119,6 +119,31 @@ def test_short_conv_at_chunk_and_channel_edges(D, W, tail):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("W", [1, 2, 3, 4])
+def test_short_conv_does_not_depend_on_how_chunks_are_split(W):
+    """Many chunks are taken whole, few in halves: the same rows come out to the bit."""
+    from cula_b200.kda import short_conv
+    gen = torch.Generator(device="cuda").manual_seed(W)
+    x = torch.randn(1, 64 * 2400 + 37, 64, device="cuda", generator=gen).to(torch.bfloat16)
+    w = torch.randn(64, W, device="cuda", generator=gen)
+    whole, _ = short_conv(x, w)
+    n = 64 * 5 + 33
+    few, _ = short_conv(x[:, :n].contiguous(), w)
+    assert torch.equal(whole[:, :n], few)
+    tail, _ = short_conv(x[:, -n:].contiguous(), w)
+    assert torch.equal(whole[:, W - 1 - n:], tail[:, W - 1:])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("words", [1, 2, 3, 4, 5, 1023, 1024, 1025, 1 << 20, (1 << 20) + 3])
+def test_clear_writes_its_words_and_no_others(words):
+    from cula_b200 import _native
+    buf = torch.full((words + 8,), 7.0, device="cuda")
+    assert _native.lib().cula_kda_clear(buf[4:].data_ptr(), 4 * words, torch.cuda.current_stream().cuda_stream) == 0
+    assert not buf[4:-4].any() and bool((buf[:4] == 7).all() and (buf[-4:] == 7).all())
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("D", [128, 256, 512, 1024])
 @pytest.mark.parametrize("R", [1, 3, 8, 9, 4099])
 def test_rms_norm_gated_row_remainders(R, D):
