@@ -68,11 +68,12 @@ void segmented_scan(const Tensor& v, const OptTensor& h0, bool want_final, const
 // step form a geometric series; the first piece's chunk-parallel stage and the last one's scan are exposed. The times are measured,
 // in us. Above half the SMs the scan leaves too little for this to gain (3 x 4096 x 32 heads: 456 -> 476 us).
 // Both stages one after the other -> in these pieces, us, cold L2, with a bf16 gate / an fp32 gate / a gate per head:
-//   1 x 4096 x 32 heads   238 -> 211     255 -> 227     214 -> 187        2 x 2048 x 32   187 -> 182     204 -> 202     163 -> 156
-//   2 x 8192 x 32         675 -> 639     726 -> 697     585 -> 537        4 x 4096 x 16   349 -> 338     378 -> 370     302 -> 275
-//   1 x 65536 x 32       3418 -> 2465   3610 -> 2719   3051 -> 2338       1 x 16384 x 48 1082 -> 932    1156 -> 1011    949 -> 810
-// The three kernels take 0.053, 0.059 and 0.042 us per tile (8192 tiles). One rate serves all: planned with its own, an fp32 gate
-// came out 1 % slower to 3 % faster and a gate per head 6 % slower to 4 % faster, for other reasons than the plan can know.
+//   1 x 4096 x 32 heads   230 -> 205     232 -> 209     206 -> 185        2 x 2048 x 32   177 -> 172     183 -> 178     155 -> 148
+//   2 x 8192 x 32         644 -> 582     660 -> 599     558 -> 498        4 x 4096 x 16   331 -> 315     339 -> 332     290 -> 260
+//   1 x 65536 x 32       3266 -> 2443   3335 -> 2525   2913 -> 2222       1 x 16384 x 48 1039 -> 896    1072 -> 929     908 -> 767
+// The three kernels take 0.048, 0.050 and 0.038 us per tile (8192 tiles; 0.0535, 0.056 and 0.043 in launches of 2048). One rate serves all:
+// planned with their rates at 8192 tiles, 2 x 2048 x 32 comes out 172 -> 180, others 1 % slower to 3 % faster, for other reasons than
+// the plan can know.
 // What keeps its intermediates (training that recomputes, B > 1 that does not) and packed batches have no pieces, and only B = 1
 // without gradients or kept intermediates has segments: few long chains are left as they are there.
 struct Plan {

@@ -29,7 +29,8 @@
 // Measured at B=2, T=2048, H=32 (2048 tiles, cold L2): 143.6 -> 119 us, 31.7 k -> 24 k warp instructions per tile against the
 // version that formed all of the Gram product as tf32 operands in shared memory, two channel halves one after the other; with the
 // q and k rows of whole chunks by TMA where their operands will stand, instead of in registers from tile to tile: 119 -> 112 us, 844 ->
-// 774 us at 4 x 8192 x 32. (Requested right at the start of a tile, where the thread that asks waits for the copies out: 789 us.)
+// 774 us at 4 x 8192 x 32 (requested right at the start of a tile, where the thread that asks waits for the copies out: 789 us); with the
+// Gram epilogue as a loop 109 us, 762 us: a tenth of the stalls are for instructions. Rolling the gates and cumulative sums too: no gain.
 #include "kda_common.cuh"
 #include "kda_params.h"
 #include "scan_common.cuh"
