@@ -238,8 +238,8 @@ Backward backward_core(const Tensor& q, const Tensor& k, const Tensor& v, const 
     r.dg = output_like(g, tab);
     r.dbeta = output_like(beta, tab);
     if (opt.gate_mode != GATE_NONE) {
-        if (dt_bias.has_value() && dt_bias->defined()) r.dbias = part_of(up.sums, 0, dt_bias->sizes());
-        r.dA = part_of(up.sums, up.sums.numel() - H, A_log->sizes());
+        if (dt_bias.has_value() && dt_bias->defined()) r.dbias = part_of(up.sums, 0, {H * DIM});
+        r.dA = part_of(up.sums, up.sums.numel() - H, {H});
     }
     check(lib.cula_kda_bwd_gated_checked(ptr(q), ptr(k), ptr(g), g_flags(g), ptr(beta), beta_flags(beta, opt.beta_logit), fptr(A_log), fptr(dt_bias),
                                          fptr(f.akk), fptr(f.mkk), fptr(scratch), fptr(work), ptr(r.dq), ptr(r.dk), ptr(r.dg), ptr(r.dbeta),
@@ -317,6 +317,8 @@ public:
             scan_left = true;
         }
         Backward b = backward_core(q, k, v, g, beta, A_log, dt_bias, o, tab ? &*tab : nullptr, f, h0.has_value(), up, scan_left, h0);
+        if (b.dA.defined()) b.dA = shaped_like(b.dA, *A_log);
+        if (b.dbias.defined()) b.dbias = shaped_like(b.dbias, *dt_bias);
         return {b.dq, b.dk, b.dv, b.dg, b.dbeta, b.dA, b.dbias, b.dh0, Tensor()};
     }
 };

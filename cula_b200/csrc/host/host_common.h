@@ -72,6 +72,13 @@ inline Tensor part_of(const Tensor& buffer, int64_t offset, at::IntArrayRef size
     t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
     return t;
 }
+// a part in the shape of the parameter that it is the gradient of
+inline Tensor shaped_like(const Tensor& part, const Tensor& parameter) {
+    if (part.numel() != parameter.numel())
+        throw std::runtime_error("a gradient of " + std::to_string(part.numel()) + " elements cannot take the shape of a parameter of " +
+                                 std::to_string(parameter.numel()));
+    return part_of(part, part.storage_offset(), parameter.sizes());
+}
 // a dual tensor of forward-mode differentiation: no operator here has a forward derivative, and only the autograd function says so
 inline bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
 inline cudaStream_t stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }

@@ -545,3 +545,28 @@ def test_stages_launched_behind_one_another_equal_stages_waited_for(B, T, H, len
     for i, grads in enumerate(queued):
         for n, a, b in zip(names, alone[i % 4], grads):
             assert torch.equal(a, b), (i, n)
+
+
+@pytest.mark.parametrize("A_shape,bias_shape,fits", [((3,), (3 * 128,), True), ((1, 1, 3, 1), (3, 128), True), ((6,), (3 * 128,), False),
+                                                     ((3,), (6 * 128,), False), ((3,), (3 * 128 + 3,), False)])
+def test_gradients_of_the_gate_parameters_have_their_shapes(A_shape, bias_shape, fits):
+    """A parameter of another size than the gradient is refused in the backward pass: its gradient may not reach past what was summed."""
+    from cula_b200.kda import chunk_kda
+    from cula_b200.kda.chunk import chunk_kda_bwd
+    from cula_b200.synthetic import make_inputs_on_device
+    d = make_inputs_on_device(1, 70, 3, torch.device("cuda"), seed=1, gate_offset=-4.0)
+    A_log, dt_bias = torch.zeros(A_shape, device="cuda", requires_grad=True), torch.zeros(bias_shape, device="cuda", requires_grad=True)
+    o, _ = chunk_kda(d["q"], d["k"], d["v"], d["g"], d["beta"], use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, safe_gate=True,
+                     lower_bound=-5.0, A_log=A_log, dt_bias=dt_bias)
+    if not fits:
+        with pytest.raises(RuntimeError, match="shape"):
+            torch.autograd.grad(o, [A_log, dt_bias], d["v"])
+        return
+    grads = torch.autograd.grad(o, [A_log, dt_bias], d["v"])
+    assert [g.shape for g in grads] == [A_log.shape, dt_bias.shape]
+    # the orchestration without autograd returns them flat, whatever the shapes of the parameters
+    r = chunk_kda_bwd(d["q"], d["k"], d["v"], d["g"], d["beta"], 128 ** -0.5, None, d["v"], None, None, None, True, True, True, -5.0,
+                      A_log.detach(), dt_bias.detach())
+    assert r[5].shape == (3,) and r[6].shape == (3 * 128,)
+    for a, b in zip(grads, r[5:7]):
+        assert err_ratio(a.flatten().cpu(), b.cpu()) < 1e-5          # summed by atomics, in another order
