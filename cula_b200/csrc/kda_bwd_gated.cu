@@ -1005,8 +1005,9 @@ extern "C" int kda_launch_bwd_gated(const kda::BwdGatedParams* p, int num_chunks
     if (e != cudaSuccess) return (int)e;
     const int sms = sm_count();
     const int tiles = num_chunks * p->H;
-    // (fixed-length: whole chunks lie inside B T = num_chunks / ceil(T / 64) T rows, of which num_chunks 64 is an upper bound too)
-    const long long rows = (long long)num_chunks * BT;
+    // whole chunks lie inside the tensors. Their length is not known for a packed batch, whose chunks may also be those of some sequences
+    // only, anywhere in it; for a fixed-length one num_chunks 64 is an upper bound
+    const long long rows = p->cu_seqlens ? 1ll << 30 : (long long)num_chunks * BT;
     BgMaps maps{};
     const bool g_rows = kind != BG_PER_HEAD, g32 = kind == BG_FP32;
     if (!make_rows_map(&maps.q, const_cast<void*>(p->q), p->H, rows) || !make_rows_map(&maps.k, const_cast<void*>(p->k), p->H, rows) ||

@@ -570,3 +570,44 @@ def test_gradients_of_the_gate_parameters_have_their_shapes(A_shape, bias_shape,
     assert r[5].shape == (3,) and r[6].shape == (3 * 128,)
     for a, b in zip(grads, r[5:7]):
         assert err_ratio(a.flatten().cpu(), b.cpu()) < 1e-5          # summed by atomics, in another order
+
+
+def gated_stage(tokens, H, cu, ci, num_chunks, first_chunk=0, g_dtype=torch.bfloat16, entry="cula_kda_bwd_gated_checked", extra=()):
+    """The gated stage alone, through the C ABI, on random records of the dense stage: (return code, status, gradients by name)."""
+    from cula_b200 import _native
+    lib = _native.lib()
+    gen = torch.Generator(device="cuda").manual_seed(tokens + H)
+    rn = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    tiles, p = ci.shape[0] * H, lambda t: t.data_ptr()  # noqa: E731
+    q, k = (F.normalize(rn(tokens, H, 128), dim=-1).bfloat16() for _ in range(2))
+    g, beta = (-0.1 * rn(tokens, H, 128).abs()).to(g_dtype), torch.rand(tokens, H, generator=gen, device="cuda")
+    akk, mkk = torch.tril(0.2 * rn(tiles, 64, 64)), torch.tril(0.2 * rn(tiles, 64, 64))
+    scratch, work = 0.1 * rn(tiles, lib.cula_kda_bwd_scratch_floats()), torch.tensor([4.0, 0.25], device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = dict(dq=torch.zeros_like(q), dk=torch.zeros_like(k), dg=torch.zeros_like(g), dbeta=torch.zeros_like(beta))
+    at = first_chunk * H
+    rc = getattr(lib, entry)(p(q), p(k), p(g), int(g_dtype == torch.float32), p(beta), 1, None, None, p(akk[at:]), p(mkk[at:]), p(scratch[at:]), p(work),
+                             *(p(t) for t in out.values()), None, None, p(cu), p(ci[first_chunk:]), num_chunks, tokens, H, 128 ** -0.5, 0, 0, 0.0,
+                             *(() if entry == "cula_kda_bwd_gated" else (p(status),)), *extra, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    return rc, int(status.item()), out
+
+
+def packed_tables(lens):
+    cu = torch.tensor([0, *np.cumsum(lens)], dtype=torch.int32, device="cuda")
+    ci = torch.tensor([(n, c) for n, length in enumerate(lens) for c in range((length + 63) // 64)], dtype=torch.int32, device="cuda")
+    return cu, ci
+
+
+@pytest.mark.parametrize("g_dtype", [torch.bfloat16, torch.float32])
+def test_gated_stage_on_the_chunks_of_some_sequences_of_a_packed_batch(g_dtype):
+    """chunk_indices may name the chunks of the last sequences only: their rows lie far behind the first num_chunks * 64 of the batch."""
+    lens, H = [640, 130, 64, 100, 128], 3
+    cu, ci = packed_tables(lens)
+    rc, status, whole = gated_stage(sum(lens), H, cu, ci, ci.shape[0], g_dtype=g_dtype)
+    assert rc == 0 and status == 0
+    first = int((ci[:, 0] < 1).sum())
+    rc, status, part = gated_stage(sum(lens), H, cu, ci, ci.shape[0] - first, first, g_dtype)
+    assert rc == 0 and status == 0
+    for n, a in whole.items():
+        assert bool(a.any()) and torch.equal(a[lens[0]:], part[n][lens[0]:]) and not part[n][:lens[0]].any(), n
