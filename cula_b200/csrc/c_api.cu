@@ -310,12 +310,11 @@ extern "C" int cula_kda_bwd_dense(const float* d_h32, const float* d_ds, const v
     return kda_launch_bwd_dense(&p, num_chunks, static_cast<cudaStream_t>(stream));
 }
 
-extern "C" int cula_kda_bwd_gated_checked(const void* d_q, const void* d_k, const void* d_g, int g_is_fp32, const void* d_beta,
-                                          int beta_is_fp32, const float* d_A_log, const float* d_dt_bias, const float* d_akk,
-                                          const float* d_mkk, const float* d_scratch, const float* d_gscale, void* d_dq, void* d_dk,
-                                          void* d_dg, void* d_dbeta, float* d_dA_log, float* d_ddt_bias, const int* d_cu_seqlens,
-                                          const int* d_chunk_indices, int num_chunks, int T, int H, float scale, int use_qk_l2norm,
-                                          int gate_mode, float lower_bound, int* d_status, void* stream) {
+static int bwd_gated(const void* d_q, const void* d_k, const void* d_g, int g_is_fp32, const void* d_beta, int beta_is_fp32, const float* d_A_log,
+                     const float* d_dt_bias, const float* d_akk, const float* d_mkk, const float* d_scratch, const float* d_gscale, void* d_dq,
+                     void* d_dk, void* d_dg, void* d_dbeta, float* d_dA_log, float* d_ddt_bias, const int* d_cu_seqlens, const int* d_chunk_indices,
+                     int num_chunks, int T, int H, float scale, int use_qk_l2norm, int gate_mode, float lower_bound, int* d_status, int max_polls,
+                     void* stream) {
     if (num_chunks == 0) return 0;
     if (!d_q || !d_k || !d_g || !d_beta || !d_akk || !d_mkk || !d_scratch || !d_gscale || !d_dq || !d_dk || !d_dg ||
         !d_dbeta || num_chunks < 0 || H <= 0)
@@ -336,7 +335,32 @@ extern "C" int cula_kda_bwd_gated_checked(const void* d_q, const void* d_k, cons
     p.beta_fp32 = beta_is_fp32 & CULA_KDA_BETA_FP32; p.beta_logit = (beta_is_fp32 & CULA_KDA_BETA_LOGIT) != 0;
     p.use_l2norm = use_qk_l2norm; p.gate_mode = gate_mode; p.lower_bound = lower_bound; p.scale = scale;
     p.status = d_status;
+    p.max_polls = max_polls;
     return kda_launch_bwd_gated(&p, num_chunks, static_cast<cudaStream_t>(stream));
+}
+
+static constexpr int GATED_POLLS = 1 << 16;      // about a second
+
+extern "C" int cula_kda_bwd_gated_checked(const void* d_q, const void* d_k, const void* d_g, int g_is_fp32, const void* d_beta,
+                                          int beta_is_fp32, const float* d_A_log, const float* d_dt_bias, const float* d_akk,
+                                          const float* d_mkk, const float* d_scratch, const float* d_gscale, void* d_dq, void* d_dk,
+                                          void* d_dg, void* d_dbeta, float* d_dA_log, float* d_ddt_bias, const int* d_cu_seqlens,
+                                          const int* d_chunk_indices, int num_chunks, int T, int H, float scale, int use_qk_l2norm,
+                                          int gate_mode, float lower_bound, int* d_status, void* stream) {
+    return bwd_gated(d_q, d_k, d_g, g_is_fp32, d_beta, beta_is_fp32, d_A_log, d_dt_bias, d_akk, d_mkk, d_scratch, d_gscale, d_dq, d_dk, d_dg, d_dbeta,
+                     d_dA_log, d_ddt_bias, d_cu_seqlens, d_chunk_indices, num_chunks, T, H, scale, use_qk_l2norm, gate_mode, lower_bound, d_status,
+                     GATED_POLLS, stream);
+}
+
+extern "C" int cula_kda_selftest_bwd_gated_wait(const void* d_q, const void* d_k, const void* d_g, int g_is_fp32, const void* d_beta,
+                                                int beta_is_fp32, const float* d_A_log, const float* d_dt_bias, const float* d_akk,
+                                                const float* d_mkk, const float* d_scratch, const float* d_gscale, void* d_dq, void* d_dk,
+                                                void* d_dg, void* d_dbeta, float* d_dA_log, float* d_ddt_bias, const int* d_cu_seqlens,
+                                                const int* d_chunk_indices, int num_chunks, int T, int H, float scale, int use_qk_l2norm,
+                                                int gate_mode, float lower_bound, int* d_status, void* stream) {
+    return bwd_gated(d_q, d_k, d_g, g_is_fp32, d_beta, beta_is_fp32, d_A_log, d_dt_bias, d_akk, d_mkk, d_scratch, d_gscale, d_dq, d_dk, d_dg, d_dbeta,
+                     d_dA_log, d_ddt_bias, d_cu_seqlens, d_chunk_indices, num_chunks, T, H, scale, use_qk_l2norm, gate_mode, lower_bound, d_status,
+                     0, stream);
 }
 
 extern "C" int cula_kda_bwd_gated(const void* d_q, const void* d_k, const void* d_g, int g_is_fp32, const void* d_beta,
@@ -345,9 +369,9 @@ extern "C" int cula_kda_bwd_gated(const void* d_q, const void* d_k, const void* 
                                   void* d_dg, void* d_dbeta, float* d_dA_log, float* d_ddt_bias, const int* d_cu_seqlens,
                                   const int* d_chunk_indices, int num_chunks, int T, int H, float scale, int use_qk_l2norm,
                                   int gate_mode, float lower_bound, void* stream) {
-    return cula_kda_bwd_gated_checked(d_q, d_k, d_g, g_is_fp32, d_beta, beta_is_fp32, d_A_log, d_dt_bias, d_akk, d_mkk, d_scratch, d_gscale,
-                                      d_dq, d_dk, d_dg, d_dbeta, d_dA_log, d_ddt_bias, d_cu_seqlens, d_chunk_indices, num_chunks, T, H, scale,
-                                      use_qk_l2norm, gate_mode, lower_bound, nullptr, stream);
+    return bwd_gated(d_q, d_k, d_g, g_is_fp32, d_beta, beta_is_fp32, d_A_log, d_dt_bias, d_akk, d_mkk, d_scratch, d_gscale, d_dq, d_dk, d_dg, d_dbeta,
+                     d_dA_log, d_ddt_bias, d_cu_seqlens, d_chunk_indices, num_chunks, T, H, scale, use_qk_l2norm, gate_mode, lower_bound, nullptr,
+                     GATED_POLLS, stream);
 }
 
 extern "C" int kda_launch_gate(const kda::GateArgs* a, int backward, cudaStream_t stream);

@@ -199,10 +199,10 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
     const uint32_t tl = tmem + ((uint32_t)(32 * qd) << 16);
 
     uint32_t par = 0;
-    // bounded wait; on expiry the CTA leaves at the next tile
+    // bounded wait; on expiry the CTA leaves at the next tile, in any case before a barrier whose phase did not end is used again
     auto wait_bar = [&](int which) {
-        bool ok = mbar_test(&bars[which], par);
-        for (int i = 0; !ok && i < (1 << 16) && !*sAbort; ++i) ok = mbar_test(&bars[which], par);
+        bool ok = false;
+        for (int i = 0; !ok && i < p.max_polls && (i == 0 || !*sAbort); ++i) ok = mbar_test(&bars[which], par);
         if (!ok) {
             if (p.status) report_status(p.status, STATUS_WAIT_TIMEOUT);
             *sAbort = 1;
@@ -308,9 +308,9 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
     };
 
     const float alpha = p.gate_mode != GATE_NONE ? __expf(alpha_log) : 0.f, bias = bias_next;
-    if (tid == 0) *sLeave = *sAbort;
     wait_bar(8);              // the token rows have landed
     wait_bar(10);             // A, dPs, dW
+    if (tid == 0) *sLeave = *sAbort;
     BG_MARK(0);
     // ---- 1. norms, gates and their sums inside a block, coefficient matrices in both orientations ----
     {
@@ -966,6 +966,11 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
     info = ninfo;
     }  // tile loop: what the next tile writes before its first barrier is read by nobody any more
     bulk_wait_all();
+    __syncthreads();
+    if (tid == 0 && *sAbort) {      // products and copies in flight end before the shared and tensor memory go away (waits bounded again)
+        const uint32_t last = par ^ 1u;        // of the last tile that was worked on; left at a tile, its inputs had been asked for
+        for (int i = 0; i < 11; ++i) mbar_wait(&bars[i], tile < num_tiles && (i == 8 || i == 10) ? par : last, 1 << 13);
+    }
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) umma::tmem_dealloc(tmem, 512);

@@ -1011,7 +1011,10 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
     }
     PHASE_MARK(11);     // W/U epilogue
     }  // tile loop
-    if (tid == MMA_THREAD) bulk_wait_all();        // staged outputs must be on their way before the shared memory goes away
+    if (tid == MMA_THREAD) {
+        if (*sAbort) mbar_wait(&bars[2], qk_parity ^ 1);      // q and k rows in flight (bounded again)
+        bulk_wait_all();                           // staged outputs must be on their way before the shared memory goes away
+    }
     __syncthreads();
     if (warp == 0) umma::tmem_dealloc(tmem, 256);
     pdl_wait();      // an overlapping launch: what follows in the stream counts on the kernel before this one as well

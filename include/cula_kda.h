@@ -315,6 +315,15 @@ int cula_kda_rms_norm_gated_bwd(const void* d_x, const void* d_g, const float* d
  */
 int cula_kda_selftest_bounded_wait(int* d_status, int max_polls, void* stream);
 
+/* The gated backward stage (arguments of cula_kda_bwd_gated_checked) with waits that give up at once, as they do after about a second
+ * where a copy or a product hangs: *d_status is set to 1, each CTA lets its copies land, frees its tensor memory and returns. */
+int cula_kda_selftest_bwd_gated_wait(const void* d_q, const void* d_k, const void* d_g, int g_is_fp32,
+                                     const void* d_beta, int beta_is_fp32, const float* d_A_log, const float* d_dt_bias,
+                                     const float* d_akk, const float* d_mkk, const float* d_scratch, const float* d_gscale,
+                                     void* d_dq, void* d_dk, void* d_dg, void* d_dbeta, float* d_dA_log, float* d_ddt_bias,
+                                     const int* d_cu_seqlens, const int* d_chunk_indices, int num_chunks, int T, int H,
+                                     float scale, int use_qk_l2norm, int gate_mode, float lower_bound, int* d_status, void* stream);
+
 /* Human-readable text for a return value of the functions above. */
 const char* cula_kda_strerror(int code);
 

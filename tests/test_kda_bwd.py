@@ -611,3 +611,17 @@ def test_gated_stage_on_the_chunks_of_some_sequences_of_a_packed_batch(g_dtype):
     assert rc == 0 and status == 0
     for n, a in whole.items():
         assert bool(a.any()) and torch.equal(a[lens[0]:], part[n][lens[0]:]) and not part[n][:lens[0]].any(), n
+
+
+@pytest.mark.parametrize("lens,H", [([64], 1), ([64 * 70, 33], 5), ([40, 17], 2)])
+@pytest.mark.parametrize("g_dtype", [torch.bfloat16, torch.float32])
+def test_gated_stage_leaves_when_a_wait_gives_up(lens, H, g_dtype):
+    """Waits that give up at once: the stage reports, lets the copies that it has asked for land and returns (chunks whole, ragged, and
+    more than SMs); the call behind it is as it was."""
+    cu, ci = packed_tables(lens)
+    rc, status, before = gated_stage(sum(lens), H, cu, ci, ci.shape[0], g_dtype=g_dtype)
+    assert rc == 0 and status == 0
+    rc, status, _ = gated_stage(sum(lens), H, cu, ci, ci.shape[0], g_dtype=g_dtype, entry="cula_kda_selftest_bwd_gated_wait")
+    assert rc == 0 and status == 1
+    rc, status, after = gated_stage(sum(lens), H, cu, ci, ci.shape[0], g_dtype=g_dtype)
+    assert rc == 0 and status == 0 and all(torch.equal(before[n], after[n]) for n in before)
