@@ -154,8 +154,40 @@ struct BgMaps {
     CUtensorMap a, m, dw, ps;             // Akk, M [tiles][64][64], dW [tiles][64][128], dPs and dAu [tiles][2 x 64][64]: 32 x 32 of fp32 at a time, 128-byte swizzle
 };
 
+// A wait gave up: what this CTA has not computed, or has computed from what had not arrived, must not pass for a gradient, with or
+// without a status word. All its tiles get NaN. (A function of its own, and the parameters by address: inlined it costs the tile loop spills.)
 template <int GK>
-__global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdGatedParams p, const int num_tiles, const __grid_constant__ BgMaps maps) {
+__device__ __noinline__ void bg_spoil(const BwdGatedParams& p, int num_tiles) {
+    const int tid = threadIdx.x;
+    const float nan = __int_as_float(0x7fffffff);
+    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+        const int c = t / p.H, h = t - c * p.H;
+        const ChunkInfo ci = chunk_info(c, p.cu_seqlens, p.chunk_indices, p.T);
+        for (int i = tid; i < ci.valid * DK; i += BG_THREADS) {
+            const size_t at = ((size_t)(ci.row0 + i / DK) * p.H + h) * DK + i % DK;
+            reinterpret_cast<__nv_bfloat16*>(p.dq)[at] = __float2bfloat16_rn(nan);
+            reinterpret_cast<__nv_bfloat16*>(p.dk)[at] = __float2bfloat16_rn(nan);
+            if (GK == BG_FP32) reinterpret_cast<float*>(p.dg)[at] = nan;
+            if (GK == BG_BF16) reinterpret_cast<__nv_bfloat16*>(p.dg)[at] = __float2bfloat16_rn(nan);
+        }
+        if (tid < ci.valid) {
+            const size_t at = (size_t)(ci.row0 + tid) * p.H + h;
+            if (p.beta_fp32) reinterpret_cast<float*>(p.dbeta)[at] = nan;
+            else reinterpret_cast<__nv_bfloat16*>(p.dbeta)[at] = __float2bfloat16_rn(nan);
+            if (GK == BG_PER_HEAD) {
+                if (p.g_fp32) reinterpret_cast<float*>(p.dg)[at] = nan;
+                else reinterpret_cast<__nv_bfloat16*>(p.dg)[at] = __float2bfloat16_rn(nan);
+            }
+        }
+        if (p.gate_mode != GATE_NONE && tid < DK) {
+            if (p.ddt_bias) atomicAdd(&p.ddt_bias[h * DK + tid], nan);
+            if (p.dA_log && tid == 0) atomicAdd(&p.dA_log[h], nan);
+        }
+    }
+}
+
+template <int GK>
+__global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const __grid_constant__ BwdGatedParams p, const int num_tiles, const __grid_constant__ BgMaps maps) {
     constexpr int NT = BG_NT, N2 = NT / 2;
     extern __shared__ unsigned char bg_smem_raw[];
     unsigned char* sm = bg_smem_raw + ((1024u - (smem_u32(bg_smem_raw) & 1023u)) & 1023u);
@@ -974,6 +1006,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const BwdG
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) umma::tmem_dealloc(tmem, 512);
+    if (*sAbort) bg_spoil<GK>(p, num_tiles);
 }
 
 }  // namespace kda

@@ -185,7 +185,8 @@ int cula_kda_bwd_gated(const void* d_q, const void* d_k, const void* d_g, int g_
                        const int* d_cu_seqlens, const int* d_chunk_indices, int num_chunks, int T, int H,
                        float scale, int use_qk_l2norm, int gate_mode, float lower_bound, void* stream);
 
-/* The same with the device status word of its bounded waits (cula_kda_bwd_gated reports nowhere). */
+/* The same with the device status word of its bounded waits. With either entry the gradients of the chunks of a CTA whose wait gave up
+ * (and d_dA_log, d_ddt_bias of their heads) are NaN; cula_kda_bwd_gated has no other way to say so. */
 int cula_kda_bwd_gated_checked(const void* d_q, const void* d_k, const void* d_g, int g_is_fp32,
                                const void* d_beta, int beta_is_fp32, const float* d_A_log, const float* d_dt_bias,
                                const float* d_akk, const float* d_mkk, const float* d_scratch, const float* d_gscale,
@@ -316,7 +317,8 @@ int cula_kda_rms_norm_gated_bwd(const void* d_x, const void* d_g, const float* d
 int cula_kda_selftest_bounded_wait(int* d_status, int max_polls, void* stream);
 
 /* The gated backward stage (arguments of cula_kda_bwd_gated_checked) with waits that give up at once, as they do after about a second
- * where a copy or a product hangs: *d_status is set to 1, each CTA lets its copies land, frees its tensor memory and returns. */
+ * where a copy or a product hangs: *d_status is set to 1, each CTA lets its copies land, frees its tensor memory, fills its gradients
+ * with NaN and returns. */
 int cula_kda_selftest_bwd_gated_wait(const void* d_q, const void* d_k, const void* d_g, int g_is_fp32,
                                      const void* d_beta, int beta_is_fp32, const float* d_A_log, const float* d_dt_bias,
                                      const float* d_akk, const float* d_mkk, const float* d_scratch, const float* d_gscale,

@@ -621,7 +621,8 @@ def test_gated_stage_leaves_when_a_wait_gives_up(lens, H, g_dtype):
     cu, ci = packed_tables(lens)
     rc, status, before = gated_stage(sum(lens), H, cu, ci, ci.shape[0], g_dtype=g_dtype)
     assert rc == 0 and status == 0
-    rc, status, _ = gated_stage(sum(lens), H, cu, ci, ci.shape[0], g_dtype=g_dtype, entry="cula_kda_selftest_bwd_gated_wait")
+    rc, status, left = gated_stage(sum(lens), H, cu, ci, ci.shape[0], g_dtype=g_dtype, entry="cula_kda_selftest_bwd_gated_wait")
     assert rc == 0 and status == 1
+    assert all(bool(t.isnan().all()) for t in left.values())          # nothing that could pass for a gradient, status word or not
     rc, status, after = gated_stage(sum(lens), H, cu, ci, ci.shape[0], g_dtype=g_dtype)
     assert rc == 0 and status == 0 and all(torch.equal(before[n], after[n]) for n in before)
