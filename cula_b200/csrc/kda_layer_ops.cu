@@ -72,7 +72,9 @@ template <int W, bool BWD, int V, int UNIT>
 __global__ void __launch_bounds__(LO_THREADS) kda_short_conv_kernel(const ConvArgs a, const int num_chunks) {
     constexpr int CH = 2 * V, GROUP = 32 * CH;               // channels of a lane, of a warp
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ch = GROUP * blockIdx.x + CH * lane, unit = CONV_WARPS * blockIdx.y + warp, c = unit / (BT / UNIT);
+    // one grid dimension for both: only the first takes more than 65535 blocks, and there may be more chunks than that
+    const int groups = (a.D + GROUP - 1) / GROUP, group = blockIdx.x % groups;
+    const int ch = GROUP * group + CH * lane, unit = CONV_WARPS * (blockIdx.x / groups) + warp, c = unit / (BT / UNIT);
     bool live = ch < a.D && c < num_chunks;
     pdl_launch_dependents();
     pdl_wait();
@@ -241,7 +243,7 @@ __global__ void __launch_bounds__(LO_THREADS) kda_short_conv_kernel(const ConvAr
     }
     if constexpr (BWD) {
         __syncthreads();
-        const int cl = threadIdx.x, cg = GROUP * blockIdx.x + cl;
+        const int cl = threadIdx.x, cg = GROUP * group + cl;
         if (cl < GROUP && cg < a.D) {
             float v[W + 1];
 #pragma unroll
@@ -395,7 +397,7 @@ extern "C" int kda_launch_short_conv(const kda::ConvArgs* a, int num_chunks, int
     const int groups = (a->D + (wide ? 127 : 63)) / (wide ? 128 : 64);
     const bool halves = wide || (long long)num_chunks * groups < 16LL * sm_count();
     const int units = num_chunks * (halves ? 2 : 1);
-    const dim3 grid(groups, (units + CONV_WARPS - 1) / CONV_WARPS);
+    const dim3 grid((unsigned)groups * ((units + CONV_WARPS - 1) / CONV_WARPS));
     void (*kernel)(const ConvArgs, const int) = nullptr;
 #define KDA_CONV_KERNEL(W)                                                                                          \
     kernel = wide ? kda_short_conv_kernel<W, true, 2, 32> : halves ? kda_short_conv_kernel<W, false, 1, 32> : kda_short_conv_kernel<W, false, 1, 64>

@@ -161,3 +161,29 @@ def test_rms_norm_gated_row_remainders(R, D):
     assert err_ratio(y_ref.detach(), y.detach().float().cpu()) < 4e-3
     for r, d, tol in zip(ref, dev, (4e-3, 4e-3, 1e-2)):
         assert err_ratio(r.grad, d.grad.float().cpu()) < tol
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens", [None, 1])
+def test_short_conv_over_more_chunks_than_a_grid_dimension_takes(lens):
+    """270,000 chunks, of one long sequence or of as many sequences of one token, forward and backward (no activation: both are
+    weighted sums of shifted rows, exact but for the rounding of the results)."""
+    from cula_b200.kda import short_conv
+    n, gen = 270_000, torch.Generator(device="cuda").manual_seed(0)
+    T = 64 * n if lens is None else n
+    x = torch.randn(1, T, 8, device="cuda", generator=gen).to(torch.bfloat16).requires_grad_(True)
+    w = torch.randn(8, 2, device="cuda", generator=gen).requires_grad_(True)
+    dy = torch.randn(1, T, 8, device="cuda", generator=gen).to(torch.bfloat16)
+    cu = None if lens is None else torch.arange(n + 1, dtype=torch.int32)
+    y, _ = short_conv(x, w, activation=None, cu_seqlens=None if cu is None else cu.cuda(), cu_seqlens_cpu=cu)
+    dx, dw = torch.autograd.grad(y, [x, w], dy)
+    far = 0.0 if cu is not None else 1.0                      # a sequence of one token has no neighbours
+    xf, dyf, w0, w1 = x.detach().float(), dy.float(), w.detach()[:, 0], w.detach()[:, 1]
+    y_ref = w1 * xf + far * w0 * F.pad(xf, (0, 0, 1, 0))[:, :T]
+    dx_ref = w1 * dyf + far * w0 * F.pad(dyf, (0, 0, 0, 1))[:, 1:]
+    dw_ref = torch.stack([far * (F.pad(xf, (0, 0, 1, 0))[:, :T].double() * dyf).sum((0, 1)), (xf.double() * dyf).sum((0, 1))], -1)
+    assert err_ratio(y_ref, y.detach()) < 4e-3 and err_ratio(dx_ref, dx) < 4e-3
+    # sums of T products of size 1 in fp32, by one atomic per four half chunks or sequences: as many roundings of up to 2^-24 of a sum that
+    # walks to a few sqrt(T), which add up like their square root (8: a few times that walk, and four sigma)
+    adds = T / 128 if cu is None else T / 4
+    assert float((dw_ref - dw).abs().max()) < 8 * T ** 0.5 * adds ** 0.5 * 2.0 ** -24
