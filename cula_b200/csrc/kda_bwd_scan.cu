@@ -479,7 +479,5 @@ extern "C" int kda_launch_bwd_scan(const kda::BwdScanParams* p, cudaStream_t str
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p->beside_forward ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, kda_bwd_scan_kernel, *p, map, map_do);
-    if (e != cudaSuccess) return (int)e;
-    return (int)cudaGetLastError();
+    return (int)launched(cudaLaunchKernelEx(&cfg, kda_bwd_scan_kernel, *p, map, map_do));
 }

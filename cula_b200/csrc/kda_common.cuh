@@ -268,6 +268,12 @@ inline int sm_count() {
     }
     return sms;
 }
+// The result of a launch. One that was refused also leaves its error for whoever asks next (torch after its own next kernel): it is
+// taken along here, since the caller gets it as the return value.
+inline cudaError_t launched(cudaError_t e) {
+    const cudaError_t left = cudaGetLastError();
+    return e != cudaSuccess ? e : left;
+}
 // A launch that may be scheduled while the kernel before it in the stream drains; the kernel calls pdl_launch_dependents() and, before it
 // touches memory, pdl_wait().
 template <typename... P, typename... A>
@@ -282,7 +288,7 @@ inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, in
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    return launched(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 // raise the dynamic shared memory limit of one kernel (a function-local static `done` per kernel holds the devices it was
 // raised on)

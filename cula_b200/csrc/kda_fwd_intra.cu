@@ -1063,7 +1063,5 @@ extern "C" int kda_launch_fwd_intra(const kda::IntraParams* p, int num_chunks, c
     IntraMaps maps;
     if (!make_half_rows_map(&maps.q, p->q, p->H) || !make_half_rows_map(&maps.k, p->k, p->H) || !make_half_rows_map(&maps.v, p->v, p->H))
         return (int)cudaErrorInvalidValue;
-    e = cudaLaunchKernelEx(&cfg, kernel, q, maps);
-    if (e != cudaSuccess) return (int)e;
-    return (int)cudaGetLastError();
+    return (int)launched(cudaLaunchKernelEx(&cfg, kernel, q, maps));
 }

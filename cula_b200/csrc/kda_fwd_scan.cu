@@ -435,9 +435,7 @@ int launch_scan(const kda::ScanParams* p, int groups, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, kda_fwd_scan_kernel, *p, map, map_o);
-    if (e != cudaSuccess) return (int)e;
-    return (int)cudaGetLastError();
+    return (int)launched(cudaLaunchKernelEx(&cfg, kda_fwd_scan_kernel, *p, map, map_o));
 }
 }  // namespace
 

@@ -396,8 +396,8 @@ extern "C" int kda_launch_short_conv(const kda::ConvArgs* a, int num_chunks, int
     const bool wide = backward;
     const int groups = (a->D + (wide ? 127 : 63)) / (wide ? 128 : 64);
     const bool halves = wide || (long long)num_chunks * groups < 16LL * sm_count();
-    const int units = num_chunks * (halves ? 2 : 1);
-    const dim3 grid((unsigned)groups * ((units + CONV_WARPS - 1) / CONV_WARPS));
+    const long long units = num_chunks * (halves ? 2LL : 1LL), blocks = groups * ((units + CONV_WARPS - 1) / CONV_WARPS);
+    const dim3 grid((unsigned)(blocks < 0xffffffffLL ? blocks : 0xffffffffLL));      // (the launch refuses what is too many)
     void (*kernel)(const ConvArgs, const int) = nullptr;
 #define KDA_CONV_KERNEL(W)                                                                                          \
     kernel = wide ? kda_short_conv_kernel<W, true, 2, 32> : halves ? kda_short_conv_kernel<W, false, 1, 32> : kda_short_conv_kernel<W, false, 1, 64>

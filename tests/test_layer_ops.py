@@ -187,3 +187,15 @@ def test_short_conv_over_more_chunks_than_a_grid_dimension_takes(lens):
     # walks to a few sqrt(T), which add up like their square root (8: a few times that walk, and four sigma)
     adds = T / 128 if cu is None else T / 4
     assert float((dw_ref - dw).abs().max()) < 8 * T ** 0.5 * adds ** 0.5 * 2.0 ** -24
+
+
+@pytest.mark.gpu
+def test_a_refused_launch_leaves_no_error_behind():
+    """More blocks than a grid takes: the call returns the error, nothing runs, and the next kernel of torch does not raise it again."""
+    from cula_b200 import _native
+    lib, stream = _native.lib(), torch.cuda.current_stream().cuda_stream
+    x, y, w = torch.zeros(64, 4096, dtype=torch.bfloat16, device="cuda"), torch.zeros(64, 4096, dtype=torch.bfloat16, device="cuda"), torch.zeros(4096, 4, device="cuda")
+    torch.cuda.synchronize()
+    p = lambda t: t.data_ptr()  # noqa: E731
+    assert lib.cula_kda_short_conv_fwd(p(x), p(w), None, None, p(y), None, None, None, 2 ** 31 - 1, 64, 4096, 4, 0, stream) > 0
+    assert torch.equal(x + 1, torch.ones_like(x))
