@@ -485,11 +485,12 @@ def test_a_sequence_does_not_read_its_neighbour(first, g_dtype):
         if poison:
             up[:, first:] = 0
         results.append([o, *torch.autograd.grad(o, leaves, up)])
-    torch.cuda.synchronize()
-    try:
-        check_status()           # NaN values of the neighbour may be reported
-    except RuntimeError:
-        pass
+        torch.cuda.synchronize()
+        try:
+            check_status()
+        except RuntimeError as e:           # NaN values of the neighbour may be reported as out of range, and nothing else
+            if not (poison and "fp16 range" in str(e)):
+                raise
     for n, a, b in zip(("o", *names), *results):
         assert torch.isfinite(b[:, :first].float()).all(), n
         assert err_ratio(a.detach().float().cpu(), b[:, :first].detach().float().cpu()) <= 1e-6, n

@@ -94,12 +94,12 @@ def test_rms_norm_gated_matches_oracle(D, act):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("D,W,tail", [(8, 1, 0), (72, 4, 5), (200, 3, 0), (64, 2, 1)])
+@pytest.mark.parametrize("D,W,tail", [(8, 1, 0), (72, 4, 5), (200, 3, 0), (64, 2, 1), (200, 4, 0)])
 def test_short_conv_at_chunk_and_channel_edges(D, W, tail):
-    """Channel counts that leave part of a warp idle, sequences that end on and around a batch of tokens and a chunk, rows
-    past the last packed token (zero, with zero gradient)."""
+    """Channel counts that leave part of a warp idle, sequences that end on and around a batch of tokens, half a chunk (an empty second
+    half, one shorter than the window) and a chunk, rows past the last packed token (zero, with zero gradient)."""
     from cula_b200.kda import short_conv
-    lens = [1, 2, 3, 4, 5, 7, 8, 9, 61, 63, 64, 65, 67, 128]
+    lens = [1, 2, 3, 4, 5, 7, 8, 9, 31, 32, 33, 34, 35, 61, 63, 64, 65, 67, 95, 96, 97, 98, 99, 128]
     cu = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32)
     T, gen = int(cu[-1]), torch.Generator().manual_seed(4)
     x, dy = (torch.randn(1, T + tail, D, generator=gen).to(torch.bfloat16) for _ in range(2))
@@ -199,3 +199,74 @@ def test_a_refused_launch_leaves_no_error_behind():
     p = lambda t: t.data_ptr()  # noqa: E731
     assert lib.cula_kda_short_conv_fwd(p(x), p(w), None, None, p(y), None, None, None, 2 ** 31 - 1, 64, 4096, 4, 0, stream) > 0
     assert torch.equal(x + 1, torch.ones_like(x))
+
+
+def layer_chain(T, H, seed):
+    """Leaves on the device and a function of them: every layer operator, forward and backward, as (results, gradients) in launch order."""
+    from cula_b200.kda import fused_beta_sigmoid, fused_kda_gate, rms_norm_gated, short_conv
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    bf = lambda *s: rn(*s).to(torch.bfloat16)  # noqa: E731
+    leaves = [bf(1, T, H * 128), 0.3 * rn(H * 128, 4), 0.1 * rn(H * 128), bf(1, T, H, 128), bf(1, T, H), rn(H), rn(H * 128), bf(1, T, H, 128),
+              bf(1, T, H, 128), 1 + 0.1 * rn(128)]
+    leaves = [t.requires_grad_(True) for t in leaves]
+    up = [bf(1, T, H * 128), rn(1, T, H, 128), rn(1, T, H), bf(1, T, H, 128)]
+
+    def run():
+        x, w, b, g, beta, A_log, dt_bias, o, og, nw = leaves
+        outs = [short_conv(x, w, b)[0], fused_kda_gate(g, A_log, dt_bias, lower_bound=-5.0), fused_beta_sigmoid(beta), rms_norm_gated(o, og, nw)]
+        return outs, torch.autograd.grad(outs, leaves, up)
+
+    return leaves, up, run
+
+
+SUMMED = (1, 2, 5, 6, 9)          # gradients that atomics add up: the order of the additions is not fixed
+
+
+def same(a, b):
+    outs = all(torch.equal(x, y) for x, y in zip(a[0], b[0]))
+    return outs and all(err_ratio(x, y) < 1e-5 if i in SUMMED else torch.equal(x, y) for i, (x, y) in enumerate(zip(a[1], b[1])))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,H", [(1, 1), (100, 3), (2048, 8)])
+def test_layer_operators_launched_behind_one_another_equal_ones_waited_for(T, H):
+    """Each kernel is launched while the one before it drains: passes queued without a pause, in memory that the passes before have just
+    given back (results dropped at once), have the results of passes that start on an idle device."""
+    chains = [layer_chain(T, H, seed) for seed in range(3)]
+    alone = []
+    for _, _, run in chains:
+        torch.cuda.synchronize()
+        alone.append(run())
+    torch.cuda.synchronize()
+    for _ in range(3):
+        for _, _, run in chains:
+            run()
+    queued = [run() for _ in range(3) for _, _, run in chains]
+    torch.cuda.synchronize()
+    for i, r in enumerate(queued):
+        assert same(alone[i % 3], r), i
+
+
+@pytest.mark.gpu
+def test_layer_operators_are_capturable_in_a_cuda_graph():
+    """A pass of all of them, with its cleared buffers and early launches, replays on other values: equal to calls outside a graph."""
+    leaves, up, run = layer_chain(300, 3, 0)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(2):
+            run()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        replayed = run()
+    for seed in (1, 2):
+        other = layer_chain(300, 3, seed)
+        with torch.no_grad():
+            for dst, src in zip([*leaves, *up], [*other[0], *other[1]]):
+                dst.copy_(src)
+        for _ in range(2):               # twice: the sums start from zero each time
+            graph.replay()
+        torch.cuda.synchronize()
+        assert same(other[2](), replayed), seed
