@@ -690,7 +690,15 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
         if (nf.y > 0) {
             fetch_g(nf);
             load_scalars(nf);
-            if (tid == INFO_THREAD && nf.y == BT) {       // the next tile's token rows towards L2
+            // the next tile's token rows towards L2: boxes of a whole chunk, the real rows of a ragged one
+            if (nf.y < BT) {
+                const int row = tid >> 2, part = tid & 3;
+                if (row < nf.y) {
+                    const size_t off = (size_t)(nf.x + row) * tok_stride + (size_t)nf.z * DK + 64 * (part & 1);
+                    prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(part < 2 ? p.q : p.k) + off);
+                    if (part < 2) prefetch_l2(reinterpret_cast<const __nv_bfloat16*>(p.v) + off);
+                }
+            } else if (tid == INFO_THREAD) {
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     tma_prefetch_3d(&maps.q, 64 * half, nf.z, nf.x);
