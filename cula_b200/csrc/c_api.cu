@@ -12,7 +12,7 @@ extern "C" int kda_launch_grad_scale(const void* d_o, size_t n_do, const float* 
                                      float* gscale, cudaStream_t stream);
 extern "C" int kda_launch_bwd_scan(const kda::BwdScanParams* p, cudaStream_t stream);
 extern "C" int kda_launch_bwd_dense(const kda::BwdDenseParams* p, int num_chunks, cudaStream_t stream);
-extern "C" int kda_launch_bwd_gated(const kda::BwdGatedParams* p, int num_chunks, cudaStream_t stream);
+extern "C" int kda_launch_bwd_gated(const kda::BwdGatedParams* p, int num_chunks, int gives_up, cudaStream_t stream);
 
 namespace {
 inline bool misaligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) != 0; }
@@ -313,7 +313,7 @@ extern "C" int cula_kda_bwd_dense(const float* d_h32, const float* d_ds, const v
 static int bwd_gated(const void* d_q, const void* d_k, const void* d_g, int g_is_fp32, const void* d_beta, int beta_is_fp32, const float* d_A_log,
                      const float* d_dt_bias, const float* d_akk, const float* d_mkk, const float* d_scratch, const float* d_gscale, void* d_dq,
                      void* d_dk, void* d_dg, void* d_dbeta, float* d_dA_log, float* d_ddt_bias, const int* d_cu_seqlens, const int* d_chunk_indices,
-                     int num_chunks, int T, int H, float scale, int use_qk_l2norm, int gate_mode, float lower_bound, int* d_status, int max_polls,
+                     int num_chunks, int T, int H, float scale, int use_qk_l2norm, int gate_mode, float lower_bound, int* d_status, bool gives_up,
                      void* stream) {
     if (num_chunks == 0) return 0;
     if (!d_q || !d_k || !d_g || !d_beta || !d_akk || !d_mkk || !d_scratch || !d_gscale || !d_dq || !d_dk || !d_dg ||
@@ -335,11 +335,8 @@ static int bwd_gated(const void* d_q, const void* d_k, const void* d_g, int g_is
     p.beta_fp32 = beta_is_fp32 & CULA_KDA_BETA_FP32; p.beta_logit = (beta_is_fp32 & CULA_KDA_BETA_LOGIT) != 0;
     p.use_l2norm = use_qk_l2norm; p.gate_mode = gate_mode; p.lower_bound = lower_bound; p.scale = scale;
     p.status = d_status;
-    p.max_polls = max_polls;
-    return kda_launch_bwd_gated(&p, num_chunks, static_cast<cudaStream_t>(stream));
+    return kda_launch_bwd_gated(&p, num_chunks, gives_up, static_cast<cudaStream_t>(stream));
 }
-
-static constexpr int GATED_POLLS = 1 << 16;      // about a second
 
 extern "C" int cula_kda_bwd_gated_checked(const void* d_q, const void* d_k, const void* d_g, int g_is_fp32, const void* d_beta,
                                           int beta_is_fp32, const float* d_A_log, const float* d_dt_bias, const float* d_akk,
@@ -349,7 +346,7 @@ extern "C" int cula_kda_bwd_gated_checked(const void* d_q, const void* d_k, cons
                                           int gate_mode, float lower_bound, int* d_status, void* stream) {
     return bwd_gated(d_q, d_k, d_g, g_is_fp32, d_beta, beta_is_fp32, d_A_log, d_dt_bias, d_akk, d_mkk, d_scratch, d_gscale, d_dq, d_dk, d_dg, d_dbeta,
                      d_dA_log, d_ddt_bias, d_cu_seqlens, d_chunk_indices, num_chunks, T, H, scale, use_qk_l2norm, gate_mode, lower_bound, d_status,
-                     GATED_POLLS, stream);
+                     false, stream);
 }
 
 extern "C" int cula_kda_selftest_bwd_gated_wait(const void* d_q, const void* d_k, const void* d_g, int g_is_fp32, const void* d_beta,
@@ -360,7 +357,7 @@ extern "C" int cula_kda_selftest_bwd_gated_wait(const void* d_q, const void* d_k
                                                 int gate_mode, float lower_bound, int* d_status, void* stream) {
     return bwd_gated(d_q, d_k, d_g, g_is_fp32, d_beta, beta_is_fp32, d_A_log, d_dt_bias, d_akk, d_mkk, d_scratch, d_gscale, d_dq, d_dk, d_dg, d_dbeta,
                      d_dA_log, d_ddt_bias, d_cu_seqlens, d_chunk_indices, num_chunks, T, H, scale, use_qk_l2norm, gate_mode, lower_bound, d_status,
-                     0, stream);
+                     true, stream);
 }
 
 extern "C" int cula_kda_bwd_gated(const void* d_q, const void* d_k, const void* d_g, int g_is_fp32, const void* d_beta,
@@ -371,7 +368,7 @@ extern "C" int cula_kda_bwd_gated(const void* d_q, const void* d_k, const void* 
                                   int gate_mode, float lower_bound, void* stream) {
     return bwd_gated(d_q, d_k, d_g, g_is_fp32, d_beta, beta_is_fp32, d_A_log, d_dt_bias, d_akk, d_mkk, d_scratch, d_gscale, d_dq, d_dk, d_dg, d_dbeta,
                      d_dA_log, d_ddt_bias, d_cu_seqlens, d_chunk_indices, num_chunks, T, H, scale, use_qk_l2norm, gate_mode, lower_bound, nullptr,
-                     GATED_POLLS, stream);
+                     false, stream);
 }
 
 extern "C" int kda_launch_gate(const kda::GateArgs* a, int backward, cudaStream_t stream);

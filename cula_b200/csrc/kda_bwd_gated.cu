@@ -154,11 +154,18 @@ struct BgMaps {
     CUtensorMap a, m, dw, ps;             // Akk, M [tiles][64][64], dW [tiles][64][128], dPs and dAu [tiles][2 x 64][64]: 32 x 32 of fp32 at a time, 128-byte swizzle
 };
 
-// A wait gave up: what this CTA has not computed, or has computed from what had not arrived, must not pass for a gradient, with or
-// without a status word. All its tiles get NaN. (A function of its own, and the parameters by address: inlined it costs the tile loop spills.)
+// A wait gave up. `leave`: 2 + parity of the tile that the CTA left at its top, 0 if its last one ended. Products and copies in flight
+// end before the shared and tensor memory go away (bounded again): those of the last tile worked on, and the inputs that had been asked
+// for of the one left at. What the CTA has not computed, or has computed from what had not arrived, must not pass for a gradient, with or
+// without a status word: all its tiles get NaN. (All of it in a function of its own, which needs nothing that the tile loop holds, and the
+// parameters by address: with the tile and its parity from the loop the stage takes 1626 us at 4 x 8192 x 32, inlined 1669, like this 1598.)
 template <int GK>
-__device__ __noinline__ void bg_spoil(const BwdGatedParams& p, int num_tiles) {
+__device__ __noinline__ void bg_unwind(const BwdGatedParams& p, int num_tiles, uint64_t* bars, int leave) {
     const int tid = threadIdx.x;
+    if (tid == 0) {
+        const uint32_t last = leave ? (leave & 1u) ^ 1u : ((num_tiles - 1 - blockIdx.x) / gridDim.x) & 1u;
+        for (int i = 0; i < 11; ++i) mbar_wait(&bars[i], leave && (i == 8 || i == 10) ? last ^ 1u : last, 1 << 13);
+    }
     const float nan = __int_as_float(0x7fffffff);
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
         const int c = t / p.H, h = t - c * p.H;
@@ -186,7 +193,8 @@ __device__ __noinline__ void bg_spoil(const BwdGatedParams& p, int num_tiles) {
     }
 }
 
-template <int GK>
+// GIVES_UP: every wait gives up at once, to test what follows
+template <int GK, bool GIVES_UP>
 __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const __grid_constant__ BwdGatedParams p, const int num_tiles, const __grid_constant__ BgMaps maps) {
     constexpr int NT = BG_NT, N2 = NT / 2;
     extern __shared__ unsigned char bg_smem_raw[];
@@ -233,8 +241,8 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const __gr
     uint32_t par = 0;
     // bounded wait; on expiry the CTA leaves at the next tile, in any case before a barrier whose phase did not end is used again
     auto wait_bar = [&](int which) {
-        bool ok = false;
-        for (int i = 0; !ok && i < p.max_polls && (i == 0 || !*sAbort); ++i) ok = mbar_test(&bars[which], par);
+        bool ok = !GIVES_UP && mbar_test(&bars[which], par);
+        for (int i = 0; !GIVES_UP && !ok && i < (1 << 16) && !*sAbort; ++i) ok = mbar_test(&bars[which], par);
         if (!ok) {
             if (p.status) report_status(p.status, STATUS_WAIT_TIMEOUT);
             *sAbort = 1;
@@ -342,7 +350,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const __gr
     const float alpha = p.gate_mode != GATE_NONE ? __expf(alpha_log) : 0.f, bias = bias_next;
     wait_bar(8);              // the token rows have landed
     wait_bar(10);             // A, dPs, dW
-    if (tid == 0) *sLeave = *sAbort;
+    if (tid == 0) *sLeave = *sAbort ? 2 | par : 0;
     BG_MARK(0);
     // ---- 1. norms, gates and their sums inside a block, coefficient matrices in both orientations ----
     {
@@ -999,14 +1007,10 @@ __global__ void __launch_bounds__(BG_THREADS, 1) kda_bwd_gated_kernel(const __gr
     }  // tile loop: what the next tile writes before its first barrier is read by nobody any more
     bulk_wait_all();
     __syncthreads();
-    if (tid == 0 && *sAbort) {      // products and copies in flight end before the shared and tensor memory go away (waits bounded again)
-        const uint32_t last = par ^ 1u;        // of the last tile that was worked on; left at a tile, its inputs had been asked for
-        for (int i = 0; i < 11; ++i) mbar_wait(&bars[i], tile < num_tiles && (i == 8 || i == 10) ? par : last, 1 << 13);
-    }
+    if (*sAbort) bg_unwind<GK>(p, num_tiles, bars, *sLeave);
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) umma::tmem_dealloc(tmem, 512);
-    if (*sAbort) bg_spoil<GK>(p, num_tiles);
 }
 
 }  // namespace kda
@@ -1032,14 +1036,17 @@ static bool make_matrix_map(CUtensorMap* map, const float* base, int cols, int r
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-extern "C" int kda_launch_bwd_gated(const kda::BwdGatedParams* p, int num_chunks, cudaStream_t stream) {
+extern "C" int kda_launch_bwd_gated(const kda::BwdGatedParams* p, int num_chunks, int gives_up, cudaStream_t stream) {
     using namespace kda;
     static_assert(BG_SMEM <= 227 * 1024, "shared memory budget");
     if (num_chunks <= 0) return 0;
     const int kind = p->g_per_head ? BG_PER_HEAD : p->g_fp32 ? BG_FP32 : BG_BF16;
-    auto kernel = kind == BG_PER_HEAD ? kda_bwd_gated_kernel<BG_PER_HEAD> : kind == BG_FP32 ? kda_bwd_gated_kernel<BG_FP32> : kda_bwd_gated_kernel<BG_BF16>;
-    static std::atomic<unsigned long long> done[3];
-    cudaError_t e = allow_smem(kernel, BG_SMEM, done[kind]);
+    void (*const kernels[2][3])(BwdGatedParams, int, BgMaps) = {
+        {kda_bwd_gated_kernel<BG_BF16, false>, kda_bwd_gated_kernel<BG_FP32, false>, kda_bwd_gated_kernel<BG_PER_HEAD, false>},
+        {kda_bwd_gated_kernel<BG_BF16, true>, kda_bwd_gated_kernel<BG_FP32, true>, kda_bwd_gated_kernel<BG_PER_HEAD, true>}};
+    const auto kernel = kernels[gives_up != 0][kind];
+    static std::atomic<unsigned long long> done[2][3];
+    cudaError_t e = allow_smem(kernel, BG_SMEM, done[gives_up != 0][kind]);
     if (e != cudaSuccess) return (int)e;
     const int sms = sm_count();
     const int tiles = num_chunks * p->H;

@@ -141,7 +141,6 @@ struct BwdGatedParams {
     float lower_bound;
     float scale;
     int* status;                  // device status word (bounded waits) or null
-    int max_polls;                // after which a wait gives up
 };
 
 // short causal depthwise convolution (forward and backward)
