@@ -20,7 +20,7 @@
 // at cula/kda/chunk_bwd.py:541-555) and the dv half of chunk_kda_bwd_kernel_dAv (cula/kda/chunk_bwd.py:63-125).
 //
 // Range: every gradient-like operand (dO, dht, dS', dVn) is carried in units of a power-of-two scale s chosen
-// from max|dO|, max|dht| (kda_grad_scale_kernel), so fp16 MMA operands neither overflow nor go subnormal.
+// from max|dO|, max|dht| (kda_grad_amax_kernel), so fp16 MMA operands neither overflow nor go subnormal.
 #include "kda_common.cuh"
 #include "kda_params.h"
 #include "scan_common.cuh"

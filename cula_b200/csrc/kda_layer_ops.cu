@@ -4,7 +4,7 @@
 // They replace flash-linear-attention's ShortConvolution / causal_conv1d (fla/modules/convolution.py) and
 // FusedRMSNormGated / rms_norm_gated (fla/modules/fused_norm_gate.py:35-120, 846-869), which the layer that calls the
 // reference's chunk_kda uses (fla/layers/kda.py:147-165, 191, 306). Each element is read and written once (the convolution
-// re-reads a halo of at most 6 tokens per 64-token chunk); the norm waits on memory, the convolution on its own instructions.
+// re-reads a halo of at most 3 tokens per chunk or half chunk, 6 per half in the backward pass); the norm waits on memory, the convolution on its own instructions.
 #include "kda_common.cuh"
 #include "kda_params.h"
 
@@ -35,7 +35,7 @@ __device__ __forceinline__ float2 sigmoid2(float2 x) {
 // Measured at 4096 tokens x 4096 channels, W = 4: forward 27.7 -> 17.8 us (67 MB: 3.8 TB/s), backward 88 -> 36 -> 25 us (101 MB: 4 TB/s;
 // the last step: four channels per lane instead of two, no checks inside a unit), 8192 x 512: 24 -> 6 us. Backward in quarters of a
 // chunk: 32 us; five CTAs per SM by a register limit spill (70 us).
-// What bounds the backward: its instructions (72 per token and warp for two channels, now about 90 for four) and the fixed latencies
+// What bounds the backward: its instructions (72 per token and warp for two channels, now 110 for four, or 55) and the fixed latencies
 // between them at four warps per scheduler, a fifth of the time memory.
 // ------------------------------------------------------------------------------------------------------------------
 constexpr int CONV_WARPS = LO_THREADS / 32;
@@ -393,14 +393,13 @@ extern "C" int kda_launch_short_conv(const kda::ConvArgs* a, int num_chunks, int
     // Backward: two pairs of channels per lane halve the instructions that do not depend on the number of channels and double the work
     // between dependent ones (rows are 16-byte pieces). Forward: one pair (two: 17.5 -> 19.5 us at 4096 x 4096), and half chunks where
     // whole ones would leave fewer than 16 warps per SM (8192 x 512: 11.5 -> 8.5 us).
-    const bool wide = backward;
-    const int groups = (a->D + (wide ? 127 : 63)) / (wide ? 128 : 64);
-    const bool halves = wide || (long long)num_chunks * groups < 16LL * sm_count();
+    const int groups = (a->D + (backward ? 127 : 63)) / (backward ? 128 : 64);
+    const bool halves = backward || (long long)num_chunks * groups < 16LL * sm_count();
     const long long units = num_chunks * (halves ? 2LL : 1LL), blocks = groups * ((units + CONV_WARPS - 1) / CONV_WARPS);
     const dim3 grid((unsigned)(blocks < 0xffffffffLL ? blocks : 0xffffffffLL));      // (the launch refuses what is too many)
     void (*kernel)(const ConvArgs, const int) = nullptr;
 #define KDA_CONV_KERNEL(W)                                                                                          \
-    kernel = wide ? kda_short_conv_kernel<W, true, 2, 32> : halves ? kda_short_conv_kernel<W, false, 1, 32> : kda_short_conv_kernel<W, false, 1, 64>
+    kernel = backward ? kda_short_conv_kernel<W, true, 2, 32> : halves ? kda_short_conv_kernel<W, false, 1, 32> : kda_short_conv_kernel<W, false, 1, 64>
     switch (a->W) {
         case 1: KDA_CONV_KERNEL(1); break;
         case 2: KDA_CONV_KERNEL(2); break;

@@ -21,7 +21,7 @@ from .build import TIMERS_LIB, build
 FWD_PHASES = ["gate activation", "barrier (block edges, norms)", "in-warp cumulative sum", "per-channel tables", "-",
               "operand generation", "wait for the Gram MMAs", "-", "triangular inverse, Y staging, Akk pack", "W/U MMA issue",
               "W/U MMA wait", "W/U epilogue", "loads issued, diagonal blocks", "Gram epilogue", "L2 norms",
-              "top of the tile (q/k loads issued)"]
+              "top of the tile"]
 DENSE_PHASES = ["half 0: operands widened into smem", "-",
                 "half 0: store read-out + wait for the states (TMA)", "half 0: MMA issue", "half 0: next operands requested",
                 "half 0: wait for the MMAs",
@@ -29,7 +29,7 @@ DENSE_PHASES = ["half 0: operands widened into smem", "-",
                 "half 1: MMA issue", "half 1: next tile's operands requested", "half 1: wait for the MMAs", "dQg, dW staged, stores issued",
                 "dKg, dPs, dAu staged, dv stored", "store read-out + end-of-tile barrier"]
 BWD_PHASES = ["inputs landed", "norms, gates, coefficients", "anchors, X, dW^T, q e", "dA", "Zw, q side read, k f, k e", "T1", "P part read",
-              "dL, cR", "R part read", "k side read", "dk, dG, sums", "S13","S11","S12","B7","top issue"]
+              "dL, cR", "R part read", "k side read", "dk, dG, sums", "norms, gate VJP, rows out"]
 
 
 def main():

@@ -123,8 +123,9 @@ int cula_kda_build_chunk_tables(const int* h_cu_seqlens, int N, int* h_chunk_ind
 
 /* ------------------------------------------------------------------------------------------------------------
  * Backward pass. The reference's backward is all Triton / flash-linear-attention kernels plus a recompute of
- * its forward intermediates (cula/kda/chunk_bwd.py:432-604); here it is four launches after re-running the two
- * forward launches with d_akk, d_mkk, d_h32_out and d_vnew_out set.
+ * its forward intermediates (cula/kda/chunk_bwd.py:432-604); here it is four calls (gradient scale, reverse scan, dense
+ * and gated stage) after re-running the two of the forward with d_akk, d_mkk, d_h32_out and d_vnew_out set. The calls that
+ * do two of these side by side: cula_kda_bwd_scale_and_intra, cula_kda_bwd_both_scans.
  * All gradient-like intermediates are carried in units of a power-of-two scale s (d_gscale = {s, 1/s}).
  * ------------------------------------------------------------------------------------------------------------ */
 
