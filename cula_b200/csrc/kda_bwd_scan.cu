@@ -479,5 +479,6 @@ extern "C" int kda_launch_bwd_scan(const kda::BwdScanParams* p, cudaStream_t str
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p->beside_forward ? 1 : 0;
-    return (int)launched(cudaLaunchKernelEx(&cfg, kda_bwd_scan_kernel, *p, map, map_do));
+    const cudaError_t launch = launched(cudaLaunchKernelEx(&cfg, kda_bwd_scan_kernel, *p, map, map_do));
+    return (int)(launch != cudaSuccess ? launch : cudaGetLastError());
 }

@@ -259,8 +259,8 @@ inline int sm_count() {
 // The result of a launch. One that was refused also leaves its error for whoever asks next (torch after its own next kernel): it is
 // taken along here, since the caller gets it as the return value.
 inline cudaError_t launched(cudaError_t e) {
-    const cudaError_t left = cudaGetLastError();
-    return e != cudaSuccess ? e : left;
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 // A launch that may be scheduled while the kernel before it in the stream drains; the kernel calls pdl_launch_dependents() and, before it
 // touches memory, pdl_wait().

@@ -1071,5 +1071,6 @@ extern "C" int kda_launch_fwd_intra(const kda::IntraParams* p, int num_chunks, c
     IntraMaps maps;
     if (!make_half_rows_map(&maps.q, p->q, p->H) || !make_half_rows_map(&maps.k, p->k, p->H) || !make_half_rows_map(&maps.v, p->v, p->H))
         return (int)cudaErrorInvalidValue;
-    return (int)launched(cudaLaunchKernelEx(&cfg, kernel, q, maps));
+    const cudaError_t launch = launched(cudaLaunchKernelEx(&cfg, kernel, q, maps));
+    return (int)(launch != cudaSuccess ? launch : cudaGetLastError());
 }

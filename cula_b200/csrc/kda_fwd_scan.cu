@@ -435,7 +435,8 @@ int launch_scan(const kda::ScanParams* p, int groups, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return (int)launched(cudaLaunchKernelEx(&cfg, kda_fwd_scan_kernel, *p, map, map_o));
+    const cudaError_t launch = launched(cudaLaunchKernelEx(&cfg, kda_fwd_scan_kernel, *p, map, map_o));
+    return (int)(launch != cudaSuccess ? launch : cudaGetLastError());
 }
 }  // namespace
 

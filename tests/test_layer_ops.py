@@ -258,3 +258,27 @@ def test_layer_operators_are_capturable_in_a_cuda_graph():
             graph.replay()
         torch.cuda.synchronize()
         assert same(other[2](), replayed), seed
+
+
+@pytest.mark.gpu
+def test_a_refused_launch_leaves_no_error_behind():
+    """The legacy stream takes no launch while a blocking stream is being captured: the call returns that error, and whoever asks the
+    runtime next (torch, after its own next kernel) does not find it a second time. Buffer and sizes are real: were it not refused, it
+    would run."""
+    import ctypes
+
+    from cula_b200 import _native
+    runtime, lib = ctypes.CDLL("libcudart.so.12"), _native.lib()          # the runtime that the library and torch share
+    buf = torch.full((1024,), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    stream, graph = ctypes.c_void_p(), ctypes.c_void_p()
+    assert runtime.cudaStreamCreate(ctypes.byref(stream)) == 0
+    assert runtime.cudaStreamBeginCapture(stream, 2) == 0                  # (relaxed)
+    rc = lib.cula_kda_clear(buf.data_ptr(), 4096, None)
+    left = runtime.cudaPeekAtLastError()
+    runtime.cudaStreamEndCapture(stream, ctypes.byref(graph))              # the refusal has ended the capture as well
+    runtime.cudaGetLastError()
+    assert runtime.cudaStreamDestroy(stream) == 0
+    assert rc > 0 and left == 0
+    assert bool((buf == 7).all())
+    assert lib.cula_kda_clear(buf.data_ptr(), 4096, torch.cuda.current_stream().cuda_stream) == 0 and not buf.any()
