@@ -5,7 +5,7 @@ checks, allocation, autograd, launches; C++ on libtorch) into the Python extensi
 
 The library is built in-tree and loaded with ctypes (cula_b200/_native.py); it has a plain C ABI
 (include/cula_kda.h) and links only against the CUDA runtime (the one driver function it needs, the tensor-map encoder
-of the dense backward stage, is looked up through the runtime's driver entry point at first use).
+of the stages that move data by TMA, is looked up through the runtime's driver entry point at first use).
 """
 from __future__ import annotations
 

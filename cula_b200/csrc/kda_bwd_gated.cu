@@ -34,7 +34,7 @@
 //
 // What bounds it: latency. 42.7 k warp instructions a tile take 37 % of the issue slots of 28 k cycles, tensor pipes 9 %, and one CTA of
 // 16 warps (all registers, all of shared and tensor memory) walks through eight CTA barriers a tile. Measured at 4 x 8192 x 32 heads:
-// 2.38 -> 1.61 ms (5.2 GB in and out, 0.8 ms at the copy peak) against mma.sync products in transposed fragments with 68.6 k warp
+// 2.38 -> 1.60 ms (5.2 GB in and out, 0.8 ms at the copy peak) against mma.sync products in transposed fragments with 68.6 k warp
 // instructions a tile, 2 x 2048 x 32: 317 -> 218 us, one tile 28.7 -> 22.5 us.
 #include "kda_common.cuh"
 #include "kda_params.h"

@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(INTRA_THREADS, 2) kda_fwd_intra_kernel(const I
     {
         const int4 nf = sInfo[par ^ 1];
         if (nf.y > 0) {
-            // (the order that spills least: a gate per head 609 -> 596 us at 4 x 8192 x 32 with the rows first, the others with them last)
+            // (the order that spills least: a gate per head 609 -> 598 us at 4 x 8192 x 32 with the rows first, the others with them last)
             if constexpr (GK == GK_PER_HEAD) prefetch_rows(nf);
             fetch_g(nf);
             load_scalars(nf);
